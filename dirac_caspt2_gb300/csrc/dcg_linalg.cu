@@ -90,7 +90,10 @@ __device__ double block_sum(double v, double *sh) {
 // A GB300 SM retires about two FP64 FMAs per clock, so the useful fraction of a tile is the
 // fraction of the GPU's FP64 rate a skinny product gets: the autotuner picks the tile.
 constexpr int kZgTiles = 3;
-constexpr int kZgTyn[kZgTiles] = {16, 8, 32};
+// Rows and columns of all tile shapes: these three, then the fine-grained ones (zgemm_fine_kernel).
+constexpr int kZgShapes = 7;
+constexpr int kZgBm[kZgShapes] = {64, 32, 128, 32, 16, 8, 8};
+constexpr int kZgBn[kZgShapes] = {64, 128, 32, 32, 16, 8, 4};
 
 template <int OPA, int OPB, int TYN>
 __global__ void __launch_bounds__(256) zgemm_kernel(int m, int n, int k, cplx alpha, const cplx *__restrict__ A,
@@ -177,6 +180,133 @@ __global__ void __launch_bounds__(256) zgemm_kernel(int m, int n, int k, cplx al
             if (use_beta) r = cadd(r, cmul(beta, C[o]));
             C[o] = r;
         }
+    }
+}
+
+// ---- fine-grained products.  A GB300 SM retires about two FP64 FMAs per clock, so a warp's FMA
+// instruction holds its quarter of the SM for 64 clocks and one complex multiply-add of 32
+// outputs for 256: shared-memory and L2 bandwidth are never the limit, padding is.  Here a warp
+// owns 8 x 4 outputs (one per lane, QN of such pieces along n), pieces outside the matrix are
+// skipped, and the chunks of K end at k, so a 14 x 14 x 14 product costs 16 x 16 x 14 instead of
+// 64 x 64 x 16.  A block is 8 warps as RM x RN pieces x KG groups of K: small outputs use
+// all four quarters of an SM on one piece by splitting K between warps (summed in a fixed
+// order through shared memory).  The next chunk is loaded into registers while the current
+// one is multiplied.  Pieces go to warps rotated by the block index, so a ragged edge does
+// not idle the same quarter of every SM.
+// Measured (whole solves, 64 x 64 tiles and up only -> with these): 4/4/12 FP64 8.66 -> 3.88 ms
+// (one 64-row product alone took 274 us), 12/8/120 real FP64 37.1 -> 25.7 ms, 14/10/230 split
+// 65.4 -> 50.8 ms, 20/12/300 split 119.6 -> 114.8 ms.
+template <int RM, int RN, int KG, int QN>
+struct ZfShape {
+    static constexpr int BM = 8 * RM, BN = 4 * RN * QN, BK = KG > 1 ? 32 : 16;
+    static constexpr int NA = (BM * BK + 255) / 256, NB = (BN * BK + 255) / 256;
+    static_assert(RM * RN * KG == 8, "eight warps");
+};
+
+// element (i, kk) of op(X) stored with leading dimension ld, (row, col) = (i, kk) for N and R
+__device__ __forceinline__ cplx zf_load(const cplx *__restrict__ X, int64_t ld, int i, int kk, int op, bool trans) {
+    cplx v = trans ? X[kk + (int64_t)i * ld] : X[i + (int64_t)kk * ld];
+    if (op == OP_C || op == OP_R) v.y = -v.y;
+    return v;
+}
+
+template <int RM, int RN, int KG, int QN>
+__global__ void __launch_bounds__(256) zgemm_fine_kernel(int m, int n, int k, int opa, int opb, cplx alpha,
+                                                         const cplx *__restrict__ A, int64_t lda, int64_t sa,
+                                                         const cplx *__restrict__ B, int64_t ldb, int64_t sb, cplx beta,
+                                                         cplx *C, int64_t ldc, int64_t sc, int zoff, int upper) {
+    using S = ZfShape<RM, RN, KG, QN>;
+    constexpr int BM = S::BM, BN = S::BN, BK = S::BK, NA = S::NA, NB = S::NB;
+    __shared__ cplx As[BK][BM + 1];
+    __shared__ cplx Bs[BK][BN + 1];
+    __shared__ cplx red[KG > 1 ? 8 * 32 * QN : 1];
+    const int64_t bz = (int64_t)blockIdx.z + zoff;
+    A += bz * sa;
+    B += bz * sb;
+    C += bz * sc;
+    const int m0 = blockIdx.x * BM, n0 = blockIdx.y * BN;
+    if (upper && m0 >= n0 + BN) return;   // tile strictly below the diagonal (Hermitian product, upper half)
+    const int tid = threadIdx.x, lane = tid & 31;
+    const int w = ((tid >> 5) + (KG > 1 ? 0 : (int)(blockIdx.x + blockIdx.y + blockIdx.z))) & 7;
+    const int kg = w % KG, sub = w / KG, rm = sub % RM, rn = sub / RM;
+    const int li = 8 * rm + (lane & 7), lj = 4 * rn + (lane >> 3);   // this lane's row and first column in the tile
+    const bool ta = opa == OP_T || opa == OP_C, tb = opb == OP_T || opb == OP_C;   // A stored k x m; B stored n x k
+    const bool rows = m0 + 8 * rm < m;
+    int nq = 0;   // pieces of this warp inside the matrix (uniform over the warp)
+#pragma unroll
+    for (int q = 0; q < QN; q++)
+        if (rows && n0 + 4 * (rn + RN * q) < n) nq = q + 1;
+    cplx acc[QN];
+#pragma unroll
+    for (int q = 0; q < QN; q++) acc[q] = mk(0.0, 0.0);
+    cplx pa[NA], pb[NB];
+    // element e of a chunk: A by rows fastest (N, R) or k fastest (T, C), B the other way round
+    auto fetch = [&](int k0) {
+#pragma unroll
+        for (int u = 0; u < NA; u++) {
+            const int e = tid + 256 * u;
+            const int i = ta ? e / BK : e % BM, kk = ta ? e % BK : e / BM;
+            pa[u] = (e < BM * BK && m0 + i < m && k0 + kk < k) ? zf_load(A, lda, m0 + i, k0 + kk, opa, ta) : mk(0.0, 0.0);
+        }
+#pragma unroll
+        for (int u = 0; u < NB; u++) {
+            const int e = tid + 256 * u;
+            const int j = tb ? e % BN : e / BK, kk = tb ? e / BN : e % BK;
+            pb[u] = (e < BN * BK && n0 + j < n && k0 + kk < k) ? zf_load(B, ldb, n0 + j, k0 + kk, opb, !tb) : mk(0.0, 0.0);
+        }
+    };
+    fetch(0);
+    for (int k0 = 0; k0 < k; k0 += BK) {
+#pragma unroll
+        for (int u = 0; u < NA; u++) {
+            const int e = tid + 256 * u;
+            if (e < BM * BK) As[ta ? e % BK : e / BM][ta ? e / BK : e % BM] = pa[u];
+        }
+#pragma unroll
+        for (int u = 0; u < NB; u++) {
+            const int e = tid + 256 * u;
+            if (e < BN * BK) Bs[tb ? e / BN : e % BK][tb ? e % BN : e / BK] = pb[u];
+        }
+        __syncthreads();
+        if (k0 + BK < k) fetch(k0 + BK);
+        const int kend = min(BK, k - k0);
+        if (nq == QN) {
+#pragma unroll 4
+            for (int kk = kg; kk < kend; kk += KG) {
+                const cplx a = As[kk][li];
+#pragma unroll
+                for (int q = 0; q < QN; q++) cfma(acc[q], a, Bs[kk][lj + 4 * RN * q]);
+            }
+        } else if (nq > 0) {
+            for (int kk = kg; kk < kend; kk += KG) {
+                const cplx a = As[kk][li];
+#pragma unroll
+                for (int q = 0; q < QN; q++)
+                    if (q < nq) cfma(acc[q], a, Bs[kk][lj + 4 * RN * q]);
+            }
+        }
+        __syncthreads();
+    }
+    if (KG > 1) {   // the K groups' sums, added in group order by group 0
+#pragma unroll
+        for (int q = 0; q < QN; q++) red[(w * QN + q) * 32 + lane] = acc[q];
+        __syncthreads();
+        if (kg != 0) return;
+        for (int g = 1; g < KG; g++)
+#pragma unroll
+            for (int q = 0; q < QN; q++) acc[q] = cadd(acc[q], red[((w + g) * QN + q) * 32 + lane]);
+    }
+    const int gi = m0 + li;
+    if (gi >= m) return;
+    const bool use_beta = (beta.x != 0.0 || beta.y != 0.0);
+#pragma unroll
+    for (int q = 0; q < QN; q++) {
+        const int gj = n0 + lj + 4 * RN * q;
+        if (gj >= n) continue;
+        cplx r = cmul(alpha, acc[q]);
+        const int64_t o = gi + (int64_t)gj * ldc;
+        if (use_beta) r = cadd(r, cmul(beta, C[o]));
+        C[o] = r;
     }
 }
 
@@ -271,6 +401,9 @@ static bool zgemm_small(Context &c, Op opa, Op opb, int m, int n, int k, cplx al
                         int64_t sa, const cplx *B, int64_t ldb, int64_t sb, cplx beta, cplx *C, int64_t ldc, int64_t sc,
                         int batch) {
     if (k < 1 || k > SMALL_D) return false;
+    // a thread forms SMALL_G outputs: below about one warp per quarter SM the fine-grained
+    // kernel, one output per thread, spreads the product further
+    if ((double)m * n * batch < 32.0 * SMALL_G * 4.0 * std::max(1, c.num_sms)) return false;
     if (opa == OP_N && (opb == OP_N || opb == OP_R) && n <= SMALL_D && m >= 64) {
         const int gy = (n + SMALL_G - 1) / SMALL_G;
         const int bx = 256 / gy;   // gy <= 4, bx >= 64
@@ -306,10 +439,31 @@ template <int OPA, int OPB>
 static void zgemm_launch(Context &c, int m, int n, int k, cplx alpha, const cplx *A, int64_t lda, int64_t sa,
                          const cplx *B, int64_t ldb, int64_t sb, cplx beta, cplx *C, int64_t ldc, int64_t sc,
                          int batch, int upper, int tile) {
-    const int bm = 4 * kZgTyn[tile], bn = 1024 / kZgTyn[tile];
+    const int bm = kZgBm[tile], bn = kZgBn[tile];
+    // the fine-grained kernel reads its operands by (row, k) and (k, column); the grid's y extent
+    // bounds the columns one launch covers
+    const int ymax = 65535;
+    if (!upper && grid1d(n, bn) > (unsigned)ymax) {
+        const int64_t nc = (int64_t)ymax * bn;
+        for (int64_t j0 = 0; j0 < n; j0 += nc) {
+            const cplx *Bj = B + (OPB == OP_N || OPB == OP_R ? j0 * ldb : j0);
+            zgemm_launch<OPA, OPB>(c, m, (int)std::min<int64_t>(nc, n - j0), k, alpha, A, lda, sa, Bj, ldb, sb, beta,
+                                   C + j0 * ldc, ldc, sc, batch, upper, tile);
+        }
+        return;
+    }
     for (int z0 = 0; z0 < batch; z0 += 65535) {
         int nz = batch - z0 < 65535 ? batch - z0 : 65535;
         dim3 grid(grid1d(m, bm), grid1d(n, bn), nz);
+#define DCG_ZF(t, rm, rn, kg, qn)                                                                                  \
+    if (tile == t) {                                                                                               \
+        zgemm_fine_kernel<rm, rn, kg, qn><<<grid, 256, 0, c.stream>>>(m, n, k, OPA, OPB, alpha, A, lda, sa, B, ldb, \
+                                                                      sb, beta, C, ldc, sc, z0, upper);            \
+        DCG_LAUNCHED(c);                                                                                           \
+        continue;                                                                                                  \
+    }
+        DCG_ZF(3, 4, 2, 1, 4) DCG_ZF(4, 2, 4, 1, 1) DCG_ZF(5, 1, 2, 4, 1) DCG_ZF(6, 1, 1, 8, 1)
+#undef DCG_ZF
         if (tile == 1)
             zgemm_kernel<OPA, OPB, 8><<<grid, 256, 0, c.stream>>>(m, n, k, alpha, A, lda, sa, B, ldb, sb, beta, C, ldc,
                                                                   sc, z0, upper);
@@ -325,7 +479,7 @@ static void zgemm_launch(Context &c, int m, int n, int k, cplx alpha, const cplx
 
 // Output tiles of a tile shape (for a Hermitian product's upper half, those touching it).
 static int64_t zg_tiles(int m, int n, int tile, int upper) {
-    const int bm = 4 * kZgTyn[tile], bn = 1024 / kZgTyn[tile];
+    const int bm = kZgBm[tile], bn = kZgBn[tile];
     const int64_t tm = (m + bm - 1) / bm, tn = (n + bn - 1) / bn;
     if (!upper) return tm * tn;
     int64_t t = 0;
@@ -378,33 +532,55 @@ static void zgemm_splitk_run(Context &c, int m, int n, int k, int nsplit, cplx a
     DCG_LAUNCHED(c);
 }
 
-// The tile shape and K split of one FP64 product.  A GEMM whose output tiles do not fill the
-// GPU is split along K into equal chunks of at least 64, computed as one batched GEMM into
-// partial products and reduced in a fixed order.  The autotuner times, per shape, every tile
-// with no split, with the occupancy heuristic min(2 SMs / tiles, k / 64) and with powers of
-// two up to k / 64 (batched products: the tiles alone); candidate 0 (64 x 64 tiles, the
-// heuristic split) is used while tuning is off and for calls that accumulate into C (beta
-// != 0, which the timed trial runs would disturb).
+// The tile shape and K split of one FP64 product.  zg_cost estimates a plan's time: the FP64
+// operations of the fullest SM (padding included; two FMAs per clock and SM) plus the latency of
+// a chunk of K per wave and of a launch.  A product whose tiles do not fill the GPU may be split
+// along K into equal chunks of at least 32, computed as one batched GEMM into partial products
+// and reduced in a fixed order.  The cheapest plan by the estimate is candidate 0, used for
+// small products, while tuning is off and for calls that accumulate into C (beta != 0, which
+// the timed trial runs would disturb); the autotuner times the plans within 1.3 of it.
 constexpr double kTuneMinFp64Flops = 1.0e9;
+constexpr int kZgMinChunk = 32;
 
 struct ZgPlan {
     int tile, nsplit;
+    double cost;   // estimated clocks
 };
+
+// Clocks of a plan on `sms` SMs.
+static double zg_cost(int sms, int m, int n, int k, int upper, int batch, int tile, int nsplit) {
+    const int bm = kZgBm[tile], bn = kZgBn[tile];
+    const int kc = (k + nsplit - 1) / nsplit;
+    const bool fine = tile >= kZgTiles;
+    // multiply-adds of one tile: whole tiles and chunks of 16 for the coarse kernels, pieces of
+    // 8 x 4 for the fine ones (their K groups share a tile, so a tile takes the same FP64 time)
+    const double tm = (m + bm - 1) / bm, tn = (n + bn - 1) / bn;
+    const double fm = fine ? 8.0 * ((m + 7) / 8) / (bm * tm) : 1.0, fn = fine ? 4.0 * ((n + 3) / 4) / (bn * tn) : 1.0;
+    const double kp = fine ? kc : 16.0 * ((kc + 15) / 16);
+    const double work = bm * bn * fm * fn * kp * 4.0 / 2.0;   // clocks of one tile alone on an SM
+    const double blocks = (double)zg_tiles(m, n, tile, upper) * nsplit * batch;
+    const double waves = std::ceil(blocks / sms);
+    // a tile alone on its SM waits for its loads once per chunk (the fine kernels prefetch)
+    const double bk = tile >= 5 ? 32.0 : 16.0;
+    const double lat = (waves <= 1.5 ? (fine ? 500.0 : 1500.0) : 100.0) * std::ceil(kc / bk);
+    double t = waves * work * (fine ? 1.04 : 1.0) + lat + 4000.0;
+    if (nsplit > 1) t += 6000.0 + (double)m * n * nsplit * 2.0 * 32.0 / (sms * 64.0);   // the reduction
+    return t;
+}
 
 static std::vector<ZgPlan> zg_candidates(Context &c, int m, int n, int k, int upper, int batch) {
     const int sms = std::max(1, c.num_sms);
-    std::vector<ZgPlan> out;
-    for (int t = 0; t < kZgTiles; t++) {
+    std::vector<ZgPlan> all, out;
+    for (int t = 0; t < kZgShapes; t++) {
         const int64_t tiles = zg_tiles(m, n, t, upper);
-        std::vector<int> ns{1};
-        if (batch == 1 && tiles < sms && k >= 128) {
-            const int heur = (int)std::min<int64_t>((2 * sms + tiles - 1) / tiles, k / 64);
-            if (heur >= 2) ns.insert(ns.begin(), heur);
-            for (int p = 2; p <= k / 64 && p <= 64; p *= 2)
-                if (std::find(ns.begin(), ns.end(), p) == ns.end()) ns.push_back(p);
-        }
-        for (int x : ns) out.push_back({t, x});
+        all.push_back({t, 1, zg_cost(sms, m, n, k, upper, batch, t, 1)});
+        if (batch != 1 || tiles >= 2 * sms) continue;
+        for (int p = 2; p <= k / kZgMinChunk && p <= 64; p *= 2)
+            all.push_back({t, p, zg_cost(sms, m, n, k, upper, batch, t, p)});
     }
+    std::stable_sort(all.begin(), all.end(), [](const ZgPlan &x, const ZgPlan &y) { return x.cost < y.cost; });
+    for (const ZgPlan &p : all)
+        if (out.empty() || (p.cost <= 1.3 * all[0].cost && out.size() < 8)) out.push_back(p);
     return out;
 }
 

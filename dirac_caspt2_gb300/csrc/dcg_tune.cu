@@ -45,7 +45,7 @@ void load_locked() {
     TuneEntry e;
     while (fscanf(fp, "%d %d %d %d %d %d %d %d %f %f", &k.kind, &k.ops, &k.m, &k.n, &k.k, &k.flags, &e.choice,
                   &e.ncand, &e.best_ms, &e.heuristic_ms) == 10)
-        if (e.choice >= 0 && e.choice < e.ncand) g_table.emplace(k, e);
+        if (e.choice >= 0 && e.choice < e.ncand) g_table[k] = e;   // the latest line of a key counts
     fclose(fp);
 }
 
@@ -66,7 +66,8 @@ int autotune_run(Context &c, const TuneKey &key, int ncand, bool trial_ok, void 
         std::lock_guard<std::mutex> lk(g_mu);
         load_locked();
         auto it = g_table.find(key);
-        if (it != g_table.end()) return it->second.choice < ncand ? it->second.choice : 0;
+        // an entry of another candidate list (a file written by another build) is not used
+        if (it != g_table.end() && it->second.ncand == ncand) return it->second.choice;
         if (mode_locked() == 0 || ncand < 2 || !trial_ok || !c.tune_trials) return 0;
     }
     // untimed pass: every candidate once (workspace growth, first-launch costs)
@@ -91,9 +92,13 @@ int autotune_run(Context &c, const TuneKey &key, int ncand, bool trial_ok, void 
     for (int q = 1; q < ncand; q++)
         if (best[q] < best[pick]) pick = q;
     std::lock_guard<std::mutex> lk(g_mu);
-    auto ins = g_table.emplace(key, TuneEntry{pick, ncand, best[pick], best[0]});
-    if (ins.second) save_locked(key, ins.first->second);
-    return ins.first->second.choice;   // a concurrent tuner of the same key may have won
+    const TuneEntry mine{pick, ncand, best[pick], best[0]};
+    auto ins = g_table.emplace(key, mine);
+    if (!ins.second && ins.first->second.ncand == ncand)
+        return ins.first->second.choice;   // a concurrent tuner of the same key won
+    ins.first->second = mine;
+    save_locked(key, mine);
+    return pick;
 }
 
 }  // namespace dcg
