@@ -2154,6 +2154,7 @@ int dcg_trim(dcg_ctx *ctx) {
         c_.dev_state = nullptr;
         for (int s = 0; s < Context::kSlots; s++) {
             c_.eig_Q[s] = nullptr;
+            c_.eig_last[s] = 0;
             c_.eig_n[s] = 0;
             c_.eig_status[s] = nullptr;
         }

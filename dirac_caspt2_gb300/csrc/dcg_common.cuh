@@ -109,10 +109,12 @@ struct Context {
     double fam_ms = 0.0, fam_work = 0.0;
     // tcgen05 shared-memory descriptor strides of the split GEMM (leading, stride byte offset)
     int split_lbo = 128, split_sbo = 256;
-    // per eigensolver slot: tridiagonal eigenvectors of the last value stage (device, n x n),
-    // their dimension and the divide-and-conquer status word
+    // per eigensolver slot: tridiagonal eigenvectors of the last value stage (device, n x n) when
+    // they are complete, the half width of the last merge when its vectors are formed on request
+    // (0 otherwise), their dimension and the divide-and-conquer status word
     static constexpr int kSlots = 32;
     const double *eig_Q[kSlots] = {};
+    int eig_last[kSlots] = {};
     int eig_n[kSlots] = {};
     int *eig_status[kSlots] = {};
     int64_t fam_launches = 0;

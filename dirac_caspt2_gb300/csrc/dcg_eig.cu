@@ -916,20 +916,387 @@ struct DcBufs {
     double *tau, *lamK;       // root offset from its origin, root value
     double *zh;               // recomputed rank-one vector
     int *outc;                // output column of each node entry in the next level
+    int *top, *bot;           // undeflated entries whose column reaches the node's first / second half
+    int *k0, *flag, *half;    // prep scratch: entries past the z test, rotation flags, halves reached
     int *kcnt, *ndef, *nrot;  // per node: undeflated count (-1: pass-through), deflated, rotations
+    int *ntop, *nbot;         // per node: lengths of top and bot
     double *rho;              // per node
     int *status;              // nonzero: a merge met an inconsistent pole order
 };
 
-__global__ void dc_leaf_kernel(int n, const double *__restrict__ d, const double *__restrict__ e, double *lam,
-                               double *Q) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    double v = d[i];
-    if (i > 0) v -= fabs(e[i - 1]);
-    if (i < n - 1) v -= fabs(e[i]);
-    lam[i] = v;
-    Q[i + (int64_t)i * n] = 1.0;
+// 1/x by two Newton steps from the hardware's ~2^-22 approximation: four FP64 operations, where
+// a division is a longer chain on a unit that retires two per clock and SM.
+__device__ __forceinline__ double dc_rcp(double x) {
+    double r;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
+    r = fma(r, fma(-x, r, 1.0), r);
+    return fma(r, fma(-x, r, 1.0), r);
+}
+
+// Sums of four values over groups of G lanes; every lane of a group gets all four.  The first two
+// exchange steps halve the number of values a lane carries, so 32 lanes take six FP64 additions
+// instead of twenty (each holds a quarter SM for 64 clocks).
+template <int G>
+__device__ __forceinline__ void dc_sum4(double &v0, double &v1, double &v2, double &v3) {
+    const int lane = threadIdx.x & 31;
+    if (G == 4) {
+        // lane g of the group ends with value g
+        const bool h2 = lane & 2, h1 = lane & 1;
+        double a = h2 ? v2 : v0, b = h2 ? v3 : v1;
+        a += __shfl_xor_sync(0xffffffffu, h2 ? v0 : v2, 2);
+        b += __shfl_xor_sync(0xffffffffu, h2 ? v1 : v3, 2);
+        double x = h1 ? b : a;
+        x += __shfl_xor_sync(0xffffffffu, h1 ? a : b, 1);
+        v0 = __shfl_sync(0xffffffffu, x, 0, 4);
+        v1 = __shfl_sync(0xffffffffu, x, 1, 4);
+        v2 = __shfl_sync(0xffffffffu, x, 2, 4);
+        v3 = __shfl_sync(0xffffffffu, x, 3, 4);
+    } else {
+        const bool hi = lane & (G / 2), lo = lane & (G / 4);
+        double a = hi ? v2 : v0, b = hi ? v3 : v1;
+        a += __shfl_xor_sync(0xffffffffu, hi ? v0 : v2, G / 2);
+        b += __shfl_xor_sync(0xffffffffu, hi ? v1 : v3, G / 2);
+        double x = lo ? b : a;
+        x += __shfl_xor_sync(0xffffffffu, lo ? a : b, G / 4);
+#pragma unroll
+        for (int o = G / 8; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+        v0 = __shfl_sync(0xffffffffu, x, 0, G);
+        v1 = __shfl_sync(0xffffffffu, x, G / 4, G);
+        v2 = __shfl_sync(0xffffffffu, x, G / 2, G);
+        v3 = __shfl_sync(0xffffffffu, x, 3 * G / 4, G);
+    }
+}
+template <int G>
+__device__ __forceinline__ double dc_group_sum(double v) {
+#pragma unroll
+    for (int o = G / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+template <int G>
+__device__ __forceinline__ double dc_group_prod(double v) {
+#pragma unroll
+    for (int o = G / 2; o > 0; o >>= 1) v *= __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+
+// Secular root j of 1/rho + sum_i z_i^2 / (d_i - lambda) = 0 by a group of G lanes (all lanes of
+// the warp call, `act` false for groups without a root).  The root lies in (d_j, d_{j+1}) (the
+// last one in (d_{k-1}, d_{k-1} + rho |z|^2)) and is found as an offset tau from the nearer pole
+// d_o, so that d_i - lambda = (d_i - d_o) - tau keeps full accuracy.  The start solves the
+// equation with its two nearest poles and the other terms frozen at the middle of the
+// interval; each step fits c + s1/(dL - x) + s2/(dR - x) to the value and slope of the two
+// partial sums at tau and takes that model's root; steps leaving the bracket bisect.  One of dL,
+// dR is zero, and with s1, s2 > 0 the root between the poles is C/q for B > 0 and q/A
+// otherwise (A x^2 - B x + C = 0, q its larger-magnitude half sum), so a step takes one square
+// root and one division besides the pole sums.  All lanes of a group hold identical scalars.
+template <int G>
+__device__ void dc_secular_root(int k, int j, bool act, const double *dk, const double *zk, double rho, int &o_out,
+                                double &tau_out, double &lam_out, int *status) {
+    const int gl = threadIdx.x & (G - 1);
+    const int kk = act ? k : 0;
+    const double rhoinv = act ? 1.0 / rho : 1.0;
+    const bool last = j >= k - 1;
+    const double dl = act ? dk[j] : 0.0, dr = act && !last ? dk[j + 1] : 0.0;
+    if (act && !last && !(dr > dl)) {   // poles out of order: give up on this root
+        if (gl == 0) atomicExch(status, 1);
+        o_out = j;
+        tau_out = 0.0;
+        lam_out = dl;
+        act = false;
+    }
+    const double hg = last ? 0.0 : 0.5 * (dr - dl);
+    const double zj2 = act ? zk[j] * zk[j] : 0.0, zr2 = act && !last ? zk[j + 1] * zk[j + 1] : 0.0;
+    double x = 0.0;   // sum of the other terms at the middle of the interval, or |z|^2
+    for (int i = gl; i < kk; i += G) {
+        const double z2 = zk[i] * zk[i];
+        if (last) x += z2;
+        else if (i != j && i != j + 1) x += z2 * dc_rcp((dk[i] - dl) - hg);
+    }
+    x = dc_group_sum<G>(x);
+    int o = j;
+    double lo = 0.0, hi = 1.0, c0 = rhoinv + x;
+    if (!last) {
+        const double g = c0 + (zr2 - zj2) / (act ? hg : 1.0);
+        if (g > 0.0) {
+            hi = hg;
+        } else {
+            o = j + 1;
+            lo = -hg;
+            hi = 0.0;
+        }
+    } else {
+        hi = rho * x;
+        // the other terms at the upper end: z_j^2 / c0 is a lower bound of the root there
+        double y = 0.0;
+        for (int i = gl; i < kk; i += G)
+            if (i != j) y += zk[i] * zk[i] * dc_rcp((dk[i] - dl) - hi);
+        c0 = y;
+    }
+    {   // uniform shuffle for the groups of both kinds
+        const double y = dc_group_sum<G>(last ? c0 : 0.0);
+        if (last) c0 = rhoinv + y;
+    }
+    const double d_o = act ? dk[o] : 0.0;
+    const double dL = dl - d_o, dR = last ? 0.0 : dr - d_o;
+    double tau;
+    {
+        const double s1 = zj2, s2 = zr2;
+        if (last) {
+            tau = fmin(s1 / c0, hi);
+        } else {
+            const double B = c0 * (dL + dR) + s1 + s2, C = s1 * dR + s2 * dL;
+            const double q = 0.5 * (B + copysign(sqrt(fmax(B * B - 4.0 * c0 * C, 0.0)), B));
+            tau = B > 0.0 ? C / q : q / c0;
+        }
+        if (!(tau > lo && (tau < hi || (last && tau == hi)))) tau = 0.5 * (lo + hi);
+    }
+    bool run = act;
+    for (int it = 0; it < kSecularMaxIter; it++) {
+        if (!__any_sync(0xffffffffu, run)) break;
+        double ps = 0.0, ph = 0.0, dps = 0.0, dph = 0.0;
+        if (run) {
+            const int nL = j + 1;
+            int i = gl;
+            for (; i < nL; i += G) {
+                const double r = dc_rcp((dk[i] - d_o) - tau);
+                const double t = zk[i] * zk[i] * r;
+                ps += t;
+                dps = fma(t, r, dps);
+            }
+            for (; i < kk; i += G) {
+                const double r = dc_rcp((dk[i] - d_o) - tau);
+                const double t = zk[i] * zk[i] * r;
+                ph += t;
+                dph = fma(t, r, dph);
+            }
+        }
+        dc_sum4<G>(ps, ph, dps, dph);
+        if (!run) continue;
+        const double g = rhoinv + ps + ph;
+        const double err = 8.0 * (ph - ps) + rhoinv + fabs(tau) * (dps + dph);
+        if (fabs(g) <= 4.0 * kUnitRoundoff * err * k || hi - lo <= 2.0 * kUnitRoundoff * fmax(fabs(lo), fabs(hi))) {
+            run = false;
+            continue;
+        }
+        if (g < 0.0) lo = tau;
+        else hi = tau;
+        const double a1 = dps * (dL - tau), s1 = a1 * (dL - tau);
+        double cc = rhoinv + ps - a1, y;
+        if (!last) {
+            const double a2 = dph * (dR - tau), s2 = a2 * (dR - tau);
+            cc += ph - a2;
+            const double B = cc * (dL + dR) + s1 + s2, C = s1 * dR + s2 * dL;
+            const double q = 0.5 * (B + copysign(sqrt(fmax(B * B - 4.0 * cc * C, 0.0)), B));
+            y = B > 0.0 ? C / q : q / cc;
+        } else {
+            y = cc > 0.0 ? fmin(dL + s1 / cc, hi) : NAN;   // the upper end itself is a root when k = 1
+        }
+        if (!(y > lo && (y < hi || (last && y == hi)))) y = 0.5 * (lo + hi);
+        tau = y;
+    }
+    if (act) {
+        o_out = o;
+        tau_out = tau;
+        lam_out = d_o + tau;
+    }
+}
+
+// Whether the rank-one components zp, zn of neighbouring poles a distance t apart combine into
+// one by a rotation (|t c s| <= tol for c = zn / |z|, s = zp / |z|), without a division.
+__device__ __forceinline__ bool dc_close(double t, double zp, double zn, double tol) {
+    return fabs(t * zp * zn) <= tol * fma(zp, zp, zn * zn);
+}
+
+// Levels up to nodes of kDcBase columns in one launch: a block of 128 threads merges its columns
+// level by level in shared memory, four lanes per secular root.  The same steps as the level
+// kernels below; separate launches took about 0.1 ms a level whatever the size (five levels
+// of a 70-column problem 0.5 ms), bound by launches, scalar FP64 chains and padded tiles.
+constexpr int kDcBase = 32;
+__global__ void __launch_bounds__(128) dc_base_kernel(int n, const double *__restrict__ d, const double *__restrict__ e,
+                                                      DcBufs b) {
+    __shared__ double Q0[kDcBase][kDcBase + 1], Q1[kDcBase][kDcBase + 1], U[kDcBase][kDcBase + 1];
+    __shared__ double lam[kDcBase], pd[kDcBase], pz[kDcBase], dk[kDcBase], zk[kDcBase], dv[kDcBase], lk[kDcBase],
+        tau[kDcBase], zh[kDcBase], s_rho[kDcBase], rc[kDcBase], rs[kDcBase], rows[kDcBase];
+    __shared__ int sp[kDcBase], st[kDcBase], kl[kDcBase], df[kDcBase], ord[kDcBase], outc[kDcBase], rp[kDcBase],
+        rn[kDcBase], kcnt[kDcBase], nrot[kDcBase];
+    const int c0 = blockIdx.x * kDcBase, nb = min(kDcBase, n - c0);
+    const int tid = threadIdx.x, lane = tid & 31;
+    double(*QA)[kDcBase + 1] = Q0, (*QB)[kDcBase + 1] = Q1;
+    for (int x = tid; x < kDcBase * kDcBase; x += 128) QA[x >> 5][x & 31] = (x >> 5) == (x & 31) ? 1.0 : 0.0;
+    if (tid < kDcBase) {
+        const int i = c0 + tid;
+        double v = 0.0;
+        if (tid < nb) {
+            v = d[i];
+            if (i > 0) v -= fabs(e[i - 1]);
+            if (i < n - 1) v -= fabs(e[i]);
+        }
+        lam[tid] = v;
+    }
+    __syncthreads();
+    for (int half = 1; half < nb; half *= 2) {
+        const int full = 2 * half;
+        for (int x = tid; x < kDcBase * kDcBase; x += 128) QB[x >> 5][x & 31] = 0.0;
+        if (tid < 32) {   // rank-one vector, merged order, deflation: lane = column, then merged position
+            const int s = lane & ~(full - 1), i = lane - s, N = min(full, nb - s);
+            const bool mrg = N > half, in = lane < nb && mrg;
+            const unsigned nodemask = (full == 32 ? 0xffffffffu : (1u << full) - 1u) << s;
+            const unsigned lt = (1u << lane) - 1u;
+            const double beta = mrg ? e[c0 + s + half - 1] : 0.0;
+            const double rho = 2.0 * fabs(beta), sg = beta < 0.0 ? -1.0 : 1.0;
+            const double vd = lane < nb ? lam[lane] : 0.0;
+            double vz = 0.0;
+            if (in) vz = (i < half ? QA[s + half - 1][lane] : sg * QA[s + half][lane]) * 0.70710678118654752440;
+            double mx = in ? fmax(fabs(vd), fabs(vz)) : 0.0;
+            for (int o = half; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+            const double tol = 8.0 * kUnitRoundoff * mx;
+            int pos = i < half ? i : i - half;
+            for (int t = 0; t < half; t++) {   // stable merge of the two ascending halves
+                const int other = i < half ? s + half + t : s + t;
+                const double u = __shfl_sync(0xffffffffu, vd, other & 31);
+                if (in && other < s + N) pos += i < half ? u < vd : u <= vd;
+            }
+            sp[lane] = lane;
+            __syncwarp();
+            if (in) sp[s + min(pos, N - 1)] = lane;
+            __syncwarp();
+            const int j = sp[lane];
+            const double dj = __shfl_sync(0xffffffffu, vd, j), zj = __shfl_sync(0xffffffffu, vz, j);
+            const bool keep = in && !(rho * fabs(zj) <= tol);
+            const unsigned km = __ballot_sync(0xffffffffu, keep) & nodemask;
+            const unsigned before = km & lt;
+            const int prev = before ? 31 - __clz(before) : lane;
+            const double dp = __shfl_sync(0xffffffffu, dj, prev), zp = __shfl_sync(0xffffffffu, zj, prev);
+            const bool close = keep && before && dc_close(dj - dp, zp, zj, tol);
+            const unsigned rm = __ballot_sync(0xffffffffu, close) & nodemask;
+            pd[lane] = dj;
+            pz[lane] = zj;
+            st[lane] = keep;
+            if (i == 0) nrot[lane] = 0;
+            __syncwarp();
+            if (i == 0 && rm) {   // a pair rotates: this node's first lane scans its merged order
+                int nr = 0, pj = -1;
+                for (int t = s; t < s + N; t++) {
+                    if (!st[t]) continue;
+                    if (pj >= 0 && dc_close(pd[t] - pd[pj], pz[pj], pz[t], tol)) {
+                        const double zt = hypot(pz[t], pz[pj]), C = pz[t] / zt, S = -pz[pj] / zt;
+                        const double a = pd[pj], c = pd[t];
+                        rp[s + nr] = sp[pj];
+                        rn[s + nr] = sp[t];
+                        rc[s + nr] = C;
+                        rs[s + nr] = S;
+                        nr++;
+                        pz[t] = zt;
+                        pd[pj] = a * C * C + c * S * S;
+                        pd[t] = a * S * S + c * C * C;
+                        st[pj] = 0;
+                    }
+                    pj = t;
+                }
+                nrot[s] = nr;
+            }
+            __syncwarp();
+            const bool kept = in && st[lane];
+            const unsigned kf = __ballot_sync(0xffffffffu, kept) & nodemask;
+            const unsigned dm = __ballot_sync(0xffffffffu, in && !kept) & nodemask;
+            if (kept) {
+                const int m = s + __popc(kf & lt);
+                kl[m] = j;
+                dk[m] = pd[lane];
+                zk[m] = pz[lane];
+            } else if (in) {
+                const int m = s + __popc(dm & lt);
+                df[m] = j;
+                dv[m] = pd[lane];
+            }
+            if (i == 0) {
+                kcnt[lane] = mrg ? __popc(kf) : -1;
+                s_rho[lane] = rho;
+            }
+        }
+        __syncthreads();
+        if (tid < nb) {   // rotations of the node's columns, one row per thread
+            const int s = tid & ~(full - 1);
+            const int nr = kcnt[s] >= 0 ? nrot[s] : 0;
+            for (int q = 0; q < nr; q++) {
+                const int p = rp[s + q], r = rn[s + q];
+                const double C = rc[s + q], S = rs[s + q], x = QA[tid][p], y = QA[tid][r];
+                QA[tid][p] = C * x + S * y;
+                QA[tid][r] = C * y - S * x;
+            }
+        }
+        const int c = tid >> 2, gl = tid & 3, s = c & ~(full - 1), i = c - s, N = min(full, nb - s);
+        const int k = c < nb ? kcnt[s] : -1;
+        int o = 0;
+        double tv = 0.0, lv = 0.0;
+        const bool root = c < nb && i < k;
+        dc_secular_root<4>(k, i, root, dk + s, zk + s, s_rho[s], o, tv, lv, b.status);
+        if (root && gl == 0) {
+            ord[c] = o;
+            tau[c] = tv;
+            lk[c] = lv;
+        }
+        __syncthreads();
+        double p = 1.0;   // zhat_i^2 = prod_j |d_i - lambda_j| / prod_{j != i} |d_i - d_j|
+        if (root) {
+            const double di = dk[c];
+            for (int j = gl; j < k; j += 4) {
+                const double dl = fabs((di - dk[s + ord[s + j]]) - tau[s + j]);
+                p *= j == i ? dl : dl / fabs(dk[s + j] - di);
+            }
+        }
+        p = dc_group_prod<4>(p);
+        if (root && gl == 0) zh[c] = copysign(sqrt(p), zk[c]);
+        const double v = c < nb && k >= 0 ? (i < k ? lk[c] : dv[c - k]) : 0.0;
+        int r = 0;   // rank in the merged ascending order
+        if (c < nb && k >= 0)
+            for (int m = gl; m < N; m += 4) {
+                const double u = m < k ? lk[s + m] : dv[s + m - k];
+                r += (u < v) || (u == v && m < i);
+            }
+        r += __shfl_xor_sync(0xffffffffu, r, 1);
+        r += __shfl_xor_sync(0xffffffffu, r, 2);
+        if (gl == 0) outc[c] = c < nb && k >= 0 ? s + min(r, N - 1) : c;
+        __syncthreads();
+        double ss = 0.0;   // eigenvectors of the merge
+        if (root) {
+            const double dO = dk[s + ord[c]], t = tau[c];
+            for (int m = gl; m < k; m += 4) {
+                const double u = zh[s + m] * dc_rcp((dk[s + m] - dO) - t);
+                U[s + m][c] = u;
+                ss = fma(u, u, ss);
+            }
+        }
+        ss = dc_group_sum<4>(ss);
+        if (root) {
+            const double inv = 1.0 / sqrt(ss);
+            for (int m = gl; m < k; m += 4) U[s + m][c] *= inv;
+        }
+        if (gl == 0 && c < nb) rows[outc[c]] = k >= 0 ? v : lam[c];
+        __syncthreads();
+        if (c < nb) {
+            const int oc = outc[c];
+            for (int row = s + gl; row < s + N; row += 4) {
+                double a = 0.0;
+                if (k < 0) a = QA[row][c];
+                else if (i >= k) a = QA[row][df[c - k]];
+                else
+                    for (int m = 0; m < k; m++) a = fma(QA[row][kl[s + m]], U[s + m][c], a);
+                QB[row][oc] = a;
+            }
+        }
+        __syncthreads();
+        if (tid < kDcBase) lam[tid] = tid < nb ? rows[tid] : 0.0;
+        double(*T)[kDcBase + 1] = QA;
+        QA = QB;
+        QB = T;
+        __syncthreads();
+    }
+    for (int x = tid; x < nb * nb; x += 128) {
+        const int r = x % nb, cc = x / nb;
+        b.QA[(c0 + r) + (int64_t)(c0 + cc) * n] = QA[r][cc];
+    }
+    if (tid < nb) b.lamA[c0 + tid] = lam[tid];
 }
 
 // Exclusive block prefix sum of one int per thread (blockDim.x <= 1024); total gets the sum.
@@ -959,12 +1326,27 @@ __device__ int dc_block_excl_scan(int v, int *wsum, int &total) {
     return base;
 }
 
-// One block per node: rank-one vector, merge order, deflation (in parallel, or thread 0
-// scanning the merged order when a pair rotation is due), rotations applied to the node's
-// eigenvector columns.  Dynamic shared memory: 20 bytes per node column.
+// One pair rotation of the deflation scan: component pj folds into nj.
+__device__ __forceinline__ void dc_rotate(double &dp, double zp, double &dn, double &zn, double &C, double &S) {
+    const double tt = hypot(zn, zp), a = dp, c = dn;
+    C = zn / tt;
+    S = -zp / tt;
+    zn = tt;
+    dp = a * C * C + c * S * S;
+    dn = a * S * S + c * C * C;
+}
+
+// One block per node: rank-one vector, merge order, deflation.  Deflation runs in parallel: the
+// z test of every entry, then the rotation test of every neighbouring kept pair on the unrotated
+// values; each maximal run of qualifying pairs is scanned by one thread, with the rotated
+// values, until a test past the run's end fails.  A scan that reaches the next run would
+// change that run's input; the block then repeats the scan in thread 0 alone.  The rotations
+// themselves are applied to the eigenvector columns by dc_merge_kernel, which has the rows
+// of the node spread over many blocks.  Dynamic shared memory: 20 bytes per node column.
 __global__ void dc_prep_kernel(int n, int half, int full, const double *__restrict__ e, DcBufs b) {
     extern __shared__ double smem[];
     __shared__ double red[32];
+    __shared__ int s_wsum[32], s_rot, s_conflict;
     const int node = blockIdx.x;
     const int s = node * full;
     const int N = min(full, n - s);
@@ -975,7 +1357,10 @@ __global__ void dc_prep_kernel(int n, int half, int full, const double *__restri
             const int r = (int)(x % N), cc = (int)(x / N);
             b.QB[(s + r) + (int64_t)(s + cc) * n] = b.QA[(s + r) + (int64_t)(s + cc) * n];
         }
-        if (threadIdx.x == 0) b.kcnt[node] = -1;
+        if (threadIdx.x == 0) {
+            b.kcnt[node] = -1;
+            b.nrot[node] = 0;
+        }
         return;
     }
     double *sd = smem, *sz = smem + N;
@@ -983,11 +1368,14 @@ __global__ void dc_prep_kernel(int n, int half, int full, const double *__restri
     const double beta = e[s + n1 - 1];
     const double rho = 2.0 * fabs(beta);
     const double sg = beta < 0.0 ? -1.0 : 1.0;
-    double mx = 0.0;
-    for (int i = threadIdx.x; i < N; i += blockDim.x) {
+    auto load = [&](int i) {
         sd[i] = b.lamA[s + i];
         const double q = i < n1 ? b.QA[(s + n1 - 1) + (int64_t)(s + i) * n] : sg * b.QA[(s + n1) + (int64_t)(s + i) * n];
         sz[i] = q * 0.70710678118654752440;
+    };
+    double mx = 0.0;
+    for (int i = threadIdx.x; i < N; i += blockDim.x) {
+        load(i);
         mx = fmax(mx, fmax(fabs(sd[i]), fabs(sz[i])));
     }
     // a valid permutation first: the merge below writes every slot exactly once for ordered
@@ -1019,260 +1407,226 @@ __global__ void dc_prep_kernel(int n, int half, int full, const double *__restri
         }
     }
     __syncthreads();
-    // Deflation, first in parallel: the z test of every entry, the compaction of the kept and
-    // deflated lists (a block scan over contiguous chunks of the merged order) and the
-    // rotation test of every neighbouring kept pair on the unrotated values.  When no pair
-    // qualifies for a rotation (the usual case) these lists are exactly the serial scan's; when
-    // one does, thread 0 runs the serial scan below, since a rotation changes later tests.  One
-    // thread scanning N entries costs N dependent FP64 chains on a unit that retires two
-    // operations per clock per SM.
-    __shared__ int s_wsum[32], s_rot;
+    int *K0 = b.k0 + s, *tf = b.flag + s, *hm = b.half + s;
+    double *rC = b.tau + s, *rS = b.lamK + s;   // scratch until the secular stage
+    const int per = (N + (int)blockDim.x - 1) / (int)blockDim.x;
+    int k0;   // entries past the z test; the others go to defl at once
     {
-        const int per = (N + (int)blockDim.x - 1) / (int)blockDim.x;
         const int t0 = min(N, (int)threadIdx.x * per), t1 = min(N, t0 + per);
         int cnt = 0;
         for (int t = t0; t < t1; t++) cnt += !(rho * fabs(sz[sp[t]]) <= tol);
-        int total;
-        int kb = dc_block_excl_scan(cnt, s_wsum, total);
+        int kb = dc_block_excl_scan(cnt, s_wsum, k0);
         for (int t = t0; t < t1; t++) {
             const int nj = sp[t];
-            if (!(rho * fabs(sz[nj]) <= tol)) b.Kl[s + kb++] = nj;
-            else b.defl[s + (t - kb)] = nj;
+            if (!(rho * fabs(sz[nj]) <= tol)) {
+                K0[kb] = nj;
+                hm[kb] = nj < n1 ? 1 : 2;
+                kb++;
+            } else {
+                b.defl[s + (t - kb)] = nj;
+            }
         }
-        if (threadIdx.x == 0) s_rot = 0;
+        if (threadIdx.x == 0) s_rot = s_conflict = 0;
         __syncthreads();
+    }
+    {   // tf[m]: the pair (m - 1, m) qualifies for a rotation
         int rot = 0;
-        for (int m = 1 + (int)threadIdx.x; m < total; m += blockDim.x) {
-            const int pj = b.Kl[s + m - 1], nj = b.Kl[s + m];
-            double S = sz[pj], C = sz[nj];
-            const double tt = hypot(C, S);
-            const double T = sd[nj] - sd[pj];
-            C /= tt;
-            S = -S / tt;
-            rot |= fabs(T * C * S) <= tol;
+        for (int m = threadIdx.x; m < k0; m += blockDim.x) {
+            int t = 0;
+            if (m > 0) {
+                const int pj = K0[m - 1], nj = K0[m];
+                t = dc_close(sd[nj] - sd[pj], sz[pj], sz[nj], tol);
+            }
+            tf[m] = t;
+            rot |= t;
         }
         if (rot) atomicOr(&s_rot, 1);
         __syncthreads();
-        if (threadIdx.x == 0 && !s_rot) {
-            b.kcnt[node] = total;
-            b.ndef[node] = N - total;
-            b.nrot[node] = 0;
+    }
+    const bool any = s_rot != 0;
+    if (any) {
+        // Bit 1 of tf[m]: entry m was folded into m + 1 (set by the scanning thread).
+        auto scan = [&](int m, bool whole) {   // from the pair (m - 1, m); returns whether it hit the next run
+            int pj = K0[m - 1], hp = hm[m - 1];
+            double dp = sd[pj], zp = sz[pj];
+            bool dirty = false;   // entry m - 1 carries rotated values
+            for (; m < k0; m++) {
+                const int nj = K0[m];
+                double dn = sd[nj], zn = sz[nj], C, S;
+                int hn = hm[m];
+                const bool inrun = (tf[m] & 1) != 0;
+                if (!whole && !inrun && !dirty) break;        // past the run's end
+                if (dc_close(dn - dp, zp, zn, tol)) {
+                    // folding into an entry whose own pair starts the next run
+                    if (!whole && !inrun && m + 1 < k0 && (tf[m + 1] & 1)) return true;
+                    dc_rotate(dp, zp, dn, zn, C, S);
+                    rC[m - 1] = C;
+                    rS[m - 1] = S;
+                    sd[pj] = dp;
+                    tf[m - 1] |= 2;
+                    hn |= hp;
+                    hm[m - 1] = hn;   // a folded column mixes both as well
+                    dirty = true;
+                    sd[nj] = dn;
+                    sz[nj] = zn;
+                    hm[m] = hn;
+                } else {
+                    dirty = false;
+                    if (!whole && !inrun) break;
+                }
+                pj = nj;
+                dp = dn;
+                zp = zn;
+                hp = hn;
+            }
+            return false;
+        };
+        for (int m = 1 + (int)threadIdx.x; m < k0; m += blockDim.x)
+            if ((tf[m] & 1) && !(tf[m - 1] & 1))
+                if (scan(m, false)) s_conflict = 1;
+        __syncthreads();
+        if (s_conflict) {
+            for (int i = threadIdx.x; i < N; i += blockDim.x) load(i);
+            for (int m = threadIdx.x; m < k0; m += blockDim.x) {
+                tf[m] &= 1;
+                hm[m] = K0[m] < n1 ? 1 : 2;
+            }
+            __syncthreads();
+            if (threadIdx.x == 0 && k0 > 1) scan(1, true);
+            __syncthreads();
+        }
+    }
+    // compaction: the undeflated entries, the folded ones and their rotations, and the entries
+    // whose columns reach each half of the node (the others are zero there)
+    {
+        const int t0 = min(k0, (int)threadIdx.x * per), t1 = min(k0, t0 + per);
+        int nf = 0, nt = 0, nbm = 0;
+        for (int m = t0; m < t1; m++) {
+            const bool fold = any && (tf[m] & 2);
+            nf += fold;
+            if (!fold) {
+                nt += hm[m] & 1;
+                nbm += hm[m] >> 1;
+            }
+        }
+        int tot_f, tot_t, tot_b;
+        int fb = dc_block_excl_scan(nf, s_wsum, tot_f);
+        int tb = dc_block_excl_scan(nt, s_wsum, tot_t);
+        int bb = dc_block_excl_scan(nbm, s_wsum, tot_b);
+        for (int m = t0; m < t1; m++) {
+            const int j = K0[m];
+            if (any && (tf[m] & 2)) {
+                b.rp[s + fb] = j;
+                b.rn[s + fb] = K0[m + 1];
+                b.rc[s + fb] = rC[m];
+                b.rs[s + fb] = rS[m];
+                b.defl[s + (N - k0) + fb] = j;
+                fb++;
+                continue;
+            }
+            const int q = m - fb;
+            b.Kl[s + q] = j;
+            b.dK[s + q] = sd[j];
+            b.zK[s + q] = sz[j];
+            if (hm[m] & 1) b.top[s + tb++] = q;
+            if (hm[m] & 2) b.bot[s + bb++] = q;
+        }
+        __syncthreads();
+        const int nd = N - k0 + tot_f;
+        for (int m = threadIdx.x; m < nd; m += blockDim.x) b.dv[s + m] = sd[b.defl[s + m]];
+        if (threadIdx.x == 0) {
+            b.kcnt[node] = k0 - tot_f;
+            b.ndef[node] = nd;
+            b.nrot[node] = tot_f;
+            b.ntop[node] = tot_t;
+            b.nbot[node] = tot_b;
             b.rho[node] = rho;
         }
     }
-    if (threadIdx.x == 0 && s_rot) {
-        int kc = 0, nd = 0, nr = 0, pj = -1;
-        for (int t = 0; t < N; t++) {
-            const int nj = sp[t];
-            if (rho * fabs(sz[nj]) <= tol) {
-                b.defl[s + nd++] = nj;
-                continue;
-            }
-            if (pj >= 0) {
-                double S = sz[pj], C = sz[nj];
-                const double tt = hypot(C, S);
-                const double T = sd[nj] - sd[pj];
-                C /= tt;
-                S = -S / tt;
-                if (fabs(T * C * S) <= tol) {
-                    sz[nj] = tt;
-                    sz[pj] = 0.0;
-                    b.rp[s + nr] = pj;
-                    b.rn[s + nr] = nj;
-                    b.rc[s + nr] = C;
-                    b.rs[s + nr] = S;
-                    nr++;
-                    const double dp = sd[pj], dn = sd[nj];
-                    sd[pj] = dp * C * C + dn * S * S;
-                    sd[nj] = dp * S * S + dn * C * C;
-                    b.defl[s + nd++] = pj;
-                    kc--;
-                }
-            }
-            b.Kl[s + kc++] = nj;
-            pj = nj;
-        }
-        b.kcnt[node] = kc;
-        b.ndef[node] = nd;
-        b.nrot[node] = nr;
-        b.rho[node] = rho;
-    }
-    __syncthreads();
-    const int kc = b.kcnt[node], nd = b.ndef[node], nr = b.nrot[node];
-    for (int m = threadIdx.x; m < kc; m += blockDim.x) {
-        const int j = b.Kl[s + m];
-        b.dK[s + m] = sd[j];
-        b.zK[s + m] = sz[j];
-    }
-    for (int m = threadIdx.x; m < nd; m += blockDim.x) b.dv[s + m] = sd[b.defl[s + m]];
-    if (nr > 0)
-        for (int r = threadIdx.x; r < N; r += blockDim.x) {
-            double *row = b.QA + (s + r);
-            for (int q = 0; q < nr; q++) {
-                const int64_t op = (int64_t)(s + b.rp[s + q]) * n, on = (int64_t)(s + b.rn[s + q]) * n;
-                const double C = b.rc[s + q], S = b.rs[s + q];
-                const double x = row[op], y = row[on];
-                row[op] = C * x + S * y;
-                row[on] = C * y - S * x;
-            }
-        }
 }
 
-// One warp per secular root: root j of 1/rho + sum_i z_i^2 / (d_i - lambda) = 0 lies in
-// (d_j, d_{j+1}) (the last one in (d_{k-1}, d_{k-1} + rho |z|^2)).  It is found as an offset
-// tau from the nearer pole d_o, so that d_i - lambda = (d_i - d_o) - tau keeps full
-// accuracy.  Each step fits c + s1/(dL - x) + s2/(dR - x) to the value and slope of the two
-// partial sums at tau and takes that model's root; steps leaving the bracket bisect.
-// All lanes hold identical scalars (lane 0's sums are broadcast), so the warp stays uniform.
+// One group of G lanes per secular root (dc_secular_root).
+template <int G>
 __global__ void dc_secular_kernel(int n, int full, DcBufs b) {
-    const int w = (int)((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5);
-    const int lane = threadIdx.x & 31;
-    if (w >= n) return;
-    const int node = w / full, s = node * full, j = w - s;
+    const int w = (int)((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) / G);
+    const int node = w < n ? w / full : 0, s = node * full, j = w - s;
     const int k = b.kcnt[node];
-    if (k < 0 || j >= k) return;
-    const double *dk = b.dK + s, *zk = b.zK + s;
-    const double rho = b.rho[node], rhoinv = 1.0 / rho;
-    int o;
-    double lo, hi;
-    if (j < k - 1) {
-        const double dl = dk[j], dr = dk[j + 1];
-        if (!(dr > dl)) {
-            if (lane == 0) {
-                atomicExch(b.status, 1);
-                b.ord[s + j] = j;
-                b.tau[s + j] = 0.0;
-                b.lamK[s + j] = dl;
-            }
-            return;
-        }
-        const double hg = 0.5 * (dr - dl);
-        double p = 0.0;
-        for (int i = lane; i < k; i += 32) p += zk[i] * zk[i] / ((dk[i] - dl) - hg);
-        const double g = rhoinv + eig_warp_sum(p);
-        if (g > 0.0) {
-            o = j;
-            lo = 0.0;
-            hi = hg;
-        } else {
-            o = j + 1;
-            lo = -hg;
-            hi = 0.0;
-        }
-    } else {
-        double p = 0.0;
-        for (int i = lane; i < k; i += 32) p += zk[i] * zk[i];
-        o = j;
-        lo = 0.0;
-        hi = rho * eig_warp_sum(p);
-    }
-    const double d_o = dk[o];
-    const int L = j, R = j + 1;
-    const double dL = dk[L] - d_o, dR = R < k ? dk[R] - d_o : 0.0;
-    double tau = 0.5 * (lo + hi);
-    for (int it = 0; it < kSecularMaxIter; it++) {
-        double ps = 0.0, ph = 0.0, dps = 0.0, dph = 0.0;
-        for (int i = lane; i < k; i += 32) {
-            // one division per pole (a GB300 FP64 division is a chain of FP64 operations on a
-            // unit that retires two per clock per SM): t = z^2 / den and t / den from 1 / den
-            const double r = 1.0 / ((dk[i] - d_o) - tau);
-            const double t = zk[i] * zk[i] * r;
-            if (i <= L) {
-                ps += t;
-                dps += t * r;
-            } else {
-                ph += t;
-                dph += t * r;
-            }
-        }
-        ps = eig_warp_sum(ps);
-        ph = eig_warp_sum(ph);
-        dps = eig_warp_sum(dps);
-        dph = eig_warp_sum(dph);
-        const double g = rhoinv + ps + ph;
-        const double err = 8.0 * (ph - ps) + rhoinv + fabs(tau) * (dps + dph);
-        if (fabs(g) <= 4.0 * kUnitRoundoff * err * k) break;
-        if (hi - lo <= 2.0 * kUnitRoundoff * fmax(fabs(lo), fabs(hi))) break;
-        if (g < 0.0) lo = tau;
-        else hi = tau;
-        const double s1 = dps * (dL - tau) * (dL - tau);
-        double cc = rhoinv + ps - s1 / (dL - tau);
-        double x;
-        if (R < k) {
-            const double s2 = dph * (dR - tau) * (dR - tau);
-            cc += ph - s2 / (dR - tau);
-            const double A = cc, B = cc * (dL + dR) + s1 + s2, C = cc * dL * dR + s1 * dR + s2 * dL;
-            if (A == 0.0) {
-                x = C / B;
-            } else {
-                const double disc = fmax(B * B - 4.0 * A * C, 0.0);
-                const double q = 0.5 * (B + copysign(sqrt(disc), B));
-                const double r1 = q / A;
-                const double r2 = q != 0.0 ? C / q : NAN;
-                x = (r1 > lo && r1 < hi) ? r1 : r2;
-            }
-        } else {
-            x = cc > 0.0 ? dL + s1 / cc : NAN;
-        }
-        if (!(x > lo && x < hi)) x = 0.5 * (lo + hi);
-        tau = x;
-    }
-    if (lane == 0) {
+    const bool act = w < n && k >= 0 && j < k;
+    int o = 0;
+    double tau = 0.0, lam = 0.0;
+    dc_secular_root<G>(k, j, act, b.dK + s, b.zK + s, act ? b.rho[node] : 1.0, o, tau, lam, b.status);
+    if (act && (threadIdx.x & (G - 1)) == 0) {
         b.ord[s + j] = o;
         b.tau[s + j] = tau;
-        b.lamK[s + j] = d_o + tau;
+        b.lamK[s + j] = lam;
     }
 }
 
-// One warp per undeflated entry i: zhat_i^2 = prod_j |d_i - lambda_j| / prod_{j != i} |d_i - d_j|
-// (up to the common factor 1/rho, which the normalisation removes); sign of z_i.
-__global__ void dc_zhat_kernel(int n, int full, DcBufs b) {
-    const int w = (int)((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5);
-    const int lane = threadIdx.x & 31;
-    if (w >= n) return;
-    const int node = w / full, s = node * full, i = w - s;
-    const int k = b.kcnt[node];
-    if (k < 0 || i >= k) return;
-    const double *dk = b.dK + s;
-    const double di = dk[i];
-    double p = 1.0;
-    for (int j = lane; j < k; j += 32) {
-        const double dl = fabs((di - dk[b.ord[s + j]]) - b.tau[s + j]);
-        p *= (j == i) ? dl : dl / fabs(dk[j] - di);
+// After the secular stage, one launch for three independent jobs, by block: [0, nz) recompute the
+// rank-one vector (one warp per undeflated entry i, zhat_i^2 = prod_j |d_i - lambda_j| /
+// prod_{j != i} |d_i - d_j| up to the common factor 1/rho, sign of z_i), [nz, 2 nz) rank the
+// node's eigenvalues (one warp per entry: its column in the next level, ties by entry index),
+// and [2 nz, ...) apply the deflation's rotations (32 rows per block; the warps take
+// contiguous shares of the rotation list cut where a new chain of columns begins).
+constexpr int DM_THREADS = 64, DM_ROT_ROWS = 32, DM_ROT_SHARES = DM_THREADS / 32;
+__global__ void __launch_bounds__(DM_THREADS) dc_merge_kernel(int n, int full, int nz, DcBufs b) {
+    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+    const int role = (int)blockIdx.x < nz ? 0 : (int)blockIdx.x < 2 * nz ? 1 : 2;
+    if (role < 2) {
+        const int g = ((int)blockIdx.x - role * nz) * (DM_THREADS / 32) + wib;
+        if (g >= n) return;
+        const int node = g / full, s = node * full, i = g - s;
+        const int k = b.kcnt[node];
+        if (k < 0) return;
+        if (role == 0) {
+            if (i >= k) return;
+            const double *dk = b.dK + s;
+            const double di = dk[i];
+            double p = 1.0;
+            for (int j = lane; j < k; j += 32) {
+                const double dl = fabs((di - dk[b.ord[s + j]]) - b.tau[s + j]);
+                p *= (j == i) ? dl : dl / fabs(dk[j] - di);
+            }
+            p = eig_warp_prod(p);
+            if (lane == 0) b.zh[s + i] = copysign(sqrt(p), b.zK[s + i]);
+            return;
+        }
+        const int N = k + b.ndef[node];
+        if (i >= N) return;
+        const double v = i < k ? b.lamK[s + i] : b.dv[s + i - k];
+        int r = 0;
+        for (int m = lane; m < N; m += 32) {
+            const double u = m < k ? b.lamK[s + m] : b.dv[s + m - k];
+            r += (u < v) || (u == v && m < i);
+        }
+        r = __reduce_add_sync(0xffffffffu, r);
+        if (lane == 0) {
+            b.lamB[s + r] = v;
+            b.outc[s + i] = s + r;
+        }
+        return;
     }
-    p = eig_warp_prod(p);
-    if (lane == 0) b.zh[s + i] = copysign(sqrt(p), b.zK[s + i]);
+    const int row = ((int)blockIdx.x - 2 * nz) * DM_ROT_ROWS + lane;
+    const int node = min(row, n - 1) / full, s = node * full;   // full >= 32: the same for the whole warp
+    const int nr = b.nrot[node];
+    if (nr == 0 || row >= n) return;
+    auto cut = [&](int q) {   // first chain start at or after q
+        while (q > 0 && q < nr && b.rp[s + q] == b.rn[s + q - 1]) q++;
+        return q;
+    };
+    const int q0 = cut((int)((int64_t)wib * nr / DM_ROT_SHARES)), q1 = cut((int)((int64_t)(wib + 1) * nr / DM_ROT_SHARES));
+    double *Q = b.QA + row + (int64_t)s * n;
+    for (int q = q0; q < q1; q++) {
+        const int64_t op = (int64_t)b.rp[s + q] * n, on = (int64_t)b.rn[s + q] * n;
+        const double C = b.rc[s + q], S = b.rs[s + q], x = Q[op], y = Q[on];
+        Q[op] = C * x + S * y;
+        Q[on] = C * y - S * x;
+    }
 }
 
-// One warp per node entry: the rank of its eigenvalue in the merged ascending order
-// (ties by entry index) gives its column in the next level.
-__global__ void dc_rank_kernel(int n, int full, DcBufs b) {
-    // one warp per entry (the N comparisons are FP64 operations: one thread per entry left a
-    // 792-entry merge on four SMs); every exit below is uniform over the warp
-    const int g = (int)(((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
-    const int lane = threadIdx.x & 31;
-    if (g >= n) return;
-    const int node = g / full, s = node * full, i = g - s;
-    const int k = b.kcnt[node];
-    if (k < 0) return;
-    const int N = k + b.ndef[node];
-    if (i >= N) return;
-    const double v = i < k ? b.lamK[s + i] : b.dv[s + i - k];
-    int r = 0;
-    for (int m = lane; m < N; m += 32) {
-        const double u = m < k ? b.lamK[s + m] : b.dv[s + m - k];
-        r += (u < v) || (u == v && m < i);
-    }
-    r = __reduce_add_sync(0xffffffffu, r);
-    if (lane == 0) {
-        b.lamB[s + r] = v;
-        b.outc[s + i] = s + r;
-    }
-}
-
-// One block per node entry: column of the merge eigenvector matrix (undeflated entries),
-// or the copy of a deflated eigenvector into its output column.
-__global__ void dc_vec_kernel(int n, int full, DcBufs b) {
+// One block per node entry with an output column in [olo, ohi): column of the merge eigenvector
+// matrix (undeflated entries), or the copy of a deflated eigenvector into its output column.
+__global__ void dc_vec_kernel(int n, int full, int olo, int ohi, DcBufs b) {
     __shared__ double red[32];
     const int g = blockIdx.x;
     const int node = g / full, s = node * full, i = g - s;
@@ -1280,75 +1634,97 @@ __global__ void dc_vec_kernel(int n, int full, DcBufs b) {
     if (k < 0) return;
     const int N = k + b.ndef[node];
     if (i >= N) return;
+    const int oc = b.outc[s + i];
+    if (oc < olo || oc >= ohi) return;
     if (i < k) {
         const double *dk = b.dK + s;
         const double dO = dk[b.ord[s + i]], t = b.tau[s + i];
+        double *u = b.U + s + (int64_t)(s + i) * n;
         double ss = 0.0;
         for (int m = threadIdx.x; m < k; m += blockDim.x) {
-            const double u = b.zh[s + m] / ((dk[m] - dO) - t);
-            ss += u * u;
+            const double v = b.zh[s + m] * dc_rcp((dk[m] - dO) - t);
+            u[m] = v;
+            ss = fma(v, v, ss);
         }
         const double inv = 1.0 / sqrt(eig_block_sum(ss, red));
-        for (int m = threadIdx.x; m < k; m += blockDim.x)
-            b.U[(s + m) + (int64_t)(s + i) * n] = b.zh[s + m] / ((dk[m] - dO) - t) * inv;
+        for (int m = threadIdx.x; m < k; m += blockDim.x) u[m] *= inv;
     } else {
-        const int64_t src = (int64_t)(s + b.defl[s + i - k]) * n, dst = (int64_t)b.outc[s + i] * n;
+        const int64_t src = (int64_t)(s + b.defl[s + i - k]) * n, dst = (int64_t)oc * n;
         for (int r = threadIdx.x; r < N; r += blockDim.x) b.QB[(s + r) + dst] = b.QA[(s + r) + src];
     }
 }
 
-// QB(rows of node, outc[j]) = QA(rows of node, Kl[m]) * U(m, j) for the undeflated entries:
-// one 64x64 output tile per block, batched over nodes (blockIdx.z).
-constexpr int DG_T = 64, DG_K = 16;
-__global__ void __launch_bounds__(256) dc_gemm_kernel(int n, int full, DcBufs b) {
+// QB(rows of node, outc[j]) = QA(rows of node, Kl[m]) * U(m, j) for the undeflated entries with
+// outc[j] in [olo, ohi), batched over nodes (blockIdx.z).  QA is block diagonal by the two halves of
+// the node, so a row of the first half sums over the entries of `top` alone and one of the
+// second half over `bot`: half the products.  One 16 x 16 output tile per block, one output per
+// thread (row tiles do not cross the halves): the FP64 unit is the limit at any tile, and
+// small tiles fill the SMs evenly (n = 791: 13 x 13 tiles of 64 left 152 SMs with one or two each).
+constexpr int DG_T = 16, DG_K = 32;
+__global__ void __launch_bounds__(256) dc_gemm_kernel(int n, int half, int full, int olo, int ohi, DcBufs b) {
     __shared__ double As[DG_K][DG_T + 1];
     __shared__ double Bs[DG_K][DG_T + 1];
+    __shared__ int s_need;
     const int node = blockIdx.z, s = node * full;
     const int k = b.kcnt[node];
     if (k <= 0) return;
     const int N = min(full, n - s);
-    const int r0 = blockIdx.x * DG_T, c0 = blockIdx.y * DG_T;
-    if (r0 >= N || c0 >= k) return;
-    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-    double acc[4][4] = {};
-    for (int m0 = 0; m0 < k; m0 += DG_K) {
-        for (int x = threadIdx.x; x < DG_T * DG_K; x += 256) {
-            const int rr = x % DG_T, kk = x / DG_T;
-            const int gr = r0 + rr, gm = m0 + kk;
-            As[kk][rr] = (gr < N && gm < k) ? b.QA[(s + gr) + (int64_t)(s + b.Kl[s + gm]) * n] : 0.0;
+    const int tt = (half + DG_T - 1) / DG_T;   // row tiles of the first half
+    const bool first = (int)blockIdx.x < tt;
+    const int r0 = first ? blockIdx.x * DG_T : half + ((int)blockIdx.x - tt) * DG_T, rend = first ? half : N;
+    const int c0 = blockIdx.y * DG_T;
+    if (r0 >= rend || c0 >= k) return;
+    const int *list = (first ? b.top : b.bot) + s;
+    const int nl = first ? b.ntop[node] : b.nbot[node];
+    const int tid = threadIdx.x, lane = tid & 31, w = ((tid >> 5) + (int)blockIdx.x + (int)blockIdx.y) & 7;
+    const int li = 8 * (w & 1) + (lane & 7), lj = 4 * (w >> 1) + (lane >> 3);
+    const int gr = r0 + li, gc = c0 + lj;
+    const int oc = gc < k ? b.outc[s + gc] : -1;
+    const bool want = gc < k && oc >= olo && oc < ohi;
+    if (tid == 0) s_need = 0;
+    __syncthreads();
+    if (want) s_need = 1;
+    __syncthreads();
+    if (!s_need) return;
+    const bool busy = __any_sync(0xffffffffu, want && gr < rend);
+    // chunk element loads: A (row fastest) and B (m fastest), two per thread
+    double pa[2], pb[2];
+    auto fetch = [&](int m0) {
+#pragma unroll
+        for (int u = 0; u < 2; u++) {
+            const int x = tid + 256 * u;
+            const int rr = x % DG_T, km = x / DG_T;
+            pa[u] = (r0 + rr < rend && m0 + km < nl) ? b.QA[(s + r0 + rr) + (int64_t)(s + b.Kl[s + list[m0 + km]]) * n] : 0.0;
+            const int kb = x % DG_K, cc = x / DG_K;
+            pb[u] = (m0 + kb < nl && c0 + cc < k) ? b.U[(s + list[m0 + kb]) + (int64_t)(s + c0 + cc) * n] : 0.0;
         }
-        for (int x = threadIdx.x; x < DG_T * DG_K; x += 256) {
-            const int kk = x % DG_K, cc = x / DG_K;
-            const int gm = m0 + kk, gc = c0 + cc;
-            Bs[kk][cc] = (gm < k && gc < k) ? b.U[(s + gm) + (int64_t)(s + gc) * n] : 0.0;
+    };
+    double a0 = 0.0, a1 = 0.0;
+    fetch(0);
+    for (int m0 = 0; m0 < nl; m0 += DG_K) {
+#pragma unroll
+        for (int u = 0; u < 2; u++) {
+            const int x = tid + 256 * u;
+            As[x / DG_T][x % DG_T] = pa[u];
+            Bs[x % DG_K][x / DG_K] = pb[u];
         }
         __syncthreads();
-#pragma unroll
-        for (int kk = 0; kk < DG_K; kk++) {
-            double a[4], bb[4];
-#pragma unroll
-            for (int q = 0; q < 4; q++) {
-                a[q] = As[kk][ty + 16 * q];
-                bb[q] = Bs[kk][tx + 16 * q];
+        if (m0 + DG_K < nl) fetch(m0 + DG_K);
+        if (busy) {
+            const int kend = min(DG_K, nl - m0);
+            if (kend == DG_K) {
+#pragma unroll 8
+                for (int q = 0; q < DG_K; q += 2) {
+                    a0 = fma(As[q][li], Bs[q][lj], a0);
+                    a1 = fma(As[q + 1][li], Bs[q + 1][lj], a1);
+                }
+            } else {
+                for (int q = 0; q < kend; q++) a0 = fma(As[q][li], Bs[q][lj], a0);
             }
-#pragma unroll
-            for (int p = 0; p < 4; p++)
-#pragma unroll
-                for (int q = 0; q < 4; q++) acc[p][q] = fma(a[p], bb[q], acc[p][q]);
         }
         __syncthreads();
     }
-#pragma unroll
-    for (int q = 0; q < 4; q++) {
-        const int gc = c0 + tx + 16 * q;
-        if (gc >= k) continue;
-        const int64_t col = (int64_t)b.outc[s + gc] * n;
-#pragma unroll
-        for (int p = 0; p < 4; p++) {
-            const int gr = r0 + ty + 16 * p;
-            if (gr < N) b.QB[(s + gr) + col] = acc[p][q];
-        }
-    }
+    if (want && gr < rend) b.QB[(s + gr) + (int64_t)oc * n] = a0 + a1;
 }
 
 // Largest divide-and-conquer dimension: the merge scan keeps 20 bytes per column in shared
@@ -1364,72 +1740,94 @@ static DcBufs dc_bufs(Context &c, int n, int slot) {
     b.QA = wsget<double>(c, nm("dc.QA"), nn);
     b.QB = wsget<double>(c, nm("dc.QB"), nn);
     b.U = wsget<double>(c, nm("dc.U"), nn);
-    b.lamA = wsget<double>(c, nm("dc.lamA"), n);
-    b.lamB = wsget<double>(c, nm("dc.lamB"), n);
-    b.dK = wsget<double>(c, nm("dc.dK"), n);
-    b.zK = wsget<double>(c, nm("dc.zK"), n);
-    b.dv = wsget<double>(c, nm("dc.dv"), n);
-    b.Kl = wsget<int>(c, nm("dc.Kl"), n);
-    b.defl = wsget<int>(c, nm("dc.defl"), n);
-    b.rp = wsget<int>(c, nm("dc.rp"), n);
-    b.rn = wsget<int>(c, nm("dc.rn"), n);
-    b.rc = wsget<double>(c, nm("dc.rc"), n);
-    b.rs = wsget<double>(c, nm("dc.rs"), n);
-    b.ord = wsget<int>(c, nm("dc.ord"), n);
-    b.tau = wsget<double>(c, nm("dc.tau"), n);
-    b.lamK = wsget<double>(c, nm("dc.lamK"), n);
-    b.zh = wsget<double>(c, nm("dc.zh"), n);
-    b.outc = wsget<int>(c, nm("dc.outc"), n);
-    b.kcnt = wsget<int>(c, nm("dc.kcnt"), n);
-    b.ndef = wsget<int>(c, nm("dc.ndef"), n);
-    b.nrot = wsget<int>(c, nm("dc.nrot"), n);
-    b.rho = wsget<double>(c, nm("dc.rho"), n);
-    b.status = wsget<int>(c, nm("dc.status"), 1);
+    // the vectors of one slot in two allocations: 10 of doubles, 16 of integers
+    const size_t m = (size_t)n + 8;
+    double *f = wsget<double>(c, nm("dc.f"), 11 * m);
+    b.lamA = f, b.lamB = f + m, b.dK = f + 2 * m, b.zK = f + 3 * m, b.dv = f + 4 * m, b.rc = f + 5 * m;
+    b.rs = f + 6 * m, b.tau = f + 7 * m, b.lamK = f + 8 * m, b.zh = f + 9 * m, b.rho = f + 10 * m;
+    int *q = wsget<int>(c, nm("dc.i"), 16 * m);
+    b.Kl = q, b.defl = q + m, b.rp = q + 2 * m, b.rn = q + 3 * m, b.ord = q + 4 * m, b.outc = q + 5 * m;
+    b.top = q + 6 * m, b.bot = q + 7 * m, b.k0 = q + 8 * m, b.flag = q + 9 * m, b.half = q + 10 * m;
+    b.kcnt = q + 11 * m, b.ndef = q + 12 * m, b.nrot = q + 13 * m, b.ntop = q + 14 * m, b.nbot = q + 15 * m;
+    b.status = b.nbot + n + 4;
     return b;
 }
 
-// Eigenvalues (ascending, into w) and eigenvectors (n x n, ld n, returned) of the
-// symmetric tridiagonal (d, e).  d and e are device arrays; e has n-1 entries.
-static const double *tridiag_dc(Context &c, int n, const double *d, const double *e, double *w, int slot) {
+// The merge eigenvectors of one level and their product with the children's, for output columns
+// [olo, ohi) of the whole matrix.
+static void dc_level_vectors(Context &c, int n, int half, int olo, int ohi, const DcBufs &b) {
+    const int full = 2 * half, nodes = (n + full - 1) / full;
+    dc_vec_kernel<<<n, 128, 0, c.stream>>>(n, full, olo, ohi, b);
+    DCG_LAUNCHED(c);
+    const int tt = (half + DG_T - 1) / DG_T, tb = (std::min(full, n) - half + DG_T - 1) / DG_T;
+    dim3 gg(tt + std::max(tb, 1), grid1d(std::min(full, n), DG_T), nodes);
+    dc_gemm_kernel<<<gg, 256, 0, c.stream>>>(n, half, full, olo, ohi, b);
+    DCG_LAUNCHED(c);
+}
+
+// Bound by latency (launches, serial FP64 chains) below a few hundred columns and by the FP64
+// pipe above.  Measured with the base kernel, four launches a level instead of six, the
+// cheaper secular steps and the merge products by halves (whole solves, before -> after):
+// 4/4/12 3.88 -> 3.05 ms, 8/6/40 8.75 -> 7.07 ms, 14/10/230 50.8 -> 41.9 ms, 20/12/300
+// 114.8 -> 104.9 ms.
+// Eigenvalues (ascending, into w) of the symmetric tridiagonal (d, e), and its eigenvectors up to
+// the last merge, whose own vectors dc_vectors forms for the columns that are asked for (most
+// of the merge products of a decomposition are the last one's).  d and e are device arrays;
+// e has n-1 entries.
+static void tridiag_dc(Context &c, int n, const double *d, const double *e, double *w, int slot) {
     if (n > kDcMaxN)
         throw Error{DCG_E_ARG, "eigensolver dimension " + std::to_string(n) + " exceeds " + std::to_string(kDcMaxN)};
     DcBufs b = dc_bufs(c, n, slot);
-    // Both buffers start at zero: a merge reads whole columns of its node block, including the
-    // cross blocks between its two children, which no earlier level writes.
+    // Both buffers start at zero: rotations and deflated copies touch whole columns of a node
+    // block, including the cross blocks between its two children, which no earlier level writes.
     DCG_CUDA(cudaMemsetAsync(b.QA, 0, sizeof(double) * (size_t)n * n, c.stream));
-    DCG_CUDA(cudaMemsetAsync(b.QB, 0, sizeof(double) * (size_t)n * n, c.stream));
+    if (n > kDcBase) DCG_CUDA(cudaMemsetAsync(b.QB, 0, sizeof(double) * (size_t)n * n, c.stream));
     DCG_CUDA(cudaMemsetAsync(b.status, 0, sizeof(int), c.stream));
-    dc_leaf_kernel<<<grid1d(n, 256), 256, 0, c.stream>>>(n, d, e, b.lamA, b.QA);
+    dc_base_kernel<<<grid1d(n, kDcBase), 128, 0, c.stream>>>(n, d, e, b);
     DCG_LAUNCHED(c);
+    c.eig_n[slot] = n;
+    c.eig_status[slot] = b.status;
+    c.eig_Q[slot] = b.QA;
+    c.eig_last[slot] = 0;
     DCG_CUDA(cudaFuncSetAttribute(dc_prep_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 20 * kDcMaxN));
-    for (int half = 1; half < n; half *= 2) {
+    for (int half = kDcBase; half < n; half *= 2) {
         const int full = 2 * half;
         const int nodes = (n + full - 1) / full;
         const int nmax = std::min(full, n);
         dc_prep_kernel<<<nodes, 256, 20 * (size_t)nmax, c.stream>>>(n, half, full, e, b);
         DCG_LAUNCHED(c);
-        // one warp per root in blocks of two warps: a 792-root merge spreads over 396 blocks,
-        // every SM (eight warps a block left 53 of 152 SMs idle on an FP64-bound kernel)
-        dc_secular_kernel<<<grid1d((int64_t)n * 32, 64), 64, 0, c.stream>>>(n, full, b);
+        // a warp per root while that is about one warp per quarter SM, half a warp for more
+        // roots (a root's scalar steps cost as much as eight poles a lane); blocks of two
+        // warps reach every SM
+        if (n <= 4 * std::max(1, c.num_sms)) dc_secular_kernel<32><<<grid1d((int64_t)n * 32, 64), 64, 0, c.stream>>>(n, full, b);
+        else dc_secular_kernel<16><<<grid1d((int64_t)n * 16, 64), 64, 0, c.stream>>>(n, full, b);
         DCG_LAUNCHED(c);
-        dc_zhat_kernel<<<grid1d((int64_t)n * 32, 64), 64, 0, c.stream>>>(n, full, b);
+        const int nz = (int)grid1d((int64_t)n * 32, DM_THREADS);
+        dc_merge_kernel<<<2 * nz + grid1d(n, DM_ROT_ROWS), DM_THREADS, 0, c.stream>>>(n, full, nz, b);
         DCG_LAUNCHED(c);
-        dc_rank_kernel<<<grid1d((int64_t)n * 32, 64), 64, 0, c.stream>>>(n, full, b);
-        DCG_LAUNCHED(c);
-        dc_vec_kernel<<<n, 128, 0, c.stream>>>(n, full, b);
-        DCG_LAUNCHED(c);
-        dim3 gg(grid1d(nmax, DG_T), grid1d(nmax, DG_T), nodes);
-        dc_gemm_kernel<<<gg, 256, 0, c.stream>>>(n, full, b);
-        DCG_LAUNCHED(c);
-        std::swap(b.QA, b.QB);
         std::swap(b.lamA, b.lamB);
+        if (full >= n) {
+            c.eig_last[slot] = half;
+            c.eig_Q[slot] = nullptr;   // formed on request
+            break;
+        }
+        dc_level_vectors(c, n, half, 0, n, b);
+        std::swap(b.QA, b.QB);
     }
     DCG_CUDA(cudaMemcpyAsync(w, b.lamA, sizeof(double) * n, cudaMemcpyDeviceToDevice, c.stream));
-    // record which buffer holds the result for the vector stage of this slot
-    c.eig_Q[slot] = b.QA;
-    c.eig_n[slot] = n;
-    c.eig_status[slot] = b.status;
-    return b.QA;
+}
+
+// Columns [vlo, vhi) of the tridiagonal's eigenvectors of the slot's last tridiag_dc (n x n,
+// ld n; other columns are undefined).
+static const double *dc_vectors(Context &c, int slot, int n, int vlo, int vhi) {
+    const int half = c.eig_last[slot];
+    if (half == 0) return c.eig_Q[slot];
+    DcBufs b = dc_bufs(c, n, slot);
+    int swaps = 0;
+    for (int h = kDcBase; h < half; h *= 2) swaps++;
+    if (swaps & 1) std::swap(b.QA, b.QB);
+    dc_level_vectors(c, n, half, vlo, vhi, b);
+    return b.QB;
 }
 
 // ===================================================================== 3. back-transformation
@@ -2241,11 +2639,11 @@ void tridiag_e2(Context &c, int slot, int n, const cplx *A, int64_t lda, const c
 void heev_vectors_slot(Context &c, int slot, int n, cplx *A, int64_t lda, int vlo, int vhi, cplx *Z, int64_t ldz) {
     const int nvec = vhi - vlo;
     if (nvec <= 0 || n <= 0 || Z == nullptr) return;
-    if (slot < 0 || slot >= kEigSlots || c.eig_Q[slot] == nullptr || c.eig_n[slot] != n)
+    if (slot < 0 || slot >= kEigSlots || (c.eig_Q[slot] == nullptr && c.eig_last[slot] == 0) || c.eig_n[slot] != n)
         throw Error{DCG_E_STATE, "eigenvectors requested without a matching eigenvalue stage"};
     HeevWork h = heev_work(c, n, slot);
-    const double *Qt = c.eig_Q[slot];
     FamScope fs(c, DCG_FAM_EIG, 8.0 * (double)n * n * nvec);
+    const double *Qt = dc_vectors(c, slot, n, vlo, vhi);
     FamScope f4(c, DCG_FAM_EIG_BACK, 8.0 * (double)n * n * nvec);
     // Many columns: the FP64 pipe is the limit, one warp per column without prefetch (fewest
     // registers).  Few columns: the n-1 sequential reflections are the limit, prefetch the next
@@ -2367,9 +2765,9 @@ void heev_vectors_only(Context &c, int n, cplx *A, int64_t lda, const double *w,
 // (device, n x n, ld n; valid until the next eigensolver call).
 const double *stedc(Context &c, int n, const double *d, const double *e, double *w) {
     if (n <= 0) return nullptr;
-    const double *Q = tridiag_dc(c, n, d, e, w, 0);
+    tridiag_dc(c, n, d, e, w, 0);
     check_dc_status(c, 0);
-    return Q;
+    return dc_vectors(c, 0, n, 0, n);
 }
 
 }  // namespace dcg
