@@ -347,6 +347,7 @@ struct EigJob {
     double *w = nullptr;
     int slot = 0;
     bool tridiag_only = false;   // stop after the reduction: for tridiag_e2 (w is not written)
+    bool real = false;           // every imaginary part is zero: the reduction skips them
 };
 void heev_values_batched(Context &c, const std::vector<EigJob> &jobs);
 void heev_vectors_slot(Context &c, int slot, int n, cplx *A, int64_t lda, int vlo, int vhi, cplx *Z, int64_t ldz);

@@ -199,7 +199,6 @@ struct GridBar {
     unsigned count;
     unsigned gen;
     int err;       // 1: a barrier wait exceeded its time limit
-    unsigned pub;  // reflectors published so far (shared-memory tridiagonalisation)
     unsigned long long limit_ns;   // time limit of one wait (set by the host before the launch)
 };
 
@@ -247,69 +246,6 @@ __device__ __forceinline__ bool grid_barrier(GridBar *gb, unsigned nblocks) {
     }
     __syncthreads();
     return s_ok != 0;
-}
-
-// Wait until gb->pub >= want (a point-to-point signal from one block instead of a grid
-// barrier); bounded like grid_barrier.  Ends with __syncthreads.
-__device__ __forceinline__ bool wait_published(GridBar *gb, unsigned want) {
-    __shared__ int s_ok2;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        int ok = 1;
-        unsigned cur;
-        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(cur) : "l"(&gb->pub) : "memory");
-        if (cur < want) {
-            const uint64_t t0 = globaltimer_ns();
-            unsigned spins = 0;
-            while (true) {
-                asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(cur) : "l"(&gb->pub) : "memory");
-                if (cur >= want) break;
-                if ((++spins & 15u) == 0) {
-                    if (*(volatile int *)&gb->err) {
-                        ok = 0;
-                        break;
-                    }
-                    if (globaltimer_ns() - t0 > gb->limit_ns) {
-                        atomicExch(&gb->err, 1);
-                        ok = 0;
-                        break;
-                    }
-                }
-            }
-        }
-        s_ok2 = ok;
-    }
-    __syncthreads();
-    return s_ok2 != 0;
-}
-
-// Two deterministic block sums in one pass (sh >= 64 doubles); every thread gets both.
-__device__ void eig_block_sum2(double &a, double &b, double *sh) {
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
-    for (int o = 16; o > 0; o >>= 1) {
-        a += __shfl_down_sync(0xffffffffu, a, o);
-        b += __shfl_down_sync(0xffffffffu, b, o);
-    }
-    __syncthreads();
-    if (lane == 0) {
-        sh[wid] = a;
-        sh[32 + wid] = b;
-    }
-    __syncthreads();
-    if (wid == 0) {
-        double x = lane < nw ? sh[lane] : 0.0, y = lane < nw ? sh[32 + lane] : 0.0;
-        for (int o = 16; o > 0; o >>= 1) {
-            x += __shfl_down_sync(0xffffffffu, x, o);
-            y += __shfl_down_sync(0xffffffffu, y, o);
-        }
-        if (lane == 0) {
-            sh[0] = x;
-            sh[32] = y;
-        }
-    }
-    __syncthreads();
-    a = sh[0];
-    b = sh[32];
 }
 
 __device__ __forceinline__ cplx ldcg(const cplx *p) { return __ldcg(p); }
@@ -462,443 +398,484 @@ __global__ void __launch_bounds__(TRD_THREADS) tridiag_persistent_kernel(int n, 
 }
 
 // ---- shared-memory-resident form (n up to kTridiagSmemMaxN): the matrix lives in the blocks'
-// shared memory for the whole reduction, block b owning columns b, b + nb, ...  Per column k
-// the global traffic is the reflector v (written by the owner of column k), the all-gathered
-// p = tau A22 v (one entry per column, from its owner) and one partial dot per block; the
-// matvec and the rank-2 update run from shared memory.  The warp that updates column k+1
-// forms the next reflector from it right away and signals it; per column one grid barrier
-// (before w) and one wait for the published reflector.
+// shared memory for the whole reduction, block b owning columns b, b + nb, ...  Per column k the
+// blocks exchange the reflector v (from the owner of column k) and x = tau A22 v (one entry per
+// column, from its owner); the matvec and the rank-2 update run from shared memory.
+//
+// What bounds it is the chain of a column (v to every block, matvec, x to every block, w, the
+// update of column k+1, its norm, the next reflector) and the FP64 unit (two FMAs per clock
+// and SM: a warp's FP64 instruction holds a quarter of the SM for 64 clocks, whether one lane
+// is active or all).  So:
+//   - v and x travel as 16-byte words that carry their own flag (the column's number beside each
+//     half of a double): a reader polls the data itself, one trip through L2 instead of data,
+//     fence, counter and data again.
+//   - every column's rows are dealt in pieces of 32 to the four quarters of the SM, shifted by
+//     the column, so matvec and update load the quarters evenly for any number of columns.
+//   - four warps (one per quarter) carry the chain: they receive v and x, form w, and in the
+//     block that owns column k+1 update that column before all others and form its reflector
+//     with one reciprocal square root and one reciprocal; the other columns follow while
+//     the reflector travels.
+//   - x^H v = conj(tau) v^H A22 v has a known phase, so only its real part is summed and
+//     w = x + al v has a real al.
+// A sum's order depends on the matrix alone (rows and pieces), never on the number of
+// blocks: the same bits alone, merged with other matrices or in a cluster.
+// Measured against a grid barrier and a published-reflector wait per column, one warp per column
+// and the reflector by one warp: all eigenvalues of order 791 20.9 -> 13.6 ms, the 20/12/300
+// solve 104.9 -> 93.9 ms, 14/10/230 41.9 -> 36.6 ms.
 constexpr int kTridiagSmemMaxN = 1400;
+constexpr int kTrdRows = (kTridiagSmemMaxN + 127) / 128;   // rows of one of the four chain warps' lanes
+constexpr int kTrdMaxJobs = 32;
 
-// reflector of x[0..m) (x[0] = alpha), by one warp; returns tau, beta, the scale for x[1:]
-__device__ __forceinline__ void warp_reflector(const cplx *x, int m, cplx &tau, double &beta, cplx &scale,
-                                               bool &skip) {
-    const int lane = threadIdx.x & 31;
-    double ss = 0.0;
-    for (int i = 1 + lane; i < m; i += 32) ss += cabs2(x[i]);
-    ss = eig_warp_sum(ss);
-    const cplx alpha = x[0];
-    const double xnorm = sqrt(ss);
-    if (xnorm == 0.0 && alpha.y == 0.0) {
-        tau = mk(0.0, 0.0);
-        beta = alpha.x;
-        scale = mk(1.0, 0.0);
-        skip = true;
-    } else {
-        const double nrm = sqrt(alpha.x * alpha.x + alpha.y * alpha.y + xnorm * xnorm);
-        beta = alpha.x >= 0.0 ? -nrm : nrm;
-        tau = mk((beta - alpha.x) / beta, -alpha.y / beta);
-        scale = cdiv(mk(1.0, 0.0), mk(alpha.x - beta, alpha.y));
-        skip = false;
-    }
-}
-
-// Column k+1 is in this block's shared memory (local slot c): write its reflector (rows k+2..)
-// to A(k+2:, k+1), and d[k+1], e[k+1], tau[k+1].  One warp.  With pub, the warp then raises
-// the published-reflector count to k1 + 1 (release order after every lane's writes).
-__device__ __forceinline__ void publish_reflector(int n, int k1, const cplx *col, cplx *A, int64_t lda, double *d,
-                                                  double *e, cplx *tau, unsigned *pub = nullptr) {
-    const int lane = threadIdx.x & 31;
-    const int m = n - k1 - 1;
-    const cplx *x = col + k1 + 1;
-    cplx t, sc;
-    double beta;
-    bool skip;
-    warp_reflector(x, m, t, beta, sc, skip);
-    cplx *g = A + (k1 + 1) + (int64_t)k1 * lda;
-    for (int i = lane; i < m; i += 32) g[i] = i == 0 ? mk(1.0, 0.0) : (skip ? x[i] : cmul(x[i], sc));
-    if (lane == 0) {
-        tau[k1] = t;
-        e[k1] = beta;
-        d[k1] = col[k1].x;
-    }
-    if (pub) {
-        __threadfence();
-        __syncwarp();
-        if (lane == 0) atomicMax(pub, (unsigned)(k1 + 1));
-    }
-}
-
-// One problem of a batched launch: its matrix, outputs, scratch and the block range
-// [b0, b0 + nb) that reduces it (with its own grid barrier).
+// One problem of a batched launch: its matrix, outputs, exchange buffers and the block range
+// [b0, b0 + nb) that reduces it.
 struct TrdJob {
     cplx *A;
     int64_t lda;
     double *d, *e;
-    cplx *tau, *pbuf;
-    double2 *part;
-    GridBar *gb;
-    int n, b0, nb;
+    cplx *tau;
+    uint4 *ll;      // trd_ll_words(n) words, zero before the launch
+    int n, b0, nb, real;
+};
+struct TrdTable {
+    TrdJob j[kTrdMaxJobs];
+    int njobs;
+    int *err;                      // per job: nonzero when a wait ran out (zero before the launch)
+    unsigned long long limit_ns;   // time limit of one wait
+};
+// exchange words of one problem: by column parity x (2 n), v (2 n) and the header (4)
+__host__ __device__ inline size_t trd_ll_words(int n) { return 8 * (size_t)n + 8; }
+
+// A double with a flag beside each of its halves in one 16-byte word.
+__device__ __forceinline__ void ll_store(uint4 *p, double v, unsigned flag) {
+    asm volatile("st.volatile.global.v4.u32 [%0], {%1, %2, %3, %4};" ::"l"(p), "r"(__double2loint(v)), "r"(flag),
+                 "r"(__double2hiint(v)), "r"(flag)
+                 : "memory");
+}
+__device__ __forceinline__ bool ll_load(const uint4 *p, unsigned flag, double &v) {
+    unsigned lo, f0, hi, f1;
+    asm volatile("ld.volatile.global.v4.u32 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(lo), "=r"(f0), "=r"(hi), "=r"(f1)
+                 : "l"(p)
+                 : "memory");
+    v = __hiloint2double((int)hi, (int)lo);
+    return f0 == flag && f1 == flag;
+}
+
+// A bounded wait of one thread (the clock and the problem's error flag are read every 4 polls).
+struct LlWait {
+    uint64_t t0 = 0;
+    unsigned spins = 0;
+    __device__ __forceinline__ bool give_up(int *err, unsigned long long limit_ns) {
+        if (spins++ == 0) t0 = globaltimer_ns();
+        if ((spins & 3u) != 0) return false;
+        if (*(volatile int *)err) return true;
+        if (globaltimer_ns() - t0 <= limit_ns) return false;
+        atomicExch(err, 1);
+        return true;
+    }
 };
 
-__device__ void tridiag_smem_body(int n, cplx *A, int64_t lda, double *d, double *e, cplx *tau, cplx *pbuf,
-                                  double2 *part, GridBar *gb, const int b, const unsigned nb) {
+// 1/x and 1/sqrt(x) from the hardware's ~2^-22 approximations by one third-order Newton step.
+__device__ __forceinline__ double fast_rcp(double x) {
+    double r;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
+    const double e = fma(-x, r, 1.0);
+    return fma(r, fma(e, e, e), r);
+}
+__device__ __forceinline__ double fast_rsqrt(double x) {
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    const double e = fma(-x * y, y, 1.0);
+    return fma(y, fma(0.375, e, 0.5) * e, y);
+}
+
+// Reflector of the column alpha, x with ss = |x|^2 (LAPACK's documented xLARFG, beta real): tau,
+// beta, the scale of x, and f = -|tau|^2 / (2 Re tau), which turns Re(x^H v) into the
+// coefficient of v in w.
+__device__ __forceinline__ void trd_scalars(cplx alpha, double ss, cplx &tau, double &beta, cplx &scale, double &f) {
+    if (ss == 0.0 && alpha.y == 0.0) {
+        tau = mk(0.0, 0.0);
+        beta = alpha.x;
+        scale = mk(1.0, 0.0);
+        f = 0.0;
+        return;
+    }
+    const double a2 = cabs2(alpha), N2 = a2 + ss;
+    if (N2 > 1e-280 && N2 < 1e280) {
+        const double rs = fast_rsqrt(N2), s = alpha.x >= 0.0 ? -1.0 : 1.0, ib = s * rs;
+        beta = s * (N2 * rs);
+        tau = mk(fma(-alpha.x, ib, 1.0), -alpha.y * ib);
+        const double gx = alpha.x - beta, r = fast_rcp(fma(gx, gx, alpha.y * alpha.y));
+        scale = mk(gx * r, -alpha.y * r);
+        f = -0.5 * cabs2(tau) * fast_rcp(tau.x);
+    } else {   // outside the safe range of the squares: the plain formulas
+        const double nrm = sqrt(N2);
+        beta = alpha.x >= 0.0 ? -nrm : nrm;
+        tau = mk((beta - alpha.x) / beta, -alpha.y / beta);
+        scale = cdiv(mk(1.0, 0.0), mk(alpha.x - beta, alpha.y));
+        f = -0.5 * cabs2(tau) / tau.x;
+    }
+}
+
+__device__ __forceinline__ void chain_sync() { asm volatile("bar.sync 1, 128;" ::: "memory"); }   // the four chain warps
+
+template <bool REAL>
+__device__ void tridiag_smem_body(const TrdJob &J, const int b, int *err, const unsigned long long limit_ns) {
     extern __shared__ cplx tsm2[];
-    __shared__ double red[64];
-    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5, nwb = blockDim.x >> 5;
-    const int nown = (n - b + (int)nb - 1) / (int)nb;   // columns b, b+nb, ...
-    cplx *cols = tsm2;                                    // nown x n
-    cplx *sv = cols + (size_t)nown * n, *sw = sv + n;
-    for (int64_t x = threadIdx.x; x < (int64_t)nown * n; x += blockDim.x) {
-        const int c = (int)(x / n), r = (int)(x % n);
-        cols[x] = A[r + (int64_t)(b + c * (int)nb) * lda];
-    }
-    __syncthreads();
-    if (b == 0 && wib == 0) {
-        if (n >= 2) publish_reflector(n, 0, cols, A, lda, d, e, tau, &gb->pub);
-        else if (lane == 0) d[0] = cols[0].x;
-    }
-    for (int k = 0; k + 1 < n; k++) {
-        // reflector k, published by the owner of column k (the only dependency on the
-        // previous column): a point-to-point wait instead of a second grid barrier.  The
-        // p / partial buffers alternate by parity, so a block that starts column k+1 early
-        // cannot overwrite what a slower block still reads for column k.
-        if (!wait_published(gb, (unsigned)(k + 1))) return;
-        cplx *pb = pbuf + (size_t)(k & 1) * (n + 1);
-        double2 *pt = part + (size_t)(k & 1) * (n + 1);   // per-column terms conj(p_j) v_j
-        const cplx t = ldcg(tau + k);
-        const bool active = (t.x != 0.0 || t.y != 0.0);
-        for (int r = k + 1 + threadIdx.x; r < n; r += blockDim.x) sv[r] = ldcg(A + r + (int64_t)k * lda);
-        __syncthreads();
-        // first owned column index > k
-        const int c0 = k + 1 > b ? (k + 1 - b + (int)nb - 1) / (int)nb : 0;
-        if (active) {
-            for (int c = c0 + wib; c < nown; c += nwb) {
-                const int j = b + c * (int)nb;
-                const cplx *col = cols + (size_t)c * n;
-                double ar = 0.0, ai = 0.0;
-                for (int r = k + 1 + lane; r < n; r += 32) {
-                    const cplx a = col[r], v = sv[r];
-                    ar += a.x * v.x + a.y * v.y;
-                    ai += a.x * v.y - a.y * v.x;
-                }
-                for (int o = 16; o > 0; o >>= 1) {
-                    ar += __shfl_down_sync(0xffffffffu, ar, o);
-                    ai += __shfl_down_sync(0xffffffffu, ai, o);
-                }
-                if (lane == 0) {
-                    const cplx xp = cmul(t, mk(ar, ai));
-                    pb[j] = xp;
-                    const cplx xv = cmul(cconj(xp), sv[j]);
-                    pt[j] = make_double2(xv.x, xv.y);
-                }
-            }
-        }
-        if (!grid_barrier(gb, nb)) return;
-        if (active) {
-            // p^H v summed over the columns in a fixed order (thread stride, then the block
-            // sum): the same bits whatever the number of blocks reducing this matrix
-            double sr = 0.0, si = 0.0;
-            for (int q = k + 1 + threadIdx.x; q < n; q += blockDim.x) {
-                const double2 v = __ldcg(pt + q);
-                sr += v.x;
-                si += v.y;
-            }
-            eig_block_sum2(sr, si, red);
-            const cplx al = cmul(mk(-0.5, 0.0), cmul(t, mk(sr, si)));
-            for (int r = k + 1 + threadIdx.x; r < n; r += blockDim.x) sw[r] = cadd(ldcg(pb + r), cmul(al, sv[r]));
-            __syncthreads();
-        }
-        // update owned columns > k; the warp that owns column k+1 then publishes its reflector
-        for (int c = c0 + wib; c < nown; c += nwb) {
-            const int j = b + c * (int)nb;
-            cplx *col = cols + (size_t)c * n;
-            if (active) {
-                const cplx vj = sv[j], wj = sw[j];
-                for (int r = k + 1 + lane; r < n; r += 32) {
-                    // a -= v_r conj(w_j) + w_r conj(v_j), as eight FMAs
-                    const cplx vr = sv[r], wr = sw[r];
-                    cplx a = col[r];
-                    a.x = fma(-vr.x, wj.x, a.x);
-                    a.x = fma(-vr.y, wj.y, a.x);
-                    a.x = fma(-wr.x, vj.x, a.x);
-                    a.x = fma(-wr.y, vj.y, a.x);
-                    a.y = fma(-vr.y, wj.x, a.y);
-                    a.y = fma(vr.x, wj.y, a.y);
-                    a.y = fma(-wr.y, vj.x, a.y);
-                    a.y = fma(wr.x, vj.y, a.y);
-                    if (r == j) a.y = 0.0;
-                    col[r] = a;
-                }
-                __syncwarp();
-            }
-            if (j == k + 1) {
-                if (k + 2 < n) publish_reflector(n, k + 1, col, A, lda, d, e, tau, &gb->pub);
-                else if (lane == 0) d[k + 1] = col[k + 1].x;
-            }
-        }
-    }
-}
-
-// ---- cluster form (n up to kTridiagClusterMaxN): the same column-cyclic reduction within one
-// thread-block cluster per matrix, the blocks exchanging through distributed shared memory
-// instead of L2.  The owner of column k keeps its reflector and tau in its shared memory;
-// each block keeps the p_j and conj(p_j) v_j of its own columns there; the others read
-// them with loads from the owner's shared-memory window.  The synchronisation (one barrier
-// and one published-reflector wait per column) runs on counters in shared memory, with
-// cluster-scope release and acquire: a few hundred cycles instead of L2 round trips, which
-// set the column time of small matrices in the cooperative form.  The arithmetic and every
-// summation order are those of tridiag_smem_body, so both give the same bits.
-constexpr int kTridiagClusterMaxN = 400;
-
-// generic address of the same shared-memory location in cluster block `rank`
-template <class T>
-__device__ __forceinline__ T *cl_map(T *p, unsigned rank) {
-    return static_cast<T *>(__cluster_map_shared_rank(static_cast<const void *>(p), rank));
-}
-__device__ __forceinline__ void cl_sync_all() {
-    __cluster_barrier_arrive();
-    __cluster_barrier_wait();
-}
-__device__ __forceinline__ unsigned cl_ld_acquire(const unsigned *p) {
-    unsigned v;
-    asm volatile("ld.acquire.cluster.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-    return v;
-}
-__device__ __forceinline__ void cl_max_relaxed(unsigned *p, unsigned x) {
-    asm volatile("red.relaxed.cluster.max.u32 [%0], %1;" ::"l"(p), "r"(x) : "memory");
-}
-__device__ __forceinline__ void cl_fence() { asm volatile("fence.acq_rel.cluster;" ::: "memory"); }
-
-// One thread: wait until *p >= want, bounded like grid_barrier (gb->limit_ns, gb->err).
-__device__ bool cl_wait_geq(const unsigned *p, unsigned want, GridBar *gb) {
-    if ((int)(cl_ld_acquire(p) - want) >= 0) return true;
-    const uint64_t t0 = globaltimer_ns();
-    unsigned spins = 0;
-    while (true) {
-        if ((int)(cl_ld_acquire(p) - want) >= 0) return true;
-        if ((++spins & 15u) == 0) {
-            if (*(volatile int *)&gb->err) return false;
-            if (globaltimer_ns() - t0 > gb->limit_ns) {
-                atomicExch(&gb->err, 1);
-                return false;
-            }
-        }
-    }
-}
-
-// Cluster-wide barrier: every block adds its arrival to the counter of every block (bar, its
-// own shared counter, mapped), then waits on its own copy, so the polling stays in local
-// shared memory instead of loading another block's; `gen` counts the barriers passed.
-__device__ __forceinline__ void cl_add_relaxed(unsigned *p, unsigned x) {
-    asm volatile("red.relaxed.cluster.add.u32 [%0], %1;" ::"l"(p), "r"(x) : "memory");
-}
-__device__ bool cl_barrier(unsigned *bar, unsigned ncta, unsigned gen, GridBar *gb, int *s_ok) {
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        cl_fence();   // the block's writes before the arrivals (one fence, then plain reductions)
-        for (unsigned r = 0; r < ncta; r++) cl_add_relaxed(cl_map(bar, r), 1u);
-        *s_ok = cl_wait_geq(bar, (gen + 1u) * ncta, gb);
-    }
-    __syncthreads();
-    return *s_ok != 0;
-}
-
-// publish_reflector for the cluster form: the reflector also goes to the owner's shared copy
-// vl (indexed by row) and tau to *stau, then the published count k1 + 1 to every block's own
-// counter (pub, mapped per block), where the waiters poll it locally.
-__device__ __forceinline__ void publish_reflector_cl(int n, int k1, const cplx *col, cplx *A, int64_t lda,
-                                                     double *d, double *e, cplx *tau, cplx *vl, cplx *stau,
-                                                     unsigned *pub, unsigned ncta) {
-    const int lane = threadIdx.x & 31;
-    const int m = n - k1 - 1;
-    const cplx *x = col + k1 + 1;
-    cplx t, sc;
-    double beta;
-    bool skip;
-    warp_reflector(x, m, t, beta, sc, skip);
-    cplx *g = A + (k1 + 1) + (int64_t)k1 * lda;
-    for (int i = lane; i < m; i += 32) {
-        const cplx v = i == 0 ? mk(1.0, 0.0) : (skip ? x[i] : cmul(x[i], sc));
-        g[i] = v;
-        vl[k1 + 1 + i] = v;
-    }
-    if (lane == 0) {
-        tau[k1] = t;
-        e[k1] = beta;
-        d[k1] = col[k1].x;
-        *stau = t;
-    }
-    __syncwarp();
-    if (lane == 0) {
-        cl_fence();   // the warp's writes before the counts
-        for (unsigned r = 0; r < ncta; r++) cl_max_relaxed(cl_map(pub, r), (unsigned)(k1 + 1));
-    }
-}
-
-// Dynamic shared memory of one cluster block: two parities of the published reflector and of
-// the block's own p and conj(p) v (compact, by owned column), then v, w and the gathered p and
-// conj(p) v of all columns (10 rows of n complex), then its columns.
-static size_t trd_cluster_bytes(int n, int ncta) { return (size_t)(((n + ncta - 1) / ncta) + 10) * n * sizeof(cplx); }
-
-// Blocks per cluster for an order-n matrix (a function of n alone, so a matrix reduces the
-// same way whichever batch it is in): more blocks share the FP64 work of larger matrices,
-// fewer keep the synchronisation short for small ones.
-static int trd_cluster_ctas(int n) {
-    if (n <= 32) return 1;
-    if (n <= 64) return 4;
-    return 16;   // a GB300 SM retires two FP64 FMAs per clock: the column work needs the blocks
-}
-
-__global__ void __launch_bounds__(TRD_THREADS) tridiag_cluster_kernel(const TrdJob *__restrict__ jobs, int njobs,
-                                                                       int ncta_expect, unsigned smem_bytes,
-                                                                       int *status) {
-    extern __shared__ cplx tsm3[];
-    __shared__ double red[64];
-    __shared__ unsigned s_bar, s_pub;
-    __shared__ cplx s_tau[2];
-    __shared__ int s_ok;
-    const unsigned ncta = __clusterSizeInBlocks();
-    const int b = (int)__clusterRelativeBlockRank();
-    // launch-shape checks, the same for every block of a cluster (none touches another block
-    // before they pass): a cluster of the expected size, a job per cluster, and room for the
-    // job's columns in the dynamic shared memory
-    if ((int)ncta != ncta_expect || gridDim.x != ncta * (unsigned)njobs) {
-        if (threadIdx.x == 0) atomicCAS(status, 0, 1);
-        return;
-    }
-    const TrdJob J = jobs[blockIdx.x / ncta];
-    const int n = J.n, nb = (int)ncta;
-    if (n < 1 || nb > TRD_THREADS / 32 || (size_t)(((n + nb - 1) / nb) + 10) * n * sizeof(cplx) > smem_bytes) {
-        if (threadIdx.x == 0) atomicCAS(status, 0, 2);
-        return;
-    }
+    __shared__ double s_sum[4], s_hdr[3];
+    __shared__ cplx s_alpha;
+    __shared__ int s_fail;
+    const int n = J.n, nb = J.nb;
     cplx *A = J.A;
     const int64_t lda = J.lda;
-    GridBar *gb = J.gb;
-    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5, nwb = blockDim.x >> 5;
+    uint4 *xb = J.ll, *vb = xb + 4 * (size_t)n, *hb = vb + 4 * (size_t)n;   // [parity][n][2], [parity][n][2], [parity][4]
+    const int tid = threadIdx.x, lane = tid & 31, q = (tid >> 5) & 3, s = tid >> 7;   // quarter, and warp within it
+    const bool chain = s == 0;
     const int nown = (n - b + nb - 1) / nb;   // columns b, b+nb, ...
-    // the buffers other blocks read come first, at the same offsets in every block (a mapped
-    // address is the same offset in another block); the block's own columns (a count that
-    // differs between blocks) come last
-    cplx *vloc = tsm3;                        // 2 x n: published reflector by parity
-    cplx *pbl = vloc + 2 * (size_t)n;         // 2 x n: p_j of own column slot c at [par n + c]
-    double2 *ptl = reinterpret_cast<double2 *>(pbl + 2 * (size_t)n);   // 2 x n: conj(p_j) v_j, same
-    cplx *sv = reinterpret_cast<cplx *>(ptl + 2 * (size_t)n), *sw = sv + n;
-    cplx *pall = sw + n;                      // p_j of every column, gathered
-    double2 *ptall = reinterpret_cast<double2 *>(pall + n);   // conj(p_j) v_j of every column
-    cplx *cols = reinterpret_cast<cplx *>(ptall + n);         // nown x n
-    if (threadIdx.x == 0) {
-        s_bar = 0;
-        s_pub = 0;
-    }
-    for (int64_t x = threadIdx.x; x < (int64_t)nown * n; x += blockDim.x) {
+    cplx *cols = tsm2;                         // nown x n
+    cplx *sv = cols + (size_t)nown * n, *sw = sv + n;
+    double *part = reinterpret_cast<double *>(sw + n);   // [nown][4 quarters][2]
+    for (int64_t x = tid; x < (int64_t)nown * n; x += blockDim.x) {
         const int c = (int)(x / n), r = (int)(x % n);
         cols[x] = A[r + (int64_t)(b + c * nb) * lda];
     }
+    if (tid == 0) s_fail = 0;
     __syncthreads();
-    cl_sync_all();   // every block's counters set before any other block touches them
-    unsigned gen = 0;   // cluster barriers passed
-    if (b == 0 && wib == 0) {
-        if (n >= 2) publish_reflector_cl(n, 0, cols, A, lda, J.d, J.e, J.tau, vloc, &s_tau[0], &s_pub, ncta);
-        else if (lane == 0) J.d[0] = cols[0].x;
+    cplx vr[kTrdRows];   // chain warps: the reflector's rows 32 (4 i + q) + lane
+    const int NI = (n + 127) / 128;
+    // Chain warps of the block that owns column k1: subtract the rank-2 term of the previous
+    // column (vr, sw) when upd, then form and publish the reflector of column k1 into vr.
+    auto panel = [&](int k1, bool upd) {
+        const cplx *col = cols + (size_t)((k1 - b) / nb) * n;
+        const int par = k1 & 1;
+        cplx vj = mk(0.0, 0.0), wj = mk(0.0, 0.0);
+        if (upd) {
+            vj = sv[k1];
+            wj = sw[k1];
+        }
+        double ss = 0.0;
+#pragma unroll
+        for (int i = 0; i < kTrdRows; i++) {
+            if (i >= NI) break;
+            const int r = 32 * (4 * i + q) + lane;
+            if (32 * (4 * i + q) + 31 < k1) continue;
+            cplx a = mk(0.0, 0.0);
+            if (r >= k1 && r < n) {
+                a = col[r];
+                if (upd) {
+                    const cplx v = vr[i], w = sw[r];
+                    a.x = fma(-v.x, wj.x, a.x);
+                    a.x = fma(-w.x, vj.x, a.x);
+                    if (!REAL) {
+                        a.x = fma(-v.y, wj.y, a.x);
+                        a.x = fma(-w.y, vj.y, a.x);
+                        a.y = fma(-v.y, wj.x, a.y);
+                        a.y = fma(v.x, wj.y, a.y);
+                        a.y = fma(-w.y, vj.x, a.y);
+                        a.y = fma(w.x, vj.y, a.y);
+                    }
+                }
+                if (r == k1) J.d[k1] = a.x;
+                if (r == k1 + 1) s_alpha = a;
+                if (r <= k1 + 1) a = mk(0.0, 0.0);
+            }
+            vr[i] = a;
+            ss = fma(a.x, a.x, ss);
+            if (!REAL) ss = fma(a.y, a.y, ss);
+        }
+        if (k1 + 1 >= n) return;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+        if (lane == 0) s_sum[q] = ss;
+        chain_sync();
+        ss = (s_sum[0] + s_sum[1]) + (s_sum[2] + s_sum[3]);
+        cplx t, sc;
+        double beta, f;
+        trd_scalars(s_alpha, ss, t, beta, sc, f);
+        uint4 *vo = vb + (size_t)par * 2 * n;
+        const unsigned flag = (unsigned)k1 + 1u;
+#pragma unroll
+        for (int i = 0; i < kTrdRows; i++) {
+            if (i >= NI) break;
+            const int r = 32 * (4 * i + q) + lane;
+            if (r <= k1 || r >= n) continue;
+            const cplx v = r == k1 + 1 ? mk(1.0, 0.0) : (REAL ? mk(vr[i].x * sc.x, 0.0) : cmul(vr[i], sc));
+            vr[i] = v;
+            if (nb > 1) {
+                ll_store(vo + 2 * (size_t)r, v.x, flag);
+                if (!REAL) ll_store(vo + 2 * (size_t)r + 1, v.y, flag);
+            }
+            A[r + (int64_t)k1 * lda] = v;
+        }
+        if (tid == 0) {
+            if (nb > 1) {
+                ll_store(hb + 4 * par, t.x, flag);
+                ll_store(hb + 4 * par + 1, t.y, flag);
+                ll_store(hb + 4 * par + 2, f, flag);
+            }
+            J.tau[k1] = t;
+            J.e[k1] = beta;
+            s_hdr[0] = t.x;   // read after the next __syncthreads
+            s_hdr[1] = t.y;
+            s_hdr[2] = f;
+        }
+    };
+    bool have = false;   // vr and s_hdr already hold this column's reflector
+    if (b == 0 && chain) {
+        panel(0, false);
+        have = true;
     }
     for (int k = 0; k + 1 < n; k++) {
-        const unsigned owner = (unsigned)(k % nb);
-        if (threadIdx.x == 0) s_ok = cl_wait_geq(&s_pub, (unsigned)(k + 1), gb);
-        __syncthreads();
-        if (!s_ok) break;
+        // first owned column index > k.  A block without one leaves: an exchange word is written
+        // again two columns later, when every block still in the loop has answered the column
+        // between (its x is needed for the next reflector), so it has read the old word.
+        const int c0 = k + 1 > b ? (k + 1 - b + nb - 1) / nb : 0;
+        if (c0 >= nown) return;
+        const unsigned flag = (unsigned)k + 1u;
         const int par = k & 1;
-        const cplx t = *cl_map(&s_tau[par], owner);
-        const bool active = (t.x != 0.0 || t.y != 0.0);
-        {
-            const cplx *vr = cl_map(vloc + (size_t)par * n, owner);
-            for (int r = k + 1 + threadIdx.x; r < n; r += blockDim.x) sv[r] = vr[r];
+        bool ok = true;
+        if (chain && !have) {   // the reflector, straight from its words
+            const uint4 *vi = vb + (size_t)par * 2 * n;
+            LlWait wt;
+            unsigned pend = 0;
+#pragma unroll
+            for (int i = 0; i < kTrdRows; i++) {
+                if (i >= NI) break;
+                const int r = 32 * (4 * i + q) + lane;
+                if (r > k && r < n) pend |= 1u << i;
+            }
+            bool hdr = tid < 3;
+            while (pend || hdr) {
+#pragma unroll
+                for (int i = 0; i < kTrdRows; i++) {
+                    if (i >= NI) break;
+                    if (!(pend >> i & 1u)) continue;
+                    const uint4 *p = vi + 2 * (size_t)(32 * (4 * i + q) + lane);
+                    double x, y = 0.0;
+                    bool got = ll_load(p, flag, x);
+                    if (!REAL) got = ll_load(p + 1, flag, y) && got;
+                    if (got) {
+                        vr[i] = mk(x, y);
+                        pend &= ~(1u << i);
+                    }
+                }
+                if (hdr) {
+                    double x;
+                    if (ll_load(hb + 4 * par + tid, flag, x)) {
+                        s_hdr[tid] = x;
+                        hdr = false;
+                    }
+                }
+                if ((pend || hdr) && wt.give_up(err, limit_ns)) {
+                    ok = false;
+                    break;
+                }
+            }
+            if (!ok) s_fail = 1;
+        }
+        __syncthreads();   // the previous column's update is done: sv may change
+        if (chain) {
+#pragma unroll
+            for (int i = 0; i < kTrdRows; i++) {
+                if (i >= NI) break;
+                const int r = 32 * (4 * i + q) + lane;
+                if (r > k && r < n) sv[r] = vr[i];
+            }
         }
         __syncthreads();
-        cplx *pb = pbl + (size_t)par * n;
-        double2 *pt = ptl + (size_t)par * n;
-        const int c0 = k + 1 > b ? (k + 1 - b + nb - 1) / nb : 0;
-        if (active) {
-            for (int c = c0 + wib; c < nown; c += nwb) {
+        if (s_fail) return;   // the only place a block gives up: no thread writes the flag before the next barrier
+        const int p0 = (k + 1) >> 5, pe = (n + 31) >> 5;   // pieces of 32 rows with rows > k
+        // matvec: conj(column) . v over this quarter's pieces, two columns at a time
+        for (int c = c0 + ((s - c0) & 3); c < nown; c += 8) {
+            double a0 = 0.0, a1 = 0.0, a2 = 0.0, a3 = 0.0;
+            const bool two = c + 4 < nown;
+            {
                 const int j = b + c * nb;
                 const cplx *col = cols + (size_t)c * n;
-                double ar = 0.0, ai = 0.0;
-                for (int r = k + 1 + lane; r < n; r += 32) {
-                    const cplx a = col[r], v = sv[r];
-                    ar += a.x * v.x + a.y * v.y;
-                    ai += a.x * v.y - a.y * v.x;
+                for (int p = p0 + ((q - j - p0) & 3); p < pe; p += 4) {
+                    const int r = 32 * p + lane;
+                    if (r > k && r < n) {
+                        const cplx a = col[r], v = sv[r];
+                        a0 = fma(a.x, v.x, a0);
+                        if (!REAL) {
+                            a0 = fma(a.y, v.y, a0);
+                            a1 = fma(a.x, v.y, a1);
+                            a1 = fma(-a.y, v.x, a1);
+                        }
+                    }
                 }
-                for (int o = 16; o > 0; o >>= 1) {
-                    ar += __shfl_down_sync(0xffffffffu, ar, o);
-                    ai += __shfl_down_sync(0xffffffffu, ai, o);
+            }
+            if (two) {
+                const int j = b + (c + 4) * nb;
+                const cplx *col = cols + (size_t)(c + 4) * n;
+                for (int p = p0 + ((q - j - p0) & 3); p < pe; p += 4) {
+                    const int r = 32 * p + lane;
+                    if (r > k && r < n) {
+                        const cplx a = col[r], v = sv[r];
+                        a2 = fma(a.x, v.x, a2);
+                        if (!REAL) {
+                            a2 = fma(a.y, v.y, a2);
+                            a3 = fma(a.x, v.y, a3);
+                            a3 = fma(-a.y, v.x, a3);
+                        }
+                    }
                 }
-                if (lane == 0) {
-                    const cplx xp = cmul(t, mk(ar, ai));
-                    pb[c] = xp;
-                    const cplx xv = cmul(cconj(xp), sv[j]);
-                    pt[c] = make_double2(xv.x, xv.y);
+            }
+            // the four sums over the warp: halves exchanged first, then eighths, so every sum is
+            // added over lane distances 16, 8, 4, 2, 1 whichever column it belongs to
+            const bool hi = lane & 16, lo = lane & 8;
+            double u = hi ? a2 : a0, w = hi ? a3 : a1;
+            if (two) {
+                u += __shfl_xor_sync(0xffffffffu, hi ? a0 : a2, 16);
+                if (!REAL) w += __shfl_xor_sync(0xffffffffu, hi ? a1 : a3, 16);
+            } else {
+                u = a0 + __shfl_xor_sync(0xffffffffu, a0, 16);
+                if (!REAL) w = a1 + __shfl_xor_sync(0xffffffffu, a1, 16);
+            }
+            double y;
+            if (REAL) {
+                y = u + __shfl_xor_sync(0xffffffffu, u, 8);
+            } else {
+                y = lo ? w : u;
+                y += __shfl_xor_sync(0xffffffffu, lo ? u : w, 8);
+            }
+            y += __shfl_xor_sync(0xffffffffu, y, 4);
+            y += __shfl_xor_sync(0xffffffffu, y, 2);
+            y += __shfl_xor_sync(0xffffffffu, y, 1);
+            if ((lane & 7) == 0 && (two || !hi)) part[((size_t)(c + (hi ? 4 : 0)) * 4 + q) * 2 + (lo ? 1 : 0)] = y;
+        }
+        __syncthreads();
+        const double tr = s_hdr[0], ti = s_hdr[1], f = s_hdr[2];
+        if (!chain) {   // x = tau p of the own columns, to every block
+            uint4 *xo = xb + (size_t)par * 2 * n;
+            const int cnt = 2 * (nown - c0);
+            for (int t = tid - 128; t < ((cnt + 31) & ~31); t += (int)blockDim.x - 128) {
+                const int c = c0 + (t >> 1), comp = t & 1;
+                double y = 0.0;
+                if (t < cnt && (!REAL || comp == 0)) {
+                    const double *p = part + (size_t)c * 8 + comp;
+                    y = (p[0] + p[2]) + (p[4] + p[6]);
+                }
+                const double z = REAL ? 0.0 : __shfl_xor_sync(0xffffffffu, y, 1);
+                if (t < cnt) {
+                    const double x = REAL ? (comp ? 0.0 : tr * y) : (comp ? fma(ti, z, tr * y) : fma(-ti, z, tr * y));
+                    const int j = b + c * nb;
+                    if (nb > 1) {
+                        if (!REAL || comp == 0) ll_store(xo + 2 * (size_t)j + comp, x, flag);
+                    } else {
+                        reinterpret_cast<double *>(sw)[2 * j + comp] = x;
+                    }
                 }
             }
         }
-        if (!cl_barrier(&s_bar, ncta, gen++, gb, &s_ok)) break;
-        if (active) {
-            // gather: warp o reads block o's compact values (contiguous, one block per warp)
-            if (wib < nb) {
-                const int o = wib, no = (n - o + nb - 1) / nb;
-                const int co = k + 1 > o ? (k + 1 - o + nb - 1) / nb : 0;
-                const cplx *rpb = cl_map(pb, (unsigned)o);
-                const double2 *rpt = cl_map(pt, (unsigned)o);
-                for (int c = co + lane; c < no; c += 32) {
-                    const int j = o + c * nb;
-                    pall[j] = rpb[c];
-                    ptall[j] = rpt[c];
+        if (nb == 1) __syncthreads();
+        if (chain) {   // gather x, w = x + al v, and the next reflector in its owner
+            const uint4 *xi = xb + (size_t)par * 2 * n;
+            double z = 0.0;
+            if (nb > 1) {
+                LlWait wt;
+                unsigned pend = 0;
+#pragma unroll
+                for (int i = 0; i < kTrdRows; i++) {
+                    if (i >= NI) break;
+                    const int r = 32 * (4 * i + q) + lane;
+                    if (r > k && r < n) pend |= 1u << i;
+                }
+                while (pend) {
+#pragma unroll
+                    for (int i = 0; i < kTrdRows; i++) {
+                        if (i >= NI) break;
+                        if (!(pend >> i & 1u)) continue;
+                        const int r = 32 * (4 * i + q) + lane;
+                        double x, y = 0.0;
+                        bool got = ll_load(xi + 2 * (size_t)r, flag, x);
+                        if (!REAL) got = ll_load(xi + 2 * (size_t)r + 1, flag, y) && got;
+                        if (got) {
+                            sw[r] = mk(x, y);
+                            pend &= ~(1u << i);
+                        }
+                    }
+                    if (pend && wt.give_up(err, limit_ns)) {
+                        s_fail = 1;
+                        break;
+                    }
                 }
             }
-            __syncthreads();
-            double sr = 0.0, si = 0.0;
-            for (int q = k + 1 + threadIdx.x; q < n; q += blockDim.x) {
-                const double2 v = ptall[q];
-                sr += v.x;
-                si += v.y;
+#pragma unroll
+            for (int i = 0; i < kTrdRows; i++) {
+                if (i >= NI) break;
+                const int r = 32 * (4 * i + q) + lane;
+                if (32 * (4 * i + q) + 31 <= k) continue;
+                if (r > k && r < n) {
+                    const cplx x = sw[r];
+                    z = fma(x.x, vr[i].x, z);
+                    if (!REAL) z = fma(x.y, vr[i].y, z);
+                }
             }
-            eig_block_sum2(sr, si, red);
-            const cplx al = cmul(mk(-0.5, 0.0), cmul(t, mk(sr, si)));
-            for (int r = k + 1 + threadIdx.x; r < n; r += blockDim.x) sw[r] = cadd(pall[r], cmul(al, sv[r]));
-            __syncthreads();
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) z += __shfl_xor_sync(0xffffffffu, z, o);
+            if (lane == 0) s_sum[q] = z;
+            chain_sync();
+            const double al = f * ((s_sum[0] + s_sum[1]) + (s_sum[2] + s_sum[3]));
+#pragma unroll
+            for (int i = 0; i < kTrdRows; i++) {
+                if (i >= NI) break;
+                const int r = 32 * (4 * i + q) + lane;
+                if (32 * (4 * i + q) + 31 <= k) continue;
+                if (r > k && r < n) {
+                    cplx x = sw[r];
+                    x.x = fma(al, vr[i].x, x.x);
+                    if (!REAL) x.y = fma(al, vr[i].y, x.y);
+                    sw[r] = x;
+                }
+            }
+            have = b == (k + 1) % nb;
+            if (have) {
+                chain_sync();   // w_{k+1} from its lane, and s_sum free again
+                panel(k + 1, true);
+            }
         }
-        for (int c = c0 + wib; c < nown; c += nwb) {
+        __syncthreads();
+        // update of the other columns, rows > k+1
+        const int c1 = k + 2 > b ? (k + 2 - b + nb - 1) / nb : 0, p1 = (k + 2) >> 5;
+        for (int c = c1 + ((s - c1) & 3); c < nown; c += 4) {
             const int j = b + c * nb;
             cplx *col = cols + (size_t)c * n;
-            if (active) {
-                const cplx vj = sv[j], wj = sw[j];
-                for (int r = k + 1 + lane; r < n; r += 32) {
-                    const cplx vr = sv[r], wr = sw[r];
+            const cplx vj = sv[j], wj = sw[j];
+            for (int p = p1 + ((q - j - p1) & 3); p < pe; p += 4) {
+                const int r = 32 * p + lane;
+                if (r > k + 1 && r < n) {
+                    // a -= v_r conj(w_j) + w_r conj(v_j), as eight FMAs
+                    const cplx v = sv[r], w = sw[r];
                     cplx a = col[r];
-                    a.x = fma(-vr.x, wj.x, a.x);
-                    a.x = fma(-vr.y, wj.y, a.x);
-                    a.x = fma(-wr.x, vj.x, a.x);
-                    a.x = fma(-wr.y, vj.y, a.x);
-                    a.y = fma(-vr.y, wj.x, a.y);
-                    a.y = fma(vr.x, wj.y, a.y);
-                    a.y = fma(-wr.y, vj.x, a.y);
-                    a.y = fma(wr.x, vj.y, a.y);
-                    if (r == j) a.y = 0.0;
+                    a.x = fma(-v.x, wj.x, a.x);
+                    a.x = fma(-w.x, vj.x, a.x);
+                    if (!REAL) {
+                        a.x = fma(-v.y, wj.y, a.x);
+                        a.x = fma(-w.y, vj.y, a.x);
+                        a.y = fma(-v.y, wj.x, a.y);
+                        a.y = fma(v.x, wj.y, a.y);
+                        a.y = fma(-w.y, vj.x, a.y);
+                        a.y = fma(w.x, vj.y, a.y);
+                        if (r == j) a.y = 0.0;
+                    }
                     col[r] = a;
                 }
-                __syncwarp();
-            }
-            if (j == k + 1) {
-                if (k + 2 < n)
-                    publish_reflector_cl(n, k + 1, col, A, lda, J.d, J.e, J.tau, vloc + (size_t)((k + 1) & 1) * n,
-                                         &s_tau[(k + 1) & 1], &s_pub, ncta);
-                else if (lane == 0) J.d[k + 1] = col[k + 1].x;
             }
         }
     }
-    cl_sync_all();   // no block leaves while another may still read its shared memory
 }
 
-// Batched tridiagonalisation: several Hermitian matrices in one cooperative launch, each
-// reduced by its own group of blocks, so the barrier-bound column loops of independent
-// problems overlap instead of running one after another.
-__global__ void __launch_bounds__(TRD_THREADS) tridiag_smem_batched_kernel(const TrdJob *__restrict__ jobs,
-                                                                            int njobs) {
+// Batched tridiagonalisation: several Hermitian matrices in one launch, each reduced by its own
+// group of blocks (all resident at once: a cooperative launch, or a cluster per matrix), so the
+// latency-bound column loops of independent problems overlap instead of running one after
+// another.
+__global__ void __launch_bounds__(TRD_THREADS) tridiag_smem_batched_kernel(const __grid_constant__ TrdTable T) {
     int j = 0;
-    while (j + 1 < njobs && (int)blockIdx.x >= jobs[j + 1].b0) j++;
-    const TrdJob J = jobs[j];
-    tridiag_smem_body(J.n, J.A, J.lda, J.d, J.e, J.tau, J.pbuf, J.part, J.gb, (int)blockIdx.x - J.b0,
-                      (unsigned)J.nb);
+    while (j + 1 < T.njobs && (int)blockIdx.x >= T.j[j + 1].b0) j++;
+    const TrdJob &J = T.j[j];
+    if (J.real) tridiag_smem_body<true>(J, (int)blockIdx.x - J.b0, T.err + j, T.limit_ns);
+    else tridiag_smem_body<false>(J, (int)blockIdx.x - J.b0, T.err + j, T.limit_ns);
 }
 
 // ===================================================================== 2. divide and conquer
@@ -923,15 +900,6 @@ struct DcBufs {
     double *rho;              // per node
     int *status;              // nonzero: a merge met an inconsistent pole order
 };
-
-// 1/x by two Newton steps from the hardware's ~2^-22 approximation: four FP64 operations, where
-// a division is a longer chain on a unit that retires two per clock and SM.
-__device__ __forceinline__ double dc_rcp(double x) {
-    double r;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
-    r = fma(r, fma(-x, r, 1.0), r);
-    return fma(r, fma(-x, r, 1.0), r);
-}
 
 // Sums of four values over groups of G lanes; every lane of a group gets all four.  The first two
 // exchange steps halve the number of values a lane carries, so 32 lanes take six FP64 additions
@@ -1010,7 +978,7 @@ __device__ void dc_secular_root(int k, int j, bool act, const double *dk, const 
     for (int i = gl; i < kk; i += G) {
         const double z2 = zk[i] * zk[i];
         if (last) x += z2;
-        else if (i != j && i != j + 1) x += z2 * dc_rcp((dk[i] - dl) - hg);
+        else if (i != j && i != j + 1) x += z2 * fast_rcp((dk[i] - dl) - hg);
     }
     x = dc_group_sum<G>(x);
     int o = j;
@@ -1029,7 +997,7 @@ __device__ void dc_secular_root(int k, int j, bool act, const double *dk, const 
         // the other terms at the upper end: z_j^2 / c0 is a lower bound of the root there
         double y = 0.0;
         for (int i = gl; i < kk; i += G)
-            if (i != j) y += zk[i] * zk[i] * dc_rcp((dk[i] - dl) - hi);
+            if (i != j) y += zk[i] * zk[i] * fast_rcp((dk[i] - dl) - hi);
         c0 = y;
     }
     {   // uniform shuffle for the groups of both kinds
@@ -1058,13 +1026,13 @@ __device__ void dc_secular_root(int k, int j, bool act, const double *dk, const 
             const int nL = j + 1;
             int i = gl;
             for (; i < nL; i += G) {
-                const double r = dc_rcp((dk[i] - d_o) - tau);
+                const double r = fast_rcp((dk[i] - d_o) - tau);
                 const double t = zk[i] * zk[i] * r;
                 ps += t;
                 dps = fma(t, r, dps);
             }
             for (; i < kk; i += G) {
-                const double r = dc_rcp((dk[i] - d_o) - tau);
+                const double r = fast_rcp((dk[i] - d_o) - tau);
                 const double t = zk[i] * zk[i] * r;
                 ph += t;
                 dph = fma(t, r, dph);
@@ -1262,7 +1230,7 @@ __global__ void __launch_bounds__(128) dc_base_kernel(int n, const double *__res
         if (root) {
             const double dO = dk[s + ord[c]], t = tau[c];
             for (int m = gl; m < k; m += 4) {
-                const double u = zh[s + m] * dc_rcp((dk[s + m] - dO) - t);
+                const double u = zh[s + m] * fast_rcp((dk[s + m] - dO) - t);
                 U[s + m][c] = u;
                 ss = fma(u, u, ss);
             }
@@ -1642,7 +1610,7 @@ __global__ void dc_vec_kernel(int n, int full, int olo, int ohi, DcBufs b) {
         double *u = b.U + s + (int64_t)(s + i) * n;
         double ss = 0.0;
         for (int m = threadIdx.x; m < k; m += blockDim.x) {
-            const double v = b.zh[s + m] * dc_rcp((dk[m] - dO) - t);
+            const double v = b.zh[s + m] * fast_rcp((dk[m] - dO) - t);
             u[m] = v;
             ss = fma(v, v, ss);
         }
@@ -2056,15 +2024,21 @@ static void tridiag_persistent(Context &c, int n, cplx *A, int64_t lda, HeevWork
 }
 
 // Shared-memory tridiagonalisation of several matrices in one cooperative launch (one job = one
-// block group).  Block counts come from a cost model: a job's FP64 work (about 4 n^3 FMAs; a
-// GB300 SM retires ~2 FP64 FMAs per clock) spreads over its blocks while the per-column grid barrier
-// and reflector wait cost more with more blocks; the jobs share the SMs, and blocks go to the job that
-// is currently the slowest.  Returns false (nothing launched) when the jobs do not fit.
-static double trd_cost(int n, int nb) {
-    return 4.0 * (double)n * n * n / (nb * 4.0e9) + 1.4 * n * (3.0e-6 + 0.02e-6 * nb);   // one barrier + one signal
+// block group).  Block counts come from a cost model: a job's FP64 work (12 FMAs per trailing
+// element and column, whole columns per block, on a unit of two FMAs per clock and SM) spreads
+// over its blocks, while every block of a column reads all of its exchanged words; the jobs
+// share the SMs, and blocks go to the job that is currently the slowest.  False (nothing
+// launched) when the jobs do not fit.
+static double trd_cost(const TrdJob &j, int nb) {
+    const double n = j.n, fma = (j.real ? 3.0 : 12.0) / 3.8e9;
+    return fma * (n * n * n / (3.0 * nb) + n * n / 4.0) + n * (3.0e-6 + (nb > 1 ? 1.5e-6 + 0.004e-6 * nb : 0.0));
 }
 
-static size_t trd_bytes_for(int n, int nbk) { return (size_t)(((n + nbk - 1) / nbk) + 2) * n * sizeof(cplx); }
+// v and w, the owned columns and their partial sums
+static size_t trd_bytes_for(int n, int nbk) {
+    const size_t nown = (size_t)(n + nbk - 1) / nbk;
+    return (nown + 2) * n * sizeof(cplx) + nown * 8 * sizeof(double);
+}
 
 // Shared-memory limit of one block of the batched kernel (its static shared memory aside).
 static size_t trd_smem_limit(const Context &c) {
@@ -2081,6 +2055,7 @@ static bool trd_plan(const Context &c, std::vector<TrdJob> &jobs, int &total, si
     const int sms = std::max(1, c.num_sms);
     const size_t limit = trd_smem_limit(c);
     total = 0;
+    if (jobs.size() > (size_t)kTrdMaxJobs) return false;
     for (TrdJob &j : jobs) {
         if (j.n > kTridiagSmemMaxN) return false;
         int nb = 1;
@@ -2090,21 +2065,26 @@ static bool trd_plan(const Context &c, std::vector<TrdJob> &jobs, int &total, si
         total += nb;
     }
     if (total > sms) return false;
-    while (total < sms) {   // give the next block to the slowest job that it helps
-        int best = -1;
+    while (total < sms) {   // give the next blocks to the slowest job that they help
+        int best = -1, add = 1;
         double worst = -1.0;
         for (size_t q = 0; q < jobs.size(); q++) {
             const TrdJob &j = jobs[q];
-            if (j.nb >= j.n || trd_cost(j.n, j.nb + 1) >= trd_cost(j.n, j.nb)) continue;
-            const double cst = trd_cost(j.n, j.nb);
+            // one block pays no exchange, so the second may only pay together with more
+            int up = 0;
+            for (int t : {1, 2, 4, 8, 16})
+                if (up == 0 && j.nb + t <= j.n && total + t <= sms && trd_cost(j, j.nb + t) < trd_cost(j, j.nb)) up = t;
+            if (up == 0) continue;
+            const double cst = trd_cost(j, j.nb);
             if (cst > worst) {
                 worst = cst;
                 best = (int)q;
+                add = up;
             }
         }
         if (best < 0) break;
-        jobs[best].nb++;
-        total++;
+        jobs[best].nb += add;
+        total += add;
     }
     smem = 0;
     int b0 = 0;
@@ -2119,22 +2099,48 @@ static bool trd_plan(const Context &c, std::vector<TrdJob> &jobs, int &total, si
     return per_sm >= 1 && total <= per_sm * sms;
 }
 
-// The cooperative launch of planned jobs on `stream` (their barriers already reset in stream
-// order), then their barrier error flags, read back after the launch completes.
-static std::vector<GridBar> trd_launch(Context &c, std::vector<TrdJob> &jobs, int total, size_t smem,
-                                       cudaStream_t stream, const char *table) {
-    TrdJob *dj = wsget<TrdJob>(c, table, jobs.size());
-    DCG_CUDA(cudaMemcpyAsync(dj, jobs.data(), jobs.size() * sizeof(TrdJob), cudaMemcpyHostToDevice, stream));
-    int nj = (int)jobs.size();
-    void *args[] = {&dj, &nj};
-    DCG_CUDA(cudaLaunchCooperativeKernel((const void *)tridiag_smem_batched_kernel, dim3(total), dim3(TRD_THREADS),
-                                         args, smem, stream));
+// The exchange words of a context's jobs start at zero, in stream order.
+static void trd_clear(Context &c, const std::vector<TrdJob> &jobs) {
+    for (const TrdJob &j : jobs)
+        if (j.nb != 1) DCG_CUDA(cudaMemsetAsync(j.ll, 0, trd_ll_words(j.n) * sizeof(uint4), c.stream));
+}
+
+// The launch of planned jobs on `stream` (their exchange words already cleared in stream order):
+// cooperative, or with ncta > 0 one cluster of ncta blocks per job.  Returns each job's error
+// flag, read back after the launch completes.
+static std::vector<int> trd_launch(Context &c, const std::vector<TrdJob> &jobs, int total, size_t smem,
+                                   cudaStream_t stream, const char *table, int ncta = 0) {
+    const size_t nj = jobs.size();
+    TrdTable T{};
+    for (size_t q = 0; q < nj; q++) T.j[q] = jobs[q];
+    T.njobs = (int)nj;
+    T.limit_ns = c.wait_limit_ns ? c.wait_limit_ns : kBarrierLimitNs;
+    T.err = wsget<int>(c, table, kTrdMaxJobs);
+    int *herr = (int *)c.ws.host(table, kTrdMaxJobs * sizeof(int));
+    DCG_CUDA(cudaMemsetAsync(T.err, 0, nj * sizeof(int), stream));
+    if (ncta > 0) {
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = (unsigned)ncta;
+        at[0].val.clusterDim.y = 1;
+        at[0].val.clusterDim.z = 1;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((unsigned)total);
+        cfg.blockDim = dim3(TRD_THREADS);
+        cfg.dynamicSmemBytes = smem;
+        cfg.stream = stream;
+        cfg.attrs = at;
+        cfg.numAttrs = 1;
+        DCG_CUDA(cudaLaunchKernelEx(&cfg, tridiag_smem_batched_kernel, T));
+    } else {
+        void *args[] = {&T};
+        DCG_CUDA(cudaLaunchCooperativeKernel((const void *)tridiag_smem_batched_kernel, dim3(total), dim3(TRD_THREADS),
+                                             args, smem, stream));
+    }
     DCG_CUDA(cudaGetLastError());
-    std::vector<GridBar> hb(jobs.size());
-    for (size_t q = 0; q < jobs.size(); q++)
-        DCG_CUDA(cudaMemcpyAsync(&hb[q], jobs[q].gb, sizeof(GridBar), cudaMemcpyDeviceToHost, stream));
+    DCG_CUDA(cudaMemcpyAsync(herr, T.err, nj * sizeof(int), cudaMemcpyDeviceToHost, stream));
     DCG_CUDA(cudaStreamSynchronize(stream));
-    return hb;
+    return std::vector<int>(herr, herr + nj);
 }
 
 // ---- merging the reductions of several contexts (the serving loop's slots)
@@ -2187,11 +2193,11 @@ static void coop_run(Context &leader, CoopBatcher &B, std::vector<CoopSub *> &ta
         size_t smem = 0;
         if (!trd_plan(leader, all, total, smem)) throw Error{DCG_E_CUDA, "merged reduction does not fit"};
         for (CoopSub *s : take) DCG_CUDA(cudaStreamWaitEvent(B.stream, s->ready, 0));
-        const std::vector<GridBar> hb = trd_launch(leader, all, total, smem, B.stream, "trd.jobs.joint");
+        const std::vector<int> he = trd_launch(leader, all, total, smem, B.stream, "trd.err.joint");
         size_t q = 0;
         for (CoopSub *s : take) {
             bool err = false;
-            for (size_t k = 0; k < s->jobs.size(); k++, q++) err = err || hb[q].err != 0;
+            for (size_t k = 0; k < s->jobs.size(); k++, q++) err = err || he[q] != 0;
             s->state = err ? 3 : 1;
             s->c->launches++;
         }
@@ -2213,7 +2219,8 @@ static bool tridiag_smem_merged(Context &c, std::vector<TrdJob> &jobs) {
         size_t smem = 0;
         if (!trd_plan(c, alone, total, smem)) return false;
     }
-    for (TrdJob &j : jobs) gridbar_reset(c, j.gb);
+    for (TrdJob &j : jobs) j.nb = 0;   // not planned yet: any block count
+    trd_clear(c, jobs);
     CoopSub me;
     me.c = &c;
     me.jobs = jobs;
@@ -2277,62 +2284,65 @@ static bool tridiag_smem_merged(Context &c, std::vector<TrdJob> &jobs) {
     return true;
 }
 
-// Cluster launch of jobs of order <= kTridiagClusterMaxN that share a cluster shape (ncta
-// blocks each): one cluster per job, no grid-wide synchronisation, so no cooperative launch
-// and no serialisation against other contexts.  False when no cluster of this shape can be
-// resident (the caller then uses the cooperative form).
+// Cluster form (an option, orders up to kTridiagClusterMaxN): the same kernel with one cluster of
+// ncta blocks per matrix instead of a cooperative launch: a cluster's blocks are resident
+// together by definition, so nothing is serialised against other contexts, and a matrix reduces
+// on the same few SMs whatever its company.
+constexpr int kTridiagClusterMaxN = 400;
+
+// Blocks per cluster for an order-n matrix (a function of n alone): more blocks share the FP64
+// work of larger matrices, fewer keep the exchange short for small ones.
+static int trd_cluster_ctas(int n) {
+    if (n <= 32) return 1;
+    if (n <= 64) return 4;
+    return 16;   // a GB300 SM retires two FP64 FMAs per clock: the column work needs the blocks
+}
+
+// Jobs of one cluster shape.  False when no cluster of this shape can be resident (the caller then
+// uses the cooperative form).
 static bool tridiag_cluster_group(Context &c, std::vector<TrdJob> &jobs, int ncta) {
     size_t smem = 0;
-    for (const TrdJob &j : jobs) smem = std::max(smem, trd_cluster_bytes(j.n, ncta));
+    for (size_t q = 0; q < jobs.size(); q++) {
+        smem = std::max(smem, trd_bytes_for(jobs[q].n, ncta));
+        jobs[q].nb = ncta;
+        jobs[q].b0 = ncta * (int)q;
+    }
     const size_t limit = trd_smem_limit(c);
-    if (smem > limit) return false;
+    if (smem > limit || jobs.size() > (size_t)kTrdMaxJobs) return false;
     // the same values from every context and thread (serving slots launch concurrently), so
     // no launch can see another's smaller limit
-    DCG_CUDA(cudaFuncSetAttribute(tridiag_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)limit));
-    DCG_CUDA(cudaFuncSetAttribute(tridiag_cluster_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    DCG_CUDA(cudaFuncSetAttribute(tridiag_smem_batched_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)limit));
+    DCG_CUDA(cudaFuncSetAttribute(tridiag_smem_batched_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeClusterDimension;
     at[0].val.clusterDim.x = (unsigned)ncta;
     at[0].val.clusterDim.y = 1;
     at[0].val.clusterDim.z = 1;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)(ncta * jobs.size()));
+    const int total = ncta * (int)jobs.size();
+    cfg.gridDim = dim3((unsigned)total);
     cfg.blockDim = dim3(TRD_THREADS);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = c.stream;
     cfg.attrs = at;
     cfg.numAttrs = 1;
     int resident = 0;
-    if (cudaOccupancyMaxActiveClusters(&resident, (const void *)tridiag_cluster_kernel, &cfg) != cudaSuccess ||
+    if (cudaOccupancyMaxActiveClusters(&resident, (const void *)tridiag_smem_batched_kernel, &cfg) != cudaSuccess ||
         resident < 1) {
         cudaGetLastError();
         return false;
     }
-    for (const TrdJob &j : jobs) gridbar_reset(c, j.gb);
-    TrdJob *dj = wsget<TrdJob>(c, "trdc.jobs" + std::to_string(ncta), jobs.size());
-    DCG_CUDA(cudaMemcpyAsync(dj, jobs.data(), jobs.size() * sizeof(TrdJob), cudaMemcpyHostToDevice, c.stream));
-    int *st = wsget<int>(c, "trdc.status", 1);
-    DCG_CUDA(cudaMemsetAsync(st, 0, sizeof(int), c.stream));
-    const TrdJob *djc = dj;
-    const int nj = (int)jobs.size();
-    DCG_CUDA(cudaLaunchKernelEx(&cfg, tridiag_cluster_kernel, djc, nj, ncta, (unsigned)smem, st));
-    DCG_LAUNCHED(c);
-    std::vector<GridBar> hb(jobs.size());
-    for (size_t q = 0; q < jobs.size(); q++)
-        DCG_CUDA(cudaMemcpyAsync(&hb[q], jobs[q].gb, sizeof(GridBar), cudaMemcpyDeviceToHost, c.stream));
-    int hst = 0;
-    DCG_CUDA(cudaMemcpyAsync(&hst, st, sizeof(int), cudaMemcpyDeviceToHost, c.stream));
-    DCG_CUDA(cudaStreamSynchronize(c.stream));
-    if (hst) throw Error{DCG_E_CUDA, "tridiagonalisation: cluster launch shape check " + std::to_string(hst)};
-    for (const GridBar &g : hb)
-        if (g.err) throw Error{DCG_E_NUMERIC, "tridiagonalisation: a cluster wait timed out"};
+    trd_clear(c, jobs);
+    const std::vector<int> he = trd_launch(c, jobs, total, smem, c.stream, "trd.err.cluster", ncta);
+    c.launches++;
+    for (int e : he)
+        if (e) throw Error{DCG_E_NUMERIC, "tridiagonalisation: a cluster wait timed out"};
     return true;
 }
 
-// Whether the cluster form takes the matrices it fits (DCG_TRD_CLUSTER=1).  Off by default:
-// on GB300 it measured slower than the cooperative form (the 300 x 300 Fock block 6.4 ms on
-// 16 SMs against 4.35 ms on 63, the B-G batch 1.84 against 1.73 ms): a 16-block cluster
-// carries four times the per-block FP64 work of a column, more than its faster exchange saves.
+// Whether the cluster form takes the matrices it fits (DCG_TRD_CLUSTER=1).  Off by default: a
+// 16-block cluster carries several times the per-block FP64 work of a column of the
+// cooperative form's larger block groups.
 static bool trd_cluster_enabled() {
     static const bool on = [] {
         const char *e = getenv("DCG_TRD_CLUSTER");
@@ -2347,11 +2357,11 @@ static bool tridiag_smem_batched(Context &c, std::vector<TrdJob> &jobs) {
     int total = 0;
     size_t smem = 0;
     if (!trd_plan(c, jobs, total, smem)) return false;
-    for (size_t q = 0; q < jobs.size(); q++) gridbar_reset(c, jobs[q].gb);
-    const std::vector<GridBar> hb = trd_launch(c, jobs, total, smem, c.stream, "trd.jobs");
+    trd_clear(c, jobs);
+    const std::vector<int> he = trd_launch(c, jobs, total, smem, c.stream, "trd.err");
     c.launches++;
-    for (const GridBar &g : hb)
-        if (g.err) throw Error{DCG_E_NUMERIC, "tridiagonalisation: a grid barrier wait timed out"};
+    for (int e : he)
+        if (e) throw Error{DCG_E_NUMERIC, "tridiagonalisation: a grid barrier wait timed out"};
     return true;
 }
 
@@ -2413,10 +2423,9 @@ void heev_values_batched(Context &c, const std::vector<EigJob> &jobs) {
             t.d = hw[q].d;
             t.e = hw[q].e;
             t.tau = hw[q].tau;
-            t.pbuf = wsget<cplx>(c, slot_name("trd.p", j.slot), 2 * ((size_t)j.n + 1));   // two parities
-            t.part = wsget<double2>(c, slot_name("trd.part", j.slot), 2 * ((size_t)j.n + 1));   // two parities
-            t.gb = wsget<GridBar>(c, slot_name("trd.bar", j.slot), 1);
+            t.ll = wsget<uint4>(c, slot_name("trd.ll", j.slot), trd_ll_words(j.n));
             t.n = j.n;
+            t.real = j.real;
             t.b0 = t.nb = 0;
             tj.push_back(t);
             who.push_back(q);
