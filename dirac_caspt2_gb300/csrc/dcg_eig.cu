@@ -1042,10 +1042,12 @@ __device__ void dc_secular_root(int k, int j, bool act, const double *dk, const 
         if (!run) continue;
         const double g = rhoinv + ps + ph;
         const double err = 8.0 * (ph - ps) + rhoinv + fabs(tau) * (dps + dph);
-        if (fabs(g) <= 4.0 * kUnitRoundoff * err * k || hi - lo <= 2.0 * kUnitRoundoff * fmax(fabs(lo), fabs(hi))) {
+        if (hi - lo <= 2.0 * kUnitRoundoff * fmax(fabs(lo), fabs(hi))) {
             run = false;
             continue;
         }
+        // close enough for this step to be the last one: the model's root is quadratically closer
+        if (fabs(g) <= 4.0 * kUnitRoundoff * err * k) run = false;
         if (g < 0.0) lo = tau;
         else hi = tau;
         const double a1 = dps * (dL - tau), s1 = a1 * (dL - tau);
@@ -1059,7 +1061,10 @@ __device__ void dc_secular_root(int k, int j, bool act, const double *dk, const 
         } else {
             y = cc > 0.0 ? fmin(dL + s1 / cc, hi) : NAN;   // the upper end itself is a root when k = 1
         }
-        if (!(y > lo && (y < hi || (last && y == hi)))) y = 0.5 * (lo + hi);
+        if (!(y > lo && (y < hi || (last && y == hi)))) {
+            if (!run) continue;   // the last step stays where it is
+            y = 0.5 * (lo + hi);
+        }
         tau = y;
     }
     if (act) {
