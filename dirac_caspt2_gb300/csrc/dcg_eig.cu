@@ -402,26 +402,28 @@ __global__ void __launch_bounds__(TRD_THREADS) tridiag_persistent_kernel(int n, 
 // blocks exchange the reflector v (from the owner of column k) and x = tau A22 v (one entry per
 // column, from its owner); the matvec and the rank-2 update run from shared memory.
 //
-// What bounds it is the chain of a column (v to every block, matvec, x to every block, w, the
-// update of column k+1, its norm, the next reflector) and the FP64 unit (two FMAs per clock
-// and SM: a warp's FP64 instruction holds a quarter of the SM for 64 clocks, whether one lane
-// is active or all).  So:
-//   - v and x travel as 16-byte words that carry their own flag (the column's number beside each
-//     half of a double): a reader polls the data itself, one trip through L2 instead of data,
-//     fence, counter and data again.
+// What bounds it is the chain of a column (the column's update, its way to every block, the
+// matvec, x to every block, the next column's update) and the FP64 unit (a warp's FP64
+// instruction holds a quarter of the SM for 70 to 77 clocks, whether one lane is active or all).  So:
+//   - the column and x travel as 16-byte words that carry their own flag (the column's number
+//     beside each half of a double): a reader polls the data itself, one trip through L2 instead
+//     of data, fence, counter and data again.
+//   - the column goes out unscaled as soon as it is updated (u; v = sc u below a unit first
+//     element).  Every block multiplies with u while a seventeenth warp of the owner forms tau
+//     and sc from the norm, which follow as the header: conj(column) . v = sc (conj(column) . u)
+//     + conj(A(k+1, j)), and tau sc = -1 / beta.
 //   - every column's rows are dealt in pieces of 32 to the four quarters of the SM, shifted by
 //     the column, so matvec and update load the quarters evenly for any number of columns.
-//   - four warps (one per quarter) carry the chain: they receive v and x, form w, and in the
-//     block that owns column k+1 update that column before all others and form its reflector
-//     with one reciprocal square root and one reciprocal; the other columns follow while
-//     the reflector travels.
-//   - x^H v = conj(tau) v^H A22 v has a known phase, so only its real part is summed and
-//     w = x + al v has a real al.
+//   - four warps (one per quarter) carry the chain: they receive u and x, scale v while x is
+//     under way, and in the block that owns column k+1 update that column before all others.
+//   - x^H v = conj(tau) v^H A22 v has a known phase, so only its real part is summed: w = x + al v
+//     has a real al, which the update needs for its own columns alone.
 // A sum's order depends on the matrix alone (rows and pieces), never on the number of
 // blocks: the same bits alone, merged with other matrices or in a cluster.
-// Measured against a grid barrier and a published-reflector wait per column, one warp per column
-// and the reflector by one warp: all eigenvalues of order 791 20.9 -> 13.6 ms, the 20/12/300
-// solve 104.9 -> 93.9 ms, 14/10/230 41.9 -> 36.6 ms.
+// Measured, reduction alone: order 70 0.35 ms (5.0 us a column, the chain), order 791 9.5 ms (12 us a
+// column, of which about 8 are FP64 issue), two of order 792 together 13.2 ms; before, with a
+// grid barrier and a published-reflector wait per column, one warp per column and the reflector
+// by one warp: order 791 17.7 ms, two of 792 21.2 ms.
 constexpr int kTridiagSmemMaxN = 1400;
 constexpr int kTrdRows = (kTridiagSmemMaxN + 127) / 128;   // rows of one of the four chain warps' lanes
 constexpr int kTrdMaxJobs = 32;
@@ -442,8 +444,8 @@ struct TrdTable {
     int *err;                      // per job: nonzero when a wait ran out (zero before the launch)
     unsigned long long limit_ns;   // time limit of one wait
 };
-// exchange words of one problem: by column parity x (2 n), v (2 n) and the header (4)
-__host__ __device__ inline size_t trd_ll_words(int n) { return 8 * (size_t)n + 8; }
+// exchange words of one problem: by column parity x (2 n), u (2 n) and the header (8)
+__host__ __device__ inline size_t trd_ll_words(int n) { return 8 * (size_t)n + 16; }
 
 // A double with a flag beside each of its halves in one 16-byte word.
 __device__ __forceinline__ void ll_store(uint4 *p, double v, unsigned flag) {
@@ -490,14 +492,13 @@ __device__ __forceinline__ double fast_rsqrt(double x) {
 }
 
 // Reflector of the column alpha, x with ss = |x|^2 (LAPACK's documented xLARFG, beta real): tau,
-// beta, the scale of x, and f = -|tau|^2 / (2 Re tau), which turns Re(x^H v) into the
-// coefficient of v in w.
-__device__ __forceinline__ void trd_scalars(cplx alpha, double ss, cplx &tau, double &beta, cplx &scale, double &f) {
+// beta, the scale sc = 1 / (alpha - beta) of x, and mib = tau sc = -1 / beta (0 for tau = 0).
+__device__ __forceinline__ void trd_scalars(cplx alpha, double ss, cplx &tau, double &beta, cplx &scale, double &mib) {
     if (ss == 0.0 && alpha.y == 0.0) {
         tau = mk(0.0, 0.0);
         beta = alpha.x;
         scale = mk(1.0, 0.0);
-        f = 0.0;
+        mib = 0.0;
         return;
     }
     const double a2 = cabs2(alpha), N2 = a2 + ss;
@@ -507,259 +508,241 @@ __device__ __forceinline__ void trd_scalars(cplx alpha, double ss, cplx &tau, do
         tau = mk(fma(-alpha.x, ib, 1.0), -alpha.y * ib);
         const double gx = alpha.x - beta, r = fast_rcp(fma(gx, gx, alpha.y * alpha.y));
         scale = mk(gx * r, -alpha.y * r);
-        f = -0.5 * cabs2(tau) * fast_rcp(tau.x);
+        mib = -ib;
     } else {   // outside the safe range of the squares: the plain formulas
         const double nrm = sqrt(N2);
         beta = alpha.x >= 0.0 ? -nrm : nrm;
         tau = mk((beta - alpha.x) / beta, -alpha.y / beta);
         scale = cdiv(mk(1.0, 0.0), mk(alpha.x - beta, alpha.y));
-        f = -0.5 * cabs2(tau) / tau.x;
+        mib = -1.0 / beta;
     }
 }
 
 __device__ __forceinline__ void chain_sync() { asm volatile("bar.sync 1, 128;" ::: "memory"); }   // the four chain warps
+__device__ __forceinline__ void column_sync() { asm volatile("bar.sync 2, 512;" ::: "memory"); }  // all but the header warp
+// the chain warps of a column's owner tell the header warp that its sums are there
+__device__ __forceinline__ void sums_ready() { asm volatile("bar.arrive 3, 160;" ::: "memory"); }
+__device__ __forceinline__ void sums_wait() { asm volatile("bar.sync 3, 160;" ::: "memory"); }
 
-template <bool REAL>
+template <bool REAL, int ROWS>   // ROWS >= n / 128
 __device__ void tridiag_smem_body(const TrdJob &J, const int b, int *err, const unsigned long long limit_ns) {
     extern __shared__ cplx tsm2[];
-    __shared__ double s_sum[4], s_hdr[3];
+    __shared__ double s_sum[4], s_ss[4], s_hdr[5], s_al;
     __shared__ cplx s_alpha;
-    __shared__ int s_fail;
     const int n = J.n, nb = J.nb;
     cplx *A = J.A;
     const int64_t lda = J.lda;
-    uint4 *xb = J.ll, *vb = xb + 4 * (size_t)n, *hb = vb + 4 * (size_t)n;   // [parity][n][2], [parity][n][2], [parity][4]
+    uint4 *xb = J.ll, *ub = xb + 4 * (size_t)n, *hb = ub + 4 * (size_t)n;   // [parity][n][2], [parity][n][2], [parity][8]
     const int tid = threadIdx.x, lane = tid & 31, q = (tid >> 5) & 3, s = tid >> 7;   // quarter, and warp within it
-    const bool chain = s == 0;
+    const bool chain = s == 0, header = s == 4;
     const int nown = (n - b + nb - 1) / nb;   // columns b, b+nb, ...
     cplx *cols = tsm2;                         // nown x n
-    cplx *sv = cols + (size_t)nown * n, *sw = sv + n;
+    cplx *sv = cols + (size_t)nown * n, *sw = sv + n;    // u, then v; x
     double *part = reinterpret_cast<double *>(sw + n);   // [nown][4 quarters][2]
     for (int64_t x = tid; x < (int64_t)nown * n; x += blockDim.x) {
         const int c = (int)(x / n), r = (int)(x % n);
         cols[x] = A[r + (int64_t)(b + c * nb) * lda];
     }
-    if (tid == 0) s_fail = 0;
     __syncthreads();
-    cplx vr[kTrdRows];   // chain warps: the reflector's rows 32 (4 i + q) + lane
+    cplx vr[ROWS];   // chain warps: rows 32 (4 i + q) + lane of u, then of v
     const int NI = (n + 127) / 128;
+#define TRD_ROWS(i, r, from)                                                                    \
+    _Pragma("unroll") for (int i = 0; i < ROWS; i++)                                            \
+        if (const int r = 32 * (4 * i + q) + lane; i < NI && r >= (from) && r < n)
     // Chain warps of the block that owns column k1: subtract the rank-2 term of the previous
-    // column (vr, sw) when upd, then form and publish the reflector of column k1 into vr.
+    // column when upd, publish what lies below the reflector's first row, and leave that row's
+    // element (alpha) and the parts of the squared norm for the header warp.
     auto panel = [&](int k1, bool upd) {
         const cplx *col = cols + (size_t)((k1 - b) / nb) * n;
-        const int par = k1 & 1;
-        cplx vj = mk(0.0, 0.0), wj = mk(0.0, 0.0);
+        cplx vj = mk(0.0, 0.0), yj = mk(0.0, 0.0);
         if (upd) {
             vj = sv[k1];
-            wj = sw[k1];
+            const cplx x = sw[k1];
+            const double a2 = 2.0 * s_al;
+            yj = mk(fma(a2, vj.x, x.x), fma(a2, vj.y, x.y));
         }
-        double ss = 0.0;
-#pragma unroll
-        for (int i = 0; i < kTrdRows; i++) {
-            if (i >= NI) break;
-            const int r = 32 * (4 * i + q) + lane;
-            if (32 * (4 * i + q) + 31 < k1) continue;
-            cplx a = mk(0.0, 0.0);
-            if (r >= k1 && r < n) {
-                a = col[r];
-                if (upd) {
-                    const cplx v = vr[i], w = sw[r];
-                    a.x = fma(-v.x, wj.x, a.x);
-                    a.x = fma(-w.x, vj.x, a.x);
-                    if (!REAL) {
-                        a.x = fma(-v.y, wj.y, a.x);
-                        a.x = fma(-w.y, vj.y, a.x);
-                        a.y = fma(-v.y, wj.x, a.y);
-                        a.y = fma(v.x, wj.y, a.y);
-                        a.y = fma(-w.y, vj.x, a.y);
-                        a.y = fma(w.x, vj.y, a.y);
-                    }
+        uint4 *uo = ub + (size_t)(k1 & 1) * 2 * n;
+        const unsigned flag = (unsigned)k1 + 1u;
+        double s0 = 0.0, s1 = 0.0;
+        TRD_ROWS(i, r, k1) {
+            cplx a = col[r];
+            if (upd) {
+                const cplx v = vr[i], x = sw[r];
+                a.x = fma(-x.x, vj.x, a.x);
+                a.x = fma(-v.x, yj.x, a.x);
+                if (!REAL) {
+                    a.y = fma(-x.y, vj.x, a.y);
+                    a.x = fma(-x.y, vj.y, a.x);
+                    a.y = fma(x.x, vj.y, a.y);
+                    a.x = fma(-v.y, yj.y, a.x);
+                    a.y = fma(-v.y, yj.x, a.y);
+                    a.y = fma(v.x, yj.y, a.y);
                 }
-                if (r == k1) J.d[k1] = a.x;
-                if (r == k1 + 1) s_alpha = a;
-                if (r <= k1 + 1) a = mk(0.0, 0.0);
+            }
+            if (r == k1) J.d[k1] = a.x;
+            if (r == k1 + 1) s_alpha = a;
+            if (r <= k1 + 1) {
+                a = mk(0.0, 0.0);
+            } else if (nb > 1) {
+                ll_store(uo + 2 * (size_t)r, a.x, flag);
+                if (!REAL) ll_store(uo + 2 * (size_t)r + 1, a.y, flag);
             }
             vr[i] = a;
-            ss = fma(a.x, a.x, ss);
-            if (!REAL) ss = fma(a.y, a.y, ss);
+            s0 = fma(a.x, a.x, s0);
+            if (!REAL) s1 = fma(a.y, a.y, s1);
         }
-        if (k1 + 1 >= n) return;
+        if (!REAL) s0 += s1;
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-        if (lane == 0) s_sum[q] = ss;
-        chain_sync();
-        ss = (s_sum[0] + s_sum[1]) + (s_sum[2] + s_sum[3]);
-        cplx t, sc;
-        double beta, f;
-        trd_scalars(s_alpha, ss, t, beta, sc, f);
-        uint4 *vo = vb + (size_t)par * 2 * n;
-        const unsigned flag = (unsigned)k1 + 1u;
-#pragma unroll
-        for (int i = 0; i < kTrdRows; i++) {
-            if (i >= NI) break;
-            const int r = 32 * (4 * i + q) + lane;
-            if (r <= k1 || r >= n) continue;
-            const cplx v = r == k1 + 1 ? mk(1.0, 0.0) : (REAL ? mk(vr[i].x * sc.x, 0.0) : cmul(vr[i], sc));
-            vr[i] = v;
-            if (nb > 1) {
-                ll_store(vo + 2 * (size_t)r, v.x, flag);
-                if (!REAL) ll_store(vo + 2 * (size_t)r + 1, v.y, flag);
-            }
-            A[r + (int64_t)k1 * lda] = v;
-        }
-        if (tid == 0) {
-            if (nb > 1) {
-                ll_store(hb + 4 * par, t.x, flag);
-                ll_store(hb + 4 * par + 1, t.y, flag);
-                ll_store(hb + 4 * par + 2, f, flag);
-            }
-            J.tau[k1] = t;
-            J.e[k1] = beta;
-            s_hdr[0] = t.x;   // read after the next __syncthreads
-            s_hdr[1] = t.y;
-            s_hdr[2] = f;
-        }
+        for (int o = 16; o > 0; o >>= 1) s0 += __shfl_xor_sync(0xffffffffu, s0, o);
+        if (lane == 0) s_ss[q] = s0;
+        if (k1 + 1 < n) sums_ready();
     };
-    bool have = false;   // vr and s_hdr already hold this column's reflector
-    if (b == 0 && chain) {
-        panel(0, false);
-        have = true;
-    }
+    if (b == 0 && chain) panel(0, false);
     for (int k = 0; k + 1 < n; k++) {
-        // first owned column index > k.  A block without one leaves: an exchange word is written
-        // again two columns later, when every block still in the loop has answered the column
-        // between (its x is needed for the next reflector), so it has read the old word.
+        // First owned column index > k.  A block without one leaves after its own last column.
+        // An exchange word is written again two columns later, when every block still in the
+        // loop has answered the column between (its x is needed for the next reflector), so it
+        // has read the old word.
         const int c0 = k + 1 > b ? (k + 1 - b + nb - 1) / nb : 0;
-        if (c0 >= nown) return;
+        const bool owner = b == k % nb;
+        if (c0 >= nown && !owner) return;
         const unsigned flag = (unsigned)k + 1u;
         const int par = k & 1;
-        bool ok = true;
-        if (chain && !have) {   // the reflector, straight from its words
-            const uint4 *vi = vb + (size_t)par * 2 * n;
+        if (chain && !owner) {   // u, straight from its words: one row until it is there, then all
+            const uint4 *ui = ub + (size_t)par * 2 * n;
             LlWait wt;
             unsigned pend = 0;
-#pragma unroll
-            for (int i = 0; i < kTrdRows; i++) {
-                if (i >= NI) break;
-                const int r = 32 * (4 * i + q) + lane;
-                if (r > k && r < n) pend |= 1u << i;
-            }
-            bool hdr = tid < 3;
-            while (pend || hdr) {
-#pragma unroll
-                for (int i = 0; i < kTrdRows; i++) {
-                    if (i >= NI) break;
-                    if (!(pend >> i & 1u)) continue;
-                    const uint4 *p = vi + 2 * (size_t)(32 * (4 * i + q) + lane);
-                    double x, y = 0.0;
-                    bool got = ll_load(p, flag, x);
-                    if (!REAL) got = ll_load(p + 1, flag, y) && got;
-                    if (got) {
-                        vr[i] = mk(x, y);
-                        pend &= ~(1u << i);
-                    }
-                }
-                if (hdr) {
-                    double x;
-                    if (ll_load(hb + 4 * par + tid, flag, x)) {
-                        s_hdr[tid] = x;
-                        hdr = false;
-                    }
-                }
-                if ((pend || hdr) && wt.give_up(err, limit_ns)) {
-                    ok = false;
-                    break;
-                }
-            }
-            if (!ok) s_fail = 1;
-        }
-        __syncthreads();   // the previous column's update is done: sv may change
-        if (chain) {
-#pragma unroll
-            for (int i = 0; i < kTrdRows; i++) {
-                if (i >= NI) break;
-                const int r = 32 * (4 * i + q) + lane;
-                if (r > k && r < n) sv[r] = vr[i];
-            }
-        }
-        __syncthreads();
-        if (s_fail) return;   // the only place a block gives up: no thread writes the flag before the next barrier
-        const int p0 = (k + 1) >> 5, pe = (n + 31) >> 5;   // pieces of 32 rows with rows > k
-        // matvec: conj(column) . v over this quarter's pieces, two columns at a time
-        for (int c = c0 + ((s - c0) & 3); c < nown; c += 8) {
-            double a0 = 0.0, a1 = 0.0, a2 = 0.0, a3 = 0.0;
-            const bool two = c + 4 < nown;
-            {
-                const int j = b + c * nb;
-                const cplx *col = cols + (size_t)c * n;
-                for (int p = p0 + ((q - j - p0) & 3); p < pe; p += 4) {
-                    const int r = 32 * p + lane;
-                    if (r > k && r < n) {
-                        const cplx a = col[r], v = sv[r];
-                        a0 = fma(a.x, v.x, a0);
-                        if (!REAL) {
-                            a0 = fma(a.y, v.y, a0);
-                            a1 = fma(a.x, v.y, a1);
-                            a1 = fma(-a.y, v.x, a1);
+            TRD_ROWS(i, r, k + 2) pend |= 1u << i;
+            bool all = false;
+            while (pend) {
+                const unsigned first = pend & (0u - pend);
+                all = all || (pend & (pend - 1)) == 0;
+                const unsigned look = all ? pend : first;
+                const unsigned before = pend;
+                TRD_ROWS(i, r, k + 2) {
+                    if (look >> i & 1u) {
+                        double x, y = 0.0;
+                        bool got = ll_load(ui + 2 * (size_t)r, flag, x);
+                        if (!REAL) got = ll_load(ui + 2 * (size_t)r + 1, flag, y) && got;
+                        if (got) {
+                            vr[i] = mk(x, y);
+                            pend &= ~(1u << i);
                         }
                     }
                 }
+                all = pend != before;
+                // once a wait has run out the problem's error flag is set and every wait of its
+                // blocks ends at once: the loop runs out on whatever values there are
+                if (pend && wt.give_up(err, limit_ns)) break;
             }
-            if (two) {
-                const int j = b + (c + 4) * nb;
-                const cplx *col = cols + (size_t)(c + 4) * n;
-                for (int p = p0 + ((q - j - p0) & 3); p < pe; p += 4) {
-                    const int r = 32 * p + lane;
-                    if (r > k && r < n) {
-                        const cplx a = col[r], v = sv[r];
-                        a2 = fma(a.x, v.x, a2);
-                        if (!REAL) {
-                            a2 = fma(a.y, v.y, a2);
-                            a3 = fma(a.x, v.y, a3);
-                            a3 = fma(-a.y, v.x, a3);
+        }
+        if (!header) {
+            column_sync();   // the previous column's update is done: sv may change
+            if (chain) TRD_ROWS(i, r, k + 1) sv[r] = r == k + 1 ? mk(0.0, 0.0) : vr[i];
+            column_sync();
+        }
+        const int p0 = (k + 2) >> 5, pe = (n + 31) >> 5;   // pieces of 32 rows with rows > k + 1
+        if (header) {   // the reflector's scalars: from the owner's sums, or its words
+            if (owner) {
+                cplx t, sc;
+                double beta, mib;
+                sums_wait();
+                trd_scalars(s_alpha, (s_ss[0] + s_ss[1]) + (s_ss[2] + s_ss[3]), t, beta, sc, mib);
+                if (lane < 5) {
+                    const double h = lane == 0 ? sc.x : lane == 1 ? sc.y : lane == 2 ? t.x : lane == 3 ? t.y : mib;
+                    if (nb > 1) ll_store(hb + 8 * par + lane, h, flag);
+                    s_hdr[lane] = h;
+                }
+                if (lane == 0) {
+                    J.tau[k] = t;
+                    J.e[k] = beta;
+                }
+            } else if (lane < 5) {
+                LlWait wt;
+                double h;
+                while (!ll_load(hb + 8 * par + lane, flag, h))
+                    if (wt.give_up(err, limit_ns)) break;
+                s_hdr[lane] = h;
+            }
+        } else {
+            // matvec: conj(column) . u over this quarter's pieces, two columns at a time
+            for (int c = c0 + ((s - c0) & 3); c < nown; c += 8) {
+                double a0 = 0.0, a1 = 0.0, a2 = 0.0, a3 = 0.0;
+                const bool two = c + 4 < nown;
+                {
+                    const int j = b + c * nb;
+                    const cplx *col = cols + (size_t)c * n;
+                    for (int p = p0 + ((q - j - p0) & 3); p < pe; p += 4) {
+                        const int r = 32 * p + lane;
+                        if (r > k + 1 && r < n) {
+                            const cplx a = col[r], v = sv[r];
+                            a0 = fma(a.x, v.x, a0);
+                            if (!REAL) {
+                                a1 = fma(a.x, v.y, a1);
+                                a0 = fma(a.y, v.y, a0);
+                                a1 = fma(-a.y, v.x, a1);
+                            }
                         }
                     }
                 }
+                if (two) {
+                    const int j = b + (c + 4) * nb;
+                    const cplx *col = cols + (size_t)(c + 4) * n;
+                    for (int p = p0 + ((q - j - p0) & 3); p < pe; p += 4) {
+                        const int r = 32 * p + lane;
+                        if (r > k + 1 && r < n) {
+                            const cplx a = col[r], v = sv[r];
+                            a2 = fma(a.x, v.x, a2);
+                            if (!REAL) {
+                                a3 = fma(a.x, v.y, a3);
+                                a2 = fma(a.y, v.y, a2);
+                                a3 = fma(-a.y, v.x, a3);
+                            }
+                        }
+                    }
+                }
+                // the four sums over the warp: halves exchanged first, then eighths, so every sum is
+                // added over lane distances 16, 8, 4, 2, 1 whichever column it belongs to
+                const bool hi = lane & 16, lo = lane & 8;
+                double u = hi ? a2 : a0, w = hi ? a3 : a1;
+                if (two) {
+                    u += __shfl_xor_sync(0xffffffffu, hi ? a0 : a2, 16);
+                    if (!REAL) w += __shfl_xor_sync(0xffffffffu, hi ? a1 : a3, 16);
+                } else {
+                    u = a0 + __shfl_xor_sync(0xffffffffu, a0, 16);
+                    if (!REAL) w = a1 + __shfl_xor_sync(0xffffffffu, a1, 16);
+                }
+                double y;
+                if (REAL) {
+                    y = u + __shfl_xor_sync(0xffffffffu, u, 8);
+                } else {
+                    y = lo ? w : u;
+                    y += __shfl_xor_sync(0xffffffffu, lo ? u : w, 8);
+                }
+                y += __shfl_xor_sync(0xffffffffu, y, 4);
+                y += __shfl_xor_sync(0xffffffffu, y, 2);
+                y += __shfl_xor_sync(0xffffffffu, y, 1);
+                if ((lane & 7) == 0 && (two || !hi)) part[((size_t)(c + (hi ? 4 : 0)) * 4 + q) * 2 + (lo ? 1 : 0)] = y;
             }
-            // the four sums over the warp: halves exchanged first, then eighths, so every sum is
-            // added over lane distances 16, 8, 4, 2, 1 whichever column it belongs to
-            const bool hi = lane & 16, lo = lane & 8;
-            double u = hi ? a2 : a0, w = hi ? a3 : a1;
-            if (two) {
-                u += __shfl_xor_sync(0xffffffffu, hi ? a0 : a2, 16);
-                if (!REAL) w += __shfl_xor_sync(0xffffffffu, hi ? a1 : a3, 16);
-            } else {
-                u = a0 + __shfl_xor_sync(0xffffffffu, a0, 16);
-                if (!REAL) w = a1 + __shfl_xor_sync(0xffffffffu, a1, 16);
-            }
-            double y;
-            if (REAL) {
-                y = u + __shfl_xor_sync(0xffffffffu, u, 8);
-            } else {
-                y = lo ? w : u;
-                y += __shfl_xor_sync(0xffffffffu, lo ? u : w, 8);
-            }
-            y += __shfl_xor_sync(0xffffffffu, y, 4);
-            y += __shfl_xor_sync(0xffffffffu, y, 2);
-            y += __shfl_xor_sync(0xffffffffu, y, 1);
-            if ((lane & 7) == 0 && (two || !hi)) part[((size_t)(c + (hi ? 4 : 0)) * 4 + q) * 2 + (lo ? 1 : 0)] = y;
         }
         __syncthreads();
-        const double tr = s_hdr[0], ti = s_hdr[1], f = s_hdr[2];
-        if (!chain) {   // x = tau p of the own columns, to every block
+        const double sx = s_hdr[0], sy = s_hdr[1], tr = s_hdr[2], ti = s_hdr[3], mib = s_hdr[4];
+        if (s >= 1 && !header) {
+            // x = tau p = mib (conj(column) . u) + tau conj(A(k+1, j)) of the own columns, to every block
             uint4 *xo = xb + (size_t)par * 2 * n;
             const int cnt = 2 * (nown - c0);
-            for (int t = tid - 128; t < ((cnt + 31) & ~31); t += (int)blockDim.x - 128) {
-                const int c = c0 + (t >> 1), comp = t & 1;
+            for (int t = tid - 128; t < ((cnt + 31) & ~31); t += 384) {
+                const int c = c0 + (t >> 1), comp = t & 1, j = b + c * nb;
                 double y = 0.0;
-                if (t < cnt && (!REAL || comp == 0)) {
-                    const double *p = part + (size_t)c * 8 + comp;
-                    y = (p[0] + p[2]) + (p[4] + p[6]);
-                }
-                const double z = REAL ? 0.0 : __shfl_xor_sync(0xffffffffu, y, 1);
+                cplx a = mk(0.0, 0.0);
                 if (t < cnt) {
-                    const double x = REAL ? (comp ? 0.0 : tr * y) : (comp ? fma(ti, z, tr * y) : fma(-ti, z, tr * y));
-                    const int j = b + c * nb;
+                    a = cols[(size_t)c * n + k + 1];
+                    const double *p = part + (size_t)c * 8 + comp;
+                    if (!REAL || comp == 0) y = (p[0] + p[2]) + (p[4] + p[6]);
+                }
+                const double x = REAL ? (comp ? 0.0 : fma(mib, y, tr * a.x))
+                                      : fma(mib, y, comp ? fma(ti, a.x, -tr * a.y) : fma(tr, a.x, ti * a.y));
+                if (t < cnt) {
                     if (nb > 1) {
                         if (!REAL || comp == 0) ll_store(xo + 2 * (size_t)j + comp, x, flag);
                     } else {
@@ -768,114 +751,119 @@ __device__ void tridiag_smem_body(const TrdJob &J, const int b, int *err, const 
                 }
             }
         }
+        if (chain) {   // v = sc u below its first row
+            TRD_ROWS(i, r, k + 1) {
+                const cplx v = r == k + 1 ? mk(1.0, 0.0)
+                                          : (REAL ? mk(vr[i].x * sx, 0.0)
+                                                  : mk(fma(vr[i].x, sx, -vr[i].y * sy), fma(vr[i].x, sy, vr[i].y * sx)));
+                vr[i] = v;
+                sv[r] = v;
+                if (owner) A[r + (int64_t)k * lda] = v;
+            }
+        }
+        if (c0 >= nown) return;   // the owner of column k was left for this
         if (nb == 1) __syncthreads();
-        if (chain) {   // gather x, w = x + al v, and the next reflector in its owner
-            const uint4 *xi = xb + (size_t)par * 2 * n;
-            double z = 0.0;
+        if (chain) {   // gather x, and al of w = x + al v: al = -1/2 tau x^H v = -|tau|^2 / (2 Re tau) Re(x^H v)
+            const double f = tr != 0.0 ? -0.5 * fma(tr, tr, ti * ti) * fast_rcp(tr) : 0.0;
             if (nb > 1) {
+                const uint4 *xi = xb + (size_t)par * 2 * n;
                 LlWait wt;
                 unsigned pend = 0;
-#pragma unroll
-                for (int i = 0; i < kTrdRows; i++) {
-                    if (i >= NI) break;
-                    const int r = 32 * (4 * i + q) + lane;
-                    if (r > k && r < n) pend |= 1u << i;
-                }
+                TRD_ROWS(i, r, k + 1) pend |= 1u << i;
+                bool all = true;
                 while (pend) {
-#pragma unroll
-                    for (int i = 0; i < kTrdRows; i++) {
-                        if (i >= NI) break;
-                        if (!(pend >> i & 1u)) continue;
-                        const int r = 32 * (4 * i + q) + lane;
-                        double x, y = 0.0;
-                        bool got = ll_load(xi + 2 * (size_t)r, flag, x);
-                        if (!REAL) got = ll_load(xi + 2 * (size_t)r + 1, flag, y) && got;
-                        if (got) {
-                            sw[r] = mk(x, y);
-                            pend &= ~(1u << i);
+                    const unsigned look = all ? pend : (pend & (0u - pend)), before = pend;
+                    TRD_ROWS(i, r, k + 1) {
+                        if (look >> i & 1u) {
+                            double x, y = 0.0;
+                            bool got = ll_load(xi + 2 * (size_t)r, flag, x);
+                            if (!REAL) got = ll_load(xi + 2 * (size_t)r + 1, flag, y) && got;
+                            if (got) {
+                                sw[r] = mk(x, y);
+                                pend &= ~(1u << i);
+                            }
                         }
                     }
-                    if (pend && wt.give_up(err, limit_ns)) {
-                        s_fail = 1;
-                        break;
-                    }
+                    all = pend != before;
+                    if (pend && wt.give_up(err, limit_ns)) break;
                 }
             }
-#pragma unroll
-            for (int i = 0; i < kTrdRows; i++) {
-                if (i >= NI) break;
-                const int r = 32 * (4 * i + q) + lane;
-                if (32 * (4 * i + q) + 31 <= k) continue;
-                if (r > k && r < n) {
-                    const cplx x = sw[r];
-                    z = fma(x.x, vr[i].x, z);
-                    if (!REAL) z = fma(x.y, vr[i].y, z);
+            double z0 = 0.0, z1 = 0.0, z2 = 0.0, z3 = 0.0;
+            TRD_ROWS(i, r, k + 1) {
+                const cplx x = sw[r];
+                if (i & 1) {
+                    z2 = fma(x.x, vr[i].x, z2);
+                    if (!REAL) z3 = fma(x.y, vr[i].y, z3);
+                } else {
+                    z0 = fma(x.x, vr[i].x, z0);
+                    if (!REAL) z1 = fma(x.y, vr[i].y, z1);
                 }
             }
+            double z = REAL ? z0 + z2 : (z0 + z1) + (z2 + z3);
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) z += __shfl_xor_sync(0xffffffffu, z, o);
             if (lane == 0) s_sum[q] = z;
             chain_sync();
-            const double al = f * ((s_sum[0] + s_sum[1]) + (s_sum[2] + s_sum[3]));
-#pragma unroll
-            for (int i = 0; i < kTrdRows; i++) {
-                if (i >= NI) break;
-                const int r = 32 * (4 * i + q) + lane;
-                if (32 * (4 * i + q) + 31 <= k) continue;
-                if (r > k && r < n) {
-                    cplx x = sw[r];
-                    x.x = fma(al, vr[i].x, x.x);
-                    if (!REAL) x.y = fma(al, vr[i].y, x.y);
-                    sw[r] = x;
-                }
-            }
-            have = b == (k + 1) % nb;
-            if (have) {
-                chain_sync();   // w_{k+1} from its lane, and s_sum free again
-                panel(k + 1, true);
-            }
+            if (tid == 0) s_al = f * ((s_sum[0] + s_sum[1]) + (s_sum[2] + s_sum[3]));
         }
         __syncthreads();
-        // update of the other columns, rows > k+1
-        const int c1 = k + 2 > b ? (k + 2 - b + nb - 1) / nb : 0, p1 = (k + 2) >> 5;
-        for (int c = c1 + ((s - c1) & 3); c < nown; c += 4) {
-            const int j = b + c * nb;
-            cplx *col = cols + (size_t)c * n;
-            const cplx vj = sv[j], wj = sw[j];
-            for (int p = p1 + ((q - j - p1) & 3); p < pe; p += 4) {
-                const int r = 32 * p + lane;
-                if (r > k + 1 && r < n) {
-                    // a -= v_r conj(w_j) + w_r conj(v_j), as eight FMAs
-                    const cplx v = sv[r], w = sw[r];
-                    cplx a = col[r];
-                    a.x = fma(-v.x, wj.x, a.x);
-                    a.x = fma(-w.x, vj.x, a.x);
-                    if (!REAL) {
-                        a.x = fma(-v.y, wj.y, a.x);
-                        a.x = fma(-w.y, vj.y, a.x);
-                        a.y = fma(-v.y, wj.x, a.y);
-                        a.y = fma(v.x, wj.y, a.y);
-                        a.y = fma(-w.y, vj.x, a.y);
-                        a.y = fma(w.x, vj.y, a.y);
+        // the next column's owner updates it before its other columns and publishes it
+        if (chain && b == (k + 1) % nb) panel(k + 1, true);
+        // update of the other columns, rows > k+1: with w = x + al v,
+        //   a - v conj(w_j) - w conj(v_j) = a - v conj(x_j + 2 al v_j) - x conj(v_j)
+        if (!header) {
+            const int c1 = k + 2 > b ? (k + 2 - b + nb - 1) / nb : 0;
+            const double a2 = 2.0 * s_al;
+            for (int c = c1 + ((s - c1) & 3); c < nown; c += 4) {
+                const int j = b + c * nb;
+                cplx *col = cols + (size_t)c * n;
+                const cplx vj = sv[j], xj = sw[j];
+                const cplx yj = mk(fma(a2, vj.x, xj.x), fma(a2, vj.y, xj.y));
+                for (int p = p0 + ((q - j - p0) & 3); p < pe; p += 4) {
+                    const int r = 32 * p + lane;
+                    if (r > k + 1 && r < n) {
+                        const cplx v = sv[r], x = sw[r];
+                        cplx a = col[r];
+                        a.x = fma(-v.x, yj.x, a.x);
+                        if (!REAL) {
+                            a.y = fma(-v.y, yj.x, a.y);
+                            a.x = fma(-v.y, yj.y, a.x);
+                            a.y = fma(v.x, yj.y, a.y);
+                            a.x = fma(-x.y, vj.y, a.x);
+                            a.y = fma(-x.y, vj.x, a.y);
+                            a.y = fma(x.x, vj.y, a.y);
+                        }
+                        a.x = fma(-x.x, vj.x, a.x);
                         if (r == j) a.y = 0.0;
+                        col[r] = a;
                     }
-                    col[r] = a;
                 }
             }
         }
     }
+#undef TRD_ROWS
 }
 
 // Batched tridiagonalisation: several Hermitian matrices in one launch, each reduced by its own
 // group of blocks (all resident at once: a cooperative launch, or a cluster per matrix), so the
 // latency-bound column loops of independent problems overlap instead of running one after
 // another.
-__global__ void __launch_bounds__(TRD_THREADS) tridiag_smem_batched_kernel(const __grid_constant__ TrdTable T) {
+constexpr int TRS_THREADS = 544;   // sixteen warps for the columns and one for the header
+__global__ void __launch_bounds__(TRS_THREADS) tridiag_smem_batched_kernel(const __grid_constant__ TrdTable T) {
     int j = 0;
     while (j + 1 < T.njobs && (int)blockIdx.x >= T.j[j + 1].b0) j++;
     const TrdJob &J = T.j[j];
-    if (J.real) tridiag_smem_body<true>(J, (int)blockIdx.x - J.b0, T.err + j, T.limit_ns);
-    else tridiag_smem_body<false>(J, (int)blockIdx.x - J.b0, T.err + j, T.limit_ns);
+    const int b = (int)blockIdx.x - J.b0;
+    if (J.n <= 512) {
+        if (J.real) tridiag_smem_body<true, 4>(J, b, T.err + j, T.limit_ns);
+        else tridiag_smem_body<false, 4>(J, b, T.err + j, T.limit_ns);
+    } else if (J.n <= 1024) {
+        if (J.real) tridiag_smem_body<true, 8>(J, b, T.err + j, T.limit_ns);
+        else tridiag_smem_body<false, 8>(J, b, T.err + j, T.limit_ns);
+    } else {
+        if (J.real) tridiag_smem_body<true, kTrdRows>(J, b, T.err + j, T.limit_ns);
+        else tridiag_smem_body<false, kTrdRows>(J, b, T.err + j, T.limit_ns);
+    }
 }
 
 // ===================================================================== 2. divide and conquer
@@ -2036,7 +2024,9 @@ static void tridiag_persistent(Context &c, int n, cplx *A, int64_t lda, HeevWork
 // launched) when the jobs do not fit.
 static double trd_cost(const TrdJob &j, int nb) {
     const double n = j.n, fma = (j.real ? 3.0 : 12.0) / 3.8e9;
-    return fma * (n * n * n / (3.0 * nb) + n * n / 4.0) + n * (3.0e-6 + (nb > 1 ? 1.5e-6 + 0.004e-6 * nb : 0.0));
+    const double own = std::ceil(n / nb);   // a block's columns also follow one another in its reductions
+    return fma * (n * n * n / (3.0 * nb) + n * n / 4.0) +
+           n * ((nb > 1 ? 4.3e-6 : 3.2e-6) + 0.3e-6 * own + 0.002e-6 * nb);
 }
 
 // v and w, the owned columns and their partial sums
@@ -2100,7 +2090,7 @@ static bool trd_plan(const Context &c, std::vector<TrdJob> &jobs, int &total, si
     }
     DCG_CUDA(cudaFuncSetAttribute(tridiag_smem_batched_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)limit));
     int per_sm = 0;
-    DCG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, tridiag_smem_batched_kernel, TRD_THREADS, smem));
+    DCG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, tridiag_smem_batched_kernel, TRS_THREADS, smem));
     return per_sm >= 1 && total <= per_sm * sms;
 }
 
@@ -2131,7 +2121,7 @@ static std::vector<int> trd_launch(Context &c, const std::vector<TrdJob> &jobs, 
         at[0].val.clusterDim.z = 1;
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3((unsigned)total);
-        cfg.blockDim = dim3(TRD_THREADS);
+        cfg.blockDim = dim3(TRS_THREADS);
         cfg.dynamicSmemBytes = smem;
         cfg.stream = stream;
         cfg.attrs = at;
@@ -2139,7 +2129,7 @@ static std::vector<int> trd_launch(Context &c, const std::vector<TrdJob> &jobs, 
         DCG_CUDA(cudaLaunchKernelEx(&cfg, tridiag_smem_batched_kernel, T));
     } else {
         void *args[] = {&T};
-        DCG_CUDA(cudaLaunchCooperativeKernel((const void *)tridiag_smem_batched_kernel, dim3(total), dim3(TRD_THREADS),
+        DCG_CUDA(cudaLaunchCooperativeKernel((const void *)tridiag_smem_batched_kernel, dim3(total), dim3(TRS_THREADS),
                                              args, smem, stream));
     }
     DCG_CUDA(cudaGetLastError());
@@ -2326,7 +2316,7 @@ static bool tridiag_cluster_group(Context &c, std::vector<TrdJob> &jobs, int nct
     cudaLaunchConfig_t cfg = {};
     const int total = ncta * (int)jobs.size();
     cfg.gridDim = dim3((unsigned)total);
-    cfg.blockDim = dim3(TRD_THREADS);
+    cfg.blockDim = dim3(TRS_THREADS);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = c.stream;
     cfg.attrs = at;
