@@ -175,7 +175,11 @@ static void set_system(Context &c, const dcg_system *s) {
             c.multb_ds[(a - 1) * n + (b - 1)] = MB(b + n, a);   // transpose(MULTB(n+1:2n, 1:n))
         }
     c.h.resize((size_t)c.nmo * c.nmo);
-    for (size_t q = 0; q < c.h.size(); q++) c.h[q] = mk(s->h_re[q], s->h_im[q]);
+    c.sys_real = c.realonly;
+    for (size_t q = 0; q < c.h.size(); q++) {
+        c.h[q] = mk(s->h_re[q], s->h_im[q]);
+        if (s->h_im[q] != 0.0) c.sys_real = false;
+    }
     c.nrec = s->nrec;
 
     DevSystem &d = dev(c);
@@ -297,6 +301,7 @@ static void ivo(Context &c, int nfsym, const double *mo_energy, int nhomo, doubl
 
 static int casci(Context &c, int nroot, double *eigen_out, double *ci_re, double *ci_im, int32_t *ndet_out) {
     if (!c.have_system) throw Error{DCG_E_STATE, "dcg_casci before dcg_set_system"};
+    RealScope real_scope(c);
     DevSystem &d = dev(c);
     c.dets = enumerate_ci(c);
     const int ndet = (int)c.dets.size();
@@ -1415,6 +1420,7 @@ namespace dcg {
 
 static int caspt2(Context &c, uint32_t skip, double e2_sub[8], double sc2_sub[8], double *e0_out, double *et_out) {
     if (!c.have_casci) throw Error{DCG_E_STATE, "dcg_caspt2 before dcg_casci"};
+    RealScope real_scope(c);
     c.gram_cholesky_blocks = 0;
     c.gram_woodbury_blocks = 0;
     DevSystem &d = dev(c);

@@ -141,6 +141,10 @@ struct Context {
     bool have_system = false;
     int ni = 0, na = 0, ns = 0, ne = 0, nmo = 0, nsym = 1, totsym = 1, selectroot = 1;
     bool realonly = false;
+    // the resident system is real throughout (realonly, and no imaginary part in h), and a solve of
+    // it is running: every matrix on the path then has zero imaginary parts, and the FP64
+    // kernels skip them (the same bits at a quarter of the FMAs)
+    bool sys_real = false, real_now = false;
     double eshift = 0.0, ecore = 0.0;
     std::vector<int> multb;   // 2n x 2n column-major
     std::vector<int> irpamo;  // nmo
@@ -183,6 +187,13 @@ struct Context {
         if (e_ != cudaSuccess)                                                          \
             throw ::dcg::Error{DCG_E_CUDA, std::string("kernel launch: ") + cudaGetErrorString(e_)}; \
     } while (0)
+
+// Sets Context::real_now for the lifetime of one solve stage.
+struct RealScope {
+    Context &c;
+    explicit RealScope(Context &cc) : c(cc) { c.real_now = c.sys_real; }
+    ~RealScope() { c.real_now = false; }
+};
 
 inline unsigned grid1d(int64_t n, int block) { return (unsigned)((n + block - 1) / block); }
 
@@ -347,7 +358,6 @@ struct EigJob {
     double *w = nullptr;
     int slot = 0;
     bool tridiag_only = false;   // stop after the reduction: for tridiag_e2 (w is not written)
-    bool real = false;           // every imaginary part is zero: the reduction skips them
 };
 void heev_values_batched(Context &c, const std::vector<EigJob> &jobs);
 void heev_vectors_slot(Context &c, int slot, int n, cplx *A, int64_t lda, int vlo, int vhi, cplx *Z, int64_t ldz);

@@ -1851,7 +1851,7 @@ __global__ void wy_tfactor_kernel(int nbp, const cplx *__restrict__ G, const cpl
 // column their partial dot products meet in double-buffered shared memory, summed in a fixed
 // order.  Columns are independent, and the FP64 work (8 FMAs per row and reflector) spreads
 // over every SM.
-template <int R, int WPC, bool PF>
+template <int R, int WPC, bool PF, bool REAL>
 __global__ void __launch_bounds__(64) backtransform_reg_kernel(int n, const cplx *__restrict__ A, int64_t lda,
                                                                 const cplx *__restrict__ tau,
                                                                 const double *__restrict__ Qt, int vlo, int nvec,
@@ -1895,20 +1895,24 @@ __global__ void __launch_bounds__(64) backtransform_reg_kernel(int n, const cplx
                 }
                 if (i & 1) {   // conj(v) z, two accumulator chains
                     s1r = fma(vv.x, z[i].x, s1r);
-                    s1r = fma(vv.y, z[i].y, s1r);
-                    s1i = fma(vv.x, z[i].y, s1i);
-                    s1i = fma(-vv.y, z[i].x, s1i);
+                    if (!REAL) {
+                        s1r = fma(vv.y, z[i].y, s1r);
+                        s1i = fma(vv.x, z[i].y, s1i);
+                        s1i = fma(-vv.y, z[i].x, s1i);
+                    }
                 } else {
                     s0r = fma(vv.x, z[i].x, s0r);
-                    s0r = fma(vv.y, z[i].y, s0r);
-                    s0i = fma(vv.x, z[i].y, s0i);
-                    s0i = fma(-vv.y, z[i].x, s0i);
+                    if (!REAL) {
+                        s0r = fma(vv.y, z[i].y, s0r);
+                        s0i = fma(vv.x, z[i].y, s0i);
+                        s0i = fma(-vv.y, z[i].x, s0i);
+                    }
                 }
             }
             double sr = s0r + s1r, si = s0i + s1i;
             for (int o = 16; o > 0; o >>= 1) {
                 sr += __shfl_down_sync(0xffffffffu, sr, o);
-                si += __shfl_down_sync(0xffffffffu, si, o);
+                if (!REAL) si += __shfl_down_sync(0xffffffffu, si, o);
             }
             if (WPC == 2) {
                 if (lane == 0) {
@@ -1922,7 +1926,8 @@ __global__ void __launch_bounds__(64) backtransform_reg_kernel(int n, const cplx
                 sr = __shfl_sync(0xffffffffu, sr, 0);
                 si = __shfl_sync(0xffffffffu, si, 0);
             }
-            const double fr = t.x * sr - t.y * si, fi = t.x * si + t.y * sr;   // f = tau (v^H z)
+            // f = tau (v^H z)
+            const double fr = REAL ? t.x * sr : t.x * sr - t.y * si, fi = REAL ? 0.0 : t.x * si + t.y * sr;
 #pragma unroll
             for (int i = 0; i < R; i++) {
                 if (i < i0) continue;
@@ -1934,9 +1939,11 @@ __global__ void __launch_bounds__(64) backtransform_reg_kernel(int n, const cplx
                     vv = (have && r > k && r < n) ? __ldg(vk + r) : mk(0.0, 0.0);
                 }
                 z[i].x = fma(-vv.x, fr, z[i].x);   // z -= v f
-                z[i].x = fma(vv.y, fi, z[i].x);
-                z[i].y = fma(-vv.x, fi, z[i].y);
-                z[i].y = fma(-vv.y, fr, z[i].y);
+                if (!REAL) {
+                    z[i].x = fma(vv.y, fi, z[i].x);
+                    z[i].y = fma(-vv.x, fi, z[i].y);
+                    z[i].y = fma(-vv.y, fr, z[i].y);
+                }
             }
         }
         if (PF) {
@@ -1957,8 +1964,8 @@ __global__ void __launch_bounds__(64) backtransform_reg_kernel(int n, const cplx
 template <int R, int WPC, bool PF>
 static void launch_bt_reg(Context &c, int n, const cplx *A, int64_t lda, const cplx *tau, const double *Qt, int vlo,
                           int nvec, cplx *Z, int64_t ldz) {
-    backtransform_reg_kernel<R, WPC, PF><<<grid1d(nvec, 2 / WPC), 64, 0, c.stream>>>(n, A, lda, tau, Qt, vlo, nvec,
-                                                                                       Z, ldz);
+    auto *kern = c.real_now ? backtransform_reg_kernel<R, WPC, PF, true> : backtransform_reg_kernel<R, WPC, PF, false>;
+    kern<<<grid1d(nvec, 2 / WPC), 64, 0, c.stream>>>(n, A, lda, tau, Qt, vlo, nvec, Z, ldz);
     DCG_LAUNCHED(c);
 }
 
@@ -2420,7 +2427,7 @@ void heev_values_batched(Context &c, const std::vector<EigJob> &jobs) {
             t.tau = hw[q].tau;
             t.ll = wsget<uint4>(c, slot_name("trd.ll", j.slot), trd_ll_words(j.n));
             t.n = j.n;
-            t.real = j.real;
+            t.real = c.real_now;
             t.b0 = t.nb = 0;
             tj.push_back(t);
             who.push_back(q);
@@ -2481,7 +2488,7 @@ void heev_values_batched(Context &c, const std::vector<EigJob> &jobs) {
 // y <- Q^H y for the columns of Y0 (written to Y), Q = H_0 H_1 ... H_{n-2} the reflectors of a
 // tridiagonal reduction (H_k = I - tau_k v_k v_k^H, v_k in column k of A below the diagonal):
 // H_0^H first.  One warp per column, the column in registers (R = ceil(n / 32)).
-template <int R, int WPC>
+template <int R, int WPC, bool REAL>
 __global__ void __launch_bounds__(64) apply_qh_kernel(int n, const cplx *__restrict__ A, int64_t lda,
                                                      const cplx *__restrict__ tau, const cplx *__restrict__ Y0,
                                                      int64_t ldy0, int ncol, cplx *Y, int64_t ldy) {
@@ -2508,12 +2515,12 @@ __global__ void __launch_bounds__(64) apply_qh_kernel(int n, const cplx *__restr
             if (i < i0) continue;
             const int r = lane + 32 * (WPC * i + wsub);
             const cplx vv = (have && r > k && r < n) ? __ldg(vk + r) : mk(0.0, 0.0);
-            sr = fma(vv.x, z[i].x, fma(vv.y, z[i].y, sr));    // conj(v) z
-            si = fma(vv.x, z[i].y, fma(-vv.y, z[i].x, si));
+            sr = fma(vv.x, z[i].x, REAL ? sr : fma(vv.y, z[i].y, sr));    // conj(v) z
+            if (!REAL) si = fma(vv.x, z[i].y, fma(-vv.y, z[i].x, si));
         }
         for (int o = 16; o > 0; o >>= 1) {
             sr += __shfl_xor_sync(0xffffffffu, sr, o);
-            si += __shfl_xor_sync(0xffffffffu, si, o);
+            if (!REAL) si += __shfl_xor_sync(0xffffffffu, si, o);
         }
         if (WPC == 2) {   // the two warps' partial dots, summed in a fixed order
             if (lane == 0) {
@@ -2524,14 +2531,15 @@ __global__ void __launch_bounds__(64) apply_qh_kernel(int n, const cplx *__restr
             sr = part[k & 1][0][0] + part[k & 1][1][0];
             si = part[k & 1][0][1] + part[k & 1][1][1];
         }
-        const double fr = t.x * sr + t.y * si, fi = t.x * si - t.y * sr;   // f = conj(tau) (v^H z)
+        // f = conj(tau) (v^H z)
+        const double fr = REAL ? t.x * sr : t.x * sr + t.y * si, fi = REAL ? 0.0 : t.x * si - t.y * sr;
 #pragma unroll
         for (int i = 0; i < R; i++) {
             if (i < i0) continue;
             const int r = lane + 32 * (WPC * i + wsub);
             const cplx vv = (have && r > k && r < n) ? __ldg(vk + r) : mk(0.0, 0.0);
-            z[i].x = fma(-vv.x, fr, fma(vv.y, fi, z[i].x));   // z -= v f
-            z[i].y = fma(-vv.x, fi, fma(-vv.y, fr, z[i].y));
+            z[i].x = fma(-vv.x, fr, REAL ? z[i].x : fma(vv.y, fi, z[i].x));   // z -= v f
+            if (!REAL) z[i].y = fma(-vv.x, fi, fma(-vv.y, fr, z[i].y));
         }
     }
     if (!have) return;
@@ -2616,15 +2624,17 @@ void tridiag_e2(Context &c, int slot, int n, const cplx *A, int64_t lda, const c
     FamScope fs(c, DCG_FAM_EIG, 8.0 * (double)n * n * nouter);
     // one warp per vector up to 256 rows; above, two warps per vector (twice the warps to hide
     // the per-reflector reduction latency) and the register chunks sized to the rows
-    if (n <= 256) {
-        apply_qh_kernel<8, 1><<<grid1d(nouter, 2), 64, 0, c.stream>>>(n, A, lda, h.tau, VC, ldvc, nouter, Y, n);
-    } else {
-        const unsigned g = (unsigned)nouter;
-        if (n <= 512) apply_qh_kernel<8, 2><<<g, 64, 0, c.stream>>>(n, A, lda, h.tau, VC, ldvc, nouter, Y, n);
-        else if (n <= 768) apply_qh_kernel<12, 2><<<g, 64, 0, c.stream>>>(n, A, lda, h.tau, VC, ldvc, nouter, Y, n);
-        else if (n <= 896) apply_qh_kernel<14, 2><<<g, 64, 0, c.stream>>>(n, A, lda, h.tau, VC, ldvc, nouter, Y, n);
-        else apply_qh_kernel<16, 2><<<g, 64, 0, c.stream>>>(n, A, lda, h.tau, VC, ldvc, nouter, Y, n);
+#define DCG_QH(r, w, g)                                                                                              \
+    {                                                                                                                \
+        auto *kern = c.real_now ? apply_qh_kernel<r, w, true> : apply_qh_kernel<r, w, false>;                        \
+        kern<<<(g), 64, 0, c.stream>>>(n, A, lda, h.tau, VC, ldvc, nouter, Y, n);                                    \
     }
+    if (n <= 256) DCG_QH(8, 1, grid1d(nouter, 2))
+    else if (n <= 512) DCG_QH(8, 2, (unsigned)nouter)
+    else if (n <= 768) DCG_QH(12, 2, (unsigned)nouter)
+    else if (n <= 896) DCG_QH(14, 2, (unsigned)nouter)
+    else DCG_QH(16, 2, (unsigned)nouter)
+#undef DCG_QH
     DCG_LAUNCHED(c);
     const size_t sz = (size_t)n * nouter;
     double *D = wsget<double>(c, slot_name("te2.D", slot), sz);

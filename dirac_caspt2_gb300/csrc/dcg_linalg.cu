@@ -183,6 +183,36 @@ __global__ void __launch_bounds__(256) zgemm_kernel(int m, int n, int k, cplx al
     }
 }
 
+// Element arithmetic of the products below: complex, or real when every imaginary part of the
+// operands is zero (Context::real_now; one FMA a multiply-add instead of four).
+template <bool REAL>
+struct ZArith {
+    using T = cplx;
+    static __device__ __forceinline__ T get(cplx v) { return v; }
+    static __device__ __forceinline__ T zero() { return mk(0.0, 0.0); }
+    static __device__ __forceinline__ void mac(T &acc, T a, T b) { cfma(acc, a, b); }
+    static __device__ __forceinline__ T add(T a, T b) { return cadd(a, b); }
+    // alpha acc (+ beta c)
+    static __device__ __forceinline__ void put(cplx *c, cplx alpha, T acc, cplx beta, bool use_beta) {
+        cplx r = cmul(alpha, acc);
+        if (use_beta) r = cadd(r, cmul(beta, *c));
+        *c = r;
+    }
+};
+template <>
+struct ZArith<true> {
+    using T = double;
+    static __device__ __forceinline__ T get(cplx v) { return v.x; }
+    static __device__ __forceinline__ T zero() { return 0.0; }
+    static __device__ __forceinline__ void mac(T &acc, T a, T b) { acc = fma(a, b, acc); }
+    static __device__ __forceinline__ T add(T a, T b) { return a + b; }
+    static __device__ __forceinline__ void put(cplx *c, cplx alpha, T acc, cplx beta, bool use_beta) {
+        double r = alpha.x * acc;
+        if (use_beta) r = fma(beta.x, c->x, r);
+        *c = mk(r, 0.0);
+    }
+};
+
 // ---- fine-grained products.  A GB300 SM retires about two FP64 FMAs per clock, so a warp's FMA
 // instruction holds its quarter of the SM for 64 clocks and one complex multiply-add of 32
 // outputs for 256: shared-memory and L2 bandwidth are never the limit, padding is.  Here a warp
@@ -210,16 +240,18 @@ __device__ __forceinline__ cplx zf_load(const cplx *__restrict__ X, int64_t ld, 
     return v;
 }
 
-template <int RM, int RN, int KG, int QN>
+template <int RM, int RN, int KG, int QN, bool REAL>
 __global__ void __launch_bounds__(256) zgemm_fine_kernel(int m, int n, int k, int opa, int opb, cplx alpha,
                                                          const cplx *__restrict__ A, int64_t lda, int64_t sa,
                                                          const cplx *__restrict__ B, int64_t ldb, int64_t sb, cplx beta,
                                                          cplx *C, int64_t ldc, int64_t sc, int zoff, int upper) {
     using S = ZfShape<RM, RN, KG, QN>;
+    using Z = ZArith<REAL>;
+    using T = typename Z::T;
     constexpr int BM = S::BM, BN = S::BN, BK = S::BK, NA = S::NA, NB = S::NB;
-    __shared__ cplx As[BK][BM + 1];
-    __shared__ cplx Bs[BK][BN + 1];
-    __shared__ cplx red[KG > 1 ? 8 * 32 * QN : 1];
+    __shared__ T As[BK][BM + 1];
+    __shared__ T Bs[BK][BN + 1];
+    __shared__ T red[KG > 1 ? 8 * 32 * QN : 1];
     const int64_t bz = (int64_t)blockIdx.z + zoff;
     A += bz * sa;
     B += bz * sb;
@@ -236,23 +268,23 @@ __global__ void __launch_bounds__(256) zgemm_fine_kernel(int m, int n, int k, in
 #pragma unroll
     for (int q = 0; q < QN; q++)
         if (rows && n0 + 4 * (rn + RN * q) < n) nq = q + 1;
-    cplx acc[QN];
+    T acc[QN];
 #pragma unroll
-    for (int q = 0; q < QN; q++) acc[q] = mk(0.0, 0.0);
-    cplx pa[NA], pb[NB];
+    for (int q = 0; q < QN; q++) acc[q] = Z::zero();
+    T pa[NA], pb[NB];
     // element e of a chunk: A by rows fastest (N, R) or k fastest (T, C), B the other way round
     auto fetch = [&](int k0) {
 #pragma unroll
         for (int u = 0; u < NA; u++) {
             const int e = tid + 256 * u;
             const int i = ta ? e / BK : e % BM, kk = ta ? e % BK : e / BM;
-            pa[u] = (e < BM * BK && m0 + i < m && k0 + kk < k) ? zf_load(A, lda, m0 + i, k0 + kk, opa, ta) : mk(0.0, 0.0);
+            pa[u] = (e < BM * BK && m0 + i < m && k0 + kk < k) ? Z::get(zf_load(A, lda, m0 + i, k0 + kk, opa, ta)) : Z::zero();
         }
 #pragma unroll
         for (int u = 0; u < NB; u++) {
             const int e = tid + 256 * u;
             const int j = tb ? e % BN : e / BK, kk = tb ? e / BN : e % BK;
-            pb[u] = (e < BN * BK && n0 + j < n && k0 + kk < k) ? zf_load(B, ldb, n0 + j, k0 + kk, opb, !tb) : mk(0.0, 0.0);
+            pb[u] = (e < BN * BK && n0 + j < n && k0 + kk < k) ? Z::get(zf_load(B, ldb, n0 + j, k0 + kk, opb, !tb)) : Z::zero();
         }
     };
     fetch(0);
@@ -273,16 +305,16 @@ __global__ void __launch_bounds__(256) zgemm_fine_kernel(int m, int n, int k, in
         if (nq == QN) {
 #pragma unroll 4
             for (int kk = kg; kk < kend; kk += KG) {
-                const cplx a = As[kk][li];
+                const T a = As[kk][li];
 #pragma unroll
-                for (int q = 0; q < QN; q++) cfma(acc[q], a, Bs[kk][lj + 4 * RN * q]);
+                for (int q = 0; q < QN; q++) Z::mac(acc[q], a, Bs[kk][lj + 4 * RN * q]);
             }
         } else if (nq > 0) {
             for (int kk = kg; kk < kend; kk += KG) {
-                const cplx a = As[kk][li];
+                const T a = As[kk][li];
 #pragma unroll
                 for (int q = 0; q < QN; q++)
-                    if (q < nq) cfma(acc[q], a, Bs[kk][lj + 4 * RN * q]);
+                    if (q < nq) Z::mac(acc[q], a, Bs[kk][lj + 4 * RN * q]);
             }
         }
         __syncthreads();
@@ -294,7 +326,7 @@ __global__ void __launch_bounds__(256) zgemm_fine_kernel(int m, int n, int k, in
         if (kg != 0) return;
         for (int g = 1; g < KG; g++)
 #pragma unroll
-            for (int q = 0; q < QN; q++) acc[q] = cadd(acc[q], red[((w + g) * QN + q) * 32 + lane]);
+            for (int q = 0; q < QN; q++) acc[q] = Z::add(acc[q], red[((w + g) * QN + q) * 32 + lane]);
     }
     const int gi = m0 + li;
     if (gi >= m) return;
@@ -302,11 +334,7 @@ __global__ void __launch_bounds__(256) zgemm_fine_kernel(int m, int n, int k, in
 #pragma unroll
     for (int q = 0; q < QN; q++) {
         const int gj = n0 + lj + 4 * RN * q;
-        if (gj >= n) continue;
-        cplx r = cmul(alpha, acc[q]);
-        const int64_t o = gi + (int64_t)gj * ldc;
-        if (use_beta) r = cadd(r, cmul(beta, C[o]));
-        C[o] = r;
+        if (gj < n) Z::put(C + gi + (int64_t)gj * ldc, alpha, acc[q], beta, use_beta);
     }
 }
 
@@ -318,12 +346,14 @@ __global__ void __launch_bounds__(256) zgemm_fine_kernel(int m, int n, int k, in
 constexpr int SMALL_D = 32, SMALL_G = 8;
 
 // C(m x n) = alpha * A(m x k) * op(B)(k x n) + beta * C, op(B) = B or conj(B); k, n <= SMALL_D.
-template <int OPB>
+template <int OPB, bool REAL>
 __global__ void __launch_bounds__(256) zgemm_rsmall_kernel(int m, int n, int k, cplx alpha, const cplx *__restrict__ A,
                                                            int64_t lda, int64_t sa, const cplx *__restrict__ B,
                                                            int64_t ldb, int64_t sb, cplx beta, cplx *C, int64_t ldc,
                                                            int64_t sc, int z0) {
-    __shared__ cplx Bs[SMALL_D][SMALL_D];
+    using Z = ZArith<REAL>;
+    using T = typename Z::T;
+    __shared__ T Bs[SMALL_D][SMALL_D];
     const int z = z0 + blockIdx.z;
     A += (int64_t)z * sa;
     B += (int64_t)z * sb;
@@ -332,67 +362,64 @@ __global__ void __launch_bounds__(256) zgemm_rsmall_kernel(int m, int n, int k, 
         const int kk = x % k, j = x / k;
         cplx v = B[kk + (int64_t)j * ldb];
         if (OPB == OP_R) v = cconj(v);
-        Bs[kk][j] = v;
+        Bs[kk][j] = Z::get(v);
     }
     __syncthreads();
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const int j0 = threadIdx.y * SMALL_G;
     if (i >= m || j0 >= n) return;
-    cplx acc[SMALL_G];
+    T acc[SMALL_G];
 #pragma unroll
-    for (int q = 0; q < SMALL_G; q++) acc[q] = mk(0.0, 0.0);
+    for (int q = 0; q < SMALL_G; q++) acc[q] = Z::zero();
     for (int kk = 0; kk < k; kk++) {
-        const cplx a = A[i + (int64_t)kk * lda];
+        const T a = Z::get(A[i + (int64_t)kk * lda]);
 #pragma unroll
         for (int q = 0; q < SMALL_G; q++)
-            if (j0 + q < n) cfma(acc[q], a, Bs[kk][j0 + q]);
+            if (j0 + q < n) Z::mac(acc[q], a, Bs[kk][j0 + q]);
     }
     const bool use_beta = (beta.x != 0.0 || beta.y != 0.0);
 #pragma unroll
     for (int q = 0; q < SMALL_G; q++) {
         if (j0 + q >= n) break;
-        const int64_t o = i + (int64_t)(j0 + q) * ldc;
-        cplx r = cmul(alpha, acc[q]);
-        if (use_beta) r = cadd(r, cmul(beta, C[o]));
-        C[o] = r;
+        Z::put(C + i + (int64_t)(j0 + q) * ldc, alpha, acc[q], beta, use_beta);
     }
 }
 
 // C(m x n) = alpha * A^H(m x k) * B(k x n) + beta * C with A (k x m); m, k <= SMALL_D.
+template <bool REAL>
 __global__ void __launch_bounds__(256) zgemm_lsmall_kernel(int m, int n, int k, cplx alpha, const cplx *__restrict__ A,
                                                            int64_t lda, int64_t sa, const cplx *__restrict__ B,
                                                            int64_t ldb, int64_t sb, cplx beta, cplx *C, int64_t ldc,
                                                            int64_t sc, int z0) {
-    __shared__ cplx As[SMALL_D][SMALL_D];   // As[kk][i] = conj(A(kk, i))
+    using Z = ZArith<REAL>;
+    using T = typename Z::T;
+    __shared__ T As[SMALL_D][SMALL_D];   // As[kk][i] = conj(A(kk, i))
     const int z = z0 + blockIdx.z;
     A += (int64_t)z * sa;
     B += (int64_t)z * sb;
     C += (int64_t)z * sc;
     for (int x = threadIdx.x + blockDim.x * threadIdx.y; x < k * m; x += blockDim.x * blockDim.y) {
         const int kk = x % k, i = x / k;
-        As[kk][i] = cconj(A[kk + (int64_t)i * lda]);
+        As[kk][i] = Z::get(cconj(A[kk + (int64_t)i * lda]));
     }
     __syncthreads();
     const int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const int i0 = threadIdx.y * SMALL_G;
     if (j >= n || i0 >= m) return;
-    cplx acc[SMALL_G];
+    T acc[SMALL_G];
 #pragma unroll
-    for (int q = 0; q < SMALL_G; q++) acc[q] = mk(0.0, 0.0);
+    for (int q = 0; q < SMALL_G; q++) acc[q] = Z::zero();
     for (int kk = 0; kk < k; kk++) {
-        const cplx b = B[kk + j * ldb];
+        const T b = Z::get(B[kk + j * ldb]);
 #pragma unroll
         for (int q = 0; q < SMALL_G; q++)
-            if (i0 + q < m) cfma(acc[q], As[kk][i0 + q], b);
+            if (i0 + q < m) Z::mac(acc[q], As[kk][i0 + q], b);
     }
     const bool use_beta = (beta.x != 0.0 || beta.y != 0.0);
 #pragma unroll
     for (int q = 0; q < SMALL_G; q++) {
         if (i0 + q >= m) break;
-        const int64_t o = (i0 + q) + j * ldc;
-        cplx r = cmul(alpha, acc[q]);
-        if (use_beta) r = cadd(r, cmul(beta, C[o]));
-        C[o] = r;
+        Z::put(C + (i0 + q) + j * ldc, alpha, acc[q], beta, use_beta);
     }
 }
 
@@ -410,12 +437,9 @@ static bool zgemm_small(Context &c, Op opa, Op opb, int m, int n, int k, cplx al
         for (int z0 = 0; z0 < batch; z0 += 65535) {
             const int nz = std::min(65535, batch - z0);
             dim3 grid(grid1d(m, bx), 1, nz), block(bx, gy);
-            if (opb == OP_N)
-                zgemm_rsmall_kernel<OP_N><<<grid, block, 0, c.stream>>>(m, n, k, alpha, A, lda, sa, B, ldb, sb, beta, C,
-                                                                        ldc, sc, z0);
-            else
-                zgemm_rsmall_kernel<OP_R><<<grid, block, 0, c.stream>>>(m, n, k, alpha, A, lda, sa, B, ldb, sb, beta, C,
-                                                                        ldc, sc, z0);
+            auto *kern = c.real_now ? zgemm_rsmall_kernel<OP_N, true>
+                         : opb == OP_N ? zgemm_rsmall_kernel<OP_N, false> : zgemm_rsmall_kernel<OP_R, false>;
+            kern<<<grid, block, 0, c.stream>>>(m, n, k, alpha, A, lda, sa, B, ldb, sb, beta, C, ldc, sc, z0);
             DCG_LAUNCHED(c);
         }
         return true;
@@ -426,8 +450,8 @@ static bool zgemm_small(Context &c, Op opa, Op opb, int m, int n, int k, cplx al
         for (int z0 = 0; z0 < batch; z0 += 65535) {
             const int nz = std::min(65535, batch - z0);
             dim3 grid(grid1d(n, bx), 1, nz), block(bx, gy);
-            zgemm_lsmall_kernel<<<grid, block, 0, c.stream>>>(m, n, k, alpha, A, lda, sa, B, ldb, sb, beta, C, ldc, sc,
-                                                              z0);
+            auto *kern = c.real_now ? zgemm_lsmall_kernel<true> : zgemm_lsmall_kernel<false>;
+            kern<<<grid, block, 0, c.stream>>>(m, n, k, alpha, A, lda, sa, B, ldb, sb, beta, C, ldc, sc, z0);
             DCG_LAUNCHED(c);
         }
         return true;
@@ -457,8 +481,8 @@ static void zgemm_launch(Context &c, int m, int n, int k, cplx alpha, const cplx
         dim3 grid(grid1d(m, bm), grid1d(n, bn), nz);
 #define DCG_ZF(t, rm, rn, kg, qn)                                                                                  \
     if (tile == t) {                                                                                               \
-        zgemm_fine_kernel<rm, rn, kg, qn><<<grid, 256, 0, c.stream>>>(m, n, k, OPA, OPB, alpha, A, lda, sa, B, ldb, \
-                                                                      sb, beta, C, ldc, sc, z0, upper);            \
+        auto *kern = c.real_now ? zgemm_fine_kernel<rm, rn, kg, qn, true> : zgemm_fine_kernel<rm, rn, kg, qn, false>; \
+        kern<<<grid, 256, 0, c.stream>>>(m, n, k, OPA, OPB, alpha, A, lda, sa, B, ldb, sb, beta, C, ldc, sc, z0, upper); \
         DCG_LAUNCHED(c);                                                                                           \
         continue;                                                                                                  \
     }
@@ -533,7 +557,7 @@ static void zgemm_splitk_run(Context &c, int m, int n, int k, int nsplit, cplx a
 }
 
 // The tile shape and K split of one FP64 product.  zg_cost estimates a plan's time: the FP64
-// operations of the fullest SM (padding included; two FMAs per clock and SM) plus the latency of
+// operations of the fullest SM (padding included; 1.66 FMAs per clock and SM) plus the latency of
 // a chunk of K per wave and of a launch.  A product whose tiles do not fill the GPU may be split
 // along K into equal chunks of at least 32, computed as one batched GEMM into partial products
 // and reduced in a fixed order.  The cheapest plan by the estimate is candidate 0, used for
@@ -548,7 +572,7 @@ struct ZgPlan {
 };
 
 // Clocks of a plan on `sms` SMs.
-static double zg_cost(int sms, int m, int n, int k, int upper, int batch, int tile, int nsplit) {
+static double zg_cost(int sms, bool real, int m, int n, int k, int upper, int batch, int tile, int nsplit) {
     const int bm = kZgBm[tile], bn = kZgBn[tile];
     const int kc = (k + nsplit - 1) / nsplit;
     const bool fine = tile >= kZgTiles;
@@ -557,7 +581,7 @@ static double zg_cost(int sms, int m, int n, int k, int upper, int batch, int ti
     const double tm = (m + bm - 1) / bm, tn = (n + bn - 1) / bn;
     const double fm = fine ? 8.0 * ((m + 7) / 8) / (bm * tm) : 1.0, fn = fine ? 4.0 * ((n + 3) / 4) / (bn * tn) : 1.0;
     const double kp = fine ? kc : 16.0 * ((kc + 15) / 16);
-    const double work = bm * bn * fm * fn * kp * 4.0 / 2.0;   // clocks of one tile alone on an SM
+    const double work = bm * bn * fm * fn * kp * (real ? 1.0 : 4.0) / 1.66;   // clocks of one tile alone on an SM
     const double blocks = (double)zg_tiles(m, n, tile, upper) * nsplit * batch;
     const double waves = std::ceil(blocks / sms);
     // a tile alone on its SM waits for its loads once per chunk (the fine kernels prefetch)
@@ -571,12 +595,12 @@ static double zg_cost(int sms, int m, int n, int k, int upper, int batch, int ti
 static std::vector<ZgPlan> zg_candidates(Context &c, int m, int n, int k, int upper, int batch) {
     const int sms = std::max(1, c.num_sms);
     std::vector<ZgPlan> all, out;
-    for (int t = 0; t < kZgShapes; t++) {
+    for (int t = c.real_now ? kZgTiles : 0; t < kZgShapes; t++) {   // the coarse kernels are complex only
         const int64_t tiles = zg_tiles(m, n, t, upper);
-        all.push_back({t, 1, zg_cost(sms, m, n, k, upper, batch, t, 1)});
+        all.push_back({t, 1, zg_cost(sms, c.real_now, m, n, k, upper, batch, t, 1)});
         if (batch != 1 || tiles >= 2 * sms) continue;
         for (int p = 2; p <= k / kZgMinChunk && p <= 64; p *= 2)
-            all.push_back({t, p, zg_cost(sms, m, n, k, upper, batch, t, p)});
+            all.push_back({t, p, zg_cost(sms, c.real_now, m, n, k, upper, batch, t, p)});
     }
     std::stable_sort(all.begin(), all.end(), [](const ZgPlan &x, const ZgPlan &y) { return x.cost < y.cost; });
     for (const ZgPlan &p : all)
@@ -597,10 +621,10 @@ static void zgemm_tuned(Context &c, int m, int n, int k, cplx alpha, const cplx 
                         const cplx *B, int64_t ldb, int64_t sb, cplx beta, cplx *C, int64_t ldc, int64_t sc, int batch,
                         int upper) {
     const std::vector<ZgPlan> cand = zg_candidates(c, m, n, k, upper, batch);
-    const TuneKey key{TUNE_ZGEMM, OPA * 8 + OPB, m, n, k, upper + 2 * std::min(batch, 1 << 20)};
+    const TuneKey key{TUNE_ZGEMM, OPA * 8 + OPB + (c.real_now ? 64 : 0), m, n, k, upper + 2 * std::min(batch, 1 << 20)};
     // products under ~1 ms of FP64 work keep the heuristic: their trials would cost more than
     // tuning can return (and a served stream meets many shapes once)
-    const double work = 8.0 * m * n * (double)k * batch;
+    const double work = (c.real_now ? 2.0 : 8.0) * m * n * (double)k * batch;
     const bool trial_ok = beta.x == 0.0 && beta.y == 0.0 && work >= kTuneMinFp64Flops;
     const int pick = autotune(c, key, (int)cand.size(), trial_ok, [&](int q) {
         zgemm_plan_run<OPA, OPB>(c, cand[q], m, n, k, alpha, A, lda, sa, B, ldb, sb, beta, C, ldc, sc, batch, upper);
