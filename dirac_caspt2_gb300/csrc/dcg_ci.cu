@@ -190,36 +190,89 @@ __global__ void casmat_kernel(int ni, int na, int ne, const uint64_t *__restrict
 // the dense kernel does; one with j < i is conj(H(j, i)) computed from det j by the same
 // arithmetic in the same order, so the matrix is Hermitian to the bit (the dense kernel
 // mirrors its upper triangle the same way).
+//
+// Finding a candidate's column dominated both passes (a binary search is log2(ndet) dependent
+// loads, 17 of them at 74,273 determinants, for 5,560 candidates a row): the determinants are
+// kept in an open-addressing table (load at most one half), one or two loads a candidate.  The
+// pairs of a candidate come from a table in shared memory, and the sums of a single over the
+// spinors share tables over the active space: heff (h and the inactive mean field) and jk.
 struct CsrRow {
     int occ[64], vir[64];
+    uint16_t pair[2048];   // (x, y) of the occupied pairs, then of the virtual ones (at most C(63, 2) together)
 };
 
-// <single excitation av <- ro of the source determinant S> (S holds ro, not av): h plus the
-// sum over S's occupied spinors (inactive, then active in increasing order), signed by the
-// excitation's phase.
-__device__ cplx single_elem(int ni, int na, const cplx *__restrict__ h, int nmo, const cplx *__restrict__ g,
-                            uint64_t S, int ro, int av) {
-    const int nmoc = ni + na;
+struct DetTable {
+    const uint64_t *key;   // ~0: empty (no determinant has 64 spinors)
+    const int *val;
+    uint64_t mask;
+};
+__device__ __forceinline__ uint64_t det_slot(uint64_t J, uint64_t mask) { return ((J * 0x9E3779B97F4A7C15ull) >> 24) & mask; }
+__device__ __forceinline__ int64_t det_find(const DetTable &t, uint64_t J) {
+    for (uint64_t q = det_slot(J, t.mask);; q = (q + 1) & t.mask) {   // ends at an empty slot: half of them are
+        const uint64_t x = __ldg(t.key + q);
+        if (x == J) return __ldg(t.val + q);
+        if (x == ~0ull) return -1;
+    }
+}
+__global__ void det_table_kernel(const uint64_t *__restrict__ dets, int ndet, uint64_t *key, int *val, uint64_t mask) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= ndet) return;
+    const uint64_t J = dets[i];
+    for (uint64_t q = det_slot(J, mask);; q = (q + 1) & mask) {
+        const unsigned long long old = atomicCAS(reinterpret_cast<unsigned long long *>(key + q), ~0ull, J);
+        if (old == ~0ull || old == J) {
+            val[q] = i;
+            return;
+        }
+    }
+}
+
+// heff[r + na a] = h(r, a) + sum over the inactive k of (ra|kk) - (rk|ka), and jk[s + na (r + na a)]
+// = (ra|ss) - (rs|sa), r, a, s active.  One thread per (r, a).
+__global__ void csr_tables_kernel(int ni, int na, const cplx *__restrict__ h, int nmo, const cplx *__restrict__ g, cplx *heff,
+                                  cplx *jk) {
+    const int e = blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= na * na) return;
+    const int nmoc = ni + na, ir = ni + e % na, ia = ni + e / na;
 #define GIDX(p, q_, r, s) ((int64_t)(p) + (int64_t)nmoc * ((q_) + (int64_t)nmoc * ((r) + (int64_t)nmoc * (s))))
-    uint64_t J;
-    int ph;
-    exct(S, av, ro, na, J, ph);
-    const int ir = ni + ro, ia = ni + av;
     cplx v = h[ir + (int64_t)nmo * ia];
     for (int k = 0; k < ni; k++) {
         v = cadd(v, g[GIDX(ir, ia, k, k)]);
         v = csub(v, g[GIDX(ir, k, k, ia)]);
     }
+    heff[e] = v;
+    for (int s = 0; s < na; s++) {
+        const int is = ni + s;
+        jk[s + (int64_t)na * e] = csub(g[GIDX(ir, ia, is, is)], g[GIDX(ir, is, is, ia)]);
+    }
+}
+
+struct CsrTables {
+    const cplx *heff, *jk;
+    DetTable dt;
+};
+
+// <single excitation av <- ro of the source determinant S> (S holds ro, not av): heff plus jk over
+// S's occupied active spinors in increasing order, signed by the excitation's phase.
+template <bool REAL>
+__device__ cplx single_elem(int na, const CsrTables &t, uint64_t S, int ro, int av) {
+    uint64_t J;
+    int ph;
+    exct(S, av, ro, na, J, ph);
+    const int64_t e = ro + (int64_t)na * av;
+    const cplx *jk = t.jk + na * e;
+    cplx v = t.heff[e];
     for (uint64_t B = S; B; B &= B - 1) {
-        const int s2 = ni + __ffsll((long long)B) - 1;
-        v = cadd(v, g[GIDX(ir, ia, s2, s2)]);
-        v = csub(v, g[GIDX(ir, s2, s2, ia)]);
+        const cplx x = __ldg(jk + __ffsll((long long)B) - 1);
+        v.x += x.x;
+        if (!REAL) v.y += x.y;
     }
     if (ph & 1) v = mk(-v.x, -v.y);
     return v;
 }
 
 // <double excitation a <- r, b <- s of S> (r < s occupied, a < b empty).
+template <bool REAL>
 __device__ cplx double_elem(int ni, int na, const cplx *__restrict__ g, uint64_t S, int r_, int s_, int a_, int b_) {
     const int nmoc = ni + na;
     uint64_t J1, J2;
@@ -227,7 +280,8 @@ __device__ cplx double_elem(int ni, int na, const cplx *__restrict__ g, uint64_t
     exct(S, a_, r_, na, J1, p1);
     exct(J1, b_, s_, na, J2, p2);
     const int ir = ni + r_, is = ni + s_, ia = ni + a_, ib = ni + b_;
-    cplx v = csub(g[GIDX(ir, ia, is, ib)], g[GIDX(ir, ib, is, ia)]);
+    const cplx *x = g + GIDX(ir, ia, is, ib), *y = g + GIDX(ir, ib, is, ia);
+    cplx v = REAL ? mk(__ldg(&x->x) - __ldg(&y->x), 0.0) : csub(__ldg(x), __ldg(y));
     if ((p1 + p2) & 1) v = mk(-v.x, -v.y);
     return v;
 #undef GIDX
@@ -235,10 +289,9 @@ __device__ cplx double_elem(int ni, int na, const cplx *__restrict__ g, uint64_t
 
 // Candidate q of row i (determinant I): false when the excitation vanishes or leaves the CI
 // space; else its column and (WANT_VAL) its element.
-template <bool WANT_VAL>
-__device__ bool casmat_candidate(int ni, int na, int ne, const uint64_t *__restrict__ dets, int ndet,
-                                 const cplx *__restrict__ h, int nmo, const cplx *__restrict__ g, int64_t i,
-                                 uint64_t I, const CsrRow &rw, int64_t q, int64_t &jout, cplx &vout) {
+template <bool WANT_VAL, bool REAL>
+__device__ bool casmat_candidate(int ni, int na, int ne, const CsrTables &t, const cplx *__restrict__ g, int64_t i, uint64_t I,
+                                 const CsrRow &rw, int64_t q, int64_t &jout, cplx &vout) {
     const int nv = na - ne;
     const int64_t nsing = (int64_t)ne * nv;
     if (q < nsing) {
@@ -246,58 +299,41 @@ __device__ bool casmat_candidate(int ni, int na, int ne, const uint64_t *__restr
         uint64_t J;
         int ph;
         if (!exct(I, av, ro, na, J, ph)) return false;
-        const int64_t j = find_sorted(dets, ndet, J);
+        const int64_t j = det_find(t.dt, J);
         if (j < 0) return false;
         jout = j;
-        if (WANT_VAL) vout = j > i ? single_elem(ni, na, h, nmo, g, I, ro, av) : cconj(single_elem(ni, na, h, nmo, g, J, av, ro));
+        if (WANT_VAL) vout = j > i ? single_elem<REAL>(na, t, I, ro, av) : cconj(single_elem<REAL>(na, t, J, av, ro));
         return true;
     }
     q -= nsing;
-    const int npv = nv * (nv - 1) / 2;
-    const int po = (int)(q / npv), pv = (int)(q % npv);
-    int x = 0, y = 0, u = 0, w2 = 0;
-    {
-        int cnt = po;
-        for (x = 0; x < ne; x++) {
-            const int rem = ne - 1 - x;
-            if (cnt < rem) {
-                y = x + 1 + cnt;
-                break;
-            }
-            cnt -= rem;
-        }
-    }
-    {
-        int cnt = pv;
-        for (u = 0; u < nv; u++) {
-            const int rem = nv - 1 - u;
-            if (cnt < rem) {
-                w2 = u + 1 + cnt;
-                break;
-            }
-            cnt -= rem;
-        }
-    }
-    const int r_ = rw.occ[x], s_ = rw.occ[y], a_ = rw.vir[u], b_ = rw.vir[w2];
-    uint64_t J1, J2;
-    int p1, p2;
-    if (!exct(I, a_, r_, na, J1, p1)) return false;
-    if (!exct(J1, b_, s_, na, J2, p2)) return false;
-    const int64_t j = find_sorted(dets, ndet, J2);
+    const int npv = nv * (nv - 1) / 2, npo = ne * (ne - 1) / 2;
+    const unsigned po = rw.pair[(int)(q / npv)], pv = rw.pair[npo + (int)(q % npv)];
+    const int r_ = rw.occ[po & 255u], s_ = rw.occ[po >> 8], a_ = rw.vir[pv & 255u], b_ = rw.vir[pv >> 8];
+    // r < s occupied and a < b empty: the excited determinant is known without the phases
+    const uint64_t J2 = I ^ (1ull << r_) ^ (1ull << s_) ^ (1ull << a_) ^ (1ull << b_);
+    const int64_t j = det_find(t.dt, J2);
     if (j < 0) return false;
     jout = j;
     // from det j the occupied pair is (a, b) and the empty pair (r, s), both increasing
-    if (WANT_VAL) vout = j > i ? double_elem(ni, na, g, I, r_, s_, a_, b_) : cconj(double_elem(ni, na, g, J2, a_, b_, r_, s_));
+    if (WANT_VAL)
+        vout = j > i ? double_elem<REAL>(ni, na, g, I, r_, s_, a_, b_) : cconj(double_elem<REAL>(ni, na, g, J2, a_, b_, r_, s_));
     return true;
 }
 
-__device__ void casmat_row_setup(int na, uint64_t I, CsrRow &rw) {
+__device__ void casmat_row_setup(int na, int ne, uint64_t I, CsrRow &rw) {
     if (threadIdx.x == 0) {
         int no = 0, nv = 0;
         for (int t = 0; t < na; t++) {
             if ((I >> t) & 1ull) rw.occ[no++] = t;
             else rw.vir[nv++] = t;
         }
+    }
+    const int nv = na - ne, npo = ne * (ne - 1) / 2;
+    for (int x = threadIdx.x; x < na; x += blockDim.x) {   // the pairs (x, y > x), x slowest
+        if (x < ne)
+            for (int y = x + 1, at = x * (2 * ne - x - 1) / 2; y < ne; y++, at++) rw.pair[at] = (uint16_t)(x | (y << 8));
+        if (x < nv)
+            for (int y = x + 1, at = npo + x * (2 * nv - x - 1) / 2; y < nv; y++, at++) rw.pair[at] = (uint16_t)(x | (y << 8));
     }
     __syncthreads();
 }
@@ -333,81 +369,93 @@ __device__ double casmat_diag(int ni, int na, int ne, const cplx *__restrict__ h
 }
 
 __global__ void __launch_bounds__(256) casmat_csr_count_kernel(int ni, int na, int ne, const uint64_t *__restrict__ dets,
-                                                               int ndet, const cplx *__restrict__ h, int nmo,
-                                                               const cplx *__restrict__ g, int64_t *counts) {
+                                                               CsrTables t, int64_t *counts) {
     __shared__ CsrRow rw;
     __shared__ int64_t red[8];
     const int i = blockIdx.x;
     const uint64_t I = dets[i];
-    casmat_row_setup(na, I, rw);
+    casmat_row_setup(na, ne, I, rw);
     const int nv = na - ne;
     const int64_t ncand = (int64_t)ne * nv + (int64_t)(ne * (ne - 1) / 2) * (nv * (nv - 1) / 2);
     int64_t cnt = 0;
     for (int64_t q = threadIdx.x; q < ncand; q += blockDim.x) {
         int64_t j;
         cplx v;
-        cnt += casmat_candidate<false>(ni, na, ne, dets, ndet, h, nmo, g, i, I, rw, q, j, v) ? 1 : 0;
+        cnt += casmat_candidate<false, false>(ni, na, ne, t, nullptr, i, I, rw, q, j, v) ? 1 : 0;
     }
     for (int o = 16; o > 0; o >>= 1) cnt += __shfl_down_sync(0xffffffffu, cnt, o);
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = cnt;
     __syncthreads();
     if (threadIdx.x == 0) {
-        int64_t t = 1;   // the diagonal
-        for (int w = 0; w < (int)(blockDim.x >> 5); w++) t += red[w];
-        counts[i] = t;
+        int64_t tot = 1;   // the diagonal
+        for (int w = 0; w < (int)(blockDim.x >> 5); w++) tot += red[w];
+        counts[i] = tot;
     }
 }
 
+template <bool REAL>
 __global__ void __launch_bounds__(256) casmat_csr_fill_kernel(int ni, int na, int ne, const uint64_t *__restrict__ dets,
-                                                              int ndet, const cplx *__restrict__ h, int nmo,
-                                                              const cplx *__restrict__ g, const int64_t *rowptr,
-                                                              int *cols, cplx *vals, double *hdiag) {
+                                                              const cplx *__restrict__ h, int nmo, const cplx *__restrict__ g,
+                                                              CsrTables t, const int64_t *rowptr, int *cols, cplx *vals,
+                                                              double *rvals, double *hdiag) {
     __shared__ CsrRow rw;
     __shared__ double red[8];
-    __shared__ int wsum[8];
-    __shared__ int64_t run;
+    __shared__ int wsum[2][8];
     const int i = blockIdx.x;
     const uint64_t I = dets[i];
-    casmat_row_setup(na, I, rw);
+    casmat_row_setup(na, ne, I, rw);
     const double dg = casmat_diag(ni, na, ne, h, nmo, g, rw, red);
+    int64_t run = rowptr[i];   // the same in every thread
     if (threadIdx.x == 0) {
-        cols[rowptr[i]] = i;
-        vals[rowptr[i]] = mk(dg, 0.0);
+        cols[run] = i;
+        if (REAL) rvals[run] = dg;
+        else vals[run] = mk(dg, 0.0);
         hdiag[i] = dg;
-        run = rowptr[i] + 1;
     }
-    __syncthreads();
+    run++;
     const int nv = na - ne;
     const int64_t ncand = (int64_t)ne * nv + (int64_t)(ne * (ne - 1) / 2) * (nv * (nv - 1) / 2);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    for (int64_t q0 = 0; q0 < ncand; q0 += blockDim.x) {
+    int buf = 0;
+    for (int64_t q0 = 0; q0 < ncand; q0 += blockDim.x, buf ^= 1) {
         const int64_t q = q0 + threadIdx.x;
         int64_t j = 0;
         cplx v = mk(0.0, 0.0);
-        const bool kept = q < ncand && casmat_candidate<true>(ni, na, ne, dets, ndet, h, nmo, g, i, I, rw, q, j, v);
+        const bool kept = q < ncand && casmat_candidate<true, REAL>(ni, na, ne, t, g, i, I, rw, q, j, v);
         const unsigned bal = __ballot_sync(0xffffffffu, kept);
-        if (lane == 0) wsum[warp] = __popc(bal);
-        __syncthreads();
+        if (lane == 0) wsum[buf][warp] = __popc(bal);
+        __syncthreads();   // the counts alternate between two rows, so one barrier a chunk is enough
         int before = 0, total = 0;
         for (int w = 0; w < nw; w++) {
-            if (w < warp) before += wsum[w];
-            total += wsum[w];
+            if (w < warp) before += wsum[buf][w];
+            total += wsum[buf][w];
         }
         before += __popc(bal & ((1u << lane) - 1u));
         if (kept) {
             cols[run + before] = (int)j;
-            vals[run + before] = v;
+            if (REAL) rvals[run + before] = v.x;
+            else vals[run + before] = v;
         }
-        __syncthreads();
-        if (threadIdx.x == 0) run += total;
-        __syncthreads();
+        run += total;
     }
 }
 
 void build_casmat_csr(Context &c, const uint64_t *dets, int ndet, const cplx *h, const cplx *g, CsrMatrix &m) {
     if (c.na > 64) throw Error{DCG_E_ARG, "casmat: more than 64 active spinors"};
+    const int na = c.na;
+    uint64_t size = 64;
+    while (size < 2 * (uint64_t)ndet) size *= 2;
+    uint64_t *key = wsget<uint64_t>(c, "csr.key", size);
+    int *val = wsget<int>(c, "csr.slot", size);
+    cplx *heff = wsget<cplx>(c, "csr.heff", (size_t)na * na), *jk = wsget<cplx>(c, "csr.jk", (size_t)na * na * na);
+    DCG_CUDA(cudaMemsetAsync(key, 0xff, sizeof(uint64_t) * size, c.stream));
+    det_table_kernel<<<grid1d(ndet, 256), 256, 0, c.stream>>>(dets, ndet, key, val, size - 1);
+    DCG_LAUNCHED(c);
+    csr_tables_kernel<<<grid1d(na * na, 64), 64, 0, c.stream>>>(c.ni, na, h, c.nmo, g, heff, jk);
+    DCG_LAUNCHED(c);
+    const CsrTables t{heff, jk, {key, val, size - 1}};
     int64_t *counts = wsget<int64_t>(c, "csr.cnt", (size_t)ndet + 1);
-    casmat_csr_count_kernel<<<ndet, 256, 0, c.stream>>>(c.ni, c.na, c.ne, dets, ndet, h, c.nmo, g, counts);
+    casmat_csr_count_kernel<<<ndet, 256, 0, c.stream>>>(c.ni, na, c.ne, dets, t, counts);
     DCG_LAUNCHED(c);
     std::vector<int64_t> hc(ndet), rp((size_t)ndet + 1, 0);
     DCG_CUDA(cudaMemcpyAsync(hc.data(), counts, sizeof(int64_t) * ndet, cudaMemcpyDeviceToHost, c.stream));
@@ -418,10 +466,11 @@ void build_casmat_csr(Context &c, const uint64_t *dets, int ndet, const cplx *h,
     m.rowptr = wsget<int64_t>(c, "csr.rp", (size_t)ndet + 1);
     DCG_CUDA(cudaMemcpyAsync(m.rowptr, rp.data(), sizeof(int64_t) * (ndet + 1), cudaMemcpyHostToDevice, c.stream));
     m.cols = wsget<int>(c, "csr.col", (size_t)m.nnz + 1);
-    m.vals = wsget<cplx>(c, "csr.val", (size_t)m.nnz + 1);
+    if (c.real_now) m.rvals = wsget<double>(c, "csr.rval", (size_t)m.nnz + 1);
+    else m.vals = wsget<cplx>(c, "csr.val", (size_t)m.nnz + 1);
     m.diag = wsget<double>(c, "csr.diag", (size_t)ndet + 1);
-    casmat_csr_fill_kernel<<<ndet, 256, 0, c.stream>>>(c.ni, c.na, c.ne, dets, ndet, h, c.nmo, g, m.rowptr, m.cols,
-                                                        m.vals, m.diag);
+    auto *fill = c.real_now ? casmat_csr_fill_kernel<true> : casmat_csr_fill_kernel<false>;
+    fill<<<ndet, 256, 0, c.stream>>>(c.ni, na, c.ne, dets, h, c.nmo, g, t, m.rowptr, m.cols, m.vals, m.rvals, m.diag);
     DCG_LAUNCHED(c);
 }
 

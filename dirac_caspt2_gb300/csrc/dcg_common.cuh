@@ -468,7 +468,8 @@ struct CsrMatrix {
     int64_t nnz = 0;
     int64_t *rowptr = nullptr;
     int *cols = nullptr;
-    cplx *vals = nullptr;
+    cplx *vals = nullptr;      // complex elements, or
+    double *rvals = nullptr;   // real ones (a real system's matrix)
     double *diag = nullptr;
 };
 // The Slater-Condon elements of the CI space as CSR (dcg_ci.cu).

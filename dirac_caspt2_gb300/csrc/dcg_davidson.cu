@@ -55,6 +55,45 @@ __device__ __forceinline__ int rr_player(int pos, int s, int np) {
     return pos == 0 ? 0 : 1 + (pos - 1 + s) % (np - 1);
 }
 
+// Element arithmetic of a real or a complex Hermitian matrix (real: every imaginary part is zero).
+template <bool REAL>
+struct JT {
+    using T = cplx;
+    static __device__ __forceinline__ T get(cplx v) { return v; }
+    static __device__ __forceinline__ cplx put(T v) { return v; }
+    static __device__ __forceinline__ double abs2(T v) { return fma(v.x, v.x, v.y * v.y); }
+    static __device__ __forceinline__ double re(T v) { return v.x; }
+    static __device__ __forceinline__ T conj(T v) { return cconj(v); }
+    static __device__ __forceinline__ T unit(double d) { return mk(d, 0.0); }
+    // c x - s y, c x + s y
+    static __device__ __forceinline__ T minus(double c, T x, T s, T y) {
+        return mk(fma(c, x.x, fma(-s.x, y.x, s.y * y.y)), fma(c, x.y, fma(-s.x, y.y, -s.y * y.x)));
+    }
+    static __device__ __forceinline__ T plus(double c, T x, T s, T y) {
+        return mk(fma(c, x.x, fma(s.x, y.x, -s.y * y.y)), fma(c, x.y, fma(s.x, y.y, s.y * y.x)));
+    }
+};
+template <>
+struct JT<true> {
+    using T = double;
+    static __device__ __forceinline__ T get(cplx v) { return v.x; }
+    static __device__ __forceinline__ cplx put(T v) { return mk(v, 0.0); }
+    static __device__ __forceinline__ double abs2(T v) { return v * v; }
+    static __device__ __forceinline__ double re(T v) { return v; }
+    static __device__ __forceinline__ T conj(T v) { return v; }
+    static __device__ __forceinline__ T unit(double d) { return d; }
+    static __device__ __forceinline__ T minus(double c, T x, T s, T y) { return fma(c, x, -s * y); }
+    static __device__ __forceinline__ T plus(double c, T x, T s, T y) { return fma(c, x, s * y); }
+};
+
+// 1/sqrt(x) from the hardware's ~2^-22 approximation by one third-order Newton step.
+__device__ __forceinline__ double jac_rsqrt(double x) {
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    const double e = fma(-x * y, y, 1.0);
+    return fma(y, fma(0.375, e, 0.5) * e, y);
+}
+
 // All eigenpairs of a small Hermitian matrix G (n <= 64, column-major, ldg; the matrix used is
 // (G + G^H)/2) by cyclic Jacobi with the parallel round-robin ordering (Golub & Van Loan,
 // Matrix Computations, 4th ed., 8.5.5): each round rotates n/2 disjoint pairs at once,
@@ -62,20 +101,29 @@ __device__ __forceinline__ int rr_player(int pos, int s, int np) {
 // by the phase e^{i phi} and rotated by the symmetric Schur step (ibid. 8.5.2), so
 // J_pp = J_qq = c, J_pq = s e^{i phi}, J_qp = -s e^{-i phi}.  Sweeps stop when the squared
 // off-diagonal Frobenius norm is below 1e-30 of the whole (status 1 after 40 sweeps).
-// Output: ascending eigenvalues w[n], eigenvectors Y (n x n, ldy).  One block.
+// Output: ascending eigenvalues w[n], eigenvectors Y (n x n, ldy).  One block, bound by its SM's
+// FP64 unit and the chain of a round's angles: the angle and phase come from FP32 arithmetic
+// (a rotated element then shrinks by ~1e-7 instead of vanishing, within the quadratic
+// convergence) and only c, s and the phase's length are made exact in FP64; a round's
+// two-sided update touches each pair of pairs once (A is Hermitian), beside the update of V.
+template <bool REAL>
 __global__ void __launch_bounds__(kJacobiThreads) jacobi_heev_kernel(int n, const int *__restrict__ n_dev,
                                                                        const cplx *__restrict__ G, int ldg,
                                                                        double *w, cplx *Y, int ldy, int *status) {
+    using Z = JT<REAL>;
+    using T = typename Z::T;
     extern __shared__ double2 jsm[];
     if (n_dev) n = *n_dev;   // dimension read on the device (graph replays of a Davidson step)
     const int np = n + (n & 1);   // padded to even: the dummy player pairs with nobody
-    cplx *A = jsm;                // np x np
-    cplx *V = A + np * np;        // np x np
-    __shared__ double cs_c[kJacobiMaxN / 2], cs_s[kJacobiMaxN / 2], cs_pr[kJacobiMaxN / 2], cs_pi[kJacobiMaxN / 2];
-    __shared__ int cs_p[kJacobiMaxN / 2], cs_q[kJacobiMaxN / 2];
+    T *A = reinterpret_cast<T *>(jsm);   // np x np
+    T *V = A + np * np;                   // np x np
+    __shared__ double cs_c[kJacobiMaxN / 2];
+    __shared__ T cs_s[kJacobiMaxN / 2];   // s e^{i phi}
+    __shared__ int cs_p[kJacobiMaxN / 2], cs_q[kJacobiMaxN / 2], cs_on[kJacobiMaxN / 2];
     __shared__ double red[32];
     __shared__ int rank_sh[kJacobiMaxN];
     const int tid = threadIdx.x, nt = blockDim.x;
+    double fro = 0.0;
     for (int e = tid; e < np * np; e += nt) {
         const int i = e % np, j = e / np;
         cplx a = mk(0.0, 0.0);
@@ -84,19 +132,18 @@ __global__ void __launch_bounds__(kJacobiThreads) jacobi_heev_kernel(int n, cons
             a = mk(0.5 * (x.x + y.x), 0.5 * (x.y - y.y));
             if (i == j) a.y = 0.0;
         }
-        A[e] = a;
-        V[e] = mk(i == j ? 1.0 : 0.0, 0.0);
+        A[e] = Z::get(a);
+        V[e] = Z::unit(i == j ? 1.0 : 0.0);
+        fro += Z::abs2(Z::get(a));
     }
-    __syncthreads();
-    double fro = 0.0;
-    for (int e = tid; e < np * np; e += nt) fro += A[e].x * A[e].x + A[e].y * A[e].y;
-    fro = block_sum_d(fro, red);
-    const int npair = np / 2;
+    fro = block_sum_d(fro, red);   // syncs the block
+    const float scale = fro > 0.0 ? (float)(1.0 / sqrt(fro)) : 1.0f;   // elements of A in FP32 range
+    const int npair = np / 2, nblk = npair * (npair + 1) / 2;
     int sweep = 0;
     for (; sweep < kJacobiMaxSweeps; sweep++) {
         double off = 0.0;
         for (int e = tid; e < np * np; e += nt)
-            if (e % np != e / np) off += A[e].x * A[e].x + A[e].y * A[e].y;
+            if (e % np < e / np) off += 2.0 * Z::abs2(A[e]);
         off = block_sum_d(off, red);
         if (off <= 1e-30 * fro || fro == 0.0) break;
         for (int s = 0; s < np - 1; s++) {
@@ -110,74 +157,98 @@ __global__ void __launch_bounds__(kJacobiThreads) jacobi_heev_kernel(int n, cons
                 }
                 cs_p[k] = p;
                 cs_q[k] = q;
-                double c = 1.0, sn = 0.0, pr = 1.0, pi = 0.0;
-                const cplx b = A[p + np * q];
-                const double ab2 = b.x * b.x + b.y * b.y;
                 // a rotation whose off-diagonal element is below 1e-34 of the squared norm is
                 // skipped (all of them together stay under the 1e-30 stopping test): the late
                 // sweeps of the quadratic convergence then cost little FP64 work
-                if (q < n && ab2 > 1e-34 * fro) {
-                    const double ab = sqrt(ab2);
-                    const double app = A[p + np * p].x, aqq = A[q + np * q].x;
-                    const double zeta = (aqq - app) / (2.0 * ab);
-                    const double t = (zeta >= 0.0 ? 1.0 : -1.0) / (fabs(zeta) + sqrt(1.0 + zeta * zeta));
-                    c = 1.0 / sqrt(1.0 + t * t);
-                    sn = t * c;
-                    pr = b.x / ab;
-                    pi = b.y / ab;
+                const T b = A[p + np * q];
+                const bool on = q < n && Z::abs2(b) > 1e-34 * fro;
+                cs_on[k] = on;
+                if (on) {
+                    const cplx bc = Z::put(b);
+                    const float bx = (float)bc.x * scale, by = REAL ? 0.0f : (float)bc.y * scale;
+                    const float d = (float)(Z::re(A[q + np * q]) - Z::re(A[p + np * p])) * scale;
+                    const float ab = REAL ? fabsf(bx) : sqrtf(fmaf(bx, bx, by * by));
+                    const float h = 0.5f * fabsf(d);
+                    const float t = copysignf(ab / (h + sqrtf(fmaf(h, h, ab * ab))), d);
+                    const double t64 = (double)t, c = jac_rsqrt(fma(t64, t64, 1.0)), sn = t64 * c;
+                    cs_c[k] = c;
+                    if constexpr (REAL) {
+                        cs_s[k] = b >= 0.0 ? sn : -sn;
+                    } else {
+                        const double px = (double)(bx / ab), py = (double)(by / ab);
+                        const double f = sn * jac_rsqrt(fma(px, px, py * py));
+                        cs_s[k] = mk(f * px, f * py);
+                    }
                 }
-                cs_c[k] = c;
-                cs_s[k] = sn;
-                cs_pr[k] = pr;
-                cs_pi[k] = pi;
             }
             __syncthreads();
-            // columns: A <- A J, V <- V J (identity rotations skipped)
-            for (int e = tid; e < np * npair; e += nt) {
-                const int i = e % np, k = e / np;
-                const double c = cs_c[k], sn = cs_s[k];
-                if (sn == 0.0) continue;
-                const int p = cs_p[k], q = cs_q[k];
-                const cplx sp = mk(sn * cs_pr[k], sn * cs_pi[k]);    // s e^{i phi}
-                const cplx sm = mk(sn * cs_pr[k], -sn * cs_pi[k]);   // s e^{-i phi}
-                const cplx ap = A[i + np * p], aq = A[i + np * q];
-                A[i + np * p] = csub(mk(c * ap.x, c * ap.y), cmul(sm, aq));
-                A[i + np * q] = cadd(cmul(sp, ap), mk(c * aq.x, c * aq.y));
-                const cplx vp = V[i + np * p], vq = V[i + np * q];
-                V[i + np * p] = csub(mk(c * vp.x, c * vp.y), cmul(sm, vq));
-                V[i + np * q] = cadd(cmul(sp, vp), mk(c * vq.x, c * vq.y));
-            }
-            __syncthreads();
-            // rows: A <- J^H A
-            for (int e = tid; e < np * npair; e += nt) {
-                const int j = e % np, k = e / np;
-                const double c = cs_c[k], sn = cs_s[k];
-                if (sn == 0.0) continue;
-                const int p = cs_p[k], q = cs_q[k];
-                const cplx sp = mk(sn * cs_pr[k], sn * cs_pi[k]);
-                const cplx sm = mk(sn * cs_pr[k], -sn * cs_pi[k]);
-                const cplx ap = A[p + np * j], aq = A[q + np * j];
-                A[p + np * j] = csub(mk(c * ap.x, c * ap.y), cmul(sp, aq));
-                A[q + np * j] = cadd(cmul(sm, ap), mk(c * aq.x, c * aq.y));
+            // A <- J^H A J, each block of a pair k and a pair l >= k once, and V <- V J
+            for (int e = tid; e < nblk + np * npair; e += nt) {
+                if (e < nblk) {
+                    int l = (int)((sqrtf(8.0f * e + 1.0f) - 1.0f) * 0.5f);
+                    while (l * (l + 1) / 2 > e) l--;
+                    while ((l + 1) * (l + 2) / 2 <= e) l++;
+                    const int k = e - l * (l + 1) / 2;
+                    if (!cs_on[k] && !cs_on[l]) continue;
+                    const int pk = cs_p[k], qk = cs_q[k], pl = cs_p[l], ql = cs_q[l];
+                    T b11 = A[pk + np * pl], b12 = A[pk + np * ql], b21 = A[qk + np * pl], b22 = A[qk + np * ql];
+                    if (cs_on[l]) {   // columns: p' = c p - conj(s) q, q' = s p + c q
+                        const double c = cs_c[l];
+                        const T sg = cs_s[l], sc = Z::conj(sg);
+                        T u = Z::minus(c, b11, sc, b12), v = Z::plus(c, b12, sg, b11);
+                        b11 = u, b12 = v;
+                        u = Z::minus(c, b21, sc, b22), v = Z::plus(c, b22, sg, b21);
+                        b21 = u, b22 = v;
+                    }
+                    if (cs_on[k]) {   // rows: p' = c p - s q, q' = conj(s) p + c q
+                        const double c = cs_c[k];
+                        const T sg = cs_s[k], sc = Z::conj(sg);
+                        T u = Z::minus(c, b11, sg, b21), v = Z::plus(c, b21, sc, b11);
+                        b11 = u, b21 = v;
+                        u = Z::minus(c, b12, sg, b22), v = Z::plus(c, b22, sc, b12);
+                        b12 = u, b22 = v;
+                    }
+                    if (k == l) {   // Hermitian to the bit
+                        b11 = Z::unit(Z::re(b11));
+                        b22 = Z::unit(Z::re(b22));
+                        A[pk + np * pk] = b11;
+                        A[qk + np * qk] = b22;
+                        A[pk + np * qk] = b12;
+                        A[qk + np * pk] = Z::conj(b12);
+                    } else {
+                        A[pk + np * pl] = b11, A[pl + np * pk] = Z::conj(b11);
+                        A[pk + np * ql] = b12, A[ql + np * pk] = Z::conj(b12);
+                        A[qk + np * pl] = b21, A[pl + np * qk] = Z::conj(b21);
+                        A[qk + np * ql] = b22, A[ql + np * qk] = Z::conj(b22);
+                    }
+                } else {
+                    const int i = (e - nblk) % np, k = (e - nblk) / np;
+                    if (!cs_on[k]) continue;
+                    const int p = cs_p[k], q = cs_q[k];
+                    const double c = cs_c[k];
+                    const T sg = cs_s[k], vp = V[i + np * p], vq = V[i + np * q];
+                    V[i + np * p] = Z::minus(c, vp, Z::conj(sg), vq);
+                    V[i + np * q] = Z::plus(c, vq, sg, vp);
+                }
             }
             __syncthreads();
         }
     }
     // ascending order (ties by index), then the outputs
     for (int i = tid; i < n; i += nt) {
-        const double di = A[i + np * i].x;
+        const double di = Z::re(A[i + np * i]);
         int r = 0;
         for (int j = 0; j < n; j++) {
-            const double dj = A[j + np * j].x;
+            const double dj = Z::re(A[j + np * j]);
             r += (dj < di) || (dj == di && j < i);
         }
         rank_sh[i] = r;
     }
     __syncthreads();
-    for (int i = tid; i < n; i += nt) w[rank_sh[i]] = A[i + np * i].x;
+    for (int i = tid; i < n; i += nt) w[rank_sh[i]] = Z::re(A[i + np * i]);
     for (int e = tid; e < n * n; e += nt) {
         const int i = e % n, j = e / n;
-        Y[i + (int64_t)ldy * rank_sh[j]] = V[i + np * j];
+        Y[i + (int64_t)ldy * rank_sh[j]] = Z::put(V[i + np * j]);
     }
     if (tid == 0 && sweep >= kJacobiMaxSweeps) *status = 1;
 }
@@ -190,63 +261,28 @@ __global__ void unit_cols_kernel(int n, int m, const int *__restrict__ idx, cplx
     X[i + ldx * c] = mk(i == idx[c] ? 1.0 : 0.0, 0.0);
 }
 
-// R[:, c] = HX[:, c] - theta[c] X[:, c]; out2[c] = |R[:, c]|^2 (one block per column, fixed
-// reduction order); T[:, c] = R[:, c] / (theta[c] - hd) with the denominator kept away from 0.
-__global__ void residual_kernel(int n, const cplx *__restrict__ HX, const cplx *__restrict__ X, int64_t ld,
-                                const double *__restrict__ theta, const double *__restrict__ hd, cplx *T,
-                                double *out2) {
-    __shared__ double sh[32];
-    const int c = blockIdx.x;
-    const double th = theta[c];
-    double acc = 0.0;
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        const cplx hx = HX[i + ld * c], x = X[i + ld * c];
-        const cplx r = mk(hx.x - th * x.x, hx.y - th * x.y);
-        acc += r.x * r.x + r.y * r.y;
-        double den = th - hd[i];
-        if (fabs(den) < 1e-4) den = den < 0.0 ? -1e-4 : 1e-4;
-        T[i + ld * c] = mk(r.x / den, r.y / den);
-    }
-    acc = block_sum_d(acc, sh);
-    if (threadIdx.x == 0) out2[c] = acc;
+// ---- vector work in chunks of kDavChunk rows, one block each: partial sums go to part[...] and
+// whoever needs the sum adds the chunks in order, so a sum depends on n alone.  One block for a
+// whole vector left 151 SMs idle on 74,273 determinants (0.2 to 1 ms a kernel).  The RAS space of
+// that size, real: whole call 310 ms before, 98 ms with the chunks, real arithmetic, the Rayleigh
+// elements of new vectors alone and the determinant table of the matrix build.
+constexpr int kDavChunk = 1024, kDavThreads = 256;
+
+// Sums of a complex (re, im) pair over the block; real vectors carry no im.
+template <bool REAL>
+__device__ __forceinline__ void dav_block_sum(double &re, double &im, double *sh) {
+    re = block_sum_d(re, sh);
+    if (!REAL) im = block_sum_d(im, sh);
 }
 
-// Y[:, c] = H X[:, c] for K vectors and a CSR H: one warp per row, the lanes striding the row's
-// entries in order and a fixed shuffle tree summing them (deterministic).
-template <int K>
-__global__ void __launch_bounds__(256) csr_hx_kernel(int n, int k, const int64_t *__restrict__ rowptr,
-                                                      const int *__restrict__ cols, const cplx *__restrict__ vals,
-                                                      const cplx *__restrict__ X, int64_t ldx, cplx *Y, int64_t ldy) {
-    const int row = (int)(((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
-    const int lane = threadIdx.x & 31;
-    if (row >= n) return;
-    double re[K], im[K];
-#pragma unroll
-    for (int c = 0; c < K; c++) re[c] = im[c] = 0.0;
-    const int64_t e1 = rowptr[row + 1];
-    for (int64_t e = rowptr[row] + lane; e < e1; e += 32) {
-        const cplx h = vals[e];
-        const int j = cols[e];
-#pragma unroll
-        for (int c = 0; c < K; c++) {
-            if (c < k) {
-                const cplx x = __ldg(X + j + ldx * c);
-                re[c] = fma(h.x, x.x, fma(-h.y, x.y, re[c]));
-                im[c] = fma(h.x, x.y, fma(h.y, x.x, im[c]));
-            }
-        }
-    }
-#pragma unroll
-    for (int c = 0; c < K; c++) {
-        for (int o = 16; o > 0; o >>= 1) {
-            re[c] += __shfl_down_sync(0xffffffffu, re[c], o);
-            im[c] += __shfl_down_sync(0xffffffffu, im[c], o);
-        }
-    }
-    if (lane == 0) {
-#pragma unroll
-        for (int c = 0; c < K; c++)
-            if (c < k) Y[row + ldy * c] = mk(re[c], im[c]);
+// conj(x) y added to (re, im)
+template <bool REAL>
+__device__ __forceinline__ void dav_dot(double &re, double &im, cplx x, cplx y) {
+    re = fma(x.x, y.x, re);
+    if (!REAL) {
+        re = fma(x.y, y.y, re);
+        im = fma(x.x, y.y, im);
+        im = fma(-x.y, y.x, im);
     }
 }
 
@@ -255,34 +291,50 @@ __global__ void __launch_bounds__(256) csr_hx_kernel(int n, int k, const int64_t
 // captured sequence (a CUDA graph) serves every step.
 struct DavState {
     int m;        // vectors in V (and W = H V)
+    int mold;     // of them, those whose Rayleigh elements G already holds
     int cand;     // new directions accepted in this step
-    int stop;     // a direction was rejected: none after it this step
-    int act;      // the direction being built is live
     int jac;      // a Jacobi solve ran out of sweeps (sticky)
+    int restarted;
+    int live[8], ok[8];   // direction q: tried, accepted
     int pad[3];
     double worst;  // largest residual norm of the wanted roots
-    double n0;     // |direction|^2 before the Gram-Schmidt passes
 };
+// Column of direction q: after the accepted ones before it.
+__device__ __forceinline__ int dav_col(const DavState *st, int q) {
+    int m = st->m;
+    for (int p = 0; p < q; p++) m += st->ok[p];
+    return m;
+}
 
-// G[i + ldg j] = V[:, i]^H W[:, j] for i, j < m (one block per element, fixed order).
-__global__ void rr_kernel(int n, const cplx *__restrict__ V, const cplx *__restrict__ W, int64_t ld, cplx *G,
-                          int ldg, const DavState *__restrict__ st) {
+// Partial G[i, j] = V[:, i]^H W[:, j], i <= j, for the columns j >= mold that G does not hold yet:
+// block (i, j - mold, chunk).
+template <bool REAL>
+__global__ void __launch_bounds__(kDavThreads) rr_part_kernel(int n, const cplx *__restrict__ V, const cplx *__restrict__ W,
+                                                              int64_t ld, cplx *part, int mmax,
+                                                              const DavState *__restrict__ st) {
     __shared__ double sh[32];
-    const int i = blockIdx.x, j = blockIdx.y, m = st->m;
-    if (i >= m || j >= m) return;
+    const int i = blockIdx.x, j = st->mold + blockIdx.y, m = st->m;
+    if (j >= m || i > j) return;
     const cplx *a = V + ld * i, *b = W + ld * j;
     double re = 0.0, im = 0.0;
-    for (int k = threadIdx.x; k < n; k += blockDim.x) {
-        const cplx x = a[k], y = b[k];
-        re += x.x * y.x + x.y * y.y;
-        im += x.x * y.y - x.y * y.x;
-    }
-    re = block_sum_d(re, sh);
-    im = block_sum_d(im, sh);
-    if (threadIdx.x == 0) G[i + (int64_t)ldg * j] = mk(re, im);
+    const int k0 = blockIdx.z * kDavChunk, k1 = min(n, k0 + kDavChunk);
+    for (int k = k0 + threadIdx.x; k < k1; k += kDavThreads) dav_dot<REAL>(re, im, a[k], b[k]);
+    dav_block_sum<REAL>(re, im, sh);
+    if (threadIdx.x == 0) part[i + (int64_t)mmax * (blockIdx.y + 16 * (int64_t)blockIdx.z)] = mk(re, im);
+}
+__global__ void rr_sum_kernel(int nchunk, const cplx *__restrict__ part, int mmax, cplx *G, int ldg,
+                              const DavState *__restrict__ st) {
+    const int i = threadIdx.x, j = st->mold + blockIdx.x;
+    if (j >= st->m || i > j) return;
+    cplx s = mk(0.0, 0.0);
+    for (int c = 0; c < nchunk; c++) s = cadd(s, part[i + (int64_t)mmax * (blockIdx.x + 16 * (int64_t)c)]);
+    if (i == j) s.y = 0.0;
+    G[i + (int64_t)ldg * j] = s;
+    G[j + (int64_t)ldg * i] = cconj(s);
 }
 
 // X = V Y[:, :nb] (z = 0) and HX = W Y[:, :nb] (z = 1) over the m columns of V and W.
+template <bool REAL>
 __global__ void ritz_kernel(int n, const cplx *__restrict__ V, const cplx *__restrict__ W, int64_t ld,
                             const cplx *__restrict__ Y, int ldy, cplx *X, cplx *HX, const DavState *__restrict__ st) {
     const int r = blockIdx.x * blockDim.x + threadIdx.x, c = blockIdx.y;
@@ -290,24 +342,64 @@ __global__ void ritz_kernel(int n, const cplx *__restrict__ V, const cplx *__res
     const cplx *A = blockIdx.z ? W : V;
     const int m = st->m;
     cplx acc = mk(0.0, 0.0);
-    for (int q = 0; q < m; q++) acc = cadd(acc, cmul(A[r + ld * q], __ldg(Y + q + (int64_t)ldy * c)));
+    for (int q = 0; q < m; q++) {
+        const cplx a = A[r + ld * q], y = __ldg(Y + q + (int64_t)ldy * c);
+        if (REAL) acc.x = fma(a.x, y.x, acc.x);
+        else cfma(acc, a, y);
+    }
     (blockIdx.z ? HX : X)[r + ld * c] = acc;
 }
 
-// The residual norms of the wanted roots; the step's direction counters reset.
-__global__ void step_begin_kernel(int nwant, const double *__restrict__ h2, DavState *st) {
-    if (threadIdx.x != 0) return;
-    double w = 0.0;
-    for (int q = 0; q < nwant; q++) w = fmax(w, sqrt(h2[q]));
-    st->worst = w;
-    st->cand = 0;
-    st->stop = 0;
+// R[:, c] = HX[:, c] - theta[c] X[:, c], its squared norm by chunks to part[chunk + nchunk c];
+// T[:, c] = R[:, c] / (theta[c] - hd) with the denominator kept away from 0.
+template <bool REAL>
+__global__ void __launch_bounds__(kDavThreads) residual_kernel(int n, const cplx *__restrict__ HX,
+                                                               const cplx *__restrict__ X, int64_t ld,
+                                                               const double *__restrict__ theta,
+                                                               const double *__restrict__ hd, cplx *T, double *part) {
+    __shared__ double sh[32];
+    const int c = blockIdx.y;
+    const double th = theta[c];
+    double acc = 0.0;
+    const int k0 = blockIdx.x * kDavChunk, k1 = min(n, k0 + kDavChunk);
+    for (int i = k0 + threadIdx.x; i < k1; i += kDavThreads) {
+        const cplx hx = HX[i + ld * c], x = X[i + ld * c];
+        const cplx r = mk(fma(-th, x.x, hx.x), REAL ? 0.0 : fma(-th, x.y, hx.y));
+        acc = fma(r.x, r.x, acc);
+        if (!REAL) acc = fma(r.y, r.y, acc);
+        double den = th - hd[i];
+        if (fabs(den) < 1e-4) den = den < 0.0 ? -1e-4 : 1e-4;
+        const double inv = 1.0 / den;
+        T[i + ld * c] = mk(r.x * inv, REAL ? 0.0 : r.y * inv);
+    }
+    acc = block_sum_d(acc, sh);
+    if (threadIdx.x == 0) part[blockIdx.x + (int64_t)gridDim.x * c] = acc;
 }
 
-// Restart on the block's Ritz vectors when the next block would not fit: V, W <- X, HX.
-__global__ void restart_copy_kernel(int n, int nb, int mmax, const cplx *__restrict__ X, const cplx *__restrict__ HX,
+// The residual norms of the block's roots (to h2), the worst of the wanted ones; the step's
+// direction flags reset, and the restart decided: the next block would not fit.
+__global__ void step_begin_kernel(int nwant, int nb, int mmax, int nchunk, const double *__restrict__ part, double *h2,
+                                  DavState *st) {
+    __shared__ double v[8];
+    if (threadIdx.x < nb) {
+        double s = 0.0;
+        for (int c = 0; c < nchunk; c++) s += part[c + (int64_t)nchunk * threadIdx.x];
+        h2[threadIdx.x] = s;
+        v[threadIdx.x] = s;
+    }
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    double w = 0.0;
+    for (int q = 0; q < nwant; q++) w = fmax(w, sqrt(v[q]));
+    st->worst = w;
+    for (int q = 0; q < 8; q++) st->live[q] = st->ok[q] = 0;
+    st->restarted = st->m + nb > mmax;
+}
+
+// Restart on the block's Ritz vectors: V, W <- X, HX.
+__global__ void restart_copy_kernel(int n, int nb, const cplx *__restrict__ X, const cplx *__restrict__ HX,
                                     cplx *V, cplx *W, int64_t ld, const DavState *__restrict__ st) {
-    if (st->m + nb <= mmax) return;
+    if (!st->restarted) return;
     const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= (int64_t)n * nb) return;
     const int i = (int)(e % n), c = (int)(e / n);
@@ -315,117 +407,169 @@ __global__ void restart_copy_kernel(int n, int nb, int mmax, const cplx *__restr
     W[i + ld * c] = HX[i + ld * c];
 }
 
-__global__ void restart_set_kernel(int nb, int mmax, DavState *st) {
-    if (threadIdx.x == 0 && st->m + nb > mmax) st->m = nb;
+__global__ void restart_set_kernel(int nb, DavState *st) {
+    if (threadIdx.x == 0 && st->restarted) st->m = nb;
 }
 
-// Direction q: live when its residual is above tol, the block has not stopped and V has room;
-// then T[:, q] goes to column m + cand of V and its squared norm to n0 (one block).
-__global__ void cand_begin_kernel(int n, int q, int mmax, double tol, const double *__restrict__ h2,
-                                  const cplx *__restrict__ T, cplx *V, int64_t ld, DavState *st) {
+// Direction q: live when its residual is above tol, no direction before it was rejected and V has
+// room; then T[:, q] goes to its column of V and its squared norm, by chunks, to part.
+template <bool REAL>
+__global__ void __launch_bounds__(kDavThreads) cand_begin_kernel(int n, int q, int mmax, double tol,
+                                                                 const double *__restrict__ h2,
+                                                                 const cplx *__restrict__ T, cplx *V, int64_t ld,
+                                                                 double *part, DavState *st) {
     __shared__ double sh[32];
-    __shared__ int live;
-    if (threadIdx.x == 0) {
-        live = !st->stop && sqrt(h2[q]) > tol && st->m + st->cand < mmax;
-        st->act = live;
-    }
-    __syncthreads();
+    bool live = sqrt(h2[q]) > tol;
+    for (int p = 0; p < q; p++)
+        if (st->live[p] && !st->ok[p]) live = false;
+    const int col = dav_col(st, q);
+    live = live && col < mmax;
+    if (blockIdx.x == 0 && threadIdx.x == 0) st->live[q] = live;
     if (!live) return;
-    cplx *dst = V + ld * (st->m + st->cand);
+    cplx *dst = V + ld * col;
     double acc = 0.0;
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
+    const int k0 = blockIdx.x * kDavChunk, k1 = min(n, k0 + kDavChunk);
+    for (int i = k0 + threadIdx.x; i < k1; i += kDavThreads) {
         const cplx x = T[i + ld * q];
         dst[i] = x;
-        acc += x.x * x.x + x.y * x.y;
+        acc = fma(x.x, x.x, acc);
+        if (!REAL) acc = fma(x.y, x.y, acc);
     }
     acc = block_sum_d(acc, sh);
-    if (threadIdx.x == 0) st->n0 = acc;
+    if (threadIdx.x == 0) part[blockIdx.x] = acc;
 }
 
-// Classical Gram-Schmidt pass of the live direction against the vectors before it.
-__global__ void cgs_dot_kernel(int n, const cplx *__restrict__ V, int64_t ld, cplx *cf, const DavState *__restrict__ st) {
+// Classical Gram-Schmidt pass of direction q against the vectors before it: the coefficients by
+// chunks (block (i, chunk)), then the subtraction, which adds the chunks and leaves the squared
+// norm of what remains by its own chunks in part2.
+template <bool REAL>
+__global__ void __launch_bounds__(kDavThreads) cgs_dot_kernel(int n, int q, const cplx *__restrict__ V, int64_t ld,
+                                                              cplx *cf, int mmax, const DavState *__restrict__ st) {
     __shared__ double sh[32];
-    const int i = blockIdx.x, mm = st->m + st->cand;
-    if (!st->act || i >= mm) return;
+    if (!st->live[q]) return;
+    const int i = blockIdx.x, mm = dav_col(st, q);
+    if (i >= mm) return;
     const cplx *a = V + ld * i, *b = V + ld * mm;
     double re = 0.0, im = 0.0;
-    for (int k = threadIdx.x; k < n; k += blockDim.x) {
-        const cplx x = a[k], y = b[k];
-        re += x.x * y.x + x.y * y.y;
-        im += x.x * y.y - x.y * y.x;
-    }
-    re = block_sum_d(re, sh);
-    im = block_sum_d(im, sh);
-    if (threadIdx.x == 0) cf[i] = mk(re, im);
+    const int k0 = blockIdx.y * kDavChunk, k1 = min(n, k0 + kDavChunk);
+    for (int k = k0 + threadIdx.x; k < k1; k += kDavThreads) dav_dot<REAL>(re, im, a[k], b[k]);
+    dav_block_sum<REAL>(re, im, sh);
+    if (threadIdx.x == 0) cf[i + (int64_t)mmax * blockIdx.y] = mk(re, im);
 }
 
-__global__ void cgs_axpy_kernel(int n, cplx *V, int64_t ld, const cplx *__restrict__ cf, const DavState *__restrict__ st) {
-    const int r = blockIdx.x * blockDim.x + threadIdx.x;
-    const int mm = st->m + st->cand;
-    if (!st->act || r >= n) return;
-    cplx acc = mk(0.0, 0.0);
-    for (int q = 0; q < mm; q++) acc = cadd(acc, cmul(V[r + ld * q], cf[q]));
-    cplx &d = V[r + ld * mm];
-    d = csub(d, acc);
-}
-
-// Accept the live direction when it kept more than 1e-10 of its length (normalised, counted),
-// else stop the block's directions here.
-__global__ void cand_end_kernel(int n, cplx *V, int64_t ld, DavState *st) {
+template <bool REAL>
+__global__ void __launch_bounds__(kDavThreads) cgs_axpy_kernel(int n, int q, cplx *V, int64_t ld,
+                                                               const cplx *__restrict__ cf, int mmax, double *part2,
+                                                               const DavState *__restrict__ st) {
     __shared__ double sh[32];
-    if (!st->act) return;
-    cplx *dst = V + ld * (st->m + st->cand);
-    double acc = 0.0;
-    for (int i = threadIdx.x; i < n; i += blockDim.x) acc += dst[i].x * dst[i].x + dst[i].y * dst[i].y;
-    acc = block_sum_d(acc, sh);
-    const bool ok = acc > 1e-20 * st->n0 && acc > 0.0;
-    if (ok) {
-        const double s = 1.0 / sqrt(acc);
-        for (int i = threadIdx.x; i < n; i += blockDim.x) dst[i] = mk(dst[i].x * s, dst[i].y * s);
+    __shared__ cplx c[kJacobiMaxN];
+    if (!st->live[q]) return;
+    const int mm = dav_col(st, q);
+    for (int i = threadIdx.x; i < mm; i += kDavThreads) {
+        cplx s = mk(0.0, 0.0);
+        for (int k = 0; k < (int)gridDim.x; k++) {
+            const cplx x = cf[i + (int64_t)mmax * k];
+            s.x += x.x;
+            if (!REAL) s.y += x.y;
+        }
+        c[i] = s;
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
-        if (ok) st->cand++;
-        else st->stop = 1;
+    cplx *dst = V + ld * mm;
+    double acc = 0.0;
+    const int k0 = blockIdx.x * kDavChunk, k1 = min(n, k0 + kDavChunk);
+    for (int r = k0 + threadIdx.x; r < k1; r += kDavThreads) {
+        cplx s = mk(0.0, 0.0);
+        for (int p = 0; p < mm; p++) {
+            const cplx v = V[r + ld * p];
+            if (REAL) s.x = fma(v.x, c[p].x, s.x);
+            else cfma(s, v, c[p]);
+        }
+        const cplx d = csub(dst[r], s);
+        dst[r] = d;
+        acc = fma(d.x, d.x, acc);
+        if (!REAL) acc = fma(d.y, d.y, acc);
     }
+    acc = block_sum_d(acc, sh);
+    if (threadIdx.x == 0) part2[blockIdx.x] = acc;
 }
 
-// W[:, m + c] = H V[:, m + c] for the cand accepted directions (CSR, one warp per row).
-template <int K>
-__global__ void __launch_bounds__(256) csr_hx_step_kernel(int n, const int64_t *__restrict__ rowptr,
-                                                           const int *__restrict__ cols, const cplx *__restrict__ vals,
-                                                           const cplx *__restrict__ V, cplx *W, int64_t ld,
-                                                           const DavState *__restrict__ st) {
+// Accept direction q when it kept more than 1e-10 of its length (normalised, counted), else no
+// direction after it is tried.
+__global__ void __launch_bounds__(kDavThreads) cand_end_kernel(int n, int q, cplx *V, int64_t ld,
+                                                               const double *__restrict__ part,
+                                                               const double *__restrict__ part2, DavState *st) {
+    if (!st->live[q]) return;
+    __shared__ double s_scale;
+    __shared__ int s_ok;
+    const int col = dav_col(st, q);
+    if (threadIdx.x == 0) {
+        double n0 = 0.0, acc = 0.0;
+        for (int k = 0; k < (int)gridDim.x; k++) {
+            n0 += part[k];
+            acc += part2[k];
+        }
+        s_ok = acc > 1e-20 * n0 && acc > 0.0;
+        s_scale = s_ok ? 1.0 / sqrt(acc) : 0.0;
+        if (blockIdx.x == 0) st->ok[q] = s_ok;   // read by later launches only
+    }
+    __syncthreads();
+    if (!s_ok) return;
+    cplx *dst = V + ld * col;
+    const double s = s_scale;
+    const int k0 = blockIdx.x * kDavChunk, k1 = min(n, k0 + kDavChunk);
+    for (int i = k0 + threadIdx.x; i < k1; i += kDavThreads) dst[i] = mk(dst[i].x * s, dst[i].y * s);
+}
+
+// Y[:, c] = H X[:, c] for K vectors and a CSR H (vals, or real rvals): one warp per row, the lanes
+// striding the row's entries in order and a fixed shuffle tree summing them (deterministic).
+// With st, X and Y are the cand accepted directions of V and W.  Bound by the FP64 unit (K FMAs
+// an entry real, 4 K complex) and, real with few vectors, by the 12 bytes an entry.
+template <int K, bool REAL>
+__global__ void __launch_bounds__(256) csr_hx_kernel(int n, int k, const int64_t *__restrict__ rowptr,
+                                                      const int *__restrict__ cols, const cplx *__restrict__ vals,
+                                                      const double *__restrict__ rvals, const cplx *__restrict__ X,
+                                                      cplx *Y, int64_t ld, const DavState *__restrict__ st) {
     const int row = (int)(((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
     const int lane = threadIdx.x & 31;
-    const int k = st->cand;
+    if (st) {
+        k = dav_col(st, 8) - st->m;
+        X += ld * st->m;
+        Y += ld * st->m;
+    }
     if (row >= n || k == 0) return;
-    const cplx *X = V + ld * st->m;
     double re[K], im[K];
 #pragma unroll
     for (int c = 0; c < K; c++) re[c] = im[c] = 0.0;
     const int64_t e1 = rowptr[row + 1];
     for (int64_t e = rowptr[row] + lane; e < e1; e += 32) {
-        const cplx h = vals[e];
-        const int j = cols[e];
+        const int j = __ldg(cols + e);
+        if (REAL) {
+            const double h = __ldg(rvals + e);
 #pragma unroll
-        for (int c = 0; c < K; c++) {
-            if (c < k) {
-                const cplx x = __ldg(X + j + ld * c);
-                re[c] = fma(h.x, x.x, fma(-h.y, x.y, re[c]));
-                im[c] = fma(h.x, x.y, fma(h.y, x.x, im[c]));
+            for (int c = 0; c < K; c++)
+                if (c < k) re[c] = fma(h, __ldg(&X[j + ld * c].x), re[c]);
+        } else {
+            const cplx h = __ldg(vals + e);
+#pragma unroll
+            for (int c = 0; c < K; c++) {
+                if (c < k) {
+                    const cplx x = __ldg(X + j + ld * c);
+                    re[c] = fma(h.x, x.x, fma(-h.y, x.y, re[c]));
+                    im[c] = fma(h.x, x.y, fma(h.y, x.x, im[c]));
+                }
             }
         }
     }
 #pragma unroll
     for (int c = 0; c < K; c++) {
-        for (int o = 16; o > 0; o >>= 1) {
-            re[c] += __shfl_down_sync(0xffffffffu, re[c], o);
-            im[c] += __shfl_down_sync(0xffffffffu, im[c], o);
-        }
+        if (c < k)
+            for (int o = 16; o > 0; o >>= 1) {
+                re[c] += __shfl_down_sync(0xffffffffu, re[c], o);
+                if (!REAL) im[c] += __shfl_down_sync(0xffffffffu, im[c], o);
+            }
     }
     if (lane == 0) {
-        cplx *Y = W + ld * st->m;
 #pragma unroll
         for (int c = 0; c < K; c++)
             if (c < k) Y[row + ld * c] = mk(re[c], im[c]);
@@ -433,42 +577,38 @@ __global__ void __launch_bounds__(256) csr_hx_step_kernel(int n, const int64_t *
 }
 
 __global__ void step_end_kernel(DavState *st) {
-    if (threadIdx.x == 0) st->m += st->cand;
+    if (threadIdx.x != 0) return;
+    const int cand = dav_col(st, 8) - st->m;
+    st->cand = cand;
+    st->mold = st->restarted ? 0 : st->m;
+    st->m += cand;
 }
 
 }  // namespace
 
-// Y (n x k) = H X for the CSR H, up to 8 vectors a launch (one pass over H for each group).
-static void csr_hx(Context &c, const CsrMatrix &H, const cplx *X, int64_t ldx, int k, cplx *Y, int64_t ldy) {
+// Y (n x k) = H X for the CSR H, up to 8 vectors (st: the accepted directions of a step, at most kmax).
+static void csr_hx(Context &c, const CsrMatrix &H, const cplx *X, cplx *Y, int64_t ld, int k, const DavState *st) {
     const int n = H.n;
     const int blocks = (int)(((int64_t)n * 32 + 255) / 256);
-    for (int c0 = 0; c0 < k; c0 += 8) {
-        const int kk = std::min(8, k - c0);
-        if (kk > 4)
-            csr_hx_kernel<8><<<blocks, 256, 0, c.stream>>>(n, kk, H.rowptr, H.cols, H.vals, X + ldx * c0, ldx,
-                                                            Y + ldy * c0, ldy);
-        else if (kk > 2)
-            csr_hx_kernel<4><<<blocks, 256, 0, c.stream>>>(n, kk, H.rowptr, H.cols, H.vals, X + ldx * c0, ldx,
-                                                            Y + ldy * c0, ldy);
-        else
-            csr_hx_kernel<2><<<blocks, 256, 0, c.stream>>>(n, kk, H.rowptr, H.cols, H.vals, X + ldx * c0, ldx,
-                                                            Y + ldy * c0, ldy);
-        DCG_LAUNCHED(c);
-    }
+    const bool real = H.rvals != nullptr;
+    auto *kern = k > 4 ? (real ? csr_hx_kernel<8, true> : csr_hx_kernel<8, false>)
+                 : k > 2 ? (real ? csr_hx_kernel<4, true> : csr_hx_kernel<4, false>)
+                         : (real ? csr_hx_kernel<2, true> : csr_hx_kernel<2, false>);
+    kern<<<blocks, 256, 0, c.stream>>>(n, k, H.rowptr, H.cols, H.vals, H.rvals, X, Y, ld, st);
 }
 
 // Lowest nwant eigenpairs of the Hermitian CSR H (its diagonal kept beside it): eigenvalues to
 // w[0..nwant), eigenvectors to the columns of Z (n x nwant, ldz = n), each with residual norm
 // <= tol_rel * max(1, max_i |H_ii|).
 //
-// One step: the Rayleigh matrix G = V^H W and its eigenpairs (Jacobi), the block's Ritz
-// vectors X = V Y and images HX = W Y, their residuals and preconditioned corrections T, a
-// restart V, W <- X, HX when the next block would not fit, then each unconverged correction
-// orthonormalised against V (classical Gram-Schmidt twice) and appended, and W extended by
-// H times the new directions.  Every size the step needs lives on the device (DavState), so
-// the step is one fixed launch sequence: captured once as a CUDA graph and replayed, with
-// one read of the state per step (the environment variable DCG_DAVIDSON_GRAPH=0 launches
-// the sequence directly instead).
+// One step: the new elements of the Rayleigh matrix G = V^H W and its eigenpairs (Jacobi), the
+// block's Ritz vectors X = V Y and images HX = W Y, their residuals and preconditioned
+// corrections T, a restart V, W <- X, HX when the next block would not fit, then each
+// unconverged correction orthonormalised against V (classical Gram-Schmidt twice) and
+// appended, and W extended by H times the new directions.  Every size the step needs lives on
+// the device (DavState), so the step is one fixed launch sequence: captured once as a CUDA
+// graph and replayed, with one read of the state per step (the environment variable
+// DCG_DAVIDSON_GRAPH=0 launches the sequence directly instead).
 void davidson_lowest_csr(Context &c, const CsrMatrix &H, int nwant, double *w, cplx *Z, double tol_rel, int maxit) {
     const int n = H.n;
     const int nb = std::min(n, nwant + 2);   // block: the wanted roots and a margin for near-degeneracy
@@ -482,7 +622,11 @@ void davidson_lowest_csr(Context &c, const CsrMatrix &H, int nwant, double *w, c
     cplx *T = wsget<cplx>(c, "dav.T", (size_t)n * nb);
     cplx *G = wsget<cplx>(c, "dav.G", (size_t)mmax * mmax);
     cplx *Y = wsget<cplx>(c, "dav.Y", (size_t)mmax * mmax);
-    cplx *cf = wsget<cplx>(c, "dav.cf", (size_t)mmax);
+    const int nchunk = (int)grid1d(n, kDavChunk);
+    cplx *cf = wsget<cplx>(c, "dav.cf", (size_t)mmax * nchunk);
+    cplx *rrp = wsget<cplx>(c, "dav.rrp", (size_t)mmax * 16 * nchunk);
+    double *part = wsget<double>(c, "dav.part", (size_t)nchunk * 10);   // residuals (8), then a direction's two norms
+    double *pn0 = part + (size_t)nchunk * 8, *pn1 = pn0 + nchunk;
     double *th = wsget<double>(c, "dav.th", mmax);
     double *h2 = wsget<double>(c, "dav.h2", (size_t)nb);
     int *idx = wsget<int>(c, "dav.idx", nb);
@@ -503,42 +647,47 @@ void davidson_lowest_csr(Context &c, const CsrMatrix &H, int nwant, double *w, c
     DCG_CUDA(cudaMemcpyAsync(idx, order.data(), sizeof(int) * nb, cudaMemcpyHostToDevice, c.stream));
     unit_cols_kernel<<<grid1d((int64_t)n * nb, 256), 256, 0, c.stream>>>(n, nb, idx, V, ld);
     DCG_LAUNCHED(c);
-    csr_hx(c, H, V, ld, nb, W, ld);
+    if (nb > 8) throw Error{DCG_E_ARG, "davidson: more than 8 directions per step"};
+    csr_hx(c, H, V, W, ld, nb, nullptr);
+    DCG_LAUNCHED(c);
     DavState s0{};
     s0.m = nb;
     DCG_CUDA(cudaMemcpyAsync(st, &s0, sizeof(DavState), cudaMemcpyHostToDevice, c.stream));
 
     const int np = mmax + (mmax & 1);
-    const size_t jsmem = 2 * sizeof(cplx) * (size_t)np * np;
-    DCG_CUDA(cudaFuncSetAttribute(jacobi_heev_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)jsmem));
-    const int hx_blocks = (int)(((int64_t)n * 32 + 255) / 256);
+    const bool real = H.rvals != nullptr;
+    const size_t jsmem = 2 * (real ? sizeof(double) : sizeof(cplx)) * (size_t)np * np;
+    auto *k_jac = real ? jacobi_heev_kernel<true> : jacobi_heev_kernel<false>;
+    DCG_CUDA(cudaFuncSetAttribute(k_jac, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  2 * (int)sizeof(cplx) * kJacobiMaxN * kJacobiMaxN));
+    auto *k_rr = real ? rr_part_kernel<true> : rr_part_kernel<false>;
+    auto *k_ritz = real ? ritz_kernel<true> : ritz_kernel<false>;
+    auto *k_res = real ? residual_kernel<true> : residual_kernel<false>;
+    auto *k_cand = real ? cand_begin_kernel<true> : cand_begin_kernel<false>;
+    auto *k_dot = real ? cgs_dot_kernel<true> : cgs_dot_kernel<false>;
+    auto *k_axpy = real ? cgs_axpy_kernel<true> : cgs_axpy_kernel<false>;
     auto enqueue_step = [&]() {
-        rr_kernel<<<dim3(mmax, mmax), 256, 0, c.stream>>>(n, V, W, ld, G, mmax, st);
-        jacobi_heev_kernel<<<1, kJacobiThreads, jsmem, c.stream>>>(mmax, &st->m, G, mmax, th, Y, mmax, &st->jac);
-        ritz_kernel<<<dim3(grid1d(n, 128), nb, 2), 128, 0, c.stream>>>(n, V, W, ld, Y, mmax, X, HX, st);
-        residual_kernel<<<nb, 256, 0, c.stream>>>(n, HX, X, ld, th, H.diag, T, h2);
-        step_begin_kernel<<<1, 32, 0, c.stream>>>(nwant, h2, st);
-        restart_copy_kernel<<<grid1d((int64_t)n * nb, 256), 256, 0, c.stream>>>(n, nb, mmax, X, HX, V, W, ld, st);
-        restart_set_kernel<<<1, 32, 0, c.stream>>>(nb, mmax, st);
+        k_rr<<<dim3(mmax, 2 * nb, nchunk), kDavThreads, 0, c.stream>>>(n, V, W, ld, rrp, mmax, st);
+        rr_sum_kernel<<<2 * nb, kJacobiMaxN, 0, c.stream>>>(nchunk, rrp, mmax, G, mmax, st);
+        k_jac<<<1, kJacobiThreads, jsmem, c.stream>>>(mmax, &st->m, G, mmax, th, Y, mmax, &st->jac);
+        k_ritz<<<dim3(grid1d(n, 128), nb, 2), 128, 0, c.stream>>>(n, V, W, ld, Y, mmax, X, HX, st);
+        k_res<<<dim3(nchunk, nb), kDavThreads, 0, c.stream>>>(n, HX, X, ld, th, H.diag, T, part);
+        step_begin_kernel<<<1, 32, 0, c.stream>>>(nwant, nb, mmax, nchunk, part, h2, st);
+        restart_copy_kernel<<<grid1d((int64_t)n * nb, 256), 256, 0, c.stream>>>(n, nb, X, HX, V, W, ld, st);
+        restart_set_kernel<<<1, 32, 0, c.stream>>>(nb, st);
         for (int q = 0; q < nb; q++) {
-            cand_begin_kernel<<<1, 256, 0, c.stream>>>(n, q, mmax, tol, h2, T, V, ld, st);
+            k_cand<<<nchunk, kDavThreads, 0, c.stream>>>(n, q, mmax, tol, h2, T, V, ld, pn0, st);
             for (int pass = 0; pass < 2; pass++) {
-                cgs_dot_kernel<<<mmax, 256, 0, c.stream>>>(n, V, ld, cf, st);
-                cgs_axpy_kernel<<<grid1d(n, 128), 128, 0, c.stream>>>(n, V, ld, cf, st);
+                k_dot<<<dim3(mmax, nchunk), kDavThreads, 0, c.stream>>>(n, q, V, ld, cf, mmax, st);
+                k_axpy<<<nchunk, kDavThreads, 0, c.stream>>>(n, q, V, ld, cf, mmax, pn1, st);
             }
-            cand_end_kernel<<<1, 256, 0, c.stream>>>(n, V, ld, st);
+            cand_end_kernel<<<nchunk, kDavThreads, 0, c.stream>>>(n, q, V, ld, pn0, pn1, st);
         }
-        if (nb > 4)
-            csr_hx_step_kernel<8><<<hx_blocks, 256, 0, c.stream>>>(n, H.rowptr, H.cols, H.vals, V, W, ld, st);
-        else if (nb > 2)
-            csr_hx_step_kernel<4><<<hx_blocks, 256, 0, c.stream>>>(n, H.rowptr, H.cols, H.vals, V, W, ld, st);
-        else
-            csr_hx_step_kernel<2><<<hx_blocks, 256, 0, c.stream>>>(n, H.rowptr, H.cols, H.vals, V, W, ld, st);
+        csr_hx(c, H, V, W, ld, nb, st);
         step_end_kernel<<<1, 32, 0, c.stream>>>(st);
         DCG_CUDA(cudaMemcpyAsync(hst, st, sizeof(DavState), cudaMemcpyDeviceToHost, c.stream));
     };
-    const int step_kernels = 9 + 6 * nb;   // kernels per step
-    if (nb > 8) throw Error{DCG_E_ARG, "davidson: more than 8 directions per step"};
+    const int step_kernels = 10 + 6 * nb;   // kernels per step
 
     static const bool use_graph = [] {
         const char *e = getenv("DCG_DAVIDSON_GRAPH");
