@@ -524,7 +524,9 @@ __device__ __forceinline__ void column_sync() { asm volatile("bar.sync 2, 512;" 
 __device__ __forceinline__ void sums_ready() { asm volatile("bar.arrive 3, 160;" ::: "memory"); }
 __device__ __forceinline__ void sums_wait() { asm volatile("bar.sync 3, 160;" ::: "memory"); }
 
-template <bool REAL, int ROWS>   // ROWS >= n / 128
+// GLB: the columns stay in global memory (L2, or HBM beyond it) and u has a row of shared memory of
+// its own; otherwise ROWS >= n / 128 and the chain warps hold u and v in registers.
+template <bool REAL, int ROWS, bool GLB>
 __device__ void tridiag_smem_body(const TrdJob &J, const int b, int *err, const unsigned long long limit_ns) {
     extern __shared__ cplx tsm2[];
     __shared__ double s_sum[4], s_ss[4], s_hdr[5], s_al;
@@ -536,24 +538,29 @@ __device__ void tridiag_smem_body(const TrdJob &J, const int b, int *err, const 
     const int tid = threadIdx.x, lane = tid & 31, q = (tid >> 5) & 3, s = tid >> 7;   // quarter, and warp within it
     const bool chain = s == 0, header = s == 4;
     const int nown = (n - b + nb - 1) / nb;   // columns b, b+nb, ...
-    cplx *cols = tsm2;                         // nown x n
-    cplx *sv = cols + (size_t)nown * n, *sw = sv + n;    // u, then v; x
-    double *part = reinterpret_cast<double *>(sw + n);   // [nown][4 quarters][2]
-    for (int64_t x = tid; x < (int64_t)nown * n; x += blockDim.x) {
-        const int c = (int)(x / n), r = (int)(x % n);
-        cols[x] = A[r + (int64_t)(b + c * nb) * lda];
+    cplx *sv = GLB ? tsm2 : tsm2 + (size_t)nown * n, *sw = sv + n;   // v (not GLB: first u) and x
+    cplx *su = GLB ? sw + n : sv;
+    double *part = reinterpret_cast<double *>(sw + (GLB ? 2 : 1) * (size_t)n);   // [nown][4 quarters][2]
+    auto column = [&](int c) { return GLB ? A + (int64_t)(b + c * nb) * lda : tsm2 + (size_t)c * n; };   // owned column
+    if (!GLB) {
+        for (int64_t x = tid; x < (int64_t)nown * n; x += blockDim.x) {
+            const int c = (int)(x / n), r = (int)(x % n);
+            tsm2[x] = A[r + (int64_t)(b + c * nb) * lda];
+        }
     }
     __syncthreads();
-    cplx vr[ROWS];   // chain warps: rows 32 (4 i + q) + lane of u, then of v
+    cplx vr[GLB ? 1 : ROWS];   // chain warps, not GLB: rows 32 (4 i + q) + lane of u, then of v
     const int NI = (n + 127) / 128;
-#define TRD_ROWS(i, r, from)                                                                    \
+    // the rows of a chain warp's lane, in groups of ROWS (not GLB: one group)
+#define TRD_GROUPS(i0) for (int i0 = 0; i0 < (GLB ? NI : 1); i0 += ROWS)
+#define TRD_ROWS(i0, i, r, from)                                                                \
     _Pragma("unroll") for (int i = 0; i < ROWS; i++)                                            \
-        if (const int r = 32 * (4 * i + q) + lane; i < NI && r >= (from) && r < n)
+        if (const int r = 32 * (4 * ((i0) + i) + q) + lane; (i0) + i < NI && r >= (from) && r < n)
     // Chain warps of the block that owns column k1: subtract the rank-2 term of the previous
     // column when upd, publish what lies below the reflector's first row, and leave that row's
     // element (alpha) and the parts of the squared norm for the header warp.
     auto panel = [&](int k1, bool upd) {
-        const cplx *col = cols + (size_t)((k1 - b) / nb) * n;
+        const cplx *col = column((k1 - b) / nb);
         cplx vj = mk(0.0, 0.0), yj = mk(0.0, 0.0);
         if (upd) {
             vj = sv[k1];
@@ -564,10 +571,10 @@ __device__ void tridiag_smem_body(const TrdJob &J, const int b, int *err, const 
         uint4 *uo = ub + (size_t)(k1 & 1) * 2 * n;
         const unsigned flag = (unsigned)k1 + 1u;
         double s0 = 0.0, s1 = 0.0;
-        TRD_ROWS(i, r, k1) {
+        TRD_GROUPS(i0) TRD_ROWS(i0, i, r, k1) {
             cplx a = col[r];
             if (upd) {
-                const cplx v = vr[i], x = sw[r];
+                const cplx v = GLB ? sv[r] : vr[GLB ? 0 : i], x = sw[r];
                 a.x = fma(-x.x, vj.x, a.x);
                 a.x = fma(-v.x, yj.x, a.x);
                 if (!REAL) {
@@ -587,7 +594,8 @@ __device__ void tridiag_smem_body(const TrdJob &J, const int b, int *err, const 
                 ll_store(uo + 2 * (size_t)r, a.x, flag);
                 if (!REAL) ll_store(uo + 2 * (size_t)r + 1, a.y, flag);
             }
-            vr[i] = a;
+            if (GLB) su[r] = a;
+            else vr[GLB ? 0 : i] = a;
             s0 = fma(a.x, a.x, s0);
             if (!REAL) s1 = fma(a.y, a.y, s1);
         }
@@ -611,34 +619,39 @@ __device__ void tridiag_smem_body(const TrdJob &J, const int b, int *err, const 
         if (chain && !owner) {   // u, straight from its words: one row until it is there, then all
             const uint4 *ui = ub + (size_t)par * 2 * n;
             LlWait wt;
-            unsigned pend = 0;
-            TRD_ROWS(i, r, k + 2) pend |= 1u << i;
-            bool all = false;
-            while (pend) {
-                const unsigned first = pend & (0u - pend);
-                all = all || (pend & (pend - 1)) == 0;
-                const unsigned look = all ? pend : first;
-                const unsigned before = pend;
-                TRD_ROWS(i, r, k + 2) {
-                    if (look >> i & 1u) {
-                        double x, y = 0.0;
-                        bool got = ll_load(ui + 2 * (size_t)r, flag, x);
-                        if (!REAL) got = ll_load(ui + 2 * (size_t)r + 1, flag, y) && got;
-                        if (got) {
-                            vr[i] = mk(x, y);
-                            pend &= ~(1u << i);
+            TRD_GROUPS(i0) {
+                unsigned pend = 0;
+                TRD_ROWS(i0, i, r, k + 2) pend |= 1u << i;
+                bool all = i0 > 0;
+                while (pend) {
+                    const unsigned first = pend & (0u - pend);
+                    all = all || (pend & (pend - 1)) == 0;
+                    const unsigned look = all ? pend : first;
+                    const unsigned before = pend;
+                    TRD_ROWS(i0, i, r, k + 2) {
+                        if (look >> i & 1u) {
+                            double x, y = 0.0;
+                            bool got = ll_load(ui + 2 * (size_t)r, flag, x);
+                            if (!REAL) got = ll_load(ui + 2 * (size_t)r + 1, flag, y) && got;
+                            if (got) {
+                                if (GLB) su[r] = mk(x, y);
+                                else vr[GLB ? 0 : i] = mk(x, y);
+                                pend &= ~(1u << i);
+                            }
                         }
                     }
+                    all = pend != before;
+                    // once a wait has run out the problem's error flag is set and every wait of its
+                    // blocks ends at once: the loop runs out on whatever values there are
+                    if (pend && wt.give_up(err, limit_ns)) break;
                 }
-                all = pend != before;
-                // once a wait has run out the problem's error flag is set and every wait of its
-                // blocks ends at once: the loop runs out on whatever values there are
-                if (pend && wt.give_up(err, limit_ns)) break;
             }
         }
         if (!header) {
-            column_sync();   // the previous column's update is done: sv may change
-            if (chain) TRD_ROWS(i, r, k + 1) sv[r] = r == k + 1 ? mk(0.0, 0.0) : vr[i];
+            if (!GLB) {
+                column_sync();   // the previous column's update is done: sv may change
+                if (chain) TRD_ROWS(0, i, r, k + 1) sv[r] = r == k + 1 ? mk(0.0, 0.0) : vr[GLB ? 0 : i];
+            }
             column_sync();
         }
         const int p0 = (k + 2) >> 5, pe = (n + 31) >> 5;   // pieces of 32 rows with rows > k + 1
@@ -671,11 +684,12 @@ __device__ void tridiag_smem_body(const TrdJob &J, const int b, int *err, const 
                 const bool two = c + 4 < nown;
                 {
                     const int j = b + c * nb;
-                    const cplx *col = cols + (size_t)c * n;
+                    const cplx *col = column(c);
+#pragma unroll 2
                     for (int p = p0 + ((q - j - p0) & 3); p < pe; p += 4) {
                         const int r = 32 * p + lane;
                         if (r > k + 1 && r < n) {
-                            const cplx a = col[r], v = sv[r];
+                            const cplx a = col[r], v = su[r];
                             a0 = fma(a.x, v.x, a0);
                             if (!REAL) {
                                 a1 = fma(a.x, v.y, a1);
@@ -687,11 +701,12 @@ __device__ void tridiag_smem_body(const TrdJob &J, const int b, int *err, const 
                 }
                 if (two) {
                     const int j = b + (c + 4) * nb;
-                    const cplx *col = cols + (size_t)(c + 4) * n;
+                    const cplx *col = column(c + 4);
+#pragma unroll 2
                     for (int p = p0 + ((q - j - p0) & 3); p < pe; p += 4) {
                         const int r = 32 * p + lane;
                         if (r > k + 1 && r < n) {
-                            const cplx a = col[r], v = sv[r];
+                            const cplx a = col[r], v = su[r];
                             a2 = fma(a.x, v.x, a2);
                             if (!REAL) {
                                 a3 = fma(a.x, v.y, a3);
@@ -736,7 +751,7 @@ __device__ void tridiag_smem_body(const TrdJob &J, const int b, int *err, const 
                 double y = 0.0;
                 cplx a = mk(0.0, 0.0);
                 if (t < cnt) {
-                    a = cols[(size_t)c * n + k + 1];
+                    a = column(c)[k + 1];
                     const double *p = part + (size_t)c * 8 + comp;
                     if (!REAL || comp == 0) y = (p[0] + p[2]) + (p[4] + p[6]);
                 }
@@ -752,11 +767,12 @@ __device__ void tridiag_smem_body(const TrdJob &J, const int b, int *err, const 
             }
         }
         if (chain) {   // v = sc u below its first row
-            TRD_ROWS(i, r, k + 1) {
+            TRD_GROUPS(i0) TRD_ROWS(i0, i, r, k + 1) {
+                const cplx u = GLB ? su[r] : vr[GLB ? 0 : i];
                 const cplx v = r == k + 1 ? mk(1.0, 0.0)
-                                          : (REAL ? mk(vr[i].x * sx, 0.0)
-                                                  : mk(fma(vr[i].x, sx, -vr[i].y * sy), fma(vr[i].x, sy, vr[i].y * sx)));
-                vr[i] = v;
+                                          : (REAL ? mk(u.x * sx, 0.0)
+                                                  : mk(fma(u.x, sx, -u.y * sy), fma(u.x, sy, u.y * sx)));
+                if (!GLB) vr[GLB ? 0 : i] = v;
                 sv[r] = v;
                 if (owner) A[r + (int64_t)k * lda] = v;
             }
@@ -768,35 +784,37 @@ __device__ void tridiag_smem_body(const TrdJob &J, const int b, int *err, const 
             if (nb > 1) {
                 const uint4 *xi = xb + (size_t)par * 2 * n;
                 LlWait wt;
-                unsigned pend = 0;
-                TRD_ROWS(i, r, k + 1) pend |= 1u << i;
-                bool all = true;
-                while (pend) {
-                    const unsigned look = all ? pend : (pend & (0u - pend)), before = pend;
-                    TRD_ROWS(i, r, k + 1) {
-                        if (look >> i & 1u) {
-                            double x, y = 0.0;
-                            bool got = ll_load(xi + 2 * (size_t)r, flag, x);
-                            if (!REAL) got = ll_load(xi + 2 * (size_t)r + 1, flag, y) && got;
-                            if (got) {
-                                sw[r] = mk(x, y);
-                                pend &= ~(1u << i);
+                TRD_GROUPS(i0) {
+                    unsigned pend = 0;
+                    TRD_ROWS(i0, i, r, k + 1) pend |= 1u << i;
+                    bool all = true;
+                    while (pend) {
+                        const unsigned look = all ? pend : (pend & (0u - pend)), before = pend;
+                        TRD_ROWS(i0, i, r, k + 1) {
+                            if (look >> i & 1u) {
+                                double x, y = 0.0;
+                                bool got = ll_load(xi + 2 * (size_t)r, flag, x);
+                                if (!REAL) got = ll_load(xi + 2 * (size_t)r + 1, flag, y) && got;
+                                if (got) {
+                                    sw[r] = mk(x, y);
+                                    pend &= ~(1u << i);
+                                }
                             }
                         }
+                        all = pend != before;
+                        if (pend && wt.give_up(err, limit_ns)) break;
                     }
-                    all = pend != before;
-                    if (pend && wt.give_up(err, limit_ns)) break;
                 }
             }
             double z0 = 0.0, z1 = 0.0, z2 = 0.0, z3 = 0.0;
-            TRD_ROWS(i, r, k + 1) {
-                const cplx x = sw[r];
+            TRD_GROUPS(i0) TRD_ROWS(i0, i, r, k + 1) {
+                const cplx x = sw[r], v = GLB ? sv[r] : vr[GLB ? 0 : i];
                 if (i & 1) {
-                    z2 = fma(x.x, vr[i].x, z2);
-                    if (!REAL) z3 = fma(x.y, vr[i].y, z3);
+                    z2 = fma(x.x, v.x, z2);
+                    if (!REAL) z3 = fma(x.y, v.y, z3);
                 } else {
-                    z0 = fma(x.x, vr[i].x, z0);
-                    if (!REAL) z1 = fma(x.y, vr[i].y, z1);
+                    z0 = fma(x.x, v.x, z0);
+                    if (!REAL) z1 = fma(x.y, v.y, z1);
                 }
             }
             double z = REAL ? z0 + z2 : (z0 + z1) + (z2 + z3);
@@ -816,9 +834,10 @@ __device__ void tridiag_smem_body(const TrdJob &J, const int b, int *err, const 
             const double a2 = 2.0 * s_al;
             for (int c = c1 + ((s - c1) & 3); c < nown; c += 4) {
                 const int j = b + c * nb;
-                cplx *col = cols + (size_t)c * n;
+                cplx *col = column(c);
                 const cplx vj = sv[j], xj = sw[j];
                 const cplx yj = mk(fma(a2, vj.x, xj.x), fma(a2, vj.y, xj.y));
+#pragma unroll 2
                 for (int p = p0 + ((q - j - p0) & 3); p < pe; p += 4) {
                     const int r = 32 * p + lane;
                     if (r > k + 1 && r < n) {
@@ -842,6 +861,7 @@ __device__ void tridiag_smem_body(const TrdJob &J, const int b, int *err, const 
         }
     }
 #undef TRD_ROWS
+#undef TRD_GROUPS
 }
 
 // Batched tridiagonalisation: several Hermitian matrices in one launch, each reduced by its own
@@ -855,15 +875,26 @@ __global__ void __launch_bounds__(TRS_THREADS) tridiag_smem_batched_kernel(const
     const TrdJob &J = T.j[j];
     const int b = (int)blockIdx.x - J.b0;
     if (J.n <= 512) {
-        if (J.real) tridiag_smem_body<true, 4>(J, b, T.err + j, T.limit_ns);
-        else tridiag_smem_body<false, 4>(J, b, T.err + j, T.limit_ns);
+        if (J.real) tridiag_smem_body<true, 4, false>(J, b, T.err + j, T.limit_ns);
+        else tridiag_smem_body<false, 4, false>(J, b, T.err + j, T.limit_ns);
     } else if (J.n <= 1024) {
-        if (J.real) tridiag_smem_body<true, 8>(J, b, T.err + j, T.limit_ns);
-        else tridiag_smem_body<false, 8>(J, b, T.err + j, T.limit_ns);
+        if (J.real) tridiag_smem_body<true, 8, false>(J, b, T.err + j, T.limit_ns);
+        else tridiag_smem_body<false, 8, false>(J, b, T.err + j, T.limit_ns);
     } else {
-        if (J.real) tridiag_smem_body<true, kTrdRows>(J, b, T.err + j, T.limit_ns);
-        else tridiag_smem_body<false, kTrdRows>(J, b, T.err + j, T.limit_ns);
+        if (J.real) tridiag_smem_body<true, kTrdRows, false>(J, b, T.err + j, T.limit_ns);
+        else tridiag_smem_body<false, kTrdRows, false>(J, b, T.err + j, T.limit_ns);
     }
+}
+
+// One matrix beyond the blocks' shared memory, over every SM: the same column loop on columns in
+// global memory.  Bound by the FP64 unit (12 FMAs an element and column: 66 ms at order 2002 at
+// 485 GFMA/s), the three passes over the trailing matrix a column from L2 or HBM beside it.
+// Measured against the kernel with two grid barriers a column that every block's reflector waits
+// for: order 1300 44 -> 27 ms, 2002 210 -> 82 ms, 2744 437 -> 191 ms.
+__global__ void __launch_bounds__(TRS_THREADS) tridiag_global_kernel(const __grid_constant__ TrdTable T) {
+    const TrdJob &J = T.j[0];
+    if (J.real) tridiag_smem_body<true, 8, true>(J, (int)blockIdx.x, T.err, T.limit_ns);
+    else tridiag_smem_body<false, 8, true>(J, (int)blockIdx.x, T.err, T.limit_ns);
 }
 
 // ===================================================================== 2. divide and conquer
@@ -2111,7 +2142,7 @@ static void trd_clear(Context &c, const std::vector<TrdJob> &jobs) {
 // cooperative, or with ncta > 0 one cluster of ncta blocks per job.  Returns each job's error
 // flag, read back after the launch completes.
 static std::vector<int> trd_launch(Context &c, const std::vector<TrdJob> &jobs, int total, size_t smem,
-                                   cudaStream_t stream, const char *table, int ncta = 0) {
+                                   cudaStream_t stream, const char *table, int ncta = 0, bool global = false) {
     const size_t nj = jobs.size();
     TrdTable T{};
     for (size_t q = 0; q < nj; q++) T.j[q] = jobs[q];
@@ -2136,8 +2167,8 @@ static std::vector<int> trd_launch(Context &c, const std::vector<TrdJob> &jobs, 
         DCG_CUDA(cudaLaunchKernelEx(&cfg, tridiag_smem_batched_kernel, T));
     } else {
         void *args[] = {&T};
-        DCG_CUDA(cudaLaunchCooperativeKernel((const void *)tridiag_smem_batched_kernel, dim3(total), dim3(TRS_THREADS),
-                                             args, smem, stream));
+        const void *kern = global ? (const void *)tridiag_global_kernel : (const void *)tridiag_smem_batched_kernel;
+        DCG_CUDA(cudaLaunchCooperativeKernel(kern, dim3(total), dim3(TRS_THREADS), args, smem, stream));
     }
     DCG_CUDA(cudaGetLastError());
     DCG_CUDA(cudaMemcpyAsync(herr, T.err, nj * sizeof(int), cudaMemcpyDeviceToHost, stream));
@@ -2367,8 +2398,40 @@ static bool tridiag_smem_batched(Context &c, std::vector<TrdJob> &jobs) {
     return true;
 }
 
-// One matrix: the L2-resident persistent kernel, or one kernel launch per column beyond it.
+// One matrix on columns in global memory (tridiag_global_kernel); false when v, x and u do not fit
+// a block's shared memory (n above about 4800).
+static bool tridiag_global(Context &c, int n, cplx *A, int64_t lda, HeevWork &h) {
+    const int nb = std::min(std::max(1, c.num_sms), n);
+    const size_t smem = 3 * sizeof(cplx) * (size_t)n + ((size_t)(n + nb - 1) / nb) * 8 * sizeof(double);
+    if (smem > trd_smem_limit(c)) return false;
+    std::lock_guard<std::mutex> coop(g_coop_mutex);
+    DCG_CUDA(cudaFuncSetAttribute(tridiag_global_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)trd_smem_limit(c)));
+    int per_sm = 0;
+    DCG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, tridiag_global_kernel, TRS_THREADS, smem));
+    if (per_sm < 1) return false;
+    TrdJob j{};
+    j.A = A;
+    j.lda = lda;
+    j.d = h.d;
+    j.e = h.e;
+    j.tau = h.tau;
+    j.ll = wsget<uint4>(c, "trd.ll.global", trd_ll_words(n));
+    j.n = n;
+    j.nb = nb;
+    j.real = c.real_now;
+    std::vector<TrdJob> jobs(1, j);
+    trd_clear(c, jobs);
+    const std::vector<int> he = trd_launch(c, jobs, nb, smem, c.stream, "trd.err.global", 0, true);
+    c.launches++;
+    if (he[0]) throw Error{DCG_E_NUMERIC, "tridiagonalisation: a grid barrier wait timed out"};
+    return true;
+}
+
+// One matrix: columns in global memory, the L2-resident persistent kernel, or one kernel launch per
+// column beyond it.
 static void tridiag_single(Context &c, int n, cplx *A, int64_t lda, HeevWork &h) {
+    if (tridiag_global(c, n, A, lda, h)) return;
     if (n <= kTridiagPersistentMaxN) {
         tridiag_persistent(c, n, A, lda, h);
         return;
