@@ -267,6 +267,15 @@ __global__ void unit_cols_kernel(int n, int m, const int *__restrict__ idx, cplx
 // that size, real: whole call 310 ms before, 98 ms with the chunks, real arithmetic, the Rayleigh
 // elements of new vectors alone and the determinant table of the matrix build.
 constexpr int kDavChunk = 1024, kDavThreads = 256;
+constexpr int kAxpyRows = 128;   // rows (and threads) of a block that subtracts: its loop over the vectors is the long one
+
+// Sum of n values by one warp in a fixed order (every lane gets it).
+__device__ __forceinline__ double warp_total(const double *x, int n, int stride = 1) {
+    double s = 0.0;
+    for (int i = threadIdx.x & 31; i < n; i += 32) s += x[(int64_t)i * stride];
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    return s;
+}
 
 // Sums of a complex (re, im) pair over the block; real vectors carry no im.
 template <bool REAL>
@@ -322,15 +331,20 @@ __global__ void __launch_bounds__(kDavThreads) rr_part_kernel(int n, const cplx 
     dav_block_sum<REAL>(re, im, sh);
     if (threadIdx.x == 0) part[i + (int64_t)mmax * (blockIdx.y + 16 * (int64_t)blockIdx.z)] = mk(re, im);
 }
+template <bool REAL>
 __global__ void rr_sum_kernel(int nchunk, const cplx *__restrict__ part, int mmax, cplx *G, int ldg,
                               const DavState *__restrict__ st) {
-    const int i = threadIdx.x, j = st->mold + blockIdx.x;
-    if (j >= st->m || i > j) return;
-    cplx s = mk(0.0, 0.0);
-    for (int c = 0; c < nchunk; c++) s = cadd(s, part[i + (int64_t)mmax * (blockIdx.x + 16 * (int64_t)c)]);
-    if (i == j) s.y = 0.0;
-    G[i + (int64_t)ldg * j] = s;
-    G[j + (int64_t)ldg * i] = cconj(s);
+    const int j = st->mold + blockIdx.x, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+    if (j >= st->m) return;
+    for (int i = threadIdx.x >> 5; i <= j; i += nw) {   // a warp per element
+        const double *x = reinterpret_cast<const double *>(part + i + (int64_t)mmax * blockIdx.x);
+        const int stride = 2 * mmax * 16;
+        const double re = warp_total(x, nchunk, stride), im = REAL || i == j ? 0.0 : warp_total(x + 1, nchunk, stride);
+        if (lane == 0) {
+            G[i + (int64_t)ldg * j] = mk(re, im);
+            G[j + (int64_t)ldg * i] = mk(re, -im);
+        }
+    }
 }
 
 // X = V Y[:, :nb] (z = 0) and HX = W Y[:, :nb] (z = 1) over the m columns of V and W.
@@ -381,11 +395,9 @@ __global__ void __launch_bounds__(kDavThreads) residual_kernel(int n, const cplx
 __global__ void step_begin_kernel(int nwant, int nb, int mmax, int nchunk, const double *__restrict__ part, double *h2,
                                   DavState *st) {
     __shared__ double v[8];
-    if (threadIdx.x < nb) {
-        double s = 0.0;
-        for (int c = 0; c < nchunk; c++) s += part[c + (int64_t)nchunk * threadIdx.x];
-        h2[threadIdx.x] = s;
-        v[threadIdx.x] = s;
+    for (int q = threadIdx.x >> 5; q < nb; q += blockDim.x >> 5) {   // a warp per root
+        const double s = warp_total(part + (int64_t)nchunk * q, nchunk);
+        if ((threadIdx.x & 31) == 0) v[q] = h2[q] = s;
     }
     __syncthreads();
     if (threadIdx.x != 0) return;
@@ -458,27 +470,27 @@ __global__ void __launch_bounds__(kDavThreads) cgs_dot_kernel(int n, int q, cons
 }
 
 template <bool REAL>
-__global__ void __launch_bounds__(kDavThreads) cgs_axpy_kernel(int n, int q, cplx *V, int64_t ld,
-                                                               const cplx *__restrict__ cf, int mmax, double *part2,
-                                                               const DavState *__restrict__ st) {
+__global__ void __launch_bounds__(kAxpyRows) cgs_axpy_kernel(int n, int q, int nchunk, cplx *V, int64_t ld,
+                                                             const cplx *__restrict__ cf, int mmax, double *part2,
+                                                             const DavState *__restrict__ st) {
     __shared__ double sh[32];
     __shared__ cplx c[kJacobiMaxN];
     if (!st->live[q]) return;
     const int mm = dav_col(st, q);
-    for (int i = threadIdx.x; i < mm; i += kDavThreads) {
-        cplx s = mk(0.0, 0.0);
-        for (int k = 0; k < (int)gridDim.x; k++) {
-            const cplx x = cf[i + (int64_t)mmax * k];
-            s.x += x.x;
-            if (!REAL) s.y += x.y;
+    if (nchunk == 1) {
+        for (int i = threadIdx.x; i < mm; i += kAxpyRows) c[i] = cf[i];
+    } else {
+        for (int i = threadIdx.x >> 5; i < mm; i += kAxpyRows / 32) {   // a warp per coefficient
+            const double *x = reinterpret_cast<const double *>(cf + i);
+            const double re = warp_total(x, nchunk, 2 * mmax), im = REAL ? 0.0 : warp_total(x + 1, nchunk, 2 * mmax);
+            if ((threadIdx.x & 31) == 0) c[i] = mk(re, im);
         }
-        c[i] = s;
     }
     __syncthreads();
     cplx *dst = V + ld * mm;
     double acc = 0.0;
-    const int k0 = blockIdx.x * kDavChunk, k1 = min(n, k0 + kDavChunk);
-    for (int r = k0 + threadIdx.x; r < k1; r += kDavThreads) {
+    const int r = blockIdx.x * kAxpyRows + threadIdx.x;
+    if (r < n) {
         cplx s = mk(0.0, 0.0);
         for (int p = 0; p < mm; p++) {
             const cplx v = V[r + ld * p];
@@ -498,20 +510,18 @@ __global__ void __launch_bounds__(kDavThreads) cgs_axpy_kernel(int n, int q, cpl
 // direction after it is tried.
 __global__ void __launch_bounds__(kDavThreads) cand_end_kernel(int n, int q, cplx *V, int64_t ld,
                                                                const double *__restrict__ part,
-                                                               const double *__restrict__ part2, DavState *st) {
+                                                               const double *__restrict__ part2, int npart2, DavState *st) {
     if (!st->live[q]) return;
     __shared__ double s_scale;
     __shared__ int s_ok;
     const int col = dav_col(st, q);
-    if (threadIdx.x == 0) {
-        double n0 = 0.0, acc = 0.0;
-        for (int k = 0; k < (int)gridDim.x; k++) {
-            n0 += part[k];
-            acc += part2[k];
+    if (threadIdx.x < 32) {
+        const double n0 = warp_total(part, (int)gridDim.x), acc = warp_total(part2, npart2);
+        if (threadIdx.x == 0) {
+            s_ok = acc > 1e-20 * n0 && acc > 0.0;
+            s_scale = s_ok ? 1.0 / sqrt(acc) : 0.0;
+            if (blockIdx.x == 0) st->ok[q] = s_ok;   // read by later launches only
         }
-        s_ok = acc > 1e-20 * n0 && acc > 0.0;
-        s_scale = s_ok ? 1.0 / sqrt(acc) : 0.0;
-        if (blockIdx.x == 0) st->ok[q] = s_ok;   // read by later launches only
     }
     __syncthreads();
     if (!s_ok) return;
@@ -612,7 +622,12 @@ static void csr_hx(Context &c, const CsrMatrix &H, const cplx *X, cplx *Y, int64
 void davidson_lowest_csr(Context &c, const CsrMatrix &H, int nwant, double *w, cplx *Z, double tol_rel, int maxit) {
     const int n = H.n;
     const int nb = std::min(n, nwant + 2);   // block: the wanted roots and a margin for near-degeneracy
-    const int mmax = std::min(n, std::min(kJacobiMaxN, std::max(24, 8 * nb)));
+    // A long subspace saves iterations (each one product with H), a short one keeps the one-block
+    // Jacobi short (its time grows with the cube): at 924 determinants 12 vectors took 20
+    // steps and 5.9 ms where 24 took 18 and 8.5; at 74,273 determinants (0.9 ms a product) the
+    // products decide.
+    const double hx_s = (double)H.nnz * nb * (H.rvals ? 1.0 : 4.0) / 4.0e11;
+    const int mmax = std::min(n, std::min(kJacobiMaxN, hx_s > 0.6e-3 ? std::max(24, 8 * nb) : std::max(12, 4 * nb)));
     if (nwant < 1 || nb > mmax || n < 2) throw Error{DCG_E_ARG, "davidson: block does not fit the subspace"};
     const int64_t ld = n;
     cplx *V = wsget<cplx>(c, "dav.V", (size_t)n * mmax);
@@ -625,7 +640,8 @@ void davidson_lowest_csr(Context &c, const CsrMatrix &H, int nwant, double *w, c
     const int nchunk = (int)grid1d(n, kDavChunk);
     cplx *cf = wsget<cplx>(c, "dav.cf", (size_t)mmax * nchunk);
     cplx *rrp = wsget<cplx>(c, "dav.rrp", (size_t)mmax * 16 * nchunk);
-    double *part = wsget<double>(c, "dav.part", (size_t)nchunk * 10);   // residuals (8), then a direction's two norms
+    const int nrow = (int)grid1d(n, kAxpyRows);
+    double *part = wsget<double>(c, "dav.part", (size_t)nchunk * 9 + nrow);   // residuals (8), then a direction's two norms
     double *pn0 = part + (size_t)nchunk * 8, *pn1 = pn0 + nchunk;
     double *th = wsget<double>(c, "dav.th", mmax);
     double *h2 = wsget<double>(c, "dav.h2", (size_t)nb);
@@ -661,6 +677,7 @@ void davidson_lowest_csr(Context &c, const CsrMatrix &H, int nwant, double *w, c
     DCG_CUDA(cudaFuncSetAttribute(k_jac, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   2 * (int)sizeof(cplx) * kJacobiMaxN * kJacobiMaxN));
     auto *k_rr = real ? rr_part_kernel<true> : rr_part_kernel<false>;
+    auto *k_rrs = real ? rr_sum_kernel<true> : rr_sum_kernel<false>;
     auto *k_ritz = real ? ritz_kernel<true> : ritz_kernel<false>;
     auto *k_res = real ? residual_kernel<true> : residual_kernel<false>;
     auto *k_cand = real ? cand_begin_kernel<true> : cand_begin_kernel<false>;
@@ -668,20 +685,20 @@ void davidson_lowest_csr(Context &c, const CsrMatrix &H, int nwant, double *w, c
     auto *k_axpy = real ? cgs_axpy_kernel<true> : cgs_axpy_kernel<false>;
     auto enqueue_step = [&]() {
         k_rr<<<dim3(mmax, 2 * nb, nchunk), kDavThreads, 0, c.stream>>>(n, V, W, ld, rrp, mmax, st);
-        rr_sum_kernel<<<2 * nb, kJacobiMaxN, 0, c.stream>>>(nchunk, rrp, mmax, G, mmax, st);
+        k_rrs<<<2 * nb, 256, 0, c.stream>>>(nchunk, rrp, mmax, G, mmax, st);
         k_jac<<<1, kJacobiThreads, jsmem, c.stream>>>(mmax, &st->m, G, mmax, th, Y, mmax, &st->jac);
         k_ritz<<<dim3(grid1d(n, 128), nb, 2), 128, 0, c.stream>>>(n, V, W, ld, Y, mmax, X, HX, st);
         k_res<<<dim3(nchunk, nb), kDavThreads, 0, c.stream>>>(n, HX, X, ld, th, H.diag, T, part);
-        step_begin_kernel<<<1, 32, 0, c.stream>>>(nwant, nb, mmax, nchunk, part, h2, st);
+        step_begin_kernel<<<1, 256, 0, c.stream>>>(nwant, nb, mmax, nchunk, part, h2, st);
         restart_copy_kernel<<<grid1d((int64_t)n * nb, 256), 256, 0, c.stream>>>(n, nb, X, HX, V, W, ld, st);
         restart_set_kernel<<<1, 32, 0, c.stream>>>(nb, st);
         for (int q = 0; q < nb; q++) {
             k_cand<<<nchunk, kDavThreads, 0, c.stream>>>(n, q, mmax, tol, h2, T, V, ld, pn0, st);
             for (int pass = 0; pass < 2; pass++) {
                 k_dot<<<dim3(mmax, nchunk), kDavThreads, 0, c.stream>>>(n, q, V, ld, cf, mmax, st);
-                k_axpy<<<nchunk, kDavThreads, 0, c.stream>>>(n, q, V, ld, cf, mmax, pn1, st);
+                k_axpy<<<nrow, kAxpyRows, 0, c.stream>>>(n, q, nchunk, V, ld, cf, mmax, pn1, st);
             }
-            cand_end_kernel<<<nchunk, kDavThreads, 0, c.stream>>>(n, q, V, ld, pn0, pn1, st);
+            cand_end_kernel<<<nchunk, kDavThreads, 0, c.stream>>>(n, q, V, ld, pn0, pn1, nrow, st);
         }
         csr_hx(c, H, V, W, ld, nb, st);
         step_end_kernel<<<1, 32, 0, c.stream>>>(st);
