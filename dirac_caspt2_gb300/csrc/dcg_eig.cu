@@ -966,6 +966,9 @@ __device__ __forceinline__ double dc_group_prod(double v) {
     return v;
 }
 
+// sqrt(max(x, 0)) for a model's discriminant: FP64 operations on the pipe are what a step costs.
+__device__ __forceinline__ double dc_sqrt(double x) { return x > 1e-280 ? x * fast_rsqrt(x) : x > 0.0 ? sqrt(x) : 0.0; }
+
 // Secular root j of 1/rho + sum_i z_i^2 / (d_i - lambda) = 0 by a group of G lanes (all lanes of
 // the warp call, `act` false for groups without a root).  The root lies in (d_j, d_{j+1}) (the
 // last one in (d_{k-1}, d_{k-1} + rho |z|^2)) and is found as an offset tau from the nearer pole
@@ -1029,11 +1032,11 @@ __device__ void dc_secular_root(int k, int j, bool act, const double *dk, const 
     {
         const double s1 = zj2, s2 = zr2;
         if (last) {
-            tau = fmin(s1 / c0, hi);
+            tau = fmin(s1 * fast_rcp(c0), hi);
         } else {
             const double B = c0 * (dL + dR) + s1 + s2, C = s1 * dR + s2 * dL;
-            const double q = 0.5 * (B + copysign(sqrt(fmax(B * B - 4.0 * c0 * C, 0.0)), B));
-            tau = B > 0.0 ? C / q : q / c0;
+            const double q = 0.5 * (B + copysign(dc_sqrt(fma(B, B, -4.0 * c0 * C)), B));
+            tau = B > 0.0 ? C * fast_rcp(q) : q * fast_rcp(c0);
         }
         if (!(tau > lo && (tau < hi || (last && tau == hi)))) tau = 0.5 * (lo + hi);
     }
@@ -1075,10 +1078,10 @@ __device__ void dc_secular_root(int k, int j, bool act, const double *dk, const 
             const double a2 = dph * (dR - tau), s2 = a2 * (dR - tau);
             cc += ph - a2;
             const double B = cc * (dL + dR) + s1 + s2, C = s1 * dR + s2 * dL;
-            const double q = 0.5 * (B + copysign(sqrt(fmax(B * B - 4.0 * cc * C, 0.0)), B));
-            y = B > 0.0 ? C / q : q / cc;
+            const double q = 0.5 * (B + copysign(dc_sqrt(fma(B, B, -4.0 * cc * C)), B));
+            y = B > 0.0 ? C * fast_rcp(q) : q * fast_rcp(cc);
         } else {
-            y = cc > 0.0 ? fmin(dL + s1 / cc, hi) : NAN;   // the upper end itself is a root when k = 1
+            y = cc > 0.0 ? fmin(fma(s1, fast_rcp(cc), dL), hi) : NAN;   // the upper end itself is a root when k = 1
         }
         if (!(y > lo && (y < hi || (last && y == hi)))) {
             if (!run) continue;   // the last step stays where it is
@@ -1097,6 +1100,24 @@ __device__ void dc_secular_root(int k, int j, bool act, const double *dk, const 
 // one by a rotation (|t c s| <= tol for c = zn / |z|, s = zp / |z|), without a division.
 __device__ __forceinline__ bool dc_close(double t, double zp, double zn, double tol) {
     return fabs(t * zp * zn) <= tol * fma(zp, zp, zn * zn);
+}
+
+// One pair rotation of the deflation scan: component zp folds into zn.
+__device__ __forceinline__ void dc_rotate(double &dp, double zp, double &dn, double &zn, double &C, double &S) {
+    const double t2 = fma(zn, zn, zp * zp), a = dp, c = dn;
+    if (t2 > 1e-280) {
+        const double ri = fast_rsqrt(t2);
+        C = zn * ri;
+        S = -zp * ri;
+        zn = t2 * ri;
+    } else {   // the squares are out of range
+        const double tt = hypot(zn, zp);
+        C = zn / tt;
+        S = -zp / tt;
+        zn = tt;
+    }
+    dp = a * C * C + c * S * S;
+    dn = a * S * S + c * C * C;
 }
 
 // Levels up to nodes of kDcBase columns in one launch: a block of 128 threads merges its columns
@@ -1171,16 +1192,16 @@ __global__ void __launch_bounds__(128) dc_base_kernel(int n, const double *__res
                 for (int t = s; t < s + N; t++) {
                     if (!st[t]) continue;
                     if (pj >= 0 && dc_close(pd[t] - pd[pj], pz[pj], pz[t], tol)) {
-                        const double zt = hypot(pz[t], pz[pj]), C = pz[t] / zt, S = -pz[pj] / zt;
-                        const double a = pd[pj], c = pd[t];
+                        double C, S, zt = pz[t], a = pd[pj], c = pd[t];
+                        dc_rotate(a, pz[pj], c, zt, C, S);
                         rp[s + nr] = sp[pj];
                         rn[s + nr] = sp[t];
                         rc[s + nr] = C;
                         rs[s + nr] = S;
                         nr++;
                         pz[t] = zt;
-                        pd[pj] = a * C * C + c * S * S;
-                        pd[t] = a * S * S + c * C * C;
+                        pd[pj] = a;
+                        pd[t] = c;
                         st[pj] = 0;
                     }
                     pj = t;
@@ -1234,7 +1255,7 @@ __global__ void __launch_bounds__(128) dc_base_kernel(int n, const double *__res
             const double di = dk[c];
             for (int j = gl; j < k; j += 4) {
                 const double dl = fabs((di - dk[s + ord[s + j]]) - tau[s + j]);
-                p *= j == i ? dl : dl / fabs(dk[s + j] - di);
+                p *= j == i ? dl : dl * fast_rcp(fabs(dk[s + j] - di));
             }
         }
         p = dc_group_prod<4>(p);
@@ -1316,16 +1337,6 @@ __device__ int dc_block_excl_scan(int v, int *wsum, int &total) {
     const int base = (wid > 0 ? wsum[wid - 1] : 0) + x - v;
     __syncthreads();
     return base;
-}
-
-// One pair rotation of the deflation scan: component pj folds into nj.
-__device__ __forceinline__ void dc_rotate(double &dp, double zp, double &dn, double &zn, double &C, double &S) {
-    const double tt = hypot(zn, zp), a = dp, c = dn;
-    C = zn / tt;
-    S = -zp / tt;
-    zn = tt;
-    dp = a * C * C + c * S * S;
-    dn = a * S * S + c * C * C;
 }
 
 // One block per node: rank-one vector, merge order, deflation.  Deflation runs in parallel: the
@@ -1577,7 +1588,7 @@ __global__ void __launch_bounds__(DM_THREADS) dc_merge_kernel(int n, int full, i
             double p = 1.0;
             for (int j = lane; j < k; j += 32) {
                 const double dl = fabs((di - dk[b.ord[s + j]]) - b.tau[s + j]);
-                p *= (j == i) ? dl : dl / fabs(dk[j] - di);
+                p *= (j == i) ? dl : dl * fast_rcp(fabs(dk[j] - di));
             }
             p = eig_warp_prod(p);
             if (lane == 0) b.zh[s + i] = copysign(sqrt(p), b.zK[s + i]);
