@@ -362,37 +362,44 @@ static int casci(Context &c, int nroot, double *eigen_out, double *ci_re, double
 // FP64-bound on a GB300 (8 M K^2 flops at ~1.2 TF/s against one pass over the class), so
 // only trivial dimensions stay on the FP64 kernels.
 constexpr int kSplitMinK = 4;
+// ... and whose FP64 work is worth it: a split product is four launches (row exponents, two
+// slicings, the product) and 12 us or more whatever its size, the time of about 5e6 FP64 FMAs
+// on the GPU (485 GFMA/s), so smaller products take the FP64 kernels: 144 launches of the
+// 8/6/40 transformation in 1.2 ms become 36.  Real systems need one FMA a multiply-add, not four.
+constexpr double kSplitMinFma = 5.0e6;
+static bool split_pays(const Context &c, double m, double n, double k, double batch = 1.0) {
+    return c.precision == DCG_PREC_SPLIT && k > kSplitMinK && m * n * k * batch * (c.real_now ? 1.0 : 4.0) >= kSplitMinFma;
+}
 
 static void transform4(Context &c, const cplx *in, cplx *out, cplx *tmp, const int dm[4], const cplx *U[4]) {
     const int64_t d0 = dm[0], d1 = dm[1], d2 = dm[2], d3 = dm[3];
     const int64_t tot = d0 * d1 * d2 * d3;
     if (tot == 0) return;
     const cplx one = mk(1.0, 0.0), zero = mk(0.0, 0.0);
-    const bool split = c.precision == DCG_PREC_SPLIT;
     const int lb = c.split_lbo, sb = c.split_sbo;
     // l: tmp = in * U4
-    if (split && d3 > kSplitMinK)
+    if (split_pays(c, (double)d0 * d1 * d2, d3, d3))
         zgemm_split(c, (int)(d0 * d1 * d2), (int)d3, (int)d3, 1, in, 1, d0 * d1 * d2, 0, U[3], d3, 0, tmp, 1,
                     d0 * d1 * d2, 0, false, lb, sb);
     else
         zgemm(c, OP_N, OP_N, (int)(d0 * d1 * d2), (int)d3, (int)d3, one, in, d0 * d1 * d2, 0, U[3], d3, 0, zero, tmp,
               d0 * d1 * d2, 0, 1);
     // k: out_l = tmp_l * conj(U3)
-    if (split && d2 > kSplitMinK)
+    if (split_pays(c, (double)d0 * d1, d2, d2, d3))
         zgemm_split(c, (int)(d0 * d1), (int)d2, (int)d2, (int)d3, tmp, 1, d0 * d1, d0 * d1 * d2, U[2], d2, 1, out, 1,
                     d0 * d1, d0 * d1 * d2, false, lb, sb);
     else
         zgemm(c, OP_N, OP_R, (int)(d0 * d1), (int)d2, (int)d2, one, tmp, d0 * d1, d0 * d1 * d2, U[2], d2, 0, zero,
               out, d0 * d1, d0 * d1 * d2, (int)d3);
     // j: tmp_kl = out_kl * U2
-    if (split && d1 > kSplitMinK)
+    if (split_pays(c, d0, d1, d1, (double)d2 * d3))
         zgemm_split(c, (int)d0, (int)d1, (int)d1, (int)(d2 * d3), out, 1, d0, d0 * d1, U[1], d1, 0, tmp, 1, d0,
                     d0 * d1, false, lb, sb);
     else
         zgemm(c, OP_N, OP_N, (int)d0, (int)d1, (int)d1, one, out, d0, d0 * d1, U[1], d1, 0, zero, tmp, d0, d0 * d1,
               (int)(d2 * d3));
     // i: out = U1^H * tmp, as out^T = tmp^T conj(U1) on the split path
-    if (split && d0 > kSplitMinK)
+    if (split_pays(c, (double)d1 * d2 * d3, d0, d0))
         zgemm_split(c, (int)(d1 * d2 * d3), (int)d0, (int)d0, 1, tmp, d0, 1, 0, U[0], d0, 1, out, d0, 1, 0, false, lb,
                     sb);
     else
@@ -479,7 +486,7 @@ static bool sroute_acc_split(const Context &c, int which) {
 // C (M x N, ld ldc) = A (M x K, ld lda) B (K x N, ld ldb)
 static void prod_nn(Context &c, bool split, int M, int N, int K, const cplx *A, int64_t lda, const cplx *B,
                     int64_t ldb, cplx *C, int64_t ldc) {
-    if (split) {
+    if (split && split_pays(c, M, N, K)) {
         zgemm_split_acc(c, M, N, K, 1, A, 1, lda, 0, B, ldb, 0, C, 1, ldc, 0, false);
     } else {
         const cplx one = mk(1.0, 0.0), zero = mk(0.0, 0.0);
@@ -490,7 +497,7 @@ static void prod_nn(Context &c, bool split, int M, int N, int K, const cplx *A, 
 // its transpose B^T conj(A)
 static void prod_cn(Context &c, bool split, int M, int N, int K, const cplx *A, int64_t lda, const cplx *B,
                     int64_t ldb, cplx *C, int64_t ldc) {
-    if (split) {
+    if (split && split_pays(c, M, N, K)) {
         zgemm_split_acc(c, N, M, K, 1, B, ldb, 1, 0, A, lda, 1, C, ldc, 1, 0, false);
     } else {
         const cplx one = mk(1.0, 0.0), zero = mk(0.0, 0.0);
@@ -748,7 +755,7 @@ static RdmBufs rdm_build(Context &c, const uint64_t *full, int64_t M, const cplx
     r.g1 = wsget<cplx>(c, "rdm.g1", (size_t)nv * na2);
     zgemm(c, OP_C, OP_N, 1, (int)(nv * na2), (int)M, one, psi, M, 0, YZ, M, 0, zero, r.g1, 1, 0, 1);
     r.gall = wsget<cplx>(c, "rdm.gall", (size_t)na2 * ncol);
-    if (c.precision == DCG_PREC_SPLIT && M > 32 && ncol >= 128) {
+    if (M > 32 && ncol >= 128 && split_pays(c, (double)na2, (double)ncol, (double)M)) {
         // gall^T = [Y|Z]^T conj(Y) on the split-precision tensor cores (rows of [Y|Z]^T are
         // its columns, contiguous along the determinant index)
         zgemm_split(c, (int)ncol, (int)na2, (int)M, 1, YZ, M, 1, 0, YZ, M, 1, r.gall, na2, 1, 0, false, c.split_lbo,
@@ -946,10 +953,12 @@ static void gram_woodbury_e2(Context &c, int Mp, int dimn, const cplx *G, cplx *
 
 // B' = P^H (D P) (dm x dm) from P and PD (Mp x dm).  Unlike the metric K and Lambda^-1 P^H G v,
 // B' is not amplified by Lambda^-1 (P is orthonormal and D diagonal), so on the split path it
-// runs on the tensor cores, as its transpose (D P)^T conj(P) written back transposed.
+// runs on the tensor cores, as its transpose (D P)^T conj(P) written back transposed.  On seven
+// slices: with five its error (2^-36 of row and column maxima, which depend on the basis P)
+// was most of the split path's distance from FP64 at 20/12/300, 1e-10 to 5e-10 of sumc2.
 static void bprime_product(Context &c, int Mp, int dm, const cplx *P, const cplx *PD, cplx *Bp) {
-    if (c.precision == DCG_PREC_SPLIT && dm > kSplitMinK) {
-        zgemm_split(c, dm, dm, Mp, 1, PD, Mp, 1, 0, P, Mp, 1, Bp, dm, 1, 0, false, c.split_lbo, c.split_sbo);
+    if (split_pays(c, dm, dm, Mp)) {
+        zgemm_split_acc(c, dm, dm, Mp, 1, PD, Mp, 1, 0, P, Mp, 1, Bp, dm, 1, 0, false);
     } else {
         const cplx one = mk(1.0, 0.0), zero = mk(0.0, 0.0);
         zgemm(c, OP_C, OP_N, dm, dm, Mp, one, P, Mp, 0, PD, Mp, 0, zero, Bp, dm, 0, 1);
@@ -972,12 +981,12 @@ static bool gram_acc_split(const Context &c, int which) {
 }
 // K = G G^H (Mp x Mp; at least the upper triangle, the caller mirrors it)
 static void gram_metric(Context &c, int Mp, int dimn, const cplx *G, cplx *K) {
-    if (gram_acc_split(c, 1)) zgemm_split_acc(c, Mp, Mp, dimn, 1, G, 1, Mp, 0, G, Mp, 3, K, 1, Mp, 0, false);
+    if (gram_acc_split(c, 1) && split_pays(c, Mp, Mp, dimn)) zgemm_split_acc(c, Mp, Mp, dimn, 1, G, 1, Mp, 0, G, Mp, 3, K, 1, Mp, 0, false);
     else zherk_upper(c, Mp, dimn, G, Mp, K, Mp);
 }
 // GV = G Vsel (Mp x nouter)
 static void gram_gv(Context &c, int Mp, int nouter, int dimn, const cplx *G, const cplx *Vsel, cplx *GV) {
-    if (gram_acc_split(c, 2)) {
+    if (gram_acc_split(c, 2) && split_pays(c, Mp, nouter, dimn)) {
         zgemm_split_acc(c, Mp, nouter, dimn, 1, G, 1, Mp, 0, Vsel, dimn, 0, GV, 1, Mp, 0, false);
     } else {
         const cplx one = mk(1.0, 0.0), zero = mk(0.0, 0.0);

@@ -353,9 +353,9 @@ void launch_woodbury_e2(Context &c, int Mp, int r, const cplx *U, int64_t ldu, c
     wb_phi_kernel<<<grid1d((int64_t)npair * Mp, 256), 256, 0, c.stream>>>(Mp, r, Ps, ldp, Phi);
     DCG_LAUNCHED(c);
     // C_i, packed: r(r+1)/2 x nouter x Mp, the largest product of the route.  On the split
-    // path it runs on the tensor cores (C_i enters a well-conditioned r x r solve, not the
-    // metric's inverse).
-    if (c.precision == DCG_PREC_SPLIT && npair >= 128)
+    // path it runs on the tensor cores unless it is smaller than their fixed cost (C_i enters a
+    // well-conditioned r x r solve, not the metric's inverse).
+    if (c.precision == DCG_PREC_SPLIT && npair >= 128 && (double)npair * nouter * Mp >= 1.25e6)
         zgemm_split(c, npair, nouter, Mp, 1, Phi, 1, npair, 0, Wm, Mp, 0, Cp, 1, npair, 0, false, c.split_lbo,
                     c.split_sbo);
     else
