@@ -370,22 +370,36 @@ struct SplitArgs {
     uint64_t wait_ns;   // limit of the pipeline waits (SP_WAIT_NS unless a test shortens it)
 };
 
+// The double with the value of an FP32 bit pattern (zero or a normal number: the accumulators are
+// sums of integers scaled by 2^-28 at least), by integer operations: a conversion instruction
+// runs on the FP64 pipe, which takes one warp instruction in 77 clocks and is what the
+// epilogue waits for.
+__device__ __forceinline__ double sp_widen(uint32_t b) {
+    const uint32_t m = b & 0x7FFFFFFFu;
+    return __hiloint2double((int)(m ? (b & 0x80000000u) | ((m >> 3) + 0x38000000u) : 0u), (int)(b << 29));
+}
+
 // g0 + g1 + g2 + g3 (FP32 bit patterns) as a double: TwoSum (Knuth) keeps g0 + g1 exact as
-// s + t, then g2 + g3 are added to t in FP32.
+// s + t, then g2 + g3 are added to t in FP32.  One FP64 instruction a value; with two
+// conversions and a comparison beside it there were four, and the first-quarter contraction
+// 6000 x 300 x 300, batch 20 took 1.83 ms instead of 1.67 (same bits), 40/14/800 1.21 s
+// instead of 1.16.
 __device__ __forceinline__ double recombine(uint32_t b0, uint32_t b1, uint32_t b2, uint32_t b3) {
     const float g0 = __uint_as_float(b0), g1 = __uint_as_float(b1);
     const float s = __fadd_rn(g0, g1);
     const float bb = __fsub_rn(s, g0);
     const float t = __fadd_rn(__fsub_rn(g0, __fsub_rn(s, bb)), __fsub_rn(g1, bb));
     const float lo = __fadd_rn(t, __fadd_rn(__uint_as_float(b2), __uint_as_float(b3)));
-    return (double)s + (double)lo;
+    return sp_widen(__float_as_uint(s)) + sp_widen(__float_as_uint(lo));
 }
 
-// v 2^sc: an integer add to the exponent field when v and the result are normal numbers.
+// v 2^sc: an integer add to the exponent field when v and the result are normal numbers, v itself
+// when it is zero (no FP64 instruction in either case).
 __device__ __forceinline__ double scale_pow2(double v, int sc) {
-    const long long bits = __double_as_longlong(v);
-    const int ex = (int)((bits >> 52) & 0x7FF);
-    if (v != 0.0 && ex > 0 && ex + sc > 0 && ex + sc < 2047) return __longlong_as_double(bits + ((long long)sc << 52));
+    const int hi = __double2hiint(v), lo = __double2loint(v);
+    const int ex = (hi >> 20) & 0x7FF;
+    if (ex > 0 && ex + sc > 0 && ex + sc < 2047) return __hiloint2double(hi + (sc << 20), lo);
+    if (((hi & 0x7FFFFFFF) | lo) == 0) return v;
     return v * ldexp(1.0, sc);
 }
 
@@ -506,8 +520,8 @@ __global__ void __launch_bounds__(SP_THREADS, 1) sp_gemm_kernel(SplitArgs a) {
                     if (j >= a.N) break;
                     // weight-2 and -3 groups are exact and their sum is kept exact as an FP32 pair
                     // (s, t); the weight >= 4 groups are 2^-14 of them and join t, rounding at ~2^-38
-                    // of the result.  Two conversions and one FP64 add per value (the FP64 pipe is
-                    // the epilogue's limit); the power-of-two scale goes into the exponent field.
+                    // of the result.  One FP64 add per value; the widening and the power-of-two scale
+                    // are integer operations on the bits.
                     const int sc = e + a.fexp[j] - 2 * SPLIT_BITS;   // each operand carries 2^-7
                     const double re = scale_pow2(recombine(g0[q], g1[q], g2[q], g3[q]), sc);
                     const double im = scale_pow2(recombine(g0[q + 1], g1[q + 1], g2[q + 1], g3[q + 1]), sc);
@@ -849,11 +863,11 @@ __global__ void __launch_bounds__(SP_THREADS, 1) sp_gemm_acc_kernel(SplitArgs a)
                     double v2[2];
 #pragma unroll
                     for (int h = 0; h < 2; h++) {
-                        double v = (double)__uint_as_float(g4[q + h]);
-                        v += (double)__uint_as_float(g3[q + h]);
-                        v += (double)__uint_as_float(g2[q + h]);
-                        v += (double)__uint_as_float(g1[q + h]);
-                        v += (double)__uint_as_float(g0[q + h]);
+                        double v = sp_widen(g4[q + h]);
+                        v += sp_widen(g3[q + h]);
+                        v += sp_widen(g2[q + h]);
+                        v += sp_widen(g1[q + h]);
+                        v += sp_widen(g0[q + h]);
                         v2[h] = scale_pow2(v, sc);
                     }
                     cplx val = mk(v2[0], v2[1]);
