@@ -23,7 +23,8 @@
 // Data movement: the slicing pre-pass writes both operands directly in the tcgen05 canonical
 // K-major, no-swizzle layout, tile by tile (128 rows x 16 real K = 4 KB per slice), so every
 // pipeline stage is filled by plain bulk copies (cp.async.bulk) completing on an mbarrier.
-// One warp produces, one thread issues the 15 MMAs per K-step, four warps read TMEM back.
+// One warp produces, one thread issues the MMAs of the 15 products per K-step, eight warps
+// read TMEM back.
 // Every wait is bounded; a wait that runs out sets an error flag and the kernel unwinds.
 #include <cuda_bf16.h>
 
@@ -44,7 +45,8 @@ constexpr int SP_STAGES = 4;
 constexpr int SP_TILE_BYTES = SP_TM * SP_TK * 2;                       // 4096
 constexpr int SP_STAGE_BYTES = 2 * SPLIT_S * SP_TILE_BYTES;            // A and B slices: 40 KB
 constexpr int SP_SMEM = SP_STAGES * SP_STAGE_BYTES + 1024;             // + alignment
-constexpr int SP_THREADS = 192;     // warps 0-3 epilogue, 4 producer, 5 MMA issuer
+constexpr int SP_EPI = 8;           // epilogue warps: two to each quarter of the TMEM lanes
+constexpr int SP_THREADS = (SP_EPI + 2) * 32;   // then the producer and the MMA issuer
 constexpr uint64_t SP_WAIT_NS = 2000000000ull;
 
 // Byte offset of element (r, kk) inside a 128 x 16 K-major tile: 8 x 8 core matrices of
@@ -310,27 +312,66 @@ __device__ __forceinline__ uint64_t sp_desc(const void *p, int lbo, int sbo) {
     const uint64_t a = (smem_u32(p) >> 4) & 0x3FFFull;
     return a | ((uint64_t)((lbo >> 4) & 0x3FFF) << 16) | ((uint64_t)((sbo >> 4) & 0x3FFF) << 32) | (1ull << 46);
 }
-// instruction descriptor: kind::f16, D f32, A/B bf16, both K-major, N = SP_TN, M = SP_TM
-constexpr uint32_t SP_IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(SP_TN >> 3) << 17) |
-                              ((uint32_t)(SP_TM >> 4) << 24);
-
-__device__ __forceinline__ void umma_f16(uint32_t dtmem, uint64_t adesc, uint64_t bdesc, uint32_t acc) {
+// instruction descriptor: kind::f16, D f32, A/B bf16, both K-major, M = SP_TM, N columns (a
+// multiple of 16 up to 256)
+__device__ __forceinline__ uint32_t sp_idesc(int n) {
+    return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(SP_TM >> 4) << 24);
+}
+__device__ __forceinline__ void umma_f16(uint32_t dtmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t acc) {
     asm volatile(
         "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
         "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(dtmem),
-        "l"(adesc), "l"(bdesc), "r"(SP_IDESC), "r"(acc));
+        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(acc));
 }
-// instruction descriptor of the persistent kernel's 128 x 64 products
-constexpr int SPP_TN = 64;
-constexpr uint32_t SPP_IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(SPP_TN >> 3) << 17) |
-                               ((uint32_t)(SP_TM >> 4) << 24);
+// real columns of a tile of tn that hold output columns, rounded to the MMA's granularity
+__device__ __forceinline__ int sp_cols(int n2, int first, int tn) { return min(tn, (n2 - first + 15) & ~15); }
 
-__device__ __forceinline__ void umma_f16_n64(uint32_t dtmem, uint64_t adesc, uint64_t bdesc, uint32_t acc) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(dtmem),
-        "l"(adesc), "l"(bdesc), "r"(SPP_IDESC), "r"(acc));
+// The 15 products p + q <= 6 (slices numbered from 1) of one K step into the four groups, tn
+// columns apart.  On a full tile the slices of B stand one below the other as one operand of up to 256 columns and the groups side
+// by side as its result, so that one MMA does a slice of A against several of B: an MMA reads
+// A again (4 KB) for every tn columns it makes, and shared memory, at 128 bytes a clock, is
+// what the mainloop waits for (128 columns: 160 -> 144 KB a K step, 64 columns: 120 -> 96 KB).
+// Each group takes its products in the same order (rising slice of A) in every form, so that all
+// forms and both kernels give the same bits.
+template <int TN>
+__device__ __forceinline__ void sp_mma_step(uint32_t acc, const uint64_t (&da)[SPLIT_S], const uint64_t (&db)[SPLIT_S],
+                                            int cols, uint32_t first) {
+    const uint32_t one = sp_idesc(cols);
+    if (cols == TN) {
+        constexpr int W = 256 / TN;   // slices of B per MMA
+        const uint32_t wide = sp_idesc(W * TN);
+        if (W == 4) {
+            umma_f16(acc, da[0], db[0], wide, first);
+            umma_f16(acc + TN, da[1], db[0], sp_idesc(192), 1u);
+            umma_f16(acc + 2 * TN, da[2], db[0], sp_idesc(128), 1u);
+        } else {
+            umma_f16(acc, da[0], db[0], wide, first);
+            umma_f16(acc + 2 * TN, da[0], db[2], wide, first);
+            umma_f16(acc + TN, da[1], db[0], wide, 1u);
+            umma_f16(acc + 3 * TN, da[1], db[2], one, 1u);
+            umma_f16(acc + 2 * TN, da[2], db[0], wide, 1u);
+        }
+        umma_f16(acc + 3 * TN, da[3], db[0], one, 1u);
+    } else {
+        umma_f16(acc, da[0], db[0], one, first);
+        umma_f16(acc + TN, da[0], db[1], one, first);
+        umma_f16(acc + TN, da[1], db[0], one, 1u);
+        umma_f16(acc + 2 * TN, da[0], db[2], one, first);
+        umma_f16(acc + 2 * TN, da[1], db[1], one, 1u);
+        umma_f16(acc + 2 * TN, da[2], db[0], one, 1u);
+        umma_f16(acc + 3 * TN, da[0], db[3], one, first);
+        umma_f16(acc + 3 * TN, da[1], db[2], one, 1u);
+        umma_f16(acc + 3 * TN, da[2], db[1], one, 1u);
+        umma_f16(acc + 3 * TN, da[3], db[0], one, 1u);
+    }
+    umma_f16(acc + 3 * TN, da[0], db[4], one, 1u);
+    umma_f16(acc + 3 * TN, da[1], db[3], one, 1u);
+    umma_f16(acc + 3 * TN, da[2], db[2], one, 1u);
+    umma_f16(acc + 3 * TN, da[3], db[1], one, 1u);
+    umma_f16(acc + 3 * TN, da[4], db[0], one, 1u);
 }
+constexpr int SPP_TN = 64;   // columns of an item of the persistent kernel
+
 __device__ __forceinline__ void mbar_arrive(uint64_t *bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
@@ -347,14 +388,12 @@ __device__ __forceinline__ void umma_commit(uint64_t *bar) {
                  : "memory");
 }
 
-#define SP_LD32(taddr, r)                                                                                        \
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15," \
-                 "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"                      \
+#define SP_LD16(taddr, r)                                                                                        \
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}," \
+                 " [%16];"                                                                                        \
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),        \
                    "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),    \
-                   "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), \
-                   "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), \
-                   "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])                                          \
+                   "=r"(r[14]), "=r"(r[15])                                                                     \
                  : "r"(taddr))
 
 struct SplitArgs {
@@ -403,6 +442,67 @@ __device__ __forceinline__ double scale_pow2(double v, int sc) {
     return v * ldexp(1.0, sc);
 }
 
+// The epilogue works on chunks of 16 real = 8 complex columns of one row a lane.  The two warps
+// of a quarter of the TMEM lanes take alternate chunks, so that one's loads and stores run
+// under the other's FP64 adds, and an accumulating product reads its C a chunk ahead, the
+// first chunk before the MMAs are done.  With four warps and the read beside each store,
+// 1.28M x 800 x 288 onto C took as long, 53.2 ms with its slicing, as the 512 terms before it,
+// 55.9; now 37.6 and 51.6 ms.
+constexpr int SP_CH = 8;   // complex columns of a chunk
+
+struct SpRow {
+    cplx *row;    // C at column 0 of the lane's row
+    int64_t sj;
+    int e;        // exponent of the row, less the operands' prescale
+    bool ok;
+};
+__device__ __forceinline__ SpRow sp_row(const SplitArgs &a, int z, int64_t i) {
+    SpRow r;
+    r.ok = i < a.M;
+    r.row = a.C + (int64_t)z * a.c_sb + (r.ok ? i : 0) * a.c_si;
+    r.sj = a.c_sj;
+    r.e = (r.ok ? a.eexp[(int64_t)z * a.M + i] : 0) - 2 * SPLIT_BITS;   // each operand carries 2^-7
+    return r;
+}
+__device__ __forceinline__ void sp_read_c(const SplitArgs &a, const SpRow &r, int j0, cplx (&old)[SP_CH]) {
+#pragma unroll
+    for (int q = 0; q < SP_CH; q++)
+        if (r.ok && j0 + q < a.N) old[q] = r.row[(int64_t)(j0 + q) * r.sj];
+}
+template <int NG>
+__device__ __forceinline__ void sp_read_tmem(uint32_t taddr, int tn, uint32_t (&g)[NG][2 * SP_CH]) {
+#pragma unroll
+    for (int p = 0; p < NG; p++) SP_LD16(taddr + (uint32_t)(p * tn), g[p]);
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+__device__ __forceinline__ double sp_value(const uint32_t (&g)[4][2 * SP_CH], int q) {
+    return recombine(g[0][q], g[1][q], g[2][q], g[3][q]);
+}
+__device__ __forceinline__ double sp_value(const uint32_t (&g)[5][2 * SP_CH], int q) {
+    double v = sp_widen(g[4][q]);
+    v += sp_widen(g[3][q]);
+    v += sp_widen(g[2][q]);
+    v += sp_widen(g[1][q]);
+    v += sp_widen(g[0][q]);
+    return v;
+}
+template <int NG>
+__device__ __forceinline__ void sp_write_c(const SplitArgs &a, const SpRow &r, int j0, const uint32_t (&g)[NG][2 * SP_CH],
+                                           const cplx (&old)[SP_CH]) {
+    if (!r.ok) return;
+    int f[SP_CH];
+#pragma unroll
+    for (int q = 0; q < SP_CH; q++) f[q] = __ldg(a.fexp + min(j0 + q, a.N - 1));
+#pragma unroll
+    for (int q = 0; q < SP_CH; q++) {
+        cplx v = mk(scale_pow2(sp_value(g, 2 * q), r.e + f[q]), scale_pow2(sp_value(g, 2 * q + 1), r.e + f[q]));
+        if (j0 + q < a.N) {
+            if (a.accumulate) v = cadd(v, old[q]);
+            r.row[(int64_t)(j0 + q) * r.sj] = v;
+        }
+    }
+}
+
 __global__ void __launch_bounds__(SP_THREADS, 1) sp_gemm_kernel(SplitArgs a) {
     extern __shared__ __align__(1024) unsigned char sp_raw[];
     __shared__ __align__(8) uint64_t bar_full[SP_STAGES], bar_empty[SP_STAGES], bar_done;
@@ -434,27 +534,28 @@ __global__ void __launch_bounds__(SP_THREADS, 1) sp_gemm_kernel(SplitArgs a) {
     asm volatile("tcgen05.fence::after_thread_sync;");
     const uint32_t tmem = s_tmem;
     const int nks = a.nks;
+    const int cols = sp_cols(2 * a.N, nb * SP_TN, SP_TN);
     int issued = 0;   // producer: stages whose copies were issued
 
-    if (warp == 4) {
+    if (warp == SP_EPI) {
         if (lane == 0) {   // producer: 2 x SPLIT_S bulk copies of 4 KB per stage
             for (int ks = 0; ks < nks; ks++) {
                 const int s = ks % SP_STAGES;
                 if (ks >= SP_STAGES && !mbar_wait(&bar_empty[s], ((ks / SP_STAGES) - 1) & 1, a.err, a.wait_ns)) break;
                 issued = ks + 1;
                 unsigned char *st = smem + s * SP_STAGE_BYTES;
-                mbar_expect_tx(&bar_full[s], SP_STAGE_BYTES);
+                mbar_expect_tx(&bar_full[s], SPLIT_S * (SP_TILE_BYTES + cols * SP_TK * 2));
                 for (int p = 0; p < SPLIT_S; p++) {
                     const int64_t ta = (((int64_t)p * a.nz + z) * a.nrb + rb) * nks + ks;
                     bulk_g2s(st + p * SP_TILE_BYTES, reinterpret_cast<const char *>(a.As) + ta * SP_TILE_BYTES,
                              SP_TILE_BYTES, &bar_full[s]);
                     const int64_t tb = ((int64_t)p * a.nnb + nb) * nks + ks;
                     bulk_g2s(st + (SPLIT_S + p) * SP_TILE_BYTES, reinterpret_cast<const char *>(a.Bs) + tb * SP_TILE_BYTES,
-                             SP_TILE_BYTES, &bar_full[s]);
+                             cols * SP_TK * 2, &bar_full[s]);
                 }
             }
         }
-    } else if (warp == 5) {
+    } else if (warp == SP_EPI + 1) {
         if (lane == 0) {   // MMA issuer
             bool ok = true;
             for (int ks = 0; ks < nks && ok; ks++) {
@@ -471,65 +572,29 @@ __global__ void __launch_bounds__(SP_THREADS, 1) sp_gemm_kernel(SplitArgs a) {
                     da[p] = sp_desc(st + p * SP_TILE_BYTES, a.lbo, a.sbo);
                     db[p] = sp_desc(st + (SPLIT_S + p) * SP_TILE_BYTES, a.lbo, a.sbo);
                 }
-                const uint32_t first = ks > 0 ? 1u : 0u;
-                // weight 2
-                umma_f16(tmem + 0 * SP_TN, da[0], db[0], first);
-                // weight 3
-                umma_f16(tmem + 1 * SP_TN, da[0], db[1], first);
-                umma_f16(tmem + 1 * SP_TN, da[1], db[0], 1u);
-                // weight 4
-                umma_f16(tmem + 2 * SP_TN, da[0], db[2], first);
-                umma_f16(tmem + 2 * SP_TN, da[1], db[1], 1u);
-                umma_f16(tmem + 2 * SP_TN, da[2], db[0], 1u);
-                // weights 5 and 6
-                umma_f16(tmem + 3 * SP_TN, da[0], db[3], first);
-                umma_f16(tmem + 3 * SP_TN, da[1], db[2], 1u);
-                umma_f16(tmem + 3 * SP_TN, da[2], db[1], 1u);
-                umma_f16(tmem + 3 * SP_TN, da[3], db[0], 1u);
-                umma_f16(tmem + 3 * SP_TN, da[0], db[4], 1u);
-                umma_f16(tmem + 3 * SP_TN, da[1], db[3], 1u);
-                umma_f16(tmem + 3 * SP_TN, da[2], db[2], 1u);
-                umma_f16(tmem + 3 * SP_TN, da[3], db[1], 1u);
-                umma_f16(tmem + 3 * SP_TN, da[4], db[0], 1u);
+                sp_mma_step<SP_TN>(tmem, da, db, cols, ks > 0 ? 1u : 0u);
                 umma_commit(&bar_empty[s]);
             }
             umma_commit(&bar_done);   // arrives once every MMA issued above has completed
         }
     } else {
-        // epilogue: warp w reads TMEM lanes 32w..32w+31 = tile rows
+        // epilogue: warp w reads TMEM lanes 32 (w % 4).. = tile rows, chunks w / 4, w / 4 + 2, ...
+        const int quad = warp & 3, half = warp >> 2;
+        const SpRow r = sp_row(a, z, (int64_t)rb * SP_TM + quad * 32 + lane);
+        const int jt = nb * (SP_TN / 2) + half * SP_CH;
+        cplx old[2][SP_CH];
+        if (a.accumulate) sp_read_c(a, r, jt, old[0]);
         const bool ok = mbar_wait(&bar_done, 0, a.err, a.wait_ns);
         asm volatile("tcgen05.fence::after_thread_sync;");
         if (ok) {
-            const int r = warp * 32 + lane;
-            const int64_t i = (int64_t)rb * SP_TM + r;
-            const bool row_ok = i < a.M;
-            const int e = row_ok ? a.eexp[(int64_t)z * a.M + i] : 0;
-            for (int c0 = 0; c0 < SP_TN; c0 += 32) {
-                uint32_t g0[32], g1[32], g2[32], g3[32];
-                const uint32_t base = tmem + ((uint32_t)(warp * 32) << 16) + c0;
-                SP_LD32(base + 0 * SP_TN, g0);
-                SP_LD32(base + 1 * SP_TN, g1);
-                SP_LD32(base + 2 * SP_TN, g2);
-                SP_LD32(base + 3 * SP_TN, g3);
-                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                if (!row_ok) continue;
 #pragma unroll
-                for (int q = 0; q < 32; q += 2) {
-                    const int jr = nb * SP_TN + c0 + q;   // real column (even: Re)
-                    const int j = jr >> 1;
-                    if (j >= a.N) break;
-                    // weight-2 and -3 groups are exact and their sum is kept exact as an FP32 pair
-                    // (s, t); the weight >= 4 groups are 2^-14 of them and join t, rounding at ~2^-38
-                    // of the result.  One FP64 add per value; the widening and the power-of-two scale
-                    // are integer operations on the bits.
-                    const int sc = e + a.fexp[j] - 2 * SPLIT_BITS;   // each operand carries 2^-7
-                    const double re = scale_pow2(recombine(g0[q], g1[q], g2[q], g3[q]), sc);
-                    const double im = scale_pow2(recombine(g0[q + 1], g1[q + 1], g2[q + 1], g3[q + 1]), sc);
-                    cplx v = mk(re, im);
-                    cplx *dst = a.C + (int64_t)z * a.c_sb + i * a.c_si + (int64_t)j * a.c_sj;
-                    if (a.accumulate) v = cadd(v, *dst);
-                    *dst = v;
-                }
+            for (int cc = 0; cc < SP_TN / (4 * SP_CH); cc++) {
+                const int j0 = jt + cc * 2 * SP_CH;
+                if (j0 >= a.N) break;
+                if (a.accumulate) sp_read_c(a, r, j0 + 2 * SP_CH, old[(cc + 1) & 1]);
+                uint32_t g[4][2 * SP_CH];
+                sp_read_tmem<4>(tmem + ((uint32_t)(quad * 32) << 16) + (cc * 2 + half) * 2 * SP_CH, SP_TN, g);
+                sp_write_c<4>(a, r, j0, g, old[cc & 1]);
             }
         }
     }
@@ -538,10 +603,10 @@ __global__ void __launch_bounds__(SP_THREADS, 1) sp_gemm_kernel(SplitArgs a) {
     // After a wait gave up, copies may still be in flight and MMAs still running: the last
     // round of each stage lands and every issued MMA completes before the CTA frees its TMEM
     // and leaves (waits bounded by SP_WAIT_NS; without an error they return at once).
-    if (warp == 4 && lane == 0)
+    if (warp == SP_EPI && lane == 0)
         for (int ks = issued - 1; ks >= 0 && ks >= issued - SP_STAGES; ks--)
             mbar_drain(&bar_full[ks % SP_STAGES], (uint32_t)((ks / SP_STAGES) & 1));
-    if (warp == 5 && lane == 0) mbar_drain(&bar_done, 0);
+    if (warp == SP_EPI + 1 && lane == 0) mbar_drain(&bar_done, 0);
     __syncthreads();
     if (warp == 0) {
         asm volatile("tcgen05.fence::after_thread_sync;");
@@ -587,7 +652,7 @@ __global__ void __launch_bounds__(SP_THREADS, 1) sp_gemm_persist_kernel(SplitArg
         }
         for (int q = 0; q < 2; q++) {
             mbar_init(&acc_full[q], 1);
-            mbar_init(&acc_empty[q], 4);   // one arrival per epilogue warp
+            mbar_init(&acc_empty[q], SP_EPI);   // one arrival per epilogue warp
         }
         mbar_init(&bar_drain, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -603,7 +668,7 @@ __global__ void __launch_bounds__(SP_THREADS, 1) sp_gemm_persist_kernel(SplitArg
     const uint32_t tmem = s_tmem;
 
     int64_t issued = 0;   // producer: stage rounds whose copies were issued
-    if (warp == 4) {
+    if (warp == SP_EPI) {
         if (lane == 0) {   // producer
             int64_t it = 0;
             bool ok = true;
@@ -611,6 +676,7 @@ __global__ void __launch_bounds__(SP_THREADS, 1) sp_gemm_persist_kernel(SplitArg
                 int z, rb, nh;
                 item_coords(t, z, rb, nh);
                 const int nb = nh >> 1, half = nh & 1;
+                const int bbytes = sp_cols(2 * a.N, nh * SPP_TN, SPP_TN) * SP_TK * 2;
                 for (int ks = 0; ks < nks; ks++, it++) {
                     const int s = (int)(it % SPP_STAGES);
                     if (it >= SPP_STAGES && !mbar_wait(&bar_empty[s], (uint32_t)(((it / SPP_STAGES) - 1) & 1), a.err, a.wait_ns)) {
@@ -618,7 +684,7 @@ __global__ void __launch_bounds__(SP_THREADS, 1) sp_gemm_persist_kernel(SplitArg
                         break;
                     }
                     unsigned char *st = smem + s * SPP_STAGE_BYTES;
-                    mbar_expect_tx(&bar_full[s], SPP_STAGE_BYTES);
+                    mbar_expect_tx(&bar_full[s], SPLIT_S * (SP_TILE_BYTES + bbytes));
                     for (int p = 0; p < SPLIT_S; p++) {
                         const int64_t ta = (((int64_t)p * a.nz + z) * a.nrb + rb) * nks + ks;
                         bulk_g2s(st + p * SP_TILE_BYTES, reinterpret_cast<const char *>(a.As) + ta * SP_TILE_BYTES,
@@ -626,13 +692,13 @@ __global__ void __launch_bounds__(SP_THREADS, 1) sp_gemm_persist_kernel(SplitArg
                         const int64_t tb = ((int64_t)p * a.nnb + nb) * nks + ks;
                         bulk_g2s(st + SPLIT_S * SP_TILE_BYTES + p * (SP_TILE_BYTES / 2),
                                  reinterpret_cast<const char *>(a.Bs) + tb * SP_TILE_BYTES + half * (SP_TILE_BYTES / 2),
-                                 SP_TILE_BYTES / 2, &bar_full[s]);
+                                 bbytes, &bar_full[s]);
                     }
                 }
             }
             issued = it;
         }
-    } else if (warp == 5) {
+    } else if (warp == SP_EPI + 1) {
         if (lane == 0) {   // MMA issuer
             int64_t it = 0, tl = 0;
             bool ok = true;
@@ -644,6 +710,9 @@ __global__ void __launch_bounds__(SP_THREADS, 1) sp_gemm_persist_kernel(SplitArg
                 }
                 asm volatile("tcgen05.fence::after_thread_sync;");
                 const uint32_t acc = tmem + (uint32_t)(b * 4 * SPP_TN);
+                int z, rb, nh;
+                item_coords(t, z, rb, nh);
+                const int cols = sp_cols(2 * a.N, nh * SPP_TN, SPP_TN);
                 for (int ks = 0; ks < nks; ks++, it++) {
                     const int s = (int)(it % SPP_STAGES);
                     if (!mbar_wait(&bar_full[s], (uint32_t)((it / SPP_STAGES) & 1), a.err, a.wait_ns)) {
@@ -658,22 +727,7 @@ __global__ void __launch_bounds__(SP_THREADS, 1) sp_gemm_persist_kernel(SplitArg
                         da[p] = sp_desc(st + p * SP_TILE_BYTES, a.lbo, a.sbo);
                         db[p] = sp_desc(st + SPLIT_S * SP_TILE_BYTES + p * (SP_TILE_BYTES / 2), a.lbo, a.sbo);
                     }
-                    const uint32_t first = ks > 0 ? 1u : 0u;
-                    umma_f16_n64(acc + 0 * SPP_TN, da[0], db[0], first);
-                    umma_f16_n64(acc + 1 * SPP_TN, da[0], db[1], first);
-                    umma_f16_n64(acc + 1 * SPP_TN, da[1], db[0], 1u);
-                    umma_f16_n64(acc + 2 * SPP_TN, da[0], db[2], first);
-                    umma_f16_n64(acc + 2 * SPP_TN, da[1], db[1], 1u);
-                    umma_f16_n64(acc + 2 * SPP_TN, da[2], db[0], 1u);
-                    umma_f16_n64(acc + 3 * SPP_TN, da[0], db[3], first);
-                    umma_f16_n64(acc + 3 * SPP_TN, da[1], db[2], 1u);
-                    umma_f16_n64(acc + 3 * SPP_TN, da[2], db[1], 1u);
-                    umma_f16_n64(acc + 3 * SPP_TN, da[3], db[0], 1u);
-                    umma_f16_n64(acc + 3 * SPP_TN, da[0], db[4], 1u);
-                    umma_f16_n64(acc + 3 * SPP_TN, da[1], db[3], 1u);
-                    umma_f16_n64(acc + 3 * SPP_TN, da[2], db[2], 1u);
-                    umma_f16_n64(acc + 3 * SPP_TN, da[3], db[1], 1u);
-                    umma_f16_n64(acc + 3 * SPP_TN, da[4], db[0], 1u);
+                    sp_mma_step<SPP_TN>(acc, da, db, cols, ks > 0 ? 1u : 0u);
                     umma_commit(&bar_empty[s]);
                 }
                 if (ok) umma_commit(&acc_full[b]);
@@ -682,45 +736,34 @@ __global__ void __launch_bounds__(SP_THREADS, 1) sp_gemm_persist_kernel(SplitArg
             mbar_drain(&bar_drain, 0);
         }
     } else {
-        // epilogue warps 0-3: warp w owns TMEM lanes 32w..32w+31 = tile rows
+        // epilogue: warp w owns TMEM lanes 32 (w % 4).. = tile rows, chunks w / 4 and w / 4 + 2
+        const int quad = warp & 3, half = warp >> 2;
         int64_t tl = 0;
         for (int64_t t = blockIdx.x; t < items; t += gridDim.x, tl++) {
             const int b = (int)(tl & 1);
-            if (!mbar_wait(&acc_full[b], (uint32_t)((tl >> 1) & 1), a.err, a.wait_ns)) break;
-            asm volatile("tcgen05.fence::after_thread_sync;");
             int z, rb, nh;
             item_coords(t, z, rb, nh);
-            const int r = warp * 32 + lane;
-            const int64_t i = (int64_t)rb * SP_TM + r;
-            const bool row_ok = i < a.M;
-            const int e = row_ok ? a.eexp[(int64_t)z * a.M + i] : 0;
-            const uint32_t base = tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(b * 4 * SPP_TN);
-            for (int c0 = 0; c0 < SPP_TN; c0 += 32) {
-                uint32_t g0[32], g1[32], g2[32], g3[32];
-                SP_LD32(base + 0 * SPP_TN + c0, g0);
-                SP_LD32(base + 1 * SPP_TN + c0, g1);
-                SP_LD32(base + 2 * SPP_TN + c0, g2);
-                SP_LD32(base + 3 * SPP_TN + c0, g3);
-                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                if (c0 + 32 >= SPP_TN) {   // the accumulator set is read: hand it back to the MMAs
+            const SpRow r = sp_row(a, z, (int64_t)rb * SP_TM + quad * 32 + lane);
+            const int jt = nh * (SPP_TN / 2) + half * SP_CH;
+            cplx old[2][SP_CH];
+            if (a.accumulate) {
+                sp_read_c(a, r, jt, old[0]);
+                sp_read_c(a, r, jt + 2 * SP_CH, old[1]);
+            }
+            if (!mbar_wait(&acc_full[b], (uint32_t)((tl >> 1) & 1), a.err, a.wait_ns)) break;
+            asm volatile("tcgen05.fence::after_thread_sync;");
+            const uint32_t base = tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(b * 4 * SPP_TN + half * 2 * SP_CH);
+#pragma unroll
+            for (int cc = 0; cc < 2; cc++) {
+                const int j0 = jt + cc * 2 * SP_CH;
+                uint32_t g[4][2 * SP_CH];
+                if (j0 < a.N) sp_read_tmem<4>(base + cc * 4 * SP_CH, SPP_TN, g);
+                if (cc == 1) {   // the accumulator set is read: hand it back to the MMAs
                     asm volatile("tcgen05.fence::before_thread_sync;");
                     __syncwarp();
                     if (lane == 0) mbar_arrive(&acc_empty[b]);
                 }
-                if (!row_ok) continue;
-#pragma unroll
-                for (int q = 0; q < 32; q += 2) {
-                    const int jr = nh * SPP_TN + c0 + q;   // real column (even: Re)
-                    const int j = jr >> 1;
-                    if (j >= a.N) break;
-                    const int sc = e + a.fexp[j] - 2 * SPLIT_BITS;
-                    const double re = scale_pow2(recombine(g0[q], g1[q], g2[q], g3[q]), sc);
-                    const double im = scale_pow2(recombine(g0[q + 1], g1[q + 1], g2[q + 1], g3[q + 1]), sc);
-                    cplx v = mk(re, im);
-                    cplx *dst = a.C + (int64_t)z * a.c_sb + i * a.c_si + (int64_t)j * a.c_sj;
-                    if (a.accumulate) v = cadd(v, *dst);
-                    *dst = v;
-                }
+                if (j0 < a.N) sp_write_c<4>(a, r, j0, g, old[cc]);
             }
         }
     }
@@ -728,7 +771,7 @@ __global__ void __launch_bounds__(SP_THREADS, 1) sp_gemm_persist_kernel(SplitArg
     __syncthreads();
     // copies still in flight after any role gave up land before the CTA leaves (the MMA issuer
     // has already waited for its MMAs through bar_drain); without an error this returns at once
-    if (warp == 4 && lane == 0)
+    if (warp == SP_EPI && lane == 0)
         for (int64_t j = issued - 1; j >= 0 && j >= issued - SPP_STAGES; j--)
             mbar_drain(&bar_full[j % SPP_STAGES], (uint32_t)((j / SPP_STAGES) & 1));
     __syncthreads();
@@ -785,9 +828,10 @@ __global__ void __launch_bounds__(SP_THREADS, 1) sp_gemm_acc_kernel(SplitArgs a)
     asm volatile("tcgen05.fence::after_thread_sync;");
     const uint32_t tmem = s_tmem;
     const int nks = a.nks;
+    const int cols = sp_cols(2 * a.N, nh * SPA_TN, SPA_TN);
     int issued = 0;
 
-    if (warp == 4) {
+    if (warp == SP_EPI) {
         if (lane == 0) {   // producer: SPA_S A tiles (4 KB) and SPA_S B half-tiles (2 KB) per stage
             for (int ks = 0; ks < nks; ks++) {
                 const int st_i = ks % SPA_STAGES;
@@ -796,7 +840,7 @@ __global__ void __launch_bounds__(SP_THREADS, 1) sp_gemm_acc_kernel(SplitArgs a)
                     break;
                 issued = ks + 1;
                 unsigned char *st = smem + st_i * SPA_STAGE_BYTES;
-                mbar_expect_tx(&bar_full[st_i], SPA_STAGE_BYTES);
+                mbar_expect_tx(&bar_full[st_i], SPA_S * (SP_TILE_BYTES + cols * SP_TK * 2));
                 for (int p = 0; p < SPA_S; p++) {
                     const int64_t ta = (((int64_t)p * a.nz + z) * a.nrb + rb) * nks + ks;
                     bulk_g2s(st + p * SP_TILE_BYTES, reinterpret_cast<const char *>(a.As) + ta * SP_TILE_BYTES,
@@ -804,11 +848,11 @@ __global__ void __launch_bounds__(SP_THREADS, 1) sp_gemm_acc_kernel(SplitArgs a)
                     const int64_t tb = ((int64_t)p * a.nnb + nb) * nks + ks;
                     bulk_g2s(st + SPA_S * SP_TILE_BYTES + p * (SP_TILE_BYTES / 2),
                              reinterpret_cast<const char *>(a.Bs) + tb * SP_TILE_BYTES + half * (SP_TILE_BYTES / 2),
-                             SP_TILE_BYTES / 2, &bar_full[st_i]);
+                             cols * SP_TK * 2, &bar_full[st_i]);
                 }
             }
         }
-    } else if (warp == 5) {
+    } else if (warp == SP_EPI + 1) {
         if (lane == 0) {   // MMA issuer: 28 products per K step, by weight p + q
             for (int ks = 0; ks < nks; ks++) {
                 const int st_i = ks % SPA_STAGES;
@@ -821,70 +865,58 @@ __global__ void __launch_bounds__(SP_THREADS, 1) sp_gemm_acc_kernel(SplitArgs a)
                     da[p] = sp_desc(st + p * SP_TILE_BYTES, a.lbo, a.sbo);
                     db[p] = sp_desc(st + SPA_S * SP_TILE_BYTES + p * (SP_TILE_BYTES / 2), a.lbo, a.sbo);
                 }
+                const uint32_t first = ks > 0 ? 1u : 0u, one = sp_idesc(cols);
+                if (cols == SPA_TN) {   // a slice of A against up to four of B, as sp_mma_step
+                    umma_f16(tmem, da[0], db[0], sp_idesc(256), first);
+                    umma_f16(tmem + 4 * SPA_TN, da[0], db[4], one, first);
+                    umma_f16(tmem + SPA_TN, da[1], db[0], sp_idesc(256), 1u);
+                    umma_f16(tmem + 2 * SPA_TN, da[2], db[0], sp_idesc(192), 1u);
+                    umma_f16(tmem + 3 * SPA_TN, da[3], db[0], sp_idesc(128), 1u);
+                    umma_f16(tmem + 4 * SPA_TN, da[4], db[0], one, 1u);
+                }
 #pragma unroll
                 for (int w = 0; w < SPA_S; w++) {
                     const int g = w < SPA_GROUPS - 1 ? w : SPA_GROUPS - 1;
+                    if (w < SPA_GROUPS && cols == SPA_TN) continue;
 #pragma unroll
-                    for (int p = 0; p <= w; p++) {
-                        // the first product into a group at the first K step overwrites it
-                        const bool first = ks == 0 && p == 0 && w < SPA_GROUPS;
-                        umma_f16_n64(tmem + (uint32_t)(g * SPA_TN), da[p], db[w - p], first ? 0u : 1u);
-                    }
+                    for (int p = 0; p <= w; p++)   // the first product into a group at the first K step overwrites it
+                        umma_f16(tmem + (uint32_t)(g * SPA_TN), da[p], db[w - p], one,
+                                 p == 0 && w < SPA_GROUPS ? first : 1u);
                 }
                 umma_commit(&bar_empty[st_i]);
             }
             umma_commit(&bar_done);   // arrives once every MMA issued above has completed
         }
     } else {
-        // epilogue: warp w reads TMEM lanes 32w..32w+31 = tile rows
+        // epilogue: as in sp_gemm_kernel, two chunks a warp
+        const int quad = warp & 3, par = warp >> 2;
+        const SpRow r = sp_row(a, z, (int64_t)rb * SP_TM + quad * 32 + lane);
+        const int jt = nh * (SPA_TN / 2) + par * SP_CH;
+        cplx old[2][SP_CH];
+        if (a.accumulate) {
+            sp_read_c(a, r, jt, old[0]);
+            sp_read_c(a, r, jt + 2 * SP_CH, old[1]);
+        }
         const bool ok = mbar_wait(&bar_done, 0, a.err, a.wait_ns);
         asm volatile("tcgen05.fence::after_thread_sync;");
         if (ok) {
-            const int r = warp * 32 + lane;
-            const int64_t i = (int64_t)rb * SP_TM + r;
-            const bool row_ok = i < a.M;
-            const int e = row_ok ? a.eexp[(int64_t)z * a.M + i] : 0;
-            for (int c0 = 0; c0 < SPA_TN; c0 += 32) {
-                uint32_t g0[32], g1[32], g2[32], g3[32], g4[32];
-                const uint32_t base = tmem + ((uint32_t)(warp * 32) << 16) + c0;
-                SP_LD32(base + 0 * SPA_TN, g0);
-                SP_LD32(base + 1 * SPA_TN, g1);
-                SP_LD32(base + 2 * SPA_TN, g2);
-                SP_LD32(base + 3 * SPA_TN, g3);
-                SP_LD32(base + 4 * SPA_TN, g4);
-                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                if (!row_ok) continue;
 #pragma unroll
-                for (int q = 0; q < 32; q += 2) {
-                    const int jr = nh * SPA_TN + c0 + q;   // real column (even: Re)
-                    const int j = jr >> 1;
-                    if (j >= a.N) break;
-                    const int sc = e + a.fexp[j] - 2 * SPLIT_BITS;
-                    double v2[2];
-#pragma unroll
-                    for (int h = 0; h < 2; h++) {
-                        double v = sp_widen(g4[q + h]);
-                        v += sp_widen(g3[q + h]);
-                        v += sp_widen(g2[q + h]);
-                        v += sp_widen(g1[q + h]);
-                        v += sp_widen(g0[q + h]);
-                        v2[h] = scale_pow2(v, sc);
-                    }
-                    cplx val = mk(v2[0], v2[1]);
-                    cplx *dst = a.C + (int64_t)z * a.c_sb + i * a.c_si + (int64_t)j * a.c_sj;
-                    if (a.accumulate) val = cadd(val, *dst);
-                    *dst = val;
-                }
+            for (int cc = 0; cc < 2; cc++) {
+                const int j0 = jt + cc * 2 * SP_CH;
+                if (j0 >= a.N) break;
+                uint32_t g[SPA_GROUPS][2 * SP_CH];
+                sp_read_tmem<SPA_GROUPS>(tmem + ((uint32_t)(quad * 32) << 16) + (cc * 2 + par) * 2 * SP_CH, SPA_TN, g);
+                sp_write_c<SPA_GROUPS>(a, r, j0, g, old[cc]);
             }
         }
     }
     asm volatile("tcgen05.fence::before_thread_sync;");
     __syncthreads();
     // after a wait gave up: copies in flight land and issued MMAs complete before TMEM is freed
-    if (warp == 4 && lane == 0)
+    if (warp == SP_EPI && lane == 0)
         for (int ks = issued - 1; ks >= 0 && ks >= issued - SPA_STAGES; ks--)
             mbar_drain(&bar_full[ks % SPA_STAGES], (uint32_t)((ks / SPA_STAGES) & 1));
-    if (warp == 5 && lane == 0) mbar_drain(&bar_done, 0);
+    if (warp == SP_EPI + 1 && lane == 0) mbar_drain(&bar_done, 0);
     __syncthreads();
     if (warp == 0) {
         asm volatile("tcgen05.fence::after_thread_sync;");
