@@ -1847,10 +1847,16 @@ __global__ void z_from_real_kernel(int n, const double *__restrict__ Qt, int vlo
     Z[i + (int64_t)c * ldz] = mk(Qt[i + (int64_t)(vlo + c) * n], 0.0);
 }
 
+// Panel p starts at this element of the packed reflectors (all panels before are full).
+__host__ __device__ __forceinline__ int64_t wy_offset(int n, int p) {
+    return (int64_t)WY_NB * ((int64_t)p * (n - 1) - (int64_t)WY_NB * p * (p - 1) / 2);
+}
+
 // Panel reflectors k0..k0+nbp-1 as a dense (m0 x nbp) matrix, m0 = n-k0-1, row r = global
-// row k0+1+r: zero above each reflector's unit entry.
-__global__ void wy_extract_kernel(int n, int k0, int nbp, const cplx *__restrict__ A, int64_t lda, cplx *Vp) {
-    const int m0 = n - k0 - 1;
+// row k0+1+r: zero above each reflector's unit entry.  blockIdx.y is the panel.
+__global__ void wy_extract_kernel(int n, const cplx *__restrict__ A, int64_t lda, cplx *Vp) {
+    const int k0 = blockIdx.y * WY_NB, nbp = min(WY_NB, n - 1 - k0), m0 = n - k0 - 1;
+    Vp += wy_offset(n, blockIdx.y);
     const int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (idx >= (int64_t)m0 * nbp) return;
     const int r = (int)(idx % m0), jj = (int)(idx / m0);
@@ -1860,10 +1866,15 @@ __global__ void wy_extract_kernel(int n, int k0, int nbp, const cplx *__restrict
     Vp[r + (int64_t)jj * m0] = v;
 }
 
-// T (nbp x nbp, ld WY_NB) from G = Vp^H Vp and tau[k0..]; one block of WY_NB threads with
-// G and T staged in shared memory (the recurrence is sequential in i).
-__global__ void wy_tfactor_kernel(int nbp, const cplx *__restrict__ G, const cplx *__restrict__ tau, int k0, cplx *T) {
+// T (nbp x nbp, ld WY_NB) from G = Vp^H Vp and tau[k0..]; one block of WY_NB threads a panel
+// with G and T staged in shared memory.  The recurrence is sequential in i and takes 0.36 ms
+// however few SMs work, so all panels go in one launch before the first is applied
+// (40/14/800: 84 launches, 30.7 ms -> 3 launches, 1 ms).
+__global__ void wy_tfactor_kernel(int n, const cplx *__restrict__ G, const cplx *__restrict__ tau, cplx *T) {
     extern __shared__ cplx wy_sm[];
+    const int k0 = blockIdx.x * WY_NB, nbp = min(WY_NB, n - 1 - k0);
+    G += (int64_t)blockIdx.x * WY_NB * WY_NB;
+    T += (int64_t)blockIdx.x * WY_NB * WY_NB;
     cplx *Gs = wy_sm, *Ts = wy_sm + WY_NB * WY_NB;
     const int j = threadIdx.x;
     for (int x = j; x < WY_NB * WY_NB; x += blockDim.x) {
@@ -2759,28 +2770,33 @@ void heev_vectors_slot(Context &c, int slot, int n, cplx *A, int64_t lda, int vl
     }
     z_from_real_kernel<<<grid1d((int64_t)n * nvec, 256), 256, 0, c.stream>>>(n, Qt, vlo, nvec, Z, ldz);
     DCG_LAUNCHED(c);
-    cplx *Vp = wsget<cplx>(c, "wy.V", (size_t)n * WY_NB);
-    cplx *G = wsget<cplx>(c, "wy.G", WY_NB * WY_NB);
-    cplx *T = wsget<cplx>(c, "wy.T", WY_NB * WY_NB);
-    cplx *W1 = wsget<cplx>(c, "wy.W1", (size_t)WY_NB * nvec);
-    cplx *W2 = wsget<cplx>(c, "wy.W2", (size_t)WY_NB * nvec);
     const cplx one = mk(1.0, 0.0), zero = mk(0.0, 0.0), mone = mk(-1.0, 0.0);
     const int nref = n - 1;
     const int npanel = (nref + WY_NB - 1) / WY_NB;
+    cplx *Vall = wsget<cplx>(c, "wy.V", (size_t)wy_offset(n, npanel - 1) + (size_t)(n - (npanel - 1) * WY_NB) * WY_NB);
+    cplx *G = wsget<cplx>(c, "wy.G", (size_t)npanel * WY_NB * WY_NB);
+    cplx *T = wsget<cplx>(c, "wy.T", (size_t)npanel * WY_NB * WY_NB);
+    cplx *W1 = wsget<cplx>(c, "wy.W1", (size_t)WY_NB * nvec);
+    cplx *W2 = wsget<cplx>(c, "wy.W2", (size_t)WY_NB * nvec);
     DCG_CUDA(cudaFuncSetAttribute(wy_tfactor_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   2 * WY_NB * WY_NB * (int)sizeof(cplx)));
+    wy_extract_kernel<<<dim3(grid1d((int64_t)nref * WY_NB, 256), npanel), 256, 0, c.stream>>>(n, A, lda, Vall);
+    DCG_LAUNCHED(c);
+    for (int p = 0; p < npanel; p++) {
+        const int nbp = std::min(WY_NB, nref - p * WY_NB), m0 = nref - p * WY_NB;
+        const cplx *Vp = Vall + wy_offset(n, p);
+        zgemm(c, OP_C, OP_N, nbp, nbp, m0, one, Vp, m0, 0, Vp, m0, 0, zero, G + (int64_t)p * WY_NB * WY_NB, nbp, 0, 1);
+    }
+    wy_tfactor_kernel<<<npanel, WY_NB, 2 * WY_NB * WY_NB * sizeof(cplx), c.stream>>>(n, G, h.tau, T);
+    DCG_LAUNCHED(c);
     for (int p = npanel - 1; p >= 0; p--) {
         const int k0 = p * WY_NB;
         const int nbp = std::min(WY_NB, nref - k0);
         const int m0 = n - k0 - 1;
-        wy_extract_kernel<<<grid1d((int64_t)m0 * nbp, 256), 256, 0, c.stream>>>(n, k0, nbp, A, lda, Vp);
-        DCG_LAUNCHED(c);
-        zgemm(c, OP_C, OP_N, nbp, nbp, m0, one, Vp, m0, 0, Vp, m0, 0, zero, G, nbp, 0, 1);
-        wy_tfactor_kernel<<<1, WY_NB, 2 * WY_NB * WY_NB * sizeof(cplx), c.stream>>>(nbp, G, h.tau, k0, T);
-        DCG_LAUNCHED(c);
+        const cplx *Vp = Vall + wy_offset(n, p), *Tp = T + (int64_t)p * WY_NB * WY_NB;
         cplx *Zs = Z + (k0 + 1);
         zgemm(c, OP_C, OP_N, nbp, nvec, m0, one, Vp, m0, 0, Zs, ldz, 0, zero, W1, nbp, 0, 1);
-        zgemm(c, OP_N, OP_N, nbp, nvec, nbp, one, T, WY_NB, 0, W1, nbp, 0, zero, W2, nbp, 0, 1);
+        zgemm(c, OP_N, OP_N, nbp, nvec, nbp, one, Tp, WY_NB, 0, W1, nbp, 0, zero, W2, nbp, 0, 1);
         zgemm(c, OP_N, OP_N, m0, nvec, nbp, mone, Vp, m0, 0, W2, nbp, 0, one, Zs, ldz, 0, 1);
     }
 }
