@@ -49,22 +49,6 @@ static std::vector<uint64_t> gosper_all(int na, int ne) {
     return out;
 }
 
-// search_cas_configuration.F90:91-110 + ras_det_check.F90:1-59
-static bool ras_ok(const Context &c, uint64_t I) {
-    if (c.ras1) {
-        const uint64_t m = (c.ras1 >= 64) ? ~0ull : ((1ull << c.ras1) - 1ull);
-        const int n1 = __builtin_popcountll(I & m);
-        if (!(c.ras1 - c.ras1_max_hole <= n1 && n1 <= c.ras1 - c.min_hole_ras1)) return false;
-    }
-    if (c.ras3) {
-        const int sh = c.ras1 + c.ras2;
-        const uint64_t hi = (sh >= 64) ? 0 : ((I >> sh) << sh);
-        const int n3 = __builtin_popcountll(I & hi);
-        if (!(n3 <= c.ras3_max_elec && c.min_elec_ras3 <= n3)) return false;
-    }
-    return true;
-}
-
 // cas_configuration_totsym (search_cas_configuration.F90:112-149)
 static int det_totsym(const Context &c, uint64_t I) {
     if (c.nsym == 1) return 1;
@@ -84,10 +68,51 @@ static int det_totsym(const Context &c, uint64_t I) {
     return ret;
 }
 
-static std::vector<uint64_t> enumerate_ci(const Context &c) {
+// Subsets of w spinors with lo to hi electrons, ascending.
+static std::vector<uint64_t> subsets_between(int w, int lo, int hi) {
     std::vector<uint64_t> out;
-    for (uint64_t I : gosper_all(c.na, c.ne))
-        if (ras_ok(c, I) && (c.nsym == 1 || det_totsym(c, I) == c.totsym)) out.push_back(I);
+    for (int n = std::max(lo, 0); n <= std::min(hi, w); n++) {
+        const std::vector<uint64_t> g = gosper_all(w, n);
+        out.insert(out.end(), g.begin(), g.end());
+    }
+    std::sort(out.begin(), out.end());
+    return out;
+}
+
+// search_cas_configuration.F90:91-110 + ras_det_check.F90:1-59: the bit strings of ne electrons
+// with their RAS1 holes and RAS3 electrons in range, ascending, put together from the parts
+// RAS3, RAS2 and RAS1 (high to low bits) instead of filtered out of all strings: 10 electrons in
+// 8 + 10 + 8 spinors with two holes and two particles are 5.3 million strings, 30 ms on the
+// host, of which 74,273 stay.
+static std::vector<uint64_t> ras_all(const Context &c) {
+    if (c.ne < 0 || c.ne > c.na || c.na > 64) return {};
+    if (!c.ras1 && !c.ras3) return gosper_all(c.na, c.ne);
+    const int w1 = std::min(c.ras1, c.na);                            // RAS1: bits 0 .. w1 - 1
+    const int sh = c.ras3 ? std::min(c.ras1 + c.ras2, c.na) : c.na;   // RAS3: bits sh .. na - 1
+    const int w2 = sh - w1, w3 = c.na - sh;
+    const int lo1 = c.ras1 ? c.ras1 - c.ras1_max_hole : 0, hi1 = c.ras1 ? c.ras1 - c.min_hole_ras1 : 0;
+    std::vector<std::vector<uint64_t>> low(w1 + 1), mid(w3 + 1);
+    for (int n = std::max(lo1, 0); n <= std::min(hi1, w1); n++) low[n] = gosper_all(w1, n);
+    std::vector<char> have(w3 + 1, 0);
+    std::vector<uint64_t> out;
+    for (uint64_t h : c.ras3 ? subsets_between(w3, c.min_elec_ras3, c.ras3_max_elec) : std::vector<uint64_t>{0}) {
+        const int n3 = __builtin_popcountll(h), rest = c.ne - n3;
+        if (!have[n3]) {
+            mid[n3] = subsets_between(w2, rest - std::min(hi1, w1), rest - std::max(lo1, 0));
+            have[n3] = 1;
+        }
+        for (uint64_t m : mid[n3])
+            for (uint64_t l : low[rest - __builtin_popcountll(m)])
+                out.push_back((w3 > 0 ? h << sh : 0) | (w2 > 0 ? m << w1 : 0) | l);
+    }
+    return out;
+}
+
+static std::vector<uint64_t> enumerate_ci(const Context &c) {
+    std::vector<uint64_t> out = ras_all(c);
+    if (c.nsym != 1)
+        out.erase(std::remove_if(out.begin(), out.end(), [&](uint64_t I) { return det_totsym(c, I) != c.totsym; }),
+                  out.end());
     return out;
 }
 
