@@ -145,28 +145,59 @@ void launch_gather_v(Context &c, const cplx *V, const int64_t *outer_off, int no
     DCG_LAUNCHED(c);
 }
 
+// 1/x to rounding: the hardware's ~2^-22 approximation and one third-order Newton step, three
+// FP64 instructions where a division takes five times as long; a division outside the range
+// in which neither x, 1/x nor the step's terms leave the normal numbers.
+__device__ __forceinline__ double e2_recip(double x) {
+    const int ex = (__double2hiint(x) >> 20) & 0x7FF;
+    if (ex < 64 || ex > 1982) return 1.0 / x;
+    double r;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
+    const double e = fma(-x, r, 1.0);
+    return fma(r, fma(e, e, e), r);
+}
+
 // e2o[o] = -sum_j |VC(j,o)|^2/(alpha_o + wb_j), sc2o[o] = sum_j |VC(j,o)|^2/(alpha_o + wb_j)^2
-// (solve_A_subspace.F90:236-261, same loop in B..G)
+// (solve_A_subspace.F90:236-261, same loop in B..G).  W lanes share an outer index.  The FP64 pipe
+// is the limit: nine instructions a term (two divisions made it about twenty).  A thread an
+// outer index needs no reduction, and is the form of many outer indices and short sums (G:
+// 12.8M of 14); a warp takes long sums, which were one serial chain, and few outer indices
+// (all of 20/12/300: 0.82 -> 0.32 ms, of 40/14/800: 10.0 -> 3.9 ms).
+template <int W>
 __global__ void e2_kernel(const cplx *__restrict__ VC, int dimm, int nouter, const double *__restrict__ alpha,
                           const double *__restrict__ wb, double *e2o, double *sc2o) {
-    const int o = blockIdx.x * blockDim.x + threadIdx.x;
-    if (o >= nouter) return;
+    const int64_t x = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const int64_t o = x / W;
+    const int l = (int)(x % W);
+    if (o >= nouter) return;   // whole warps when W = 32
     const double al = alpha[o];
     double e = 0.0, s = 0.0;
-    for (int j = 0; j < dimm; j++) {
-        const double a2 = cabs2(VC[j + (int64_t)dimm * o]);
-        const double den = al + wb[j];
-        e -= a2 / den;
-        s += a2 / (den * den);
+    for (int j = l; j < dimm; j += W) {
+        const double r = e2_recip(al + wb[j]);
+        const double t = cabs2(VC[j + (int64_t)dimm * o]) * r;
+        e -= t;
+        s = fma(t, r, s);
     }
-    e2o[o] = e;
-    sc2o[o] = s;
+    if (W == 32)
+        for (int q = 16; q > 0; q >>= 1) {
+            e += __shfl_down_sync(0xffffffffu, e, q);
+            s += __shfl_down_sync(0xffffffffu, s, q);
+        }
+    if (l == 0) {
+        e2o[o] = e;
+        sc2o[o] = s;
+    }
 }
 
 void launch_e2(Context &c, const cplx *VC, int dimm, int nouter, const double *alpha, const double *wb, double *e2o,
                double *sc2o) {
     if (nouter == 0) return;
-    e2_kernel<<<grid1d(nouter, 128), 128, 0, c.stream>>>(VC, dimm, nouter, alpha, wb, e2o, sc2o);
+    // a warp costs ten shuffled adds, a thread a chain of nine instructions a term: below 4096
+    // outer indices the chip is not full either way and the chain is what counts
+    if (dimm >= 32 || nouter < 4096)
+        e2_kernel<32><<<grid1d((int64_t)nouter * 32, 128), 128, 0, c.stream>>>(VC, dimm, nouter, alpha, wb, e2o, sc2o);
+    else
+        e2_kernel<1><<<grid1d(nouter, 128), 128, 0, c.stream>>>(VC, dimm, nouter, alpha, wb, e2o, sc2o);
     DCG_LAUNCHED(c);
 }
 
@@ -478,18 +509,29 @@ void launch_F_pack(Context &c, const cplx *Fc, int ns, int na, cplx *Fp) {
 // One block per (b, i), i >= 1: its threads run over the (j < i, a > b) pairs with a fastest, so
 // both operands, (a i|b j) and (a j|b i), are contiguous runs over a and every element of the
 // a > b half of the class is read exactly once (streaming loads); the a < b half is never read.
-// The FP64 pipe, not HBM, bounds this kernel on GB300 (about two FP64 operations per clock per
-// SM): per element two subtractions and |V|^2, the denominator, a reciprocal and the two
-// accumulations.  The reciprocal is the FP32 one widened and refined by one Newton-Raphson step
-// for 1/e, r = r0 + r0 (1 - e r0), whose relative error is the square of the FP32 error
-// (<= 2^-48) plus rounding; a denominator outside the FP32 normal range takes 1.0 / e.
+// The FP64 pipe, not HBM, bounds this kernel on GB300 (a warp instruction in 77 clocks and SM
+// quarter): per element two subtractions and |V|^2, the denominator, a reciprocal and the two
+// accumulations, ten instructions.  The reciprocal is the FP32 one widened and refined by one
+// Newton-Raphson step for 1/e, r = r0 + r0 (1 - e r0), whose relative error is the square of the
+// FP32 error (<= 2^-46) plus rounding; a denominator outside the FP32 normal range takes 1.0 / e.
+// The narrowing cuts the bits and the widening shifts them: as conversions both would run on the
+// FP64 pipe (20 inactive, 300 secondary spinors: 0.285 ms with them and with the denominator in
+// two additions, 0.249 now).
 __device__ __forceinline__ double h_recip(double e) {
-    const float ef = __double2float_rn(e);
-    const float af = fabsf(ef);
-    if (!(af >= 1.1754944e-38f && af <= 3.0e38f)) return 1.0 / e;
-    const double r0 = (double)__frcp_rn(ef);
+    const int hi = __double2hiint(e);
+    const int ex = ((hi >> 20) & 0x7FF) - 896;   // exponent field in FP32
+    if (ex < 3 || ex > 250) return 1.0 / e;
+    // e rounded to 23 fraction bits: half a unit of them added to the bits (a carry goes on into
+    // the exponent)
+    const uint32_t lo = (uint32_t)__double2loint(e), lo2 = lo + 0x10000000u;
+    const uint32_t h2 = (uint32_t)hi + (lo2 < lo ? 1u : 0u);
+    const uint32_t m = ((h2 & 0x7FFFFFFFu) - (896u << 20)) << 3 | lo2 >> 29;
+    const uint32_t r = __float_as_uint(__frcp_rn(__uint_as_float((h2 & 0x80000000u) | m)));
+    const double r0 = __hiloint2double((int)((r & 0x80000000u) | (((r & 0x7FFFFFFFu) >> 3) + (896u << 20))), (int)(r << 29));
     return fma(r0, fma(-e, r0, 1.0), r0);
 }
+
+constexpr int kHDen = 512;
 
 __global__ void __launch_bounds__(256) h_stream_kernel(const cplx *__restrict__ Hc, int ni, int ns,
                                                        const double *__restrict__ eps_i,
@@ -497,6 +539,7 @@ __global__ void __launch_bounds__(256) h_stream_kernel(const cplx *__restrict__ 
                                                        const int *__restrict__ irp_i, const int *__restrict__ irp_s,
                                                        const int *__restrict__ md, const int *__restrict__ msy,
                                                        int nsym, double eshift, double *e2part, double *sc2part) {
+    __shared__ double h_den[kHDen];   // eps_b - eps_i + eshift - eps_j of the first j
     __shared__ double sh[2][8];
     const int b = blockIdx.x, i = blockIdx.y + 1;
     const int64_t S = ns, I = ni;
@@ -504,6 +547,8 @@ __global__ void __launch_bounds__(256) h_stream_kernel(const cplx *__restrict__ 
     const int tot = i * nab;       // (j, a) pairs of this block
     const double cbi = eps_s[b] - eps_i[i] + eshift;
     const int irb = irp_s[b], iri = irp_i[i];
+    for (int j = threadIdx.x; j < min(i, kHDen); j += blockDim.x) h_den[j] = cbi - eps_i[j];
+    __syncthreads();
     const cplx *row1 = Hc + (b + 1) + S * (i + I * (int64_t)b);   // (a i|b j) = row1[a' + S I S j]
     const cplx *row2 = Hc + (b + 1) + S * I * (b + S * (int64_t)i);   // (a j|b i) = row2[a' + S j]
     double e2 = 0.0, sc2 = 0.0;
@@ -518,7 +563,7 @@ __global__ void __launch_bounds__(256) h_stream_kernel(const cplx *__restrict__ 
         const cplx x2 = __ldcs(row2 + a1 + S * (int64_t)j);
         const double vr = x1.x - x2.x, vi = x1.y - x2.y;
         const double a2 = fma(vr, vr, vi * vi);
-        const double e = __ldg(eps_s + a) + (cbi - __ldg(eps_i + j));
+        const double e = __ldg(eps_s + a) + (j < kHDen ? h_den[j] : cbi - __ldg(eps_i + j));
         const double r = h_recip(e);
         const double t = a2 * r;
         e2 -= t;
