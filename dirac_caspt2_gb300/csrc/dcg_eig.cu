@@ -922,7 +922,7 @@ struct DcBufs {
 
 // Sums of four values over groups of G lanes; every lane of a group gets all four.  The first two
 // exchange steps halve the number of values a lane carries, so 32 lanes take six FP64 additions
-// instead of twenty (each holds a quarter SM for 64 clocks).
+// instead of twenty (each holds a quarter SM for 77 clocks).
 template <int G>
 __device__ __forceinline__ void dc_sum4(double &v0, double &v1, double &v2, double &v3) {
     const int lane = threadIdx.x & 31;
@@ -1896,6 +1896,43 @@ __global__ void wy_tfactor_kernel(int n, const cplx *__restrict__ G, const cplx 
     for (int x = j; x < WY_NB * WY_NB; x += blockDim.x) T[x] = Ts[x];
 }
 
+// f = t (sum of s over the column's WPC warps), the same in every lane.  The lower half of a
+// warp sums the real part and the upper half the imaginary part, and each forms its part of f:
+// 8 FP64 instructions where both in every lane take 16 of the 72 of a 791-row reflector in
+// two warps (two times 791 vectors of order 791: 9.8 -> 9.3 ms).  `part` alternates
+// between two buffers, so one barrier a reflector is enough.
+template <int WPC, bool REAL>
+__device__ __forceinline__ void bt_scale(double sr, double si, cplx t, int wsub, double (&part)[2][2], double &fr,
+                                         double &fi) {
+    const int lane = threadIdx.x & 31;
+    if (REAL) {
+        for (int o = 16; o > 0; o >>= 1) sr += __shfl_xor_sync(0xffffffffu, sr, o);
+        if (WPC == 2) {
+            if (lane == 0) part[wsub][0] = sr;
+            __syncthreads();
+            sr = part[0][0] + part[1][0];
+        }
+        fr = t.x * sr;
+        fi = 0.0;
+        return;
+    }
+    const int h = lane >> 4;
+    double s = h ? si : sr;
+    s += __shfl_xor_sync(0xffffffffu, h ? sr : si, 16);
+    for (int o = 8; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (WPC == 2) {   // the two warps' sums, in a fixed order
+        if ((lane & 15) == 0) part[wsub][h] = s;
+        __syncthreads();
+        s = part[0][h] + part[1][h];
+    }
+    const double other = __shfl_xor_sync(0xffffffffu, s, 16);
+    // Re f = t.x Re s - t.y Im s, Im f = t.x Im s + t.y Re s
+    const double ty = __hiloint2double(__double2hiint(t.y) ^ (h ? 0 : (int)0x80000000), __double2loint(t.y));
+    const double f = fma(t.x, s, ty * other);
+    fr = __shfl_sync(0xffffffffu, f, 0);
+    fi = __shfl_sync(0xffffffffu, f, 16);
+}
+
 // Register-resident back-transformation (n <= 32 R WPC): WPC warps per eigenvector column,
 // the column held in registers (warp w, lane l owns rows l + 32 (WPC i + w)), the reflectors
 // applied from the last to the first.  Reflector k-1 is loaded into registers while reflector
@@ -1962,25 +1999,8 @@ __global__ void __launch_bounds__(64) backtransform_reg_kernel(int n, const cplx
                     }
                 }
             }
-            double sr = s0r + s1r, si = s0i + s1i;
-            for (int o = 16; o > 0; o >>= 1) {
-                sr += __shfl_down_sync(0xffffffffu, sr, o);
-                if (!REAL) si += __shfl_down_sync(0xffffffffu, si, o);
-            }
-            if (WPC == 2) {
-                if (lane == 0) {
-                    part[k & 1][wsub][0] = sr;
-                    part[k & 1][wsub][1] = si;
-                }
-                __syncthreads();
-                sr = part[k & 1][0][0] + part[k & 1][1][0];
-                si = part[k & 1][0][1] + part[k & 1][1][1];
-            } else {
-                sr = __shfl_sync(0xffffffffu, sr, 0);
-                si = __shfl_sync(0xffffffffu, si, 0);
-            }
-            // f = tau (v^H z)
-            const double fr = REAL ? t.x * sr : t.x * sr - t.y * si, fi = REAL ? 0.0 : t.x * si + t.y * sr;
+            double fr, fi;   // f = tau (v^H z)
+            bt_scale<WPC, REAL>(s0r + s1r, REAL ? 0.0 : s0i + s1i, t, wsub, part[k & 1], fr, fi);
 #pragma unroll
             for (int i = 0; i < R; i++) {
                 if (i < i0) continue;
@@ -2603,21 +2623,8 @@ __global__ void __launch_bounds__(64) apply_qh_kernel(int n, const cplx *__restr
             sr = fma(vv.x, z[i].x, REAL ? sr : fma(vv.y, z[i].y, sr));    // conj(v) z
             if (!REAL) si = fma(vv.x, z[i].y, fma(-vv.y, z[i].x, si));
         }
-        for (int o = 16; o > 0; o >>= 1) {
-            sr += __shfl_xor_sync(0xffffffffu, sr, o);
-            if (!REAL) si += __shfl_xor_sync(0xffffffffu, si, o);
-        }
-        if (WPC == 2) {   // the two warps' partial dots, summed in a fixed order
-            if (lane == 0) {
-                part[k & 1][wsub][0] = sr;
-                part[k & 1][wsub][1] = si;
-            }
-            __syncthreads();
-            sr = part[k & 1][0][0] + part[k & 1][1][0];
-            si = part[k & 1][0][1] + part[k & 1][1][1];
-        }
-        // f = conj(tau) (v^H z)
-        const double fr = REAL ? t.x * sr : t.x * sr + t.y * si, fi = REAL ? 0.0 : t.x * si - t.y * sr;
+        double fr, fi;   // f = conj(tau) (v^H z)
+        bt_scale<WPC, REAL>(sr, si, mk(t.x, -t.y), wsub, part[k & 1], fr, fi);
 #pragma unroll
         for (int i = 0; i < R; i++) {
             if (i < i0) continue;
