@@ -258,8 +258,8 @@ int dcg_zgemm(dcg_ctx *ctx, int precision, int32_t M, int32_t N, int32_t K, int3
 #define DCG_FAM_EIG_BACK 9    /*   back-transformation (FLOPs 8 n^2 m)                            */
 #define DCG_FAM_SPLIT_MMA 10  /* tcgen05 split-precision GEMM kernel; work = BF16 tensor FLOPs      */
 
-/* Time limit of the context's device-side waits that can give up: the grid barriers and the
- * published-reflector waits of the Householder tridiagonalisation (default 5 s) and the
+/* Time limit of the context's device-side waits that can give up: the waits of the
+ * Householder tridiagonalisation for the other blocks' flagged words (default 5 s) and the
  * pipeline waits of the tensor-core GEMM kernels (default 2 s).  A wait that runs out sets an
  * error flag; the kernel's other blocks leave at their next wait, copies still in flight land
  * and issued tensor-core operations complete (waits bounded by the default limits) before a
@@ -371,8 +371,9 @@ int dcg_merged_reduction_stats(int device, int64_t out[3]);
 int dcg_casci_energy_check(dcg_ctx *ctx, double out[8]);
 
 /* ------------------------------------------------------------------------ autotuner
- * Shape-dependent launch choices (today: the tile shape, 64x64, 32x128 or 128x32, and the
- * K-split of the FP64 GEMMs; for the split-precision tensor-core GEMMs the kernel, one tile
+ * Shape-dependent launch choices (today: the tile shape, from 64x64, 32x128 and 128x32 down to
+ * 8x4, and the K-split of the FP64 GEMMs, the candidates a cost model puts within 1.3 times
+ * the best; for the split-precision tensor-core GEMMs the kernel, one tile
  * per CTA or persistent CTAs whose epilogue overlaps the next tile's MMAs, and the CTA
  * raster, row-block or column-block major, which decides which operand tiles meet in L2) are
  * tuned on first use, for products of at least ~1 ms of work:
