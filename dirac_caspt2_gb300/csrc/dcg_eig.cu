@@ -496,6 +496,10 @@ __device__ __forceinline__ double fast_rsqrt(double x) {
     return fma(y, fma(0.375, e, 0.5) * e, y);
 }
 
+}  // namespace dcg
+#include "dcg_deflate.cuh"
+namespace dcg {
+
 // Reflector of the column alpha, x with ss = |x|^2 (LAPACK's documented xLARFG, beta real): tau,
 // beta, the scale sc = 1 / (alpha - beta) of x, and mib = tau sc = -1 / beta (0 for tau = 0).
 __device__ __forceinline__ void trd_scalars(cplx alpha, double ss, cplx &tau, double &beta, cplx &scale, double &mib) {
@@ -918,7 +922,7 @@ struct DcBufs {
     double *zh;               // recomputed rank-one vector
     int *outc;                // output column of each node entry in the next level
     int *top, *bot;           // undeflated entries whose column reaches the node's first / second half
-    int *k0, *flag, *half;    // prep scratch: entries past the z test, rotation flags, halves reached
+    int *k0, *flag, *half;    // prep scratch: entries past the z test, close pairs, halves reached
     int *kcnt, *ndef, *nrot;  // per node: undeflated count (-1: pass-through), deflated, rotations
     int *ntop, *nbot;         // per node: lengths of top and bot
     double *rho;              // per node
@@ -1099,30 +1103,6 @@ __device__ void dc_secular_root(int k, int j, bool act, const double *dk, const 
         tau_out = tau;
         lam_out = d_o + tau;
     }
-}
-
-// Whether the rank-one components zp, zn of neighbouring poles a distance t apart combine into
-// one by a rotation (|t c s| <= tol for c = zn / |z|, s = zp / |z|), without a division.
-__device__ __forceinline__ bool dc_close(double t, double zp, double zn, double tol) {
-    return fabs(t * zp * zn) <= tol * fma(zp, zp, zn * zn);
-}
-
-// One pair rotation of the deflation scan: component zp folds into zn.
-__device__ __forceinline__ void dc_rotate(double &dp, double zp, double &dn, double &zn, double &C, double &S) {
-    const double t2 = fma(zn, zn, zp * zp), a = dp, c = dn;
-    if (t2 > 1e-280) {
-        const double ri = fast_rsqrt(t2);
-        C = zn * ri;
-        S = -zp * ri;
-        zn = t2 * ri;
-    } else {   // the squares are out of range
-        const double tt = hypot(zn, zp);
-        C = zn / tt;
-        S = -zp / tt;
-        zn = tt;
-    }
-    dp = a * C * C + c * S * S;
-    dn = a * S * S + c * C * C;
 }
 
 // Levels up to nodes of kDcBase columns in one launch: a block of 128 threads merges its columns
@@ -1347,8 +1327,8 @@ __device__ int dc_block_excl_scan(int v, int *wsum, int &total) {
 // One block per node: rank-one vector, merge order, deflation.  Deflation runs in parallel: the
 // z test of every entry, then the rotation test of every neighbouring kept pair on the unrotated
 // values; each maximal run of qualifying pairs is scanned by one thread, with the rotated
-// values, until a test past the run's end fails.  A scan that reaches the next run would
-// change that run's input; the block then repeats the scan in thread 0 alone.  The rotations
+// values, until a test past the run's end fails (dc_deflate_scan).  A scan that reaches the next
+// run would change that run's input; the block then repeats the scan in thread 0 alone.  The rotations
 // themselves are applied to the eigenvector columns by dc_merge_kernel, which has the rows
 // of the node spread over many blocks.  Dynamic shared memory: 20 bytes per node column.
 __global__ void dc_prep_kernel(int n, int half, int full, const double *__restrict__ e, DcBufs b) {
@@ -1376,14 +1356,14 @@ __global__ void dc_prep_kernel(int n, int half, int full, const double *__restri
     const double beta = e[s + n1 - 1];
     const double rho = 2.0 * fabs(beta);
     const double sg = beta < 0.0 ? -1.0 : 1.0;
-    auto load = [&](int i) {
-        sd[i] = b.lamA[s + i];
+    auto source = [&](int i, double &dv, double &zv) {   // pole and component of column i, unrotated
+        dv = b.lamA[s + i];
         const double q = i < n1 ? b.QA[(s + n1 - 1) + (int64_t)(s + i) * n] : sg * b.QA[(s + n1) + (int64_t)(s + i) * n];
-        sz[i] = q * 0.70710678118654752440;
+        zv = q * 0.70710678118654752440;
     };
     double mx = 0.0;
     for (int i = threadIdx.x; i < N; i += blockDim.x) {
-        load(i);
+        source(i, sd[i], sz[i]);
         mx = fmax(mx, fmax(fabs(sd[i]), fabs(sz[i])));
     }
     // a valid permutation first: the merge below writes every slot exactly once for ordered
@@ -1415,8 +1395,9 @@ __global__ void dc_prep_kernel(int n, int half, int full, const double *__restri
         }
     }
     __syncthreads();
-    int *K0 = b.k0 + s, *tf = b.flag + s, *hm = b.half + s;
-    double *rC = b.tau + s, *rS = b.lamK + s;   // scratch until the secular stage
+    int *K0 = b.k0 + s, *close = b.flag + s, *hm = b.half + s;
+    int *fold = b.ord + s;                    // scratch until the secular stage, as the next two
+    double *rC = b.tau + s, *rS = b.lamK + s;
     const int per = (N + (int)blockDim.x - 1) / (int)blockDim.x;
     int k0;   // entries past the z test; the others go to defl at once
     {
@@ -1437,7 +1418,7 @@ __global__ void dc_prep_kernel(int n, int half, int full, const double *__restri
         if (threadIdx.x == 0) s_rot = s_conflict = 0;
         __syncthreads();
     }
-    {   // tf[m]: the pair (m - 1, m) qualifies for a rotation
+    {   // close[m]: the pair (m - 1, m) qualifies for a rotation
         int rot = 0;
         for (int m = threadIdx.x; m < k0; m += blockDim.x) {
             int t = 0;
@@ -1445,7 +1426,8 @@ __global__ void dc_prep_kernel(int n, int half, int full, const double *__restri
                 const int pj = K0[m - 1], nj = K0[m];
                 t = dc_close(sd[nj] - sd[pj], sz[pj], sz[nj], tol);
             }
-            tf[m] = t;
+            close[m] = t;
+            fold[m] = 0;
             rot |= t;
         }
         if (rot) atomicOr(&s_rot, 1);
@@ -1453,54 +1435,19 @@ __global__ void dc_prep_kernel(int n, int half, int full, const double *__restri
     }
     const bool any = s_rot != 0;
     if (any) {
-        // Bit 1 of tf[m]: entry m was folded into m + 1 (set by the scanning thread).
-        auto scan = [&](int m, bool whole) {   // from the pair (m - 1, m); returns whether it hit the next run
-            int pj = K0[m - 1], hp = hm[m - 1];
-            double dp = sd[pj], zp = sz[pj];
-            bool dirty = false;   // entry m - 1 carries rotated values
-            for (; m < k0; m++) {
-                const int nj = K0[m];
-                double dn = sd[nj], zn = sz[nj], C, S;
-                int hn = hm[m];
-                const bool inrun = (tf[m] & 1) != 0;
-                if (!whole && !inrun && !dirty) break;        // past the run's end
-                if (dc_close(dn - dp, zp, zn, tol)) {
-                    // folding into an entry whose own pair starts the next run
-                    if (!whole && !inrun && m + 1 < k0 && (tf[m + 1] & 1)) return true;
-                    dc_rotate(dp, zp, dn, zn, C, S);
-                    rC[m - 1] = C;
-                    rS[m - 1] = S;
-                    sd[pj] = dp;
-                    tf[m - 1] |= 2;
-                    hn |= hp;
-                    hm[m - 1] = hn;   // a folded column mixes both as well
-                    dirty = true;
-                    sd[nj] = dn;
-                    sz[nj] = zn;
-                    hm[m] = hn;
-                } else {
-                    dirty = false;
-                    if (!whole && !inrun) break;
-                }
-                pj = nj;
-                dp = dn;
-                zp = zn;
-                hp = hn;
-            }
-            return false;
-        };
+        const DeflScan a{K0, close, fold, hm, sd, sz, rC, rS, k0, n1, tol};
         for (int m = 1 + (int)threadIdx.x; m < k0; m += blockDim.x)
-            if ((tf[m] & 1) && !(tf[m - 1] & 1))
-                if (scan(m, false)) s_conflict = 1;
+            if (close[m] && !close[m - 1])
+                if (dc_deflate_scan(a, m, false, source)) atomicOr(&s_conflict, 1);
         __syncthreads();
         if (s_conflict) {
-            for (int i = threadIdx.x; i < N; i += blockDim.x) load(i);
+            for (int i = threadIdx.x; i < N; i += blockDim.x) source(i, sd[i], sz[i]);
             for (int m = threadIdx.x; m < k0; m += blockDim.x) {
-                tf[m] &= 1;
+                fold[m] = 0;
                 hm[m] = K0[m] < n1 ? 1 : 2;
             }
             __syncthreads();
-            if (threadIdx.x == 0 && k0 > 1) scan(1, true);
+            if (threadIdx.x == 0 && k0 > 1) dc_deflate_scan(a, 1, true, source);
             __syncthreads();
         }
     }
@@ -1510,9 +1457,9 @@ __global__ void dc_prep_kernel(int n, int half, int full, const double *__restri
         const int t0 = min(k0, (int)threadIdx.x * per), t1 = min(k0, t0 + per);
         int nf = 0, nt = 0, nbm = 0;
         for (int m = t0; m < t1; m++) {
-            const bool fold = any && (tf[m] & 2);
-            nf += fold;
-            if (!fold) {
+            const bool gone = any && fold[m];
+            nf += gone;
+            if (!gone) {
                 nt += hm[m] & 1;
                 nbm += hm[m] >> 1;
             }
@@ -1523,7 +1470,7 @@ __global__ void dc_prep_kernel(int n, int half, int full, const double *__restri
         int bb = dc_block_excl_scan(nbm, s_wsum, tot_b);
         for (int m = t0; m < t1; m++) {
             const int j = K0[m];
-            if (any && (tf[m] & 2)) {
+            if (any && fold[m]) {
                 b.rp[s + fb] = j;
                 b.rn[s + fb] = K0[m + 1];
                 b.rc[s + fb] = rC[m];
