@@ -1851,8 +1851,12 @@ __global__ void wy_tfactor_kernel(int n, const cplx *__restrict__ G, const cplx 
 // f = t (sum of s over the column's WPC warps), the same in every lane.  The lower half of a
 // warp sums the real part and the upper half the imaginary part, and each forms its part of f:
 // 8 FP64 instructions where both in every lane take 16 of the 72 of a 791-row reflector in
-// two warps (two times 791 vectors of order 791: 9.8 -> 9.3 ms).  `part` alternates
-// between two buffers, so one barrier a reflector is enough.
+// two warps (two times 791 vectors of order 791: 9.8 -> 9.3 ms).  The caller alternates `part`
+// between two buffers from one applied reflector to the next, so one barrier each is enough: a
+// buffer is written again only after the barrier of the reflector between, which the other warp
+// reaches when it has read the old sums.  Reflectors with tau = 0 are skipped and have no
+// barrier, so they do not count (by the reflector's number, two applied ones around a skipped
+// one would share a buffer with nothing between them).
 template <int WPC, bool REAL>
 __device__ __forceinline__ void bt_scale(double sr, double si, cplx t, int wsub, double (&part)[2][2], double &fr,
                                          double &fi) {
@@ -1898,7 +1902,7 @@ __global__ void __launch_bounds__(64) backtransform_reg_kernel(int n, const cplx
                                                                 const cplx *__restrict__ tau,
                                                                 const double *__restrict__ Qt, int vlo, int nvec,
                                                                 cplx *Z, int64_t ldz) {
-    __shared__ double part[2][2][2];   // [parity][warp][re, im]
+    __shared__ double part[2][2][2];   // [buffer][warp][re, im]
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int wsub = warp % WPC;                               // warp within its column
     const int col = blockIdx.x * (2 / WPC) + warp / WPC;       // 64 threads: 2 / WPC columns
@@ -1918,6 +1922,7 @@ __global__ void __launch_bounds__(64) backtransform_reg_kernel(int n, const cplx
         }                                                                                    \
     }
     if (PF && n >= 2) BT_LOAD(n - 2, vc);
+    int applied = 0;   // reflectors that were not skipped
     for (int k = n - 2; k >= 0; k--) {
         if (PF && k >= 1) BT_LOAD(k - 1, vn);
         const cplx t = __ldg(tau + k);
@@ -1952,7 +1957,7 @@ __global__ void __launch_bounds__(64) backtransform_reg_kernel(int n, const cplx
                 }
             }
             double fr, fi;   // f = tau (v^H z)
-            bt_scale<WPC, REAL>(s0r + s1r, REAL ? 0.0 : s0i + s1i, t, wsub, part[k & 1], fr, fi);
+            bt_scale<WPC, REAL>(s0r + s1r, REAL ? 0.0 : s0i + s1i, t, wsub, part[applied++ & 1], fr, fi);
 #pragma unroll
             for (int i = 0; i < R; i++) {
                 if (i < i0) continue;
@@ -2549,7 +2554,7 @@ template <int R, int WPC, bool REAL>
 __global__ void __launch_bounds__(64) apply_qh_kernel(int n, const cplx *__restrict__ A, int64_t lda,
                                                      const cplx *__restrict__ tau, const cplx *__restrict__ Y0,
                                                      int64_t ldy0, int ncol, cplx *Y, int64_t ldy) {
-    __shared__ double part[2][2][2];   // [parity][warp][re, im]
+    __shared__ double part[2][2][2];   // [buffer][warp][re, im]
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int wsub = warp % WPC;                              // warp within its column
     const int col = blockIdx.x * (2 / WPC) + warp / WPC;      // 64 threads: 2 / WPC columns
@@ -2561,6 +2566,7 @@ __global__ void __launch_bounds__(64) apply_qh_kernel(int n, const cplx *__restr
         const int r = lane + 32 * (WPC * i + wsub);
         z[i] = (have && r < n) ? Y0[r + (int64_t)col * ldy0] : mk(0.0, 0.0);
     }
+    int applied = 0;   // reflectors that were not skipped
     for (int k = 0; k + 1 < n; k++) {
         const cplx t = __ldg(tau + k);
         if (t.x == 0.0 && t.y == 0.0) continue;   // uniform over the block
@@ -2576,7 +2582,7 @@ __global__ void __launch_bounds__(64) apply_qh_kernel(int n, const cplx *__restr
             if (!REAL) si = fma(vv.x, z[i].y, fma(-vv.y, z[i].x, si));
         }
         double fr, fi;   // f = conj(tau) (v^H z)
-        bt_scale<WPC, REAL>(sr, si, mk(t.x, -t.y), wsub, part[k & 1], fr, fi);
+        bt_scale<WPC, REAL>(sr, si, mk(t.x, -t.y), wsub, part[applied++ & 1], fr, fi);
 #pragma unroll
         for (int i = 0; i < R; i++) {
             if (i < i0) continue;
