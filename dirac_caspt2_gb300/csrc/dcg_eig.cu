@@ -406,7 +406,7 @@ __global__ void __launch_bounds__(TRD_THREADS) tridiag_persistent_kernel(int n, 
 // matvec, x to every block, the next column's update) and the FP64 unit (a warp's FP64
 // instruction holds a quarter of the SM for 70 to 77 clocks, whether one lane is active or all).  So:
 //   - the column and x travel as 16-byte words that carry their own flag (the column's number
-//     beside each half of a double): a reader polls the data itself, one trip through L2 instead
+//     above each half of a double): a reader polls the data itself, one trip through L2 instead
 //     of data, fence, counter and data again.
 //   - the column goes out unscaled as soon as it is updated (u; v = sc u below a unit first
 //     element).  Every block multiplies with u while a seventeenth warp of the owner forms tau
@@ -435,7 +435,7 @@ struct TrdJob {
     int64_t lda;
     double *d, *e;
     cplx *tau;
-    uint4 *ll;      // trd_ll_words(n) words, zero before the launch
+    ulonglong2 *ll;      // trd_ll_words(n) words, zero before the launch
     int n, b0, nb, real;
 };
 struct TrdTable {
@@ -447,20 +447,21 @@ struct TrdTable {
 // exchange words of one problem: by column parity x (2 n), u (2 n) and the header (8)
 __host__ __device__ inline size_t trd_ll_words(int n) { return 8 * (size_t)n + 16; }
 
-// A double with a flag beside each of its halves in one 16-byte word.
-__device__ __forceinline__ void ll_store(uint4 *p, double v, unsigned flag) {
-    asm volatile("st.volatile.global.v4.u32 [%0], {%1, %2, %3, %4};" ::"l"(p), "r"(__double2loint(v)), "r"(flag),
-                 "r"(__double2hiint(v)), "r"(flag)
+// A double in one 16-byte word: two 64-bit elements, each a half of it with the flag above it.  (Data
+// words that carry their own flag are the low-latency exchange known from communication
+// libraries.)  A vector access is one access per element in no given order, and a 64-bit element
+// is read and written whole, so each flag vouches for the half beside it.
+__device__ __forceinline__ void ll_store(ulonglong2 *p, double v, unsigned flag) {
+    const unsigned long long f = (unsigned long long)flag << 32;
+    asm volatile("st.volatile.global.v2.b64 [%0], {%1, %2};" ::"l"(p), "l"(f | (unsigned)__double2loint(v)),
+                 "l"(f | (unsigned)__double2hiint(v))
                  : "memory");
 }
-__device__ __forceinline__ bool ll_load(const uint4 *p, unsigned flag, double &v) {
-    unsigned lo, f0, hi, f1;
-    asm volatile("ld.volatile.global.v4.u32 {%0, %1, %2, %3}, [%4];"
-                 : "=r"(lo), "=r"(f0), "=r"(hi), "=r"(f1)
-                 : "l"(p)
-                 : "memory");
-    v = __hiloint2double((int)hi, (int)lo);
-    return f0 == flag && f1 == flag;
+__device__ __forceinline__ bool ll_load(const ulonglong2 *p, unsigned flag, double &v) {
+    unsigned long long lo, hi;
+    asm volatile("ld.volatile.global.v2.b64 {%0, %1}, [%2];" : "=l"(lo), "=l"(hi) : "l"(p) : "memory");
+    v = __hiloint2double((int)(unsigned)hi, (int)(unsigned)lo);
+    return (unsigned)(lo >> 32) == flag && (unsigned)(hi >> 32) == flag;
 }
 
 // A bounded wait of one thread (the clock and the problem's error flag are read every 4 polls).
@@ -543,7 +544,7 @@ __device__ void tridiag_smem_body(const TrdJob &J, const int b, int *err, const 
     const int n = J.n, nb = J.nb;
     cplx *A = J.A;
     const int64_t lda = J.lda;
-    uint4 *xb = J.ll, *ub = xb + 4 * (size_t)n, *hb = ub + 4 * (size_t)n;   // [parity][n][2], [parity][n][2], [parity][8]
+    ulonglong2 *xb = J.ll, *ub = xb + 4 * (size_t)n, *hb = ub + 4 * (size_t)n;   // [parity][n][2], [parity][n][2], [parity][8]
     const int tid = threadIdx.x, lane = tid & 31, q = (tid >> 5) & 3, s = tid >> 7;   // quarter, and warp within it
     const bool chain = s == 0, header = s == 4;
     const int nown = (n - b + nb - 1) / nb;   // columns b, b+nb, ...
@@ -577,7 +578,7 @@ __device__ void tridiag_smem_body(const TrdJob &J, const int b, int *err, const 
             const double a2 = 2.0 * s_al;
             yj = mk(fma(a2, vj.x, x.x), fma(a2, vj.y, x.y));
         }
-        uint4 *uo = ub + (size_t)(k1 & 1) * 2 * n;
+        ulonglong2 *uo = ub + (size_t)(k1 & 1) * 2 * n;
         const unsigned flag = (unsigned)k1 + 1u;
         double s0 = 0.0, s1 = 0.0;
         TRD_GROUPS(i0) TRD_ROWS(i0, i, r, k1) {
@@ -626,7 +627,7 @@ __device__ void tridiag_smem_body(const TrdJob &J, const int b, int *err, const 
         const unsigned flag = (unsigned)k + 1u;
         const int par = k & 1;
         if (chain && !owner) {   // u, straight from its words: one row until it is there, then all
-            const uint4 *ui = ub + (size_t)par * 2 * n;
+            const ulonglong2 *ui = ub + (size_t)par * 2 * n;
             LlWait wt;
             TRD_GROUPS(i0) {
                 unsigned pend = 0;
@@ -753,7 +754,7 @@ __device__ void tridiag_smem_body(const TrdJob &J, const int b, int *err, const 
         const double sx = s_hdr[0], sy = s_hdr[1], tr = s_hdr[2], ti = s_hdr[3], mib = s_hdr[4];
         if (s >= 1 && !header) {
             // x = tau p = mib (conj(column) . u) + tau conj(A(k+1, j)) of the own columns, to every block
-            uint4 *xo = xb + (size_t)par * 2 * n;
+            ulonglong2 *xo = xb + (size_t)par * 2 * n;
             const int cnt = 2 * (nown - c0);
             for (int t = tid - 128; t < ((cnt + 31) & ~31); t += 384) {
                 const int c = c0 + (t >> 1), comp = t & 1, j = b + c * nb;
@@ -791,7 +792,7 @@ __device__ void tridiag_smem_body(const TrdJob &J, const int b, int *err, const 
         if (chain) {   // gather x, and al of w = x + al v: al = -1/2 tau x^H v = -|tau|^2 / (2 Re tau) Re(x^H v)
             const double f = tr != 0.0 ? -0.5 * fma(tr, tr, ti * ti) * fast_rcp(tr) : 0.0;
             if (nb > 1) {
-                const uint4 *xi = xb + (size_t)par * 2 * n;
+                const ulonglong2 *xi = xb + (size_t)par * 2 * n;
                 LlWait wt;
                 TRD_GROUPS(i0) {
                     unsigned pend = 0;
@@ -2134,7 +2135,7 @@ static bool trd_plan(const Context &c, std::vector<TrdJob> &jobs, int &total, si
 // The exchange words of a context's jobs start at zero, in stream order.
 static void trd_clear(Context &c, const std::vector<TrdJob> &jobs) {
     for (const TrdJob &j : jobs)
-        if (j.nb != 1) DCG_CUDA(cudaMemsetAsync(j.ll, 0, trd_ll_words(j.n) * sizeof(uint4), c.stream));
+        if (j.nb != 1) DCG_CUDA(cudaMemsetAsync(j.ll, 0, trd_ll_words(j.n) * sizeof(ulonglong2), c.stream));
 }
 
 // The launch of planned jobs on `stream` (their exchange words already cleared in stream order):
@@ -2415,7 +2416,7 @@ static bool tridiag_global(Context &c, int n, cplx *A, int64_t lda, HeevWork &h)
     j.d = h.d;
     j.e = h.e;
     j.tau = h.tau;
-    j.ll = wsget<uint4>(c, "trd.ll.global", trd_ll_words(n));
+    j.ll = wsget<ulonglong2>(c, "trd.ll.global", trd_ll_words(n));
     j.n = n;
     j.nb = nb;
     j.real = c.real_now;
@@ -2487,7 +2488,7 @@ void heev_values_batched(Context &c, const std::vector<EigJob> &jobs) {
             t.d = hw[q].d;
             t.e = hw[q].e;
             t.tau = hw[q].tau;
-            t.ll = wsget<uint4>(c, slot_name("trd.ll", j.slot), trd_ll_words(j.n));
+            t.ll = wsget<ulonglong2>(c, slot_name("trd.ll", j.slot), trd_ll_words(j.n));
             t.n = j.n;
             t.real = c.real_now;
             t.b0 = t.nb = 0;
