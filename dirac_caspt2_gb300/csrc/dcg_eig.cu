@@ -436,13 +436,13 @@ struct TrdJob {
     double *d, *e;
     cplx *tau;
     ulonglong2 *ll;      // trd_ll_words(n) words, zero before the launch
+    unsigned long long limit_ns;   // time limit of one wait (its context's, also in a merged launch)
     int n, b0, nb, real;
 };
 struct TrdTable {
     TrdJob j[kTrdMaxJobs];
     int njobs;
-    int *err;                      // per job: nonzero when a wait ran out (zero before the launch)
-    unsigned long long limit_ns;   // time limit of one wait
+    int *err;   // per job: nonzero when a wait ran out (zero before the launch)
 };
 // exchange words of one problem: by column parity x (2 n), u (2 n) and the header (8)
 __host__ __device__ inline size_t trd_ll_words(int n) { return 8 * (size_t)n + 16; }
@@ -537,11 +537,12 @@ __device__ __forceinline__ void sums_wait() { asm volatile("bar.sync 3, 160;" ::
 // GLB: the columns stay in global memory (L2, or HBM beyond it) and u has a row of shared memory of
 // its own; otherwise ROWS >= n / 128 and the chain warps hold u and v in registers.
 template <bool REAL, int ROWS, bool GLB>
-__device__ void tridiag_smem_body(const TrdJob &J, const int b, int *err, const unsigned long long limit_ns) {
+__device__ void tridiag_smem_body(const TrdJob &J, const int b, int *err) {
     extern __shared__ cplx tsm2[];
     __shared__ double s_sum[4], s_ss[4], s_hdr[5], s_al;
     __shared__ cplx s_alpha;
     const int n = J.n, nb = J.nb;
+    const unsigned long long limit_ns = J.limit_ns;
     cplx *A = J.A;
     const int64_t lda = J.lda;
     ulonglong2 *xb = J.ll, *ub = xb + 4 * (size_t)n, *hb = ub + 4 * (size_t)n;   // [parity][n][2], [parity][n][2], [parity][8]
@@ -885,14 +886,14 @@ __global__ void __launch_bounds__(TRS_THREADS) tridiag_smem_batched_kernel(const
     const TrdJob &J = T.j[j];
     const int b = (int)blockIdx.x - J.b0;
     if (J.n <= 512) {
-        if (J.real) tridiag_smem_body<true, 4, false>(J, b, T.err + j, T.limit_ns);
-        else tridiag_smem_body<false, 4, false>(J, b, T.err + j, T.limit_ns);
+        if (J.real) tridiag_smem_body<true, 4, false>(J, b, T.err + j);
+        else tridiag_smem_body<false, 4, false>(J, b, T.err + j);
     } else if (J.n <= 1024) {
-        if (J.real) tridiag_smem_body<true, 8, false>(J, b, T.err + j, T.limit_ns);
-        else tridiag_smem_body<false, 8, false>(J, b, T.err + j, T.limit_ns);
+        if (J.real) tridiag_smem_body<true, 8, false>(J, b, T.err + j);
+        else tridiag_smem_body<false, 8, false>(J, b, T.err + j);
     } else {
-        if (J.real) tridiag_smem_body<true, kTrdRows, false>(J, b, T.err + j, T.limit_ns);
-        else tridiag_smem_body<false, kTrdRows, false>(J, b, T.err + j, T.limit_ns);
+        if (J.real) tridiag_smem_body<true, kTrdRows, false>(J, b, T.err + j);
+        else tridiag_smem_body<false, kTrdRows, false>(J, b, T.err + j);
     }
 }
 
@@ -903,8 +904,8 @@ __global__ void __launch_bounds__(TRS_THREADS) tridiag_smem_batched_kernel(const
 // for: order 1300 44 -> 27 ms, 2002 210 -> 82 ms, 2744 437 -> 191 ms.
 __global__ void __launch_bounds__(TRS_THREADS) tridiag_global_kernel(const __grid_constant__ TrdTable T) {
     const TrdJob &J = T.j[0];
-    if (J.real) tridiag_smem_body<true, 8, true>(J, (int)blockIdx.x, T.err, T.limit_ns);
-    else tridiag_smem_body<false, 8, true>(J, (int)blockIdx.x, T.err, T.limit_ns);
+    if (J.real) tridiag_smem_body<true, 8, true>(J, (int)blockIdx.x, T.err);
+    else tridiag_smem_body<false, 8, true>(J, (int)blockIdx.x, T.err);
 }
 
 // ===================================================================== 2. divide and conquer
@@ -2022,11 +2023,13 @@ static HeevWork heev_work(Context &c, int n, int slot) {
 // kernels must never wait for each other's SMs.
 static std::mutex g_coop_mutex;
 
+static uint64_t trd_wait_limit(const Context &c) { return c.wait_limit_ns ? c.wait_limit_ns : kBarrierLimitNs; }
+
 // A fresh barrier (counters and error flag zero) with the context's wait limit, written in
 // stream order (a copy from pageable host memory is staged before the call returns).
 static void gridbar_reset(Context &c, GridBar *gb) {
     GridBar x{};
-    x.limit_ns = c.wait_limit_ns ? c.wait_limit_ns : kBarrierLimitNs;
+    x.limit_ns = trd_wait_limit(c);
     DCG_CUDA(cudaMemcpyAsync(gb, &x, sizeof(GridBar), cudaMemcpyHostToDevice, c.stream));
 }
 
@@ -2147,7 +2150,6 @@ static std::vector<int> trd_launch(Context &c, const std::vector<TrdJob> &jobs, 
     TrdTable T{};
     for (size_t q = 0; q < nj; q++) T.j[q] = jobs[q];
     T.njobs = (int)nj;
-    T.limit_ns = c.wait_limit_ns ? c.wait_limit_ns : kBarrierLimitNs;
     T.err = wsget<int>(c, table, kTrdMaxJobs);
     int *herr = (int *)c.ws.host(table, kTrdMaxJobs * sizeof(int));
     DCG_CUDA(cudaMemsetAsync(T.err, 0, nj * sizeof(int), stream));
@@ -2417,6 +2419,7 @@ static bool tridiag_global(Context &c, int n, cplx *A, int64_t lda, HeevWork &h)
     j.e = h.e;
     j.tau = h.tau;
     j.ll = wsget<ulonglong2>(c, "trd.ll.global", trd_ll_words(n));
+    j.limit_ns = trd_wait_limit(c);
     j.n = n;
     j.nb = nb;
     j.real = c.real_now;
@@ -2489,6 +2492,7 @@ void heev_values_batched(Context &c, const std::vector<EigJob> &jobs) {
             t.e = hw[q].e;
             t.tau = hw[q].tau;
             t.ll = wsget<ulonglong2>(c, slot_name("trd.ll", j.slot), trd_ll_words(j.n));
+            t.limit_ns = trd_wait_limit(c);
             t.n = j.n;
             t.real = c.real_now;
             t.b0 = t.nb = 0;
