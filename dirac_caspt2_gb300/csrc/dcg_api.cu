@@ -21,6 +21,7 @@
 
 #include "dcg_common.cuh"
 #include "dcg_kernels.cuh"
+#include "dcg_strings.h"
 
 struct dcg_ctx {
     dcg::Context c;
@@ -29,26 +30,6 @@ struct dcg_ctx {
 namespace dcg {
 
 // ------------------------------------------------------------------------- host helpers
-static std::vector<uint64_t> gosper_all(int na, int ne) {
-    std::vector<uint64_t> out;
-    if (ne < 0 || ne > na || na > 64) return out;
-    if (ne == 0) {
-        out.push_back(0);
-        return out;
-    }
-    uint64_t cur = (ne == 64) ? ~0ull : ((1ull << ne) - 1ull);
-    const uint64_t lim = (na == 64) ? 0 : (1ull << na);
-    while (true) {
-        out.push_back(cur);
-        uint64_t t = (cur | (cur - 1)) + 1;
-        uint64_t nxt = t | ((((t & (~t + 1)) / (cur & (~cur + 1))) >> 1) - 1);
-        if (nxt <= cur) break;
-        if (na < 64 && nxt >= lim) break;
-        cur = nxt;
-    }
-    return out;
-}
-
 // cas_configuration_totsym (search_cas_configuration.F90:112-149)
 static int det_totsym(const Context &c, uint64_t I) {
     if (c.nsym == 1) return 1;
@@ -68,48 +49,8 @@ static int det_totsym(const Context &c, uint64_t I) {
     return ret;
 }
 
-// Subsets of w spinors with lo to hi electrons, ascending.
-static std::vector<uint64_t> subsets_between(int w, int lo, int hi) {
-    std::vector<uint64_t> out;
-    for (int n = std::max(lo, 0); n <= std::min(hi, w); n++) {
-        const std::vector<uint64_t> g = gosper_all(w, n);
-        out.insert(out.end(), g.begin(), g.end());
-    }
-    std::sort(out.begin(), out.end());
-    return out;
-}
-
-// search_cas_configuration.F90:91-110 + ras_det_check.F90:1-59: the bit strings of ne electrons
-// with their RAS1 holes and RAS3 electrons in range, ascending, put together from the parts
-// RAS3, RAS2 and RAS1 (high to low bits) instead of filtered out of all strings: 10 electrons in
-// 8 + 10 + 8 spinors with two holes and two particles are 5.3 million strings, 30 ms on the
-// host, of which 74,273 stay.
-static std::vector<uint64_t> ras_all(const Context &c) {
-    if (c.ne < 0 || c.ne > c.na || c.na > 64) return {};
-    if (!c.ras1 && !c.ras3) return gosper_all(c.na, c.ne);
-    const int w1 = std::min(c.ras1, c.na);                            // RAS1: bits 0 .. w1 - 1
-    const int sh = c.ras3 ? std::min(c.ras1 + c.ras2, c.na) : c.na;   // RAS3: bits sh .. na - 1
-    const int w2 = sh - w1, w3 = c.na - sh;
-    const int lo1 = c.ras1 ? c.ras1 - c.ras1_max_hole : 0, hi1 = c.ras1 ? c.ras1 - c.min_hole_ras1 : 0;
-    std::vector<std::vector<uint64_t>> low(w1 + 1), mid(w3 + 1);
-    for (int n = std::max(lo1, 0); n <= std::min(hi1, w1); n++) low[n] = gosper_all(w1, n);
-    std::vector<char> have(w3 + 1, 0);
-    std::vector<uint64_t> out;
-    for (uint64_t h : c.ras3 ? subsets_between(w3, c.min_elec_ras3, c.ras3_max_elec) : std::vector<uint64_t>{0}) {
-        const int n3 = __builtin_popcountll(h), rest = c.ne - n3;
-        if (!have[n3]) {
-            mid[n3] = subsets_between(w2, rest - std::min(hi1, w1), rest - std::max(lo1, 0));
-            have[n3] = 1;
-        }
-        for (uint64_t m : mid[n3])
-            for (uint64_t l : low[rest - __builtin_popcountll(m)])
-                out.push_back((w3 > 0 ? h << sh : 0) | (w2 > 0 ? m << w1 : 0) | l);
-    }
-    return out;
-}
-
 static std::vector<uint64_t> enumerate_ci(const Context &c) {
-    std::vector<uint64_t> out = ras_all(c);
+    std::vector<uint64_t> out = ras_strings(c.na, c.ne, {c.ras1, c.ras2, c.ras3, c.ras1_max_hole, c.min_hole_ras1, c.ras3_max_elec, c.min_elec_ras3});
     if (c.nsym != 1)
         out.erase(std::remove_if(out.begin(), out.end(), [&](uint64_t I) { return det_totsym(c, I) != c.totsym; }),
                   out.end());
