@@ -65,6 +65,7 @@ struct JT {
     static __device__ __forceinline__ double re(T v) { return v.x; }
     static __device__ __forceinline__ T conj(T v) { return cconj(v); }
     static __device__ __forceinline__ T unit(double d) { return mk(d, 0.0); }
+    static __device__ __forceinline__ T times(double f, T v) { return mk(f * v.x, f * v.y); }
     // c x - s y, c x + s y
     static __device__ __forceinline__ T minus(double c, T x, T s, T y) {
         return mk(fma(c, x.x, fma(-s.x, y.x, s.y * y.y)), fma(c, x.y, fma(-s.x, y.y, -s.y * y.x)));
@@ -82,6 +83,7 @@ struct JT<true> {
     static __device__ __forceinline__ double re(T v) { return v; }
     static __device__ __forceinline__ T conj(T v) { return v; }
     static __device__ __forceinline__ T unit(double d) { return d; }
+    static __device__ __forceinline__ T times(double f, T v) { return f * v; }
     static __device__ __forceinline__ T minus(double c, T x, T s, T y) { return fma(c, x, -s * y); }
     static __device__ __forceinline__ T plus(double c, T x, T s, T y) { return fma(c, x, s * y); }
 };
@@ -137,6 +139,17 @@ __global__ void __launch_bounds__(kJacobiThreads) jacobi_heev_kernel(int n, cons
         fro += Z::abs2(Z::get(a));
     }
     fro = block_sum_d(fro, red);   // syncs the block
+    // a norm whose FP32 reciprocal could leave the range: the matrix is scaled by a power of two
+    // (exact) and the eigenvalues back
+    const int ex = (((__double2hiint(fro) >> 20) & 0x7FF) - 1023) / 2;
+    const bool rescale = fro > 0.0 && (ex < -60 || ex > 60) && ex < 512;
+    const double up = rescale ? __hiloint2double((1023 - ex) << 20, 0) : 1.0;
+    const double down = rescale ? __hiloint2double((1023 + ex) << 20, 0) : 1.0;
+    if (rescale) {
+        for (int e = tid; e < np * np; e += nt) A[e] = Z::times(up, A[e]);
+        fro = fro * up * up;
+        __syncthreads();
+    }
     const float scale = fro > 0.0 ? (float)(1.0 / sqrt(fro)) : 1.0f;   // elements of A in FP32 range
     const int npair = np / 2, nblk = npair * (npair + 1) / 2;
     int sweep = 0;
@@ -245,7 +258,7 @@ __global__ void __launch_bounds__(kJacobiThreads) jacobi_heev_kernel(int n, cons
         rank_sh[i] = r;
     }
     __syncthreads();
-    for (int i = tid; i < n; i += nt) w[rank_sh[i]] = Z::re(A[i + np * i]);
+    for (int i = tid; i < n; i += nt) w[rank_sh[i]] = down * Z::re(A[i + np * i]);
     for (int e = tid; e < n * n; e += nt) {
         const int i = e % n, j = e / n;
         Y[i + (int64_t)ldy * rank_sh[j]] = Z::put(V[i + np * j]);
