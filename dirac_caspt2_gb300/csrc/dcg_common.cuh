@@ -226,6 +226,9 @@ std::vector<T> download(Context &c, const T *p, size_t n) {
 // and keeps the fastest; later calls of the key, in any context, reuse it.  Candidate 0 is the
 // built-in heuristic, used while tuning is off (dcg_autotune_mode) and for keys first met
 // without trial_ok.  The trial runs must leave the same result as the final run.
+// A choice is an index into the caller's list of candidates.  Where the list itself depends on
+// the shape, the SM count or the build, `list` identifies its contents: a stored choice of
+// another list is not used (0: the list is fixed).
 enum TuneKind { TUNE_ZGEMM = 1, TUNE_SPLIT_KERNEL = 2 };
 struct TuneKey {
     int kind, ops, m, n, k, flags;
@@ -238,11 +241,11 @@ struct TuneKey {
         return flags < o.flags;
     }
 };
-int autotune_run(Context &c, const TuneKey &key, int ncand, bool trial_ok, void (*fn)(void *, int), void *arg);
+int autotune_run(Context &c, const TuneKey &key, int ncand, unsigned list, bool trial_ok, void (*fn)(void *, int), void *arg);
 template <typename F>
-int autotune(Context &c, const TuneKey &key, int ncand, bool trial_ok, F &&run) {
+int autotune(Context &c, const TuneKey &key, int ncand, unsigned list, bool trial_ok, F &&run) {
     using Fn = typename std::remove_reference<F>::type;
-    return autotune_run(c, key, ncand, trial_ok, [](void *p, int q) { (*static_cast<Fn *>(p))(q); },
+    return autotune_run(c, key, ncand, list, trial_ok, [](void *p, int q) { (*static_cast<Fn *>(p))(q); },
                         const_cast<void *>(static_cast<const void *>(&run)));
 }
 

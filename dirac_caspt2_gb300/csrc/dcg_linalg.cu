@@ -608,6 +608,14 @@ static std::vector<ZgPlan> zg_candidates(Context &c, int m, int n, int k, int up
     return out;
 }
 
+// What a list of plans holds, for the autotuner's stored choices (FNV-1a; never 0).
+static unsigned zg_list_id(const std::vector<ZgPlan> &cand) {
+    unsigned h = 2166136261u;
+    for (const ZgPlan &p : cand)
+        for (int v : {kZgBm[p.tile], kZgBn[p.tile], p.nsplit}) h = (h ^ (unsigned)v) * 16777619u;
+    return h ? h : 1u;
+}
+
 template <int OPA, int OPB>
 static void zgemm_plan_run(Context &c, const ZgPlan &p, int m, int n, int k, cplx alpha, const cplx *A, int64_t lda,
                            int64_t sa, const cplx *B, int64_t ldb, int64_t sb, cplx beta, cplx *C, int64_t ldc,
@@ -626,7 +634,7 @@ static void zgemm_tuned(Context &c, int m, int n, int k, cplx alpha, const cplx 
     // tuning can return (and a served stream meets many shapes once)
     const double work = (c.real_now ? 2.0 : 8.0) * m * n * (double)k * batch;
     const bool trial_ok = beta.x == 0.0 && beta.y == 0.0 && work >= kTuneMinFp64Flops;
-    const int pick = autotune(c, key, (int)cand.size(), trial_ok, [&](int q) {
+    const int pick = autotune(c, key, (int)cand.size(), zg_list_id(cand), trial_ok, [&](int q) {
         zgemm_plan_run<OPA, OPB>(c, cand[q], m, n, k, alpha, A, lda, sa, B, ldb, sb, beta, C, ldc, sc, batch, upper);
     });
     zgemm_plan_run<OPA, OPB>(c, cand[pick], m, n, k, alpha, A, lda, sa, B, ldb, sb, beta, C, ldc, sc, batch, upper);

@@ -1014,7 +1014,7 @@ void zgemm_split(Context &c, int M, int N, int K, int batch, const cplx *A, int6
     int pick;
     const char *force = getenv("DCG_SPLIT_KERNEL");   // diagnostic: a fixed candidate 0-3
     if (force && force[0] >= '0' && force[0] <= '3' && force[1] == 0) pick = force[0] - '0';
-    else pick = autotune(c, key, 4, !accumulate && tensor_work >= 1.0e11, launch);
+    else pick = autotune(c, key, 4, 0, !accumulate && tensor_work >= 1.0e11, launch);
     {
         // tensor work: 15 slice products, each a real GEMM of M x 2N x 2K
         FamScope fs(c, DCG_FAM_SPLIT_MMA, tensor_work);

@@ -12,6 +12,7 @@ namespace {
 
 struct TuneEntry {
     int choice, ncand;
+    unsigned list;
     float best_ms, heuristic_ms;
 };
 
@@ -29,7 +30,8 @@ int mode_locked() {
 }
 
 // With DCG_TUNE_FILE set, the table persists in that text file, one entry per line
-// ("kind ops m n k flags choice ncand best_ms heuristic_ms"): entries are read at the first
+// ("kind ops m n k flags choice ncand best_ms heuristic_ms list"; without the last, of a list
+// that is fixed): entries are read at the first
 // lookup and every new entry is appended, so another process (a profiler's run of the same
 // workload, a service restart) reuses the choices without trials.
 const char *tune_file() { return getenv("DCG_TUNE_FILE"); }
@@ -43,9 +45,13 @@ void load_locked() {
     if (!fp) return;
     TuneKey k;
     TuneEntry e;
-    while (fscanf(fp, "%d %d %d %d %d %d %d %d %f %f", &k.kind, &k.ops, &k.m, &k.n, &k.k, &k.flags, &e.choice,
-                  &e.ncand, &e.best_ms, &e.heuristic_ms) == 10)
-        if (e.choice >= 0 && e.choice < e.ncand) g_table[k] = e;   // the latest line of a key counts
+    char line[256];
+    while (fgets(line, sizeof line, fp)) {
+        e.list = 0;
+        const int got = sscanf(line, "%d %d %d %d %d %d %d %d %f %f %u", &k.kind, &k.ops, &k.m, &k.n, &k.k, &k.flags,
+                               &e.choice, &e.ncand, &e.best_ms, &e.heuristic_ms, &e.list);
+        if (got >= 10 && e.choice >= 0 && e.choice < e.ncand) g_table[k] = e;   // the latest line of a key counts
+    }
     fclose(fp);
 }
 
@@ -54,20 +60,20 @@ void save_locked(const TuneKey &k, const TuneEntry &e) {
     if (!f || !f[0]) return;
     FILE *fp = fopen(f, "a");
     if (!fp) return;
-    fprintf(fp, "%d %d %d %d %d %d %d %d %.6f %.6f\n", k.kind, k.ops, k.m, k.n, k.k, k.flags, e.choice, e.ncand,
-            e.best_ms, e.heuristic_ms);
+    fprintf(fp, "%d %d %d %d %d %d %d %d %.6f %.6f %u\n", k.kind, k.ops, k.m, k.n, k.k, k.flags, e.choice, e.ncand,
+            e.best_ms, e.heuristic_ms, e.list);
     fclose(fp);
 }
 
 }  // namespace
 
-int autotune_run(Context &c, const TuneKey &key, int ncand, bool trial_ok, void (*fn)(void *, int), void *arg) {
+int autotune_run(Context &c, const TuneKey &key, int ncand, unsigned list, bool trial_ok, void (*fn)(void *, int), void *arg) {
     {
         std::lock_guard<std::mutex> lk(g_mu);
         load_locked();
         auto it = g_table.find(key);
-        // an entry of another candidate list (a file written by another build) is not used
-        if (it != g_table.end() && it->second.ncand == ncand) return it->second.choice;
+        // an entry of another candidate list (a file of another build or GPU) is not used
+        if (it != g_table.end() && it->second.ncand == ncand && it->second.list == list) return it->second.choice;
         if (mode_locked() == 0 || ncand < 2 || !trial_ok || !c.tune_trials) return 0;
     }
     // untimed pass: every candidate once (workspace growth, first-launch costs)
@@ -92,9 +98,9 @@ int autotune_run(Context &c, const TuneKey &key, int ncand, bool trial_ok, void 
     for (int q = 1; q < ncand; q++)
         if (best[q] < best[pick]) pick = q;
     std::lock_guard<std::mutex> lk(g_mu);
-    const TuneEntry mine{pick, ncand, best[pick], best[0]};
+    const TuneEntry mine{pick, ncand, list, best[pick], best[0]};
     auto ins = g_table.emplace(key, mine);
-    if (!ins.second && ins.first->second.ncand == ncand)
+    if (!ins.second && ins.first->second.ncand == ncand && ins.first->second.list == list)
         return ins.first->second.choice;   // a concurrent tuner of the same key won
     ins.first->second = mine;
     save_locked(key, mine);

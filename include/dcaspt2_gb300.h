@@ -381,7 +381,8 @@ int dcg_casci_energy_check(dcg_ctx *ctx, double out[8]);
  * is kept in a process-wide table that every context then uses.  Different choices change
  * only the summation order of the products.
  * With the environment variable DCG_TUNE_FILE naming a text file, the table is read from it
- * at first use and each new entry appended to it, so later processes reuse the choices.
+ * at first use and each new entry appended to it, so later processes reuse the choices
+ * (those whose list of candidates is the same; others are tuned again).
  * mode: 1 tune (default; environment DCG_AUTOTUNE=0 starts with 0), 0 use the built-in
  * heuristics for keys not yet tuned, 2 clear the table (mode unchanged), other values only
  * query.  Returns the mode before the call. */
