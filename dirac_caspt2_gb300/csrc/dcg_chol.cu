@@ -13,14 +13,6 @@ namespace {
 constexpr int CH_NB = 48;   // panel width: the 48 x 49 complex tile fits the 48 KB of static shared memory
 constexpr int CH_SLAB = 256;   // columns of one trailing update: below a few slabs the square costs no more than its launches
 
-// 1/sqrt(x) from the hardware's ~2^-22 approximation by one third-order Newton step.
-__device__ __forceinline__ double ch_rsqrt(double x) {
-    double y;
-    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-    const double e = fma(-x * y, y, 1.0);
-    return fma(y, fma(0.375, e, 0.5) * e, y);
-}
-
 // a -= x conj(y) and a -= x y, complex or real
 template <bool REAL>
 __device__ __forceinline__ void ch_sub_conj(cplx &a, cplx x, cplx y) {
@@ -58,7 +50,7 @@ __global__ void __launch_bounds__(512) chol_panel_kernel(int kb, int k0, cplx *A
                 if (lane == 0) bad = k0 + j + 1;
             } else {
                 const bool safe = piv > 1e-290 && piv < 1e290;
-                const double ri = safe ? ch_rsqrt(piv) : 1.0 / sqrt(piv);
+                const double ri = safe ? fast_rsqrt(piv) : 1.0 / sqrt(piv);
                 if (lane == 0) {
                     s_r[0] = ri;
                     s_r[1] = piv * ri;

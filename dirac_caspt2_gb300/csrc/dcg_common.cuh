@@ -14,6 +14,7 @@
 #include <vector>
 
 #include "../../include/dcaspt2_gb300.h"
+#include "dcg_recip.cuh"
 
 namespace dcg {
 

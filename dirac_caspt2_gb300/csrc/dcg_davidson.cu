@@ -88,14 +88,6 @@ struct JT<true> {
     static __device__ __forceinline__ T plus(double c, T x, T s, T y) { return fma(c, x, s * y); }
 };
 
-// 1/sqrt(x) from the hardware's ~2^-22 approximation by one third-order Newton step.
-__device__ __forceinline__ double jac_rsqrt(double x) {
-    double y;
-    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-    const double e = fma(-x * y, y, 1.0);
-    return fma(y, fma(0.375, e, 0.5) * e, y);
-}
-
 // All eigenpairs of a small Hermitian matrix G (n <= 64, column-major, ldg; the matrix used is
 // (G + G^H)/2) by cyclic Jacobi with the parallel round-robin ordering (Golub & Van Loan,
 // Matrix Computations, 4th ed., 8.5.5): each round rotates n/2 disjoint pairs at once,
@@ -183,13 +175,13 @@ __global__ void __launch_bounds__(kJacobiThreads) jacobi_heev_kernel(int n, cons
                     const float ab = REAL ? fabsf(bx) : sqrtf(fmaf(bx, bx, by * by));
                     const float h = 0.5f * fabsf(d);
                     const float t = copysignf(ab / (h + sqrtf(fmaf(h, h, ab * ab))), d);
-                    const double t64 = (double)t, c = jac_rsqrt(fma(t64, t64, 1.0)), sn = t64 * c;
+                    const double t64 = (double)t, c = fast_rsqrt(fma(t64, t64, 1.0)), sn = t64 * c;
                     cs_c[k] = c;
                     if constexpr (REAL) {
                         cs_s[k] = b >= 0.0 ? sn : -sn;
                     } else {
                         const double px = (double)(bx / ab), py = (double)(by / ab);
-                        const double f = sn * jac_rsqrt(fma(px, px, py * py));
+                        const double f = sn * fast_rsqrt(fma(px, px, py * py));
                         cs_s[k] = mk(f * px, f * py);
                     }
                 }

@@ -30,6 +30,7 @@
 #include <map>
 
 #include "dcg_common.cuh"
+#include "dcg_deflate.cuh"
 
 namespace dcg {
 
@@ -477,29 +478,6 @@ struct LlWait {
         return true;
     }
 };
-
-// 1/x and 1/sqrt(x) from the hardware's ~2^-22 approximations by one third-order Newton step.
-__device__ __forceinline__ double fast_rcp(double x) {
-    double r;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
-    const double e = fma(-x, r, 1.0);
-    return fma(r, fma(e, e, e), r);
-}
-// The same for any x: a division where x, 1/x or the step's terms could leave the normal numbers.
-__device__ __forceinline__ double safe_rcp(double x) {
-    const int ex = (__double2hiint(x) >> 20) & 0x7FF;
-    return ex < 64 || ex > 1982 ? 1.0 / x : fast_rcp(x);
-}
-__device__ __forceinline__ double fast_rsqrt(double x) {
-    double y;
-    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-    const double e = fma(-x * y, y, 1.0);
-    return fma(y, fma(0.375, e, 0.5) * e, y);
-}
-
-}  // namespace dcg
-#include "dcg_deflate.cuh"
-namespace dcg {
 
 // Reflector of the column alpha, x with ss = |x|^2 (LAPACK's documented xLARFG, beta real): tau,
 // beta, the scale sc = 1 / (alpha - beta) of x, and mib = tau sc = -1 / beta (0 for tau = 0).

@@ -145,18 +145,6 @@ void launch_gather_v(Context &c, const cplx *V, const int64_t *outer_off, int no
     DCG_LAUNCHED(c);
 }
 
-// 1/x to rounding: the hardware's ~2^-22 approximation and one third-order Newton step, three
-// FP64 instructions where a division takes five times as long; a division outside the range
-// in which neither x, 1/x nor the step's terms leave the normal numbers.
-__device__ __forceinline__ double e2_recip(double x) {
-    const int ex = (__double2hiint(x) >> 20) & 0x7FF;
-    if (ex < 64 || ex > 1982) return 1.0 / x;
-    double r;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
-    const double e = fma(-x, r, 1.0);
-    return fma(r, fma(e, e, e), r);
-}
-
 // e2o[o] = -sum_j |VC(j,o)|^2/(alpha_o + wb_j), sc2o[o] = sum_j |VC(j,o)|^2/(alpha_o + wb_j)^2
 // (solve_A_subspace.F90:236-261, same loop in B..G).  W lanes share an outer index.  The FP64 pipe
 // is the limit: nine instructions a term (two divisions made it about twenty).  A thread an
@@ -173,7 +161,7 @@ __global__ void e2_kernel(const cplx *__restrict__ VC, int dimm, int nouter, con
     const double al = alpha[o];
     double e = 0.0, s = 0.0;
     for (int j = l; j < dimm; j += W) {
-        const double r = e2_recip(al + wb[j]);
+        const double r = safe_rcp(al + wb[j]);
         const double t = cabs2(VC[j + (int64_t)dimm * o]) * r;
         e -= t;
         s = fma(t, r, s);
@@ -511,26 +499,9 @@ void launch_F_pack(Context &c, const cplx *Fc, int ns, int na, cplx *Fp) {
 // a > b half of the class is read exactly once (streaming loads); the a < b half is never read.
 // The FP64 pipe, not HBM, bounds this kernel on GB300 (a warp instruction in 77 clocks and SM
 // quarter): per element two subtractions and |V|^2, the denominator, a reciprocal and the two
-// accumulations, ten instructions.  The reciprocal is the FP32 one widened and refined by one
-// Newton-Raphson step for 1/e, r = r0 + r0 (1 - e r0), whose relative error is the square of the
-// FP32 error (<= 2^-46) plus rounding; a denominator outside the FP32 normal range takes 1.0 / e.
-// The narrowing cuts the bits and the widening shifts them: as conversions both would run on the
-// FP64 pipe (20 inactive, 300 secondary spinors: 0.285 ms with them and with the denominator in
+// accumulations, ten instructions.  The reciprocal is the refined FP32 one (h_recip; 20 inactive,
+// 300 secondary spinors: 0.285 ms with conversion instructions in it and with the denominator in
 // two additions, 0.249 now).
-__device__ __forceinline__ double h_recip(double e) {
-    const int hi = __double2hiint(e);
-    const int ex = ((hi >> 20) & 0x7FF) - 896;   // exponent field in FP32
-    if (ex < 3 || ex > 250) return 1.0 / e;
-    // e rounded to 23 fraction bits: half a unit of them added to the bits (a carry goes on into
-    // the exponent)
-    const uint32_t lo = (uint32_t)__double2loint(e), lo2 = lo + 0x10000000u;
-    const uint32_t h2 = (uint32_t)hi + (lo2 < lo ? 1u : 0u);
-    const uint32_t m = ((h2 & 0x7FFFFFFFu) - (896u << 20)) << 3 | lo2 >> 29;
-    const uint32_t r = __float_as_uint(__frcp_rn(__uint_as_float((h2 & 0x80000000u) | m)));
-    const double r0 = __hiloint2double((int)((r & 0x80000000u) | (((r & 0x7FFFFFFFu) >> 3) + (896u << 20))), (int)(r << 29));
-    return fma(r0, fma(-e, r0, 1.0), r0);
-}
-
 constexpr int kHDen = 512;
 
 __global__ void __launch_bounds__(256) h_stream_kernel(const cplx *__restrict__ Hc, int ni, int ns,
