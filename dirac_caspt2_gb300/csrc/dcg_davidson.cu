@@ -272,6 +272,7 @@ __global__ void unit_cols_kernel(int n, int m, const int *__restrict__ idx, cplx
 // that size, real: whole call 310 ms before, 98 ms with the chunks, real arithmetic, the Rayleigh
 // elements of new vectors alone and the determinant table of the matrix build.
 constexpr int kDavChunk = 1024, kDavThreads = 256;
+constexpr int kDavShortSteps = 250;   // steps with the short subspace before V may grow to the long one
 constexpr int kAxpyRows = 128;   // rows (and threads) of a block that subtracts: its loop over the vectors is the long one
 
 // Sum of n values by one warp in a fixed order (every lane gets it).
@@ -310,7 +311,8 @@ struct DavState {
     int jac;      // a Jacobi solve ran out of sweeps (sticky)
     int restarted;
     int live[8], ok[8];   // direction q: tried, accepted
-    int pad[3];
+    int cap;      // vectors that V may hold now (at most mmax)
+    int pad[2];
     double worst;  // largest residual norm of the wanted roots
 };
 // Column of direction q: after the accepted ones before it.
@@ -397,7 +399,7 @@ __global__ void __launch_bounds__(kDavThreads) residual_kernel(int n, const cplx
 
 // The residual norms of the block's roots (to h2), the worst of the wanted ones; the step's
 // direction flags reset, and the restart decided: the next block would not fit.
-__global__ void step_begin_kernel(int nwant, int nb, int mmax, int nchunk, const double *__restrict__ part, double *h2,
+__global__ void step_begin_kernel(int nwant, int nb, int nchunk, const double *__restrict__ part, double *h2,
                                   DavState *st) {
     __shared__ double v[8];
     for (int q = threadIdx.x >> 5; q < nb; q += blockDim.x >> 5) {   // a warp per root
@@ -410,7 +412,7 @@ __global__ void step_begin_kernel(int nwant, int nb, int mmax, int nchunk, const
     for (int q = 0; q < nwant; q++) w = fmax(w, sqrt(v[q]));
     st->worst = w;
     for (int q = 0; q < 8; q++) st->live[q] = st->ok[q] = 0;
-    st->restarted = st->m + nb > mmax;
+    st->restarted = st->m + nb > st->cap;
 }
 
 // Restart on the block's Ritz vectors: V, W <- X, HX.
@@ -431,7 +433,7 @@ __global__ void restart_set_kernel(int nb, DavState *st) {
 // Direction q: live when its residual is above tol, no direction before it was rejected and V has
 // room; then T[:, q] goes to its column of V and its squared norm, by chunks, to part.
 template <bool REAL>
-__global__ void __launch_bounds__(kDavThreads) cand_begin_kernel(int n, int q, int mmax, double tol,
+__global__ void __launch_bounds__(kDavThreads) cand_begin_kernel(int n, int q, double tol,
                                                                  const double *__restrict__ h2,
                                                                  const cplx *__restrict__ T, cplx *V, int64_t ld,
                                                                  double *part, DavState *st) {
@@ -440,7 +442,7 @@ __global__ void __launch_bounds__(kDavThreads) cand_begin_kernel(int n, int q, i
     for (int p = 0; p < q; p++)
         if (st->live[p] && !st->ok[p]) live = false;
     const int col = dav_col(st, q);
-    live = live && col < mmax;
+    live = live && col < st->cap;
     if (blockIdx.x == 0 && threadIdx.x == 0) st->live[q] = live;
     if (!live) return;
     cplx *dst = V + ld * col;
@@ -628,12 +630,18 @@ void davidson_lowest_csr(Context &c, const CsrMatrix &H, int nwant, double *w, c
     const int n = H.n;
     const int nb = std::min(n, nwant + 2);   // block: the wanted roots and a margin for near-degeneracy
     // A long subspace saves iterations (each one product with H), a short one keeps the one-block
-    // Jacobi short (its time grows with the cube): at 924 determinants 12 vectors took 20
-    // steps and 5.9 ms where 24 took 18 and 8.5; at 74,273 determinants (0.9 ms a product) the
-    // products decide.
+    // Jacobi short (its time grows with the cube): at 924 determinants and one root 12 vectors
+    // took 16 steps and 4.9 ms where 24 took 14 and 6.8; at 74,273 determinants (0.9 ms a product)
+    // the products decide.  Restarts every few steps can stall on nearly degenerate levels: of 240
+    // runs (60 spectra of 252 to 8008 determinants, one to six roots) three with two roots at 8008
+    // did not converge in 400 steps with the short one and took 124 to 259 with the long one.  So
+    // V may grow to the long one after kDavShortSteps, with maxit steps from there.  Almost every
+    // run is done by then; growing after 60 steps helped two roots (113 -> 79 ms) and cost six (179 ->
+    // 229 ms, their 64 vectors).
     const double hx_s = (double)H.nnz * nb * (H.rvals ? 1.0 : 4.0) / 4.0e11;
-    const int mmax = std::min(n, std::min(kJacobiMaxN, hx_s > 0.6e-3 ? std::max(24, 8 * nb) : std::max(12, 4 * nb)));
-    if (nwant < 1 || nb > mmax || n < 2) throw Error{DCG_E_ARG, "davidson: block does not fit the subspace"};
+    const int mmax = std::min(n, std::min(kJacobiMaxN, std::max(24, 8 * nb)));
+    const int mshort = hx_s > 0.6e-3 ? mmax : std::min(mmax, std::max(12, 4 * nb));
+    if (nwant < 1 || nb > mshort || n < 2) throw Error{DCG_E_ARG, "davidson: block does not fit the subspace"};
     const int64_t ld = n;
     cplx *V = wsget<cplx>(c, "dav.V", (size_t)n * mmax);
     cplx *W = wsget<cplx>(c, "dav.W", (size_t)n * mmax);
@@ -673,6 +681,7 @@ void davidson_lowest_csr(Context &c, const CsrMatrix &H, int nwant, double *w, c
     DCG_LAUNCHED(c);
     DavState s0{};
     s0.m = nb;
+    s0.cap = mshort;
     DCG_CUDA(cudaMemcpyAsync(st, &s0, sizeof(DavState), cudaMemcpyHostToDevice, c.stream));
 
     const int np = mmax + (mmax & 1);
@@ -694,11 +703,11 @@ void davidson_lowest_csr(Context &c, const CsrMatrix &H, int nwant, double *w, c
         k_jac<<<1, kJacobiThreads, jsmem, c.stream>>>(mmax, &st->m, G, mmax, th, Y, mmax, &st->jac);
         k_ritz<<<dim3(grid1d(n, 128), nb, 2), 128, 0, c.stream>>>(n, V, W, ld, Y, mmax, X, HX, st);
         k_res<<<dim3(nchunk, nb), kDavThreads, 0, c.stream>>>(n, HX, X, ld, th, H.diag, T, part);
-        step_begin_kernel<<<1, 256, 0, c.stream>>>(nwant, nb, mmax, nchunk, part, h2, st);
+        step_begin_kernel<<<1, 256, 0, c.stream>>>(nwant, nb, nchunk, part, h2, st);
         restart_copy_kernel<<<grid1d((int64_t)n * nb, 256), 256, 0, c.stream>>>(n, nb, X, HX, V, W, ld, st);
         restart_set_kernel<<<1, 32, 0, c.stream>>>(nb, st);
         for (int q = 0; q < nb; q++) {
-            k_cand<<<nchunk, kDavThreads, 0, c.stream>>>(n, q, mmax, tol, h2, T, V, ld, pn0, st);
+            k_cand<<<nchunk, kDavThreads, 0, c.stream>>>(n, q, tol, h2, T, V, ld, pn0, st);
             for (int pass = 0; pass < 2; pass++) {
                 k_dot<<<dim3(mmax, nchunk), kDavThreads, 0, c.stream>>>(n, q, V, ld, cf, mmax, st);
                 k_axpy<<<nrow, kAxpyRows, 0, c.stream>>>(n, q, nchunk, V, ld, cf, mmax, pn1, st);
@@ -734,7 +743,10 @@ void davidson_lowest_csr(Context &c, const CsrMatrix &H, int nwant, double *w, c
 
     bool converged = false;
     c.casci_iters = 0;
+    if (mshort < mmax) maxit += kDavShortSteps;
     for (int it = 0; it < maxit; it++) {
+        if (it == kDavShortSteps && mshort < mmax)
+            DCG_CUDA(cudaMemcpyAsync(&st->cap, &mmax, sizeof(int), cudaMemcpyHostToDevice, c.stream));
         if (exec) {
             DCG_CUDA(cudaGraphLaunch(exec, c.stream));
             c.launches += step_kernels;
