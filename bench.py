@@ -187,12 +187,12 @@ def run_reference(args, cfg_name):
 
 
 def _traffic(family, cfg_name):
-    """DRAM bytes per launch of the family, from the ncu capture summarised under profiles/
-    (dram__bytes_read.sum + dram__bytes_write.sum, mean over one solve's launches)."""
+    """DRAM bytes of the family's largest launch, from the ncu capture summarised under profiles/
+    (dram__bytes_read.sum + dram__bytes_write.sum of one launch)."""
     import re
     if family != "split_mma":
         return None
-    p = os.path.join(os.path.dirname(os.path.abspath(__file__)), "profiles", f"launch_list_{cfg_name}_split.md")
+    p = os.path.join(os.path.dirname(os.path.abspath(__file__)), "profiles", f"sp_gemm_kernel_quarter_{cfg_name}.md")
     if not os.path.exists(p):
         return None
     m = re.search(r"^traffic_bytes_per_launch = (\d+)", open(p).read(), re.M)
@@ -395,8 +395,9 @@ def run_ours(args, cfg_name):
         achieved = fam_work / (fam_ms * 1e-3) / 1e12
         roof = {"bound": "fp64", "achieved": achieved, "peak": None, "unit": "TFLOP/s", "frac": None,
                 "work": "FP64 FLOPs; GB300 has no FP64 tensor rate to compare against"}
-    roof.update({"traffic": _traffic(family, cfg_name), "kernel_family": family, "launches_timed": fam_launch,
-                 "mean_launch_ms": fam_ms / max(1, fam_launch),
+    roof.update({"traffic": _traffic(family, cfg_name),
+                 "traffic_note": "DRAM bytes of one launch, the largest transformation quarter (ncu)",
+                 "kernel_family": family, "launches_timed": fam_launch, "mean_launch_ms": fam_ms / max(1, fam_launch),
                  "peak_source": f"{src} MEASURED_PEAKS.json ({'sustained' if roof['unit'] == 'TFLOP/s' else 'burst'})"})
     e_casci, e2_last, e_tot = res_v[-1]
     energies = [r[2] for r in res_v + res_e]
