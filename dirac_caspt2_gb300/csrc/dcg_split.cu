@@ -591,7 +591,7 @@ __global__ void __launch_bounds__(SP_THREADS, 1) sp_gemm_kernel(SplitArgs a) {
             for (int cc = 0; cc < SP_TN / (4 * SP_CH); cc++) {
                 const int j0 = jt + cc * 2 * SP_CH;
                 if (j0 >= a.N) break;
-                if (a.accumulate) sp_read_c(a, r, j0 + 2 * SP_CH, old[(cc + 1) & 1]);
+                if (a.accumulate && cc + 1 < SP_TN / (4 * SP_CH)) sp_read_c(a, r, j0 + 2 * SP_CH, old[(cc + 1) & 1]);
                 uint32_t g[4][2 * SP_CH];
                 sp_read_tmem<4>(tmem + ((uint32_t)(quad * 32) << 16) + (cc * 2 + half) * 2 * SP_CH, SP_TN, g);
                 sp_write_c<4>(a, r, j0, g, old[cc & 1]);
