@@ -406,7 +406,7 @@ def run_ours(args, cfg_name):
             "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
             "dtype": ("c128 (f64)" if prec == api.DCG_PREC_FP64 else
                       "c128: transformation on BF16 tensor cores as 5-slice split products with FP64 "
-                      "recombination; eigensolvers, densities and E2 in f64"),
+                      "recombination, densities, metric and B' as 7-slice ones; eigensolvers and E2 in f64"),
             "data": "synthetic (seeded Kramers-paired complex spinor system; replicas only)",
             "config": {"workload": cfg_name, "ninact": cfg.ninact, "nact": cfg.nact, "nsec": cfg.nsec,
                        "nelec": cfg.nelec, "root": 1, "records": int(len(S.rec_val)),

@@ -86,8 +86,7 @@ __global__ void __launch_bounds__(512) chol_panel_kernel(int kb, int k0, cplx *A
 //   CH_BACKWARD L11^H X = B
 // Column by column: the element's owner divides, every later element subtracts its multiple.
 // One thread a vector took 300 us for any number of vectors (1,128 complex multiply-adds in a
-// row at 77 clocks an FP64 instruction); this form takes 40 us.  With the panel, 14/10/230 split
-// 35.2 -> 29.3 ms, 12/8/120 real 12.2 -> 10.3 ms.
+// row at 77 clocks an FP64 instruction); this form takes 40 us.
 constexpr int CH_RHS = 8;
 enum ChSolve { CH_ROWS, CH_FORWARD, CH_BACKWARD };
 template <bool REAL, int MODE>

@@ -95,8 +95,8 @@ struct Context {
     std::string err;
     int64_t launches = 0;
     int num_sms = 0;
-    // limit of the device-side waits that can give up (grid barriers of the tridiagonalisation,
-    // pipeline waits of the tensor-core GEMM), ns; 0 = each kernel's default (dcg_set_wait_limit)
+    // limit of the device-side waits that can give up (flagged words and grid barriers of the
+    // tridiagonalisation, pipeline waits of the tensor-core GEMM), ns; 0 = each kernel's default (dcg_set_wait_limit)
     uint64_t wait_limit_ns = 0;
     bool tune_trials = true;     // may run autotuner trials (off for serving slots)
     // hand batched tridiagonal reductions to the device's batcher, which merges those of all
@@ -144,7 +144,8 @@ struct Context {
     bool realonly = false;
     // the resident system is real throughout (realonly, and no imaginary part in h), and a solve of
     // it is running: every matrix on the path then has zero imaginary parts, and the FP64
-    // kernels skip them (the same bits at a quarter of the FMAs)
+    // kernels skip them: a quarter of the FMAs (other tiles and K splits may pay then, so sums
+    // may run in another order than in complex arithmetic)
     bool sys_real = false, real_now = false;
     double eshift = 0.0, ecore = 0.0;
     std::vector<int> multb;   // 2n x 2n column-major

@@ -268,9 +268,7 @@ __global__ void unit_cols_kernel(int n, int m, const int *__restrict__ idx, cplx
 
 // ---- vector work in chunks of kDavChunk rows, one block each: partial sums go to part[...] and
 // whoever needs the sum adds the chunks in order, so a sum depends on n alone.  One block for a
-// whole vector left 151 SMs idle on 74,273 determinants (0.2 to 1 ms a kernel).  The RAS space of
-// that size, real: whole call 310 ms before, 98 ms with the chunks, real arithmetic, the Rayleigh
-// elements of new vectors alone and the determinant table of the matrix build.
+// whole vector left 151 SMs idle on 74,273 determinants (0.2 to 1 ms a kernel).
 constexpr int kDavChunk = 1024, kDavThreads = 256;
 constexpr int kDavShortSteps = 250;   // steps with the short subspace before V may grow to the long one
 constexpr int kAxpyRows = 128;   // rows (and threads) of a block that subtracts: its loop over the vectors is the long one

@@ -1675,7 +1675,7 @@ static DcBufs dc_bufs(Context &c, int n, int slot) {
     b.QA = wsget<double>(c, nm("dc.QA"), nn);
     b.QB = wsget<double>(c, nm("dc.QB"), nn);
     b.U = wsget<double>(c, nm("dc.U"), nn);
-    // the vectors of one slot in two allocations: 10 of doubles, 16 of integers
+    // the vectors of one slot in two allocations: 11 of doubles, 16 of integers
     const size_t m = (size_t)n + 8;
     double *f = wsget<double>(c, nm("dc.f"), 11 * m);
     b.lamA = f, b.lamB = f + m, b.dK = f + 2 * m, b.zK = f + 3 * m, b.dv = f + 4 * m, b.rc = f + 5 * m;
@@ -1701,10 +1701,9 @@ static void dc_level_vectors(Context &c, int n, int half, int olo, int ohi, cons
 }
 
 // Bound by latency (launches, serial FP64 chains) below a few hundred columns and by the FP64
-// pipe above.  Measured with the base kernel, four launches a level instead of six, the
-// cheaper secular steps and the merge products by halves (whole solves, before -> after):
-// 4/4/12 3.88 -> 3.05 ms, 8/6/40 8.75 -> 7.07 ms, 14/10/230 50.8 -> 41.9 ms, 20/12/300
-// 114.8 -> 104.9 ms.
+// pipe above.  Order 791, values: 2.4 ms with the base kernel, four launches a level, the short
+// secular steps and the merge products by halves; 6 ms with six launches a level from 1 x 1
+// leaves and divisions.
 // Eigenvalues (ascending, into w) of the symmetric tridiagonal (d, e), and its eigenvectors up to
 // the last merge, whose own vectors dc_vectors forms for the columns that are asked for (most
 // of the merge products of a decomposition are the last one's).  d and e are device arrays;
@@ -2037,7 +2036,7 @@ static void tridiag_persistent(Context &c, int n, cplx *A, int64_t lda, HeevWork
 
 // Shared-memory tridiagonalisation of several matrices in one cooperative launch (one job = one
 // block group).  Block counts come from a cost model: a job's FP64 work (12 FMAs per trailing
-// element and column, whole columns per block, on a unit of two FMAs per clock and SM) spreads
+// element and column, whole columns per block, on a unit of 1.66 FMAs per clock and SM) spreads
 // over its blocks, while every block of a column reads all of its exchanged words; the jobs
 // share the SMs, and blocks go to the job that is currently the slowest.  False (nothing
 // launched) when the jobs do not fit.
@@ -2161,8 +2160,8 @@ static std::vector<int> trd_launch(Context &c, const std::vector<TrdJob> &jobs, 
 // instead of launching it.  The first waiting thread that finds the batcher idle becomes the
 // leader: it takes, in arrival order, the submissions whose jobs fit one launch together, makes
 // a batcher stream wait for each submission's ready event, launches them as one cooperative
-// kernel (each job its own block group and barrier) and hands every submission its result.
-// Requests that run concurrently then overlap their barrier-bound column loops inside one kernel
+// kernel (each job its own block group and words) and hands every submission its result.
+// Requests that run concurrently then overlap their exchange-bound column loops inside one kernel
 // instead of queueing on the cooperative-launch lock.  The block-group sizes change with the
 // company, the arithmetic of a job does not: its partial sums do not depend on the number of
 // blocks reducing it, so a matrix gets the same bits alone and merged.
@@ -2292,7 +2291,7 @@ static bool tridiag_smem_merged(Context &c, std::vector<TrdJob> &jobs) {
     }
     cudaEventDestroy(me.ready);
     if (me.state == 2) return false;
-    if (me.state == 3) throw Error{DCG_E_NUMERIC, "tridiagonalisation: a grid barrier wait timed out"};
+    if (me.state == 3) throw Error{DCG_E_NUMERIC, "tridiagonalisation: a wait for another block's words timed out"};
     if (me.state == 4) throw Error{DCG_E_CUDA, "merged tridiagonalisation: " + me.msg};
     return true;
 }
@@ -2308,7 +2307,7 @@ constexpr int kTridiagClusterMaxN = 400;
 static int trd_cluster_ctas(int n) {
     if (n <= 32) return 1;
     if (n <= 64) return 4;
-    return 16;   // a GB300 SM retires two FP64 FMAs per clock: the column work needs the blocks
+    return 16;   // a GB300 SM retires 1.66 FP64 FMAs per clock: the column work needs the blocks
 }
 
 // Jobs of one cluster shape.  False when no cluster of this shape can be resident (the caller then
@@ -2349,7 +2348,7 @@ static bool tridiag_cluster_group(Context &c, std::vector<TrdJob> &jobs, int nct
     const std::vector<int> he = trd_launch(c, jobs, total, smem, c.stream, "trd.err.cluster", ncta);
     c.launches++;
     for (int e : he)
-        if (e) throw Error{DCG_E_NUMERIC, "tridiagonalisation: a cluster wait timed out"};
+        if (e) throw Error{DCG_E_NUMERIC, "tridiagonalisation: a wait for another block's words timed out"};
     return true;
 }
 
@@ -2374,7 +2373,7 @@ static bool tridiag_smem_batched(Context &c, std::vector<TrdJob> &jobs) {
     const std::vector<int> he = trd_launch(c, jobs, total, smem, c.stream, "trd.err");
     c.launches++;
     for (int e : he)
-        if (e) throw Error{DCG_E_NUMERIC, "tridiagonalisation: a grid barrier wait timed out"};
+        if (e) throw Error{DCG_E_NUMERIC, "tridiagonalisation: a wait for another block's words timed out"};
     return true;
 }
 
@@ -2405,7 +2404,7 @@ static bool tridiag_global(Context &c, int n, cplx *A, int64_t lda, HeevWork &h)
     trd_clear(c, jobs);
     const std::vector<int> he = trd_launch(c, jobs, nb, smem, c.stream, "trd.err.global", 0, true);
     c.launches++;
-    if (he[0]) throw Error{DCG_E_NUMERIC, "tridiagonalisation: a grid barrier wait timed out"};
+    if (he[0]) throw Error{DCG_E_NUMERIC, "tridiagonalisation: a wait for another block's words timed out"};
     return true;
 }
 

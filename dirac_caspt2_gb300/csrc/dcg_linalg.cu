@@ -87,7 +87,7 @@ __device__ double block_sum(double v, double *sh) {
 // ===================================================================== ZGEMM
 // 256 threads as TYN x (256 / TYN), each owning a 4 x 4 block of outputs spaced TYN rows and
 // 256/TYN columns apart: tiles of 64 x 64 (TYN 16), 32 x 128 (TYN 8) or 128 x 32 (TYN 32).
-// A GB300 SM retires about two FP64 FMAs per clock, so the useful fraction of a tile is the
+// A GB300 SM retires 1.66 FP64 FMAs per clock, so the useful fraction of a tile is the
 // fraction of the GPU's FP64 rate a skinny product gets: the autotuner picks the tile.
 constexpr int kZgTiles = 3;
 // Rows and columns of all tile shapes: these three, then the fine-grained ones (zgemm_fine_kernel).
@@ -223,9 +223,8 @@ struct ZArith<true> {
 // order through shared memory).  The next chunk is loaded into registers while the current
 // one is multiplied.  Pieces go to warps rotated by the block index, so a ragged edge does
 // not idle the same quarter of every SM.
-// Measured (whole solves, 64 x 64 tiles and up only -> with these): 4/4/12 FP64 8.66 -> 3.88 ms
-// (one 64-row product alone took 274 us), 12/8/120 real FP64 37.1 -> 25.7 ms, 14/10/230 split
-// 65.4 -> 50.8 ms, 20/12/300 split 119.6 -> 114.8 ms.
+// Measured: the small products of a solve take under 10 us a launch where tiles of 64 x 64 and up
+// took 70 to 274 us.
 template <int RM, int RN, int KG, int QN>
 struct ZfShape {
     static constexpr int BM = 8 * RM, BN = 4 * RN * QN, BK = KG > 1 ? 32 : 16;

@@ -259,7 +259,8 @@ int dcg_zgemm(dcg_ctx *ctx, int precision, int32_t M, int32_t N, int32_t K, int3
 #define DCG_FAM_SPLIT_MMA 10  /* tcgen05 split-precision GEMM kernel; work = BF16 tensor FLOPs      */
 
 /* Time limit of the context's device-side waits that can give up: the waits of the
- * Householder tridiagonalisation for the other blocks' flagged words (default 5 s) and the
+ * Householder tridiagonalisation for the other blocks (flagged words, and grid barriers above
+ * about 4,750 rows; default 5 s; also in a merged launch each context's own) and the
  * pipeline waits of the tensor-core GEMM kernels (default 2 s).  A wait that runs out sets an
  * error flag; the kernel's other blocks leave at their next wait, copies still in flight land
  * and issued tensor-core operations complete (waits bounded by the default limits) before a
