@@ -897,7 +897,7 @@ struct DcBufs {
     int *Kl, *defl;           // node-local column of each undeflated / deflated entry
     int *rp, *rn;             // Givens rotation column pairs
     double *rc, *rs;          // and their cosines / sines
-    int *ord;                 // origin pole of each secular root
+    int *ord;                 // origin pole of each secular root (before that, the folded entries)
     double *tau, *lamK;       // root offset from its origin, root value
     double *zh;               // recomputed rank-one vector
     int *outc;                // output column of each node entry in the next level
